@@ -1,4 +1,4 @@
-"""The workloads whose speed this framework is judged by, and how their results are compared.
+"""The workloads this framework's speed is measured on, and how their results are compared.
 
 Every case is one call a user makes on a compiled model: ``CompiledModel.train_step(inputs, labels)`` (forward, loss,
 backward, optimizer, and the loss read back) or ``CompiledModel.forward(inputs)`` on a model compiled for inference.
