@@ -14,6 +14,7 @@ from typing import Dict, Optional, Union
 import torch
 
 from . import _ffcore as core
+from .ops import kernels as K
 from .runtime.executor import ExecConfig, Executable, OptimizerConfig
 
 
@@ -47,8 +48,11 @@ class CompiledModel:
         if not return_loss:
             self.d2h_bytes_last_step = 0
             return None
-        mean = ex.loss_rows.mean(dtype=torch.float32).reshape(1)
-        self._loss_host.copy_(mean, non_blocking=False)
+        if ex.loss_rows.is_cuda:
+            K.loss_mean(ex.loss_rows, self._loss_host)
+            torch.cuda.current_stream().synchronize()
+        else:
+            self._loss_host.copy_(ex.loss_rows.mean(dtype=torch.float32).reshape(1))
         self.d2h_bytes_last_step = 4
         return float(self._loss_host[0])
 

@@ -719,6 +719,8 @@ def _decl_tensor_ops(l):
         "ffk_topk_bwd": [P, P, P, I, I, I, I, I, S],
         "ffk_reverse": [P, P, L, L, L, I, S],
         "ffk_load_rows": [P, P, P, L, L, L, L, S],
+        "ffk_stage_batch": [P, S],
+        "ffk_loss_mean": [P, L, P, S],
     }
     for name, args in sig.items():
         fn = getattr(l, name)
@@ -814,6 +816,56 @@ def load_rows(dataset, out, indices=None, first=0):
     _check(_tlib().ffk_load_rows(dataset.data_ptr(), None if indices is None else indices.data_ptr(), out.data_ptr(), n, row_bytes, int(first),
                                  dataset.shape[0], _stream()), "ffk_load_rows")
     return out
+
+
+class _StageSeg(ctypes.Structure):
+    _fields_ = [("src", c_void_p), ("dst", c_void_p), ("n", c_longlong), ("kind", c_int), ("first_block", c_int)]
+
+
+_STAGE_MAX = 16
+
+
+class _StageArgs(ctypes.Structure):
+    _fields_ = [("seg", _StageSeg * _STAGE_MAX), ("nseg", c_int), ("alpha", c_float), ("alpha_ptr", c_void_p),
+                ("seed", c_ulonglong), ("seed_ptr", c_void_p)]
+
+
+_STAGE_KINDS = {(torch.float32, torch.bfloat16): 1, (torch.int64, torch.int32): 2, (torch.int32, torch.int64): 3}
+
+
+def stage_batch(pairs, scalars=None):
+    """Every (source, destination) pair copied, cast where the types differ, and the step's scalars
+    ``(alpha, its device tensor or None, seed, its device tensor)`` set, in one launch (one per 16 pairs).  Pairs the kernel does not
+    cover (host memory, another device, strided sources, rare casts) go through ``Tensor.copy_``."""
+    a = _StageArgs()
+    k = 0
+    if scalars is not None:
+        a.alpha, a.alpha_ptr, a.seed, a.seed_ptr = scalars[0], _p(scalars[1]), scalars[2], scalars[3].data_ptr()
+    launch = _tlib().ffk_stage_batch
+    for src, dst in pairs:
+        kind = 0 if src.dtype == dst.dtype else _STAGE_KINDS.get((src.dtype, dst.dtype), -1)
+        if kind < 0 or src.device != dst.device or not src.is_contiguous() or src.numel() != dst.numel():
+            dst.copy_(src.reshape(dst.shape), non_blocking=True)
+            continue
+        if k == _STAGE_MAX:
+            a.nseg = k
+            _check(launch(ctypes.byref(a), _stream()), "ffk_stage_batch")
+            k = 0
+            a.alpha_ptr = a.seed_ptr = None
+        n = src.numel()
+        a.seg[k] = (src.data_ptr(), dst.data_ptr(), n if kind else n * src.element_size(), kind, 0)
+        k += 1
+    if k or a.seed_ptr:
+        a.nseg = k
+        _check(launch(ctypes.byref(a), _stream()), "ffk_stage_batch")
+
+
+def loss_mean(rows, out_host):
+    """Mean of the fp32 device tensor `rows` into the page-locked host scalar `out_host`; valid once the stream has caught up."""
+    _cuda_contig(rows)
+    if rows.dtype != torch.float32 or out_host.dtype != torch.float32 or not out_host.is_pinned():
+        raise KernelError("loss_mean: fp32 rows and a page-locked fp32 host scalar expected")
+    _check(_tlib().ffk_loss_mean(rows.data_ptr(), rows.numel(), out_host.data_ptr(), _stream()), "ffk_loss_mean")
 
 
 def gather(x, idx, out, dim):

@@ -1525,14 +1525,18 @@ class Executable:
 
     # ---- execution
     def set_inputs(self, inputs: Dict[str, torch.Tensor], labels: Optional[torch.Tensor] = None):
-        for nid, name in self._input_nodes:
-            if name in inputs:
-                dst = self.values[(nid, "OUTPUT")].data
-                src = inputs[name]
-                dst.copy_(src.reshape(dst.shape), non_blocking=True)
+        self._stage(inputs, labels, None)
+
+    def _stage(self, inputs, labels, scalars):
+        """Copies the batch into the plan's buffers; on the GPU together with the step's scalars in one launch."""
+        pairs = [(inputs[name], self.values[(nid, "OUTPUT")].data) for nid, name in self._input_nodes if name in inputs]
         if labels is not None and self.labels is not None:
-            labels = self.local_label_rows(labels, self.labels.shape[0])
-            self.labels.copy_(labels.reshape(self.labels.shape), non_blocking=True)
+            pairs.append((self.local_label_rows(labels, self.labels.shape[0]), self.labels))
+        if self.on_gpu:
+            K.stage_batch(pairs, scalars)
+            return
+        for src, dst in pairs:
+            dst.copy_(src.reshape(dst.shape), non_blocking=True)
 
     def forward(self):
         if self.cfg.profile_layers:
@@ -1656,15 +1660,20 @@ class Executable:
             K.sgd_update(self.master[sl], self.opt_m[sl] if self.opt_m is not None else None, self.grads[sl], shadow, o.lr, o.momentum,
                          o.nesterov, o.weight_decay)
 
-    def _pre_step(self):
-        """Per-step scalars that a captured graph reads from device memory."""
+    def _step_scalars(self):
+        """Per-step scalars that a captured graph reads from device memory: (step size, its tensor, dropout seed, its tensor)."""
         o = self.cfg.optimizer
         t = self.step_count + 1
-        if o.kind == "adam":
-            alpha_t = o.lr * math.sqrt(1.0 - o.beta2 ** t) / (1.0 - o.beta1 ** t)
-            self.alpha_tensor.fill_(alpha_t)
-        if self.seed_tensor is not None:
-            self.seed_tensor.fill_((self.cfg.seed * 7919 + t * 104729) & 0x7FFFFFFFFFFFFFFF)
+        seed = (self.cfg.seed * 7919 + t * 104729) & 0x7FFFFFFFFFFFFFFF
+        if o.kind != "adam":
+            return 0.0, None, seed, self.seed_tensor
+        return o.lr * math.sqrt(1.0 - o.beta2 ** t) / (1.0 - o.beta1 ** t), self.alpha_tensor, seed, self.seed_tensor
+
+    def _pre_step(self):
+        if self.on_gpu:
+            K.stage_batch((), self._step_scalars())
+        elif self.cfg.optimizer.kind == "adam":
+            self.alpha_tensor.fill_(self._step_scalars()[0])
 
     def _step_body(self):
         self.forward()
@@ -1675,9 +1684,12 @@ class Executable:
 
     def train_step(self, inputs: Optional[Dict[str, torch.Tensor]] = None, labels: Optional[torch.Tensor] = None):
         """One optimisation step; returns the per-row loss tensor (device)."""
-        if inputs is not None or labels is not None:
-            self.set_inputs(inputs or {}, labels)
-        self._pre_step()
+        if self.on_gpu and self.dist is None:
+            self._stage(inputs or {}, labels, self._step_scalars())
+        else:
+            if inputs is not None or labels is not None:
+                self.set_inputs(inputs or {}, labels)
+            self._pre_step()
         if self.cfg.use_cuda_graph and self.on_gpu:
             if not getattr(self, "_warmed", False):
                 # the first step runs eagerly (lazy library initialisation must not happen during capture);

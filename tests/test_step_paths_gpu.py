@@ -6,6 +6,7 @@ pytestmark = pytest.mark.gpu
 
 from flexflow_train_b200 import _ffcore as core  # noqa: E402
 from flexflow_train_b200 import api  # noqa: E402
+from flexflow_train_b200.ops import kernels as K  # noqa: E402
 from flexflow_train_b200.runtime.executor import ExecConfig, Executable  # noqa: E402
 
 LM = {"num_features": 128, "sequence_length": 48, "batch_size": 3, "dim_feedforward": 256, "num_heads": 2, "num_decoder_layers": 2,
@@ -37,3 +38,28 @@ def test_forward_inside_a_callers_capture():
         y = m.forward({"input": x})
     g.replay()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("n", [1, 7, 4096, 4099, 16384 * 3 + 5])
+@pytest.mark.parametrize("offset", [0, 1])  # 1: no 16-byte alignment
+def test_stage_batch_copies_and_casts_like_copy(n, offset):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    f = torch.randn(n + offset, generator=gen, device="cuda")[offset:]
+    i = torch.randint(-2**31, 2**31 - 1, (n + offset,), generator=gen, device="cuda", dtype=torch.int64)[offset:]
+    pairs = []
+    for src, dt in ((f, torch.bfloat16), (f, torch.float32), (i, torch.int32), (i, torch.int64), (i.int(), torch.int64), (f.half(), torch.float16),
+                    (i.int(), torch.int32), (f > 0, torch.bool), (f.double(), torch.float32), (f.cpu(), torch.bfloat16)):
+        pairs.append((src, torch.zeros(n + offset, dtype=dt, device="cuda")[offset:]))
+    alpha, seed = torch.zeros(1, device="cuda"), torch.zeros(1, dtype=torch.int64, device="cuda")
+    K.stage_batch(pairs * 2, (0.25, alpha, 2**62 + 3, seed))  # 20 pairs: more than one launch holds
+    for src, dst in pairs:
+        assert torch.equal(dst, src.to("cuda").to(dst.dtype)), (src.dtype, dst.dtype)
+    assert alpha.item() == 0.25 and seed.item() == 2**62 + 3
+
+
+@pytest.mark.parametrize("n", [1, 33, 4096, 32771])
+def test_loss_mean(n):
+    rows, out = torch.rand(n, device="cuda") + 1, torch.zeros(1).pin_memory()
+    K.loss_mean(rows, out)
+    torch.cuda.current_stream().synchronize()
+    assert abs(out.item() - rows.double().mean().item()) < 1e-6 * 2  # 32 partial sums of n / 1024 terms each
