@@ -8,6 +8,7 @@
 // statistics in fp32.
 #include "common.cuh"
 #include "rowwise_vec.cuh"
+#include "tcgen05.cuh"
 
 namespace {
 
@@ -186,62 +187,155 @@ __global__ void softmax_ce_kernel(const T *__restrict__ logits, const L *__restr
   }
 }
 
-// bf16 rows with cols % 8 == 0: 16-byte accesses; one pass finds the row maximum and the sum of exponentials
-// together (online softmax), a second pass over the (cache-resident) row writes the gradient.
-template <typename L>
-__global__ void softmax_ce_vec_kernel(const bf16 *__restrict__ logits, const L *__restrict__ labels, bf16 *__restrict__ probs,
-                                      bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols, float grad_scale) {
-  __shared__ float2 red[32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+// bf16 rows with cols % 8 == 0: the row stays in registers between the loss and the gradient (one block per row, see
+// rowwise_vec.cuh).
+template <int VPT, typename L>
+__global__ void __launch_bounds__(512, 2) softmax_ce_row_kernel(const bf16 *__restrict__ logits, const L *__restrict__ labels,
+                                                                bf16 *__restrict__ probs, bf16 *__restrict__ dlogits,
+                                                                float *__restrict__ loss, int cols, float grad_scale) {
+  __shared__ float red[64];
   const int nvec = cols >> 3;
-  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
-    const bf16 *px = logits + (long long)row * cols;
-    const long long label = (long long)labels[row];
-    float m = -INFINITY, s = 0.f;
-    for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+  const long long base = (long long)blockIdx.x * cols;
+  uint4 u[VPT];
+  vec::row_load<VPT>(logits + base, nvec, u);
+  const long long label = (long long)labels[blockIdx.x];
+  const bool valid = label >= 0 && label < cols;
+  const float at_label = valid ? bf2f(logits[base + label]) : 0.f;  // before dlogits is written: it may be the same buffer
+  float m, s;
+  vec::row_max_sum<VPT>(u, nvec, 1.f, red, m, s);
+  const float inv = 1.f / s;
+  if (threadIdx.x == 0 && loss) loss[blockIdx.x] = valid ? (__logf(s) + m - at_label) : 0.f;
+  if (!probs && !dlogits) return;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = i * blockDim.x + threadIdx.x;
+    if (c < nvec) {
       float v[8];
-      vec::ld8(px + i * 8, v);
-      float vm = v[0];
+      vec::unpack8(u[i], v);
 #pragma unroll
-      for (int j = 1; j < 8; ++j) vm = fmaxf(vm, v[j]);
-      const float nm = fmaxf(m, vm);
-      float acc = 0.f;
+      for (int j = 0; j < 8; ++j) v[j] = __expf(v[j] - m) * inv;
+      if (probs) vec::st8(probs + base + c * 8, v);
+      if (dlogits) {
+        const int hit = valid ? (int)label - c * 8 : -1;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc += __expf(v[j] - nm);
-      s = s * __expf(m - nm) + acc;
-      m = nm;
+        for (int j = 0; j < 8; ++j) v[j] = valid ? (v[j] - (j == hit ? 1.f : 0.f)) * grad_scale : 0.f;
+        vec::st8(dlogits + base + c * 8, v);
+      }
     }
-    // combine (m, s) pairs: warp, then block
+  }
+}
+
+// Wide rows (4096 < cols <= 32768, a vocabulary): persistent blocks whose next rows travel into a ring in shared memory by bulk
+// copies while the current one is reduced and written.  Bound by HBM (one read, one write per element).  Holding the row in
+// registers alone leaves nothing in flight between a block's phases (cross-entropy of 8192 x 30528: 294 us; a running maximum with
+// the row read twice: 254 us; softmax of 4004 x 32000: 144 us, three passes of 2-byte loads: 549 us), and forming each
+// exponential twice makes the special-function unit (16 a clock and SM) as slow as the memory.  Here each is formed once, in
+// fp32 registers: four 16-byte pieces per thread, 1024 threads per SM in blocks of 256, 512 or 1024 (113 us for the softmax).
+constexpr int WIDE_VPT = 4;
+constexpr int WIDE_SMEM = 220 * 1024;   // of one SM, shared by its blocks
+__device__ int g_rows_err = 0;
+template <bool CE, typename L>
+__global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__restrict__ x, const L *__restrict__ labels, bf16 *__restrict__ probs,
+                                                               bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols,
+                                                               float scale, float grad_scale, int depth) {
+  extern __shared__ __align__(128) uint8_t wide_smem[];
+  __shared__ float red[64];
+  __shared__ uint64_t full[4];
+  __shared__ int abort_flag;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nvec = cols >> 3;
+  const uint32_t row_bytes = (uint32_t)cols * 2u;
+  auto fetch = [&](int row, int stage) {   // one thread; row_bytes and both addresses are multiples of 16
+    mbar_expect_tx(&full[stage], row_bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(wide_smem) + (uint32_t)stage * row_bytes),
+                 "l"(x + (long long)row * cols), "r"(row_bytes), "r"(smem_u32(&full[stage]))
+                 : "memory");
+  };
+  if (threadIdx.x == 0) {
+    abort_flag = 0;
+    for (int s = 0; s < depth; ++s) mbar_init(&full[s], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int s = 0; s < depth; ++s)
+      if ((long long)blockIdx.x + (long long)s * gridDim.x < rows) fetch(blockIdx.x + s * gridDim.x, s);
+  }
+  __syncthreads();
+  int stage = 0;
+  uint32_t phase = 0;
+  for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+    const bool ok = mbar_wait(&full[stage], phase, &abort_flag, &g_rows_err, FFK_ERR_TIMEOUT_PRODUCER);
+    const uint4 *src = reinterpret_cast<const uint4 *>(wide_smem + (size_t)stage * row_bytes);
+    float v[WIDE_VPT][8];
+    float m = -INFINITY;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
-      const float nm = fmaxf(m, om);
-      s = (nm == -INFINITY) ? 0.f : s * __expf(m - nm) + os * __expf(om - nm);
-      m = nm;
-    }
-    __syncthreads();  // the previous row's readers are done with `red`
-    if (lane == 0) red[wid] = make_float2(m, s);
-    __syncthreads();
-    float M = -INFINITY, S = 0.f;
-    for (int k = 0; k < nw; ++k) M = fmaxf(M, red[k].x);
-    for (int k = 0; k < nw; ++k) S += (red[k].x == -INFINITY) ? 0.f : red[k].y * __expf(red[k].x - M);
-    const float inv = 1.f / S;
-    const bool valid = label >= 0 && label < cols;
-    if (threadIdx.x == 0 && loss) loss[row] = valid ? (__logf(S) + M - bf2f(px[valid ? label : 0])) : 0.f;
-    if (probs || dlogits) {
-      for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-        float v[8], g[8];
-        vec::ld8(px + i * 8, v);
+    for (int i = 0; i < WIDE_VPT; ++i) {
+      const int c = i * blockDim.x + threadIdx.x;
+      if (c < nvec) {
+        vec::unpack8(src[c], v[i]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __expf(v[j] - M) * inv;
-        if (probs) vec::st8(probs + (long long)row * cols + i * 8, v);
-        if (dlogits) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) g[j] = valid ? (v[j] - ((long long)(i * 8 + j) == label ? 1.f : 0.f)) * grad_scale : 0.f;
-          vec::st8(dlogits + (long long)row * cols + i * 8, g);
+        for (int j = 0; j < 8; ++j) {
+          v[i][j] *= scale;
+          m = fmaxf(m, v[i][j]);
         }
       }
     }
+    long long label = -1;
+    bool valid = false;
+    float at_label = 0.f;
+    if (CE) {
+      label = (long long)labels[row];
+      valid = label >= 0 && label < cols;
+      if (valid && threadIdx.x == 0) at_label = bf2f(reinterpret_cast<const bf16 *>(src)[label]);
+    }
+    m = warp_max(m);
+    if (lane == 0) red[wid] = m;
+    // past this barrier the row's stage is free; a copy that never came (ok is false) ends the block here
+    if (__syncthreads_or(!ok)) {
+      if (threadIdx.x == 0)   // the other stages' copies land, or a second limit runs out, before the shared memory goes away
+        for (int k = 0; k < depth; ++k) {
+          const uint64_t t0 = ffk_globaltimer();
+          while (!mbar_try_wait(&full[k], k >= stage ? phase : phase ^ 1) && ffk_globaltimer() - t0 < WAIT_LIMIT_NS) {}
+        }
+      __syncthreads();
+      return;
+    }
+    if (threadIdx.x == 0 && row + (long long)depth * gridDim.x < rows) fetch((int)(row + (long long)depth * gridDim.x), stage);
+    m = warp_max(red[lane < nw ? lane : 0]);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < WIDE_VPT; ++i)
+      if (i * blockDim.x + threadIdx.x < nvec) {
+        float a = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          v[i][j] = __expf(v[i][j] - m);
+          a += v[i][j];
+        }
+        s += a;
+      }
+    s = warp_sum(s);
+    if (lane == 0) red[32 + wid] = s;
+    __syncthreads();
+    s = warp_sum(lane < nw ? red[32 + lane] : 0.f);
+    const float inv = 1.f / s;
+    if (CE && threadIdx.x == 0 && loss) loss[row] = valid ? (__logf(s) + m - at_label) : 0.f;
+    const long long base = row * cols;
+#pragma unroll
+    for (int i = 0; i < WIDE_VPT; ++i) {
+      const int c = i * blockDim.x + threadIdx.x;
+      if (c < nvec) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[i][j] *= inv;
+        if (probs) vec::st8(probs + base + c * 8, v[i]);
+        if (CE && dlogits) {
+          const int hit = valid ? (int)label - c * 8 : -1;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[i][j] = valid ? (v[i][j] - (j == hit ? 1.f : 0.f)) * grad_scale : 0.f;
+          vec::st8(dlogits + base + c * 8, v[i]);
+        }
+      }
+    }
+    if (++stage == depth) { stage = 0; phase ^= 1; }
   }
 }
 
@@ -408,60 +502,116 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
   return (int)cudaGetLastError();
 }
 
-template <int VPT>
-static void launch_softmax_fwd_warp(const void *x, void *y, void *yd, int rows, float scale, int causal_q, float p, unsigned long long salt,
-                                    const unsigned long long *seed_ptr, cudaStream_t st) {
-  int blocks = (rows + 7) / 8;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  vec::softmax_fwd_warp_kernel<VPT><<<blocks, 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (bf16 *)yd, rows, scale, causal_q, p, salt, seed_ptr);
+// Rows of up to 4096 bf16 elements at a pitch of whole 16-byte pieces: one warp per row.
+static bool softmax_warp_ok(int cols, int ld, int dt, const void *a, const void *b, const void *c) {
+  return dt == 1 && cols > 0 && cols <= 4096 && ld >= cols && ld % 8 == 0 && aligned16(a) && aligned16(b) && aligned16(c);
 }
-template <int VPT>
-static void launch_softmax_bwd_warp(const void *dy, const void *y, void *dx, int rows, float scale, float p, unsigned long long salt,
-                                    const unsigned long long *seed_ptr, cudaStream_t st) {
-  int blocks = (rows + 7) / 8;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  vec::softmax_bwd_warp_kernel<VPT><<<blocks, 256, 0, st>>>((const bf16 *)dy, (const bf16 *)y, (bf16 *)dx, rows, scale, p, salt, seed_ptr);
+// vectors of 8 per lane that hold a row: the next of 1, 2, 3, 4, 6, 8, 16
+static int softmax_vpt(int cols) {
+  const int v = (cols + 255) / 256;
+  return v <= 4 ? v : v <= 6 ? 6 : v <= 8 ? 8 : 16;
 }
-static bool softmax_vec_ok(int cols, int dt, const void *a, const void *b, const void *c) {
-  return dt == 1 && cols % 256 == 0 && cols <= 4096 && (cols / 256 == 1 || cols / 256 == 2 || cols / 256 == 4 || cols / 256 == 8 || cols / 256 == 16) &&
-         aligned16(a) && aligned16(b) && aligned16(c);
-}
-// y = softmax(scale * x); yd (optional, bf16 rows of 256*k columns only) = dropout(y, p) with the mask
-// hash(salt, *seed_ptr, element index).  Returns -3 when yd is requested for a shape the fused path cannot take.
-FFK_API int ffk_softmax_dropout_fwd(const void *x, void *y, void *yd, int rows, int cols, float scale, int causal_q, float p,
+// y = softmax(scale * x) over rows of `cols` at pitch `ld`; yd (optional) = dropout(y, p) with the mask
+// hash(salt, *seed_ptr, row * cols + column).  Returns -3 for rows the one-warp-per-row kernel cannot take.
+FFK_API int ffk_softmax_dropout_fwd(const void *x, void *y, void *yd, int rows, int cols, int ld, float scale, int causal_q, float p,
                                     unsigned long long salt, const unsigned long long *seed_ptr, int dt, cudaStream_t st) {
   if (rows <= 0) return 0;
-  if (!softmax_vec_ok(cols, dt, x, y, yd)) return -3;
-  switch (cols / 256) {
-    case 1: launch_softmax_fwd_warp<1>(x, y, yd, rows, scale, causal_q, p, salt, seed_ptr, st); break;
-    case 2: launch_softmax_fwd_warp<2>(x, y, yd, rows, scale, causal_q, p, salt, seed_ptr, st); break;
-    case 4: launch_softmax_fwd_warp<4>(x, y, yd, rows, scale, causal_q, p, salt, seed_ptr, st); break;
-    case 8: launch_softmax_fwd_warp<8>(x, y, yd, rows, scale, causal_q, p, salt, seed_ptr, st); break;
-    default: launch_softmax_fwd_warp<16>(x, y, yd, rows, scale, causal_q, p, salt, seed_ptr, st); break;
-  }
+  if (!softmax_warp_ok(cols, ld, dt, x, y, yd)) return -3;
+  const int grid = ffk_blocks(rows, 8);
+#define SM_FWD(V)                                                                                                                        \
+  case V:                                                                                                                                \
+    if (cols == 256 * V && ld == cols)                                                                                                   \
+      vec::softmax_fwd_warp_kernel<V, true><<<grid, 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (bf16 *)yd, rows, cols, ld, scale, causal_q, \
+                                                                  p, salt, seed_ptr);                                                    \
+    else                                                                                                                                 \
+      vec::softmax_fwd_warp_kernel<V, false><<<grid, 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (bf16 *)yd, rows, cols, ld, scale, causal_q, \
+                                                                   p, salt, seed_ptr);                                                   \
+    break;
+  switch (softmax_vpt(cols)) { SM_FWD(1) SM_FWD(2) SM_FWD(3) SM_FWD(4) SM_FWD(6) SM_FWD(8) SM_FWD(16) }
+#undef SM_FWD
   return (int)cudaGetLastError();
 }
-// dx = scale * y * (g - sum(g*y)) with g = dropout_backward(dy) (p = 0: g = dy).  Same shape limits as above.
-FFK_API int ffk_softmax_dropout_bwd(const void *dy, const void *y, void *dx, int rows, int cols, float scale, float p,
+// dx = scale * y * (g - sum(g*y)) with g = dropout_backward(dy) (p = 0: g = dy).  Same rows as above.
+FFK_API int ffk_softmax_dropout_bwd(const void *dy, const void *y, void *dx, int rows, int cols, int ld, float scale, float p,
                                     unsigned long long salt, const unsigned long long *seed_ptr, int dt, cudaStream_t st) {
   if (rows <= 0) return 0;
-  if (!softmax_vec_ok(cols, dt, dy, y, dx)) return -3;
-  switch (cols / 256) {
-    case 1: launch_softmax_bwd_warp<1>(dy, y, dx, rows, scale, p, salt, seed_ptr, st); break;
-    case 2: launch_softmax_bwd_warp<2>(dy, y, dx, rows, scale, p, salt, seed_ptr, st); break;
-    case 4: launch_softmax_bwd_warp<4>(dy, y, dx, rows, scale, p, salt, seed_ptr, st); break;
-    case 8: launch_softmax_bwd_warp<8>(dy, y, dx, rows, scale, p, salt, seed_ptr, st); break;
-    default: launch_softmax_bwd_warp<16>(dy, y, dx, rows, scale, p, salt, seed_ptr, st); break;
-  }
+  if (!softmax_warp_ok(cols, ld, dt, dy, y, dx)) return -3;
+  const int grid = ffk_blocks(rows, 8);
+#define SM_BWD(V)                                                                                                                       \
+  case V:                                                                                                                               \
+    if (cols == 256 * V && ld == cols)                                                                                                  \
+      vec::softmax_bwd_warp_kernel<V, true><<<grid, 256, 0, st>>>((const bf16 *)dy, (const bf16 *)y, (bf16 *)dx, rows, cols, ld, scale, p, \
+                                                                  salt, seed_ptr);                                                      \
+    else                                                                                                                                \
+      vec::softmax_bwd_warp_kernel<V, false><<<grid, 256, 0, st>>>((const bf16 *)dy, (const bf16 *)y, (bf16 *)dx, rows, cols, ld, scale, p, \
+                                                                   salt, seed_ptr);                                                     \
+    break;
+  switch (softmax_vpt(cols)) { SM_BWD(1) SM_BWD(2) SM_BWD(3) SM_BWD(4) SM_BWD(6) SM_BWD(8) SM_BWD(16) }
+#undef SM_BWD
   return (int)cudaGetLastError();
+}
+// y = dropout(x) over bf16 rows of `cols` at pitch `ld`: the dropped copy ffk_softmax_dropout_fwd would write.
+FFK_API int ffk_dropout_rows(const void *x, void *y, long long rows, int cols, int ld, float p, unsigned long long salt,
+                             const unsigned long long *seed_ptr, cudaStream_t st) {
+  if (rows <= 0) return 0;
+  if (!softmax_warp_ok(cols, ld, 1, x, y, nullptr)) return -3;
+  vec::dropout_rows_kernel<<<ffk_blocks(rows * (ld / 8), 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, rows, cols, ld, p, salt, seed_ptr);
+  return (int)cudaGetLastError();
+}
+
+// Block size and vectors per thread of the one-block-per-row kernels: at most 512 threads, the fewest that hold the row in
+// four vectors each (several small blocks per SM overlap one's loads with another's stores).  0 = the row is too long.
+static int row_block(int cols, int &threads) {
+  const int nvec = cols / 8;
+  threads = nvec <= 512 ? 128 : nvec <= 1024 ? 256 : 512;
+  const int v = (nvec + threads - 1) / threads;
+  return v <= 1 ? 1 : v <= 2 ? 2 : v <= 4 ? 4 : v <= 8 ? 8 : v <= 16 ? 16 : 0;
+}
+// The wide-row kernel takes rows of whole 16-byte pieces that fill its threads at least to half and its ring at least twice.
+static bool softmax_wide_ok(int cols, int dt) { return dt == 1 && cols % 8 == 0 && cols > 4096 && cols <= 32768; }
+template <bool CE, typename L>
+static int launch_softmax_wide(const void *x, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols, float scale,
+                               float grad_scale, cudaStream_t st) {
+  auto kern = softmax_wide_kernel<CE, L>;
+  static bool attr_done = false;
+  if (!attr_done) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WIDE_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    attr_done = true;
+  }
+  const int threads = cols <= 8192 ? 256 : cols <= 16384 ? 512 : 1024;   // at most four pieces of 8 per thread
+  const int per_sm = 1024 / threads;
+  int depth = WIDE_SMEM / per_sm / (cols * 2);
+  if (depth > 4) depth = 4;
+  const int grid = rows < 148 * per_sm ? rows : 148 * per_sm;
+  kern<<<grid, threads, (size_t)depth * cols * 2, st>>>((const bf16 *)x, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss, rows, cols,
+                                                        scale, grad_scale, depth);
+  return (int)cudaGetLastError();
+}
+// Error word of the wide-row kernel's bounded waits (read and cleared; synchronises the device).
+FFK_API int ffk_softmax_last_error() {
+  int v = 0, z = 0;
+  if (cudaDeviceSynchronize() != cudaSuccess) return -1;
+  cudaMemcpyFromSymbol(&v, g_rows_err, sizeof(int));
+  cudaMemcpyToSymbol(g_rows_err, &z, sizeof(int));
+  return v;
 }
 
 FFK_API int ffk_softmax_fwd(const void *x, void *y, int rows, int cols, float scale, int causal_q, int dt,
                             cudaStream_t st) {
   if (rows <= 0) return 0;
-  if (softmax_vec_ok(cols, dt, x, y, nullptr))
-    return ffk_softmax_dropout_fwd(x, y, nullptr, rows, cols, scale, causal_q, 0.f, 0, nullptr, dt, st);
-  int threads = cols >= 1024 ? 256 : 128;
+  if (softmax_warp_ok(cols, cols, dt, x, y, nullptr))
+    return ffk_softmax_dropout_fwd(x, y, nullptr, rows, cols, cols, scale, causal_q, 0.f, 0, nullptr, dt, st);
+  if (softmax_wide_ok(cols, dt) && causal_q <= 0 && aligned16(x) && aligned16(y))
+    return launch_softmax_wide<false, int>(x, nullptr, y, nullptr, nullptr, rows, cols, scale, 1.f, st);
+  int threads, vpt;
+  if (dt == 1 && cols % 8 == 0 && causal_q <= 0 && aligned16(x) && aligned16(y) && (vpt = row_block(cols, threads)) != 0) {
+    // only rows beyond the wide kernel's come here (the shorter ones took the warp kernel)
+    if (vpt <= 8) vec::softmax_fwd_row_kernel<8><<<rows, threads, 0, st>>>((const bf16 *)x, (bf16 *)y, cols, scale);
+    else vec::softmax_fwd_row_kernel<16><<<rows, threads, 0, st>>>((const bf16 *)x, (bf16 *)y, cols, scale);
+    return (int)cudaGetLastError();
+  }
+  threads = cols >= 1024 ? 256 : 128;
   DISPATCH_FLOAT(dt, (softmax_fwd_kernel<T><<<rows < 148 * 16 ? rows : 148 * 16, threads, 0, st>>>(
                          (const T *)x, (T *)y, rows, cols, scale, causal_q)));
   return (int)cudaGetLastError();
@@ -469,30 +619,43 @@ FFK_API int ffk_softmax_fwd(const void *x, void *y, int rows, int cols, float sc
 FFK_API int ffk_softmax_bwd(const void *dy, const void *y, void *dx, int rows, int cols, float scale, int dt,
                             cudaStream_t st) {
   if (rows <= 0) return 0;
-  if (softmax_vec_ok(cols, dt, dy, y, dx))
-    return ffk_softmax_dropout_bwd(dy, y, dx, rows, cols, scale, 0.f, 0, nullptr, dt, st);
+  if (softmax_warp_ok(cols, cols, dt, dy, y, dx))
+    return ffk_softmax_dropout_bwd(dy, y, dx, rows, cols, cols, scale, 0.f, 0, nullptr, dt, st);
   int threads = cols >= 1024 ? 256 : 128;
   DISPATCH_FLOAT(dt, (softmax_bwd_kernel<T><<<rows < 148 * 16 ? rows : 148 * 16, threads, 0, st>>>(
                          (const T *)dy, (const T *)y, (T *)dx, rows, cols, scale)));
   return (int)cudaGetLastError();
 }
+template <int VPT>
+static void launch_softmax_ce_row(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols,
+                                  float grad_scale, int label_dt, int threads, cudaStream_t st) {
+  if (label_dt == 3)
+    softmax_ce_row_kernel<VPT, long long><<<rows, threads, 0, st>>>((const bf16 *)logits, (const long long *)labels, (bf16 *)probs,
+                                                                    (bf16 *)dlogits, loss, cols, grad_scale);
+  else
+    softmax_ce_row_kernel<VPT, int><<<rows, threads, 0, st>>>((const bf16 *)logits, (const int *)labels, (bf16 *)probs, (bf16 *)dlogits, loss,
+                                                              cols, grad_scale);
+}
 // label_dt: 2 = int32, 3 = int64
 FFK_API int ffk_softmax_ce(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows,
                            int cols, float grad_scale, int dt, int label_dt, cudaStream_t st) {
   if (rows <= 0) return 0;
-  int threads = cols >= 4096 ? 1024 : 256;
-  int grid = rows < 148 * 4 ? rows : 148 * 4;
-  if (dt == 1 && cols % 8 == 0 && (((uintptr_t)logits | (uintptr_t)probs | (uintptr_t)dlogits) & 15) == 0) {
-    int vthreads = cols >= 8192 ? 512 : 256;
-    int vgrid = rows < 148 * 8 ? rows : 148 * 8;
-    if (label_dt == 3)
-      softmax_ce_vec_kernel<long long><<<vgrid, vthreads, 0, st>>>((const bf16 *)logits, (const long long *)labels, (bf16 *)probs,
-                                                                   (bf16 *)dlogits, loss, rows, cols, grad_scale);
-    else
-      softmax_ce_vec_kernel<int><<<vgrid, vthreads, 0, st>>>((const bf16 *)logits, (const int *)labels, (bf16 *)probs, (bf16 *)dlogits, loss,
-                                                             rows, cols, grad_scale);
+  if (softmax_wide_ok(cols, dt) && aligned16(logits) && aligned16(probs) && aligned16(dlogits))
+    return label_dt == 3 ? launch_softmax_wide<true, long long>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st)
+                         : launch_softmax_wide<true, int>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st);
+  int threads, vpt;
+  if (dt == 1 && cols % 8 == 0 && aligned16(logits) && aligned16(probs) && aligned16(dlogits) && (vpt = row_block(cols, threads)) != 0) {
+    switch (vpt) {
+      case 1: launch_softmax_ce_row<1>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
+      case 2: launch_softmax_ce_row<2>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
+      case 4: launch_softmax_ce_row<4>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
+      case 8: launch_softmax_ce_row<8>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
+      default: launch_softmax_ce_row<16>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
+    }
     return (int)cudaGetLastError();
   }
+  threads = cols >= 4096 ? 1024 : 256;
+  const int grid = rows < 148 * 4 ? rows : 148 * 4;
   DISPATCH_FLOAT(dt, {
     if (label_dt == 3)
       softmax_ce_kernel<T, long long><<<grid, threads, 0, st>>>((const T *)logits, (const long long *)labels,

@@ -24,25 +24,38 @@ __device__ __forceinline__ void st8(bf16 *p, const float *v) {
 }
 
 // ---------------------------------------------------------------- softmax: one warp per row
-// cols = 256 * VPT.  y = softmax(scale * x); yd (optional) = dropout(y) with keep mask hash(seed, element index).
-template <int VPT>
-__global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, bf16 *__restrict__ yd, int rows, float scale,
-                                        int causal_q, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
-  constexpr int COLS = 256 * VPT;
+// Keep flags of the 8 elements from flat index e on (two group words where the row length is a multiple of 4, and e with it;
+// otherwise element by element, the same function of (seed, flat index) as the stand-alone dropout kernel).
+__device__ __forceinline__ uint32_t keep8(unsigned long long seed, unsigned long long e, bool grouped, uint32_t thr) {
+  if (grouped) return ffk_keep4(seed, e >> 2, thr) | (ffk_keep4(seed, (e >> 2) + 1, thr) << 4);
+  uint32_t k = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) k |= (ffk_keep(seed, e + j, thr) ? 1u : 0u) << j;
+  return k;
+}
+// Rows of `cols` elements at a pitch of `ld` (a multiple of 8, at least cols); 256 * (VPT - 1) < cols <= 256 * VPT; FULL: cols
+// fills the vectors and ld == cols.  y = softmax(scale * x); yd (optional) = dropout(y) with keep mask hash(seed, row * cols +
+// column); the pitch's tail columns of y / yd are written as zeros.  Bound by HBM: the row is read once into registers.  Rows
+// that are no multiple of 256 (sequence 500, 128 x 500 x 500 scores) used to take the block-per-row scalar kernel, which reads
+// the row three times in 2-byte pieces and left the dropped copy to a second kernel: 104 + 28 us.
+template <int VPT, bool FULL>
+__global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, bf16 *__restrict__ yd, int rows, int cols, int ld,
+                                        float scale, int causal_q, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   unsigned long long seed = salt;
   if (seed_ptr) seed = salt * 0x9E3779B97F4A7C15ull + *seed_ptr;
   const float keep_scale = p_drop < 1.f ? 1.f / (1.f - p_drop) : 0.f;
   const uint32_t thr = ffk_drop_threshold(p_drop);
+  const bool grouped = FULL || (cols & 3) == 0;
   for (long long row = (long long)blockIdx.x * wpb + wib; row < rows; row += (long long)gridDim.x * wpb) {
-    const bf16 *px = x + row * COLS;
+    const bf16 *px = x + row * ld;
     float v[VPT][8];
-    const int limit = causal_q > 0 ? (int)(row % causal_q) + 1 : COLS;
+    const int limit = causal_q > 0 ? min(cols, (int)(row % causal_q) + 1) : cols;
     float mx = -INFINITY;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       int c0 = (i * 32 + lane) * 8;
-      ld8(px + c0, v[i]);
+      if (FULL || c0 < cols) ld8(px + c0, v[i]);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         v[i][j] = (c0 + j < limit) ? v[i][j] * scale : -INFINITY;
@@ -56,6 +69,7 @@ __global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__rest
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         v[i][j] = __expf(v[i][j] - mx);
+        if (!FULL && (i * 32 + lane) * 8 + j >= cols) v[i][j] = 0.f;  // also when the row's maximum is -inf
         s += v[i][j];
       }
     s = warp_sum(s);
@@ -63,45 +77,49 @@ __global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__rest
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       int c0 = (i * 32 + lane) * 8;
+      if (!FULL && c0 >= cols) continue;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[i][j] *= inv;
-      st8(y + row * COLS + c0, v[i]);
+      for (int j = 0; j < 8; ++j) v[i][j] = (FULL || c0 + j < cols) ? v[i][j] * inv : 0.f;
+      st8(y + row * ld + c0, v[i]);
       if (yd) {
         float d[8];
-        const unsigned long long g4 = (unsigned long long)(row * COLS + c0) >> 2;
-        const uint32_t keep = ffk_keep4(seed, g4, thr) | (ffk_keep4(seed, g4 + 1, thr) << 4);
+        const uint32_t keep = keep8(seed, (unsigned long long)(row * cols + c0), grouped, thr);
 #pragma unroll
         for (int j = 0; j < 8; ++j) d[j] = (keep >> j) & 1u ? v[i][j] * keep_scale : 0.f;
-        st8(yd + row * COLS + c0, d);
+        st8(yd + row * ld + c0, d);
       }
     }
   }
 }
-// dx = scale * y * (g - sum(g * y)), g = dy (optionally first passed back through the dropout mask)
-template <int VPT>
-__global__ void softmax_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ y, bf16 *__restrict__ dx, int rows,
-                                        float scale, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
-  constexpr int COLS = 256 * VPT;
+// dx = scale * y * (g - sum(g * y)), g = dy (optionally first passed back through the dropout mask); rows as above
+template <int VPT, bool FULL>
+__global__ void softmax_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ y, bf16 *__restrict__ dx, int rows, int cols,
+                                        int ld, float scale, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   unsigned long long seed = salt;
   if (seed_ptr) seed = salt * 0x9E3779B97F4A7C15ull + *seed_ptr;
   const float keep_scale = p_drop < 1.f ? 1.f / (1.f - p_drop) : 0.f;
   const uint32_t thr = ffk_drop_threshold(p_drop);
+  const bool grouped = FULL || (cols & 3) == 0;
   for (long long row = (long long)blockIdx.x * wpb + wib; row < rows; row += (long long)gridDim.x * wpb) {
     float g[VPT][8], p[VPT][8];
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       int c0 = (i * 32 + lane) * 8;
-      ld8(dy + row * COLS + c0, g[i]);
-      ld8(y + row * COLS + c0, p[i]);
-      uint32_t keep = 0xFFu;
-      if (p_drop > 0.f) {
-        const unsigned long long g4 = (unsigned long long)(row * COLS + c0) >> 2;
-        keep = ffk_keep4(seed, g4, thr) | (ffk_keep4(seed, g4 + 1, thr) << 4);
+      if (FULL || c0 < cols) {
+        ld8(dy + row * ld + c0, g[i]);
+        ld8(y + row * ld + c0, p[i]);
       }
+    }
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      int c0 = (i * 32 + lane) * 8;
+      uint32_t keep = 0xFFu;
+      if (p_drop > 0.f && (FULL || c0 < cols)) keep = keep8(seed, (unsigned long long)(row * cols + c0), grouped, thr);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
+        if (!FULL && c0 + j >= cols) { g[i][j] = 0.f; p[i][j] = 0.f; }
         if (p_drop > 0.f) g[i][j] = (keep >> j) & 1u ? g[i][j] * keep_scale : 0.f;
         s += g[i][j] * p[i][j];
       }
@@ -110,9 +128,100 @@ __global__ void softmax_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       int c0 = (i * 32 + lane) * 8;
+      if (!FULL && c0 >= cols) continue;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) g[i][j] = scale * p[i][j] * (g[i][j] - s);
-      st8(dx + row * COLS + c0, g[i]);
+      for (int j = 0; j < 8; ++j) g[i][j] = (FULL || c0 + j < cols) ? scale * p[i][j] * (g[i][j] - s) : 0.f;
+      st8(dx + row * ld + c0, g[i]);
+    }
+  }
+}
+// y = dropout(x) over rows of `cols` at pitch `ld`, the mask of softmax_fwd_warp_kernel's yd; a thread per 8 elements
+static __global__ void dropout_rows_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, long long rows, int cols, int ld, float p_drop,
+                                           unsigned long long salt, const unsigned long long *seed_ptr) {
+  const unsigned long long seed = seed_ptr ? salt * 0x9E3779B97F4A7C15ull + *seed_ptr : salt;
+  const float keep_scale = p_drop < 1.f ? 1.f / (1.f - p_drop) : 0.f;
+  const uint32_t thr = ffk_drop_threshold(p_drop);
+  const int nv = ld >> 3;
+  const long long total = rows * nv;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+    const long long row = t / nv;
+    const int c0 = (int)(t - row * nv) * 8;
+    float v[8];
+    ld8(x + t * 8, v);
+    const uint32_t keep = keep8(seed, (unsigned long long)(row * cols + c0), (cols & 3) == 0, thr);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = ((keep >> j) & 1u) && c0 + j < cols ? v[j] * keep_scale : 0.f;
+    st8(y + t * 8, v);
+  }
+}
+
+// ---------------------------------------------------------------- softmax over rows of one block each
+// The row (cols % 8 == 0, up to 8 * VPT * blockDim.x) stays packed in registers between the maximum, the sum and the result, so
+// HBM sees one read and one write.
+template <int VPT>
+__device__ __forceinline__ void row_load(const bf16 *p, int nvec, uint4 (&u)[VPT]) {
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = i * blockDim.x + threadIdx.x;
+    if (c < nvec) u[i] = reinterpret_cast<const uint4 *>(p)[c];
+  }
+}
+// maximum of the row's values times scale, and the sum of exp(value * scale - maximum); `red`: 64 floats of shared memory
+template <int VPT>
+__device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, float scale, float *red, float &mx, float &sum) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  float m = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (i * blockDim.x + threadIdx.x < nvec) {
+      float v[8];
+      unpack8(u[i], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m = fmaxf(m, v[j] * scale);
+    }
+  m = warp_max(m);
+  if (lane == 0) red[wid] = m;
+  __syncthreads();
+  m = red[0];
+  for (int k = 1; k < nw; ++k) m = fmaxf(m, red[k]);
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i)
+    if (i * blockDim.x + threadIdx.x < nvec) {
+      float v[8];
+      unpack8(u[i], v);
+      float a = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a += __expf(v[j] * scale - m);
+      s += a;
+    }
+  s = warp_sum(s);
+  if (lane == 0) red[32 + wid] = s;
+  __syncthreads();
+  s = 0.f;
+  for (int k = 0; k < nw; ++k) s += red[32 + k];
+  mx = m;
+  sum = s;
+}
+template <int VPT>
+__global__ void __launch_bounds__(512, 2) softmax_fwd_row_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, int cols, float scale) {
+  __shared__ float red[64];
+  const int nvec = cols >> 3;
+  const long long base = (long long)blockIdx.x * cols;
+  uint4 u[VPT];
+  row_load<VPT>(x + base, nvec, u);
+  float m, s;
+  row_max_sum<VPT>(u, nvec, scale, red, m, s);
+  const float inv = 1.f / s;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = i * blockDim.x + threadIdx.x;
+    if (c < nvec) {
+      float v[8];
+      unpack8(u[i], v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __expf(v[j] * scale - m) * inv;
+      st8(y + base + c * 8, v);
     }
   }
 }

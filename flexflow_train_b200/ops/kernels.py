@@ -927,17 +927,32 @@ def reverse(x, out, axis):
 
 
 # --------------------------------------------------------------------------- fused softmax + dropout (attention probabilities)
-def softmax_dropout_supported(t) -> bool:
-    cols = t.shape[-1]
-    return t.dtype == torch.bfloat16 and cols % 256 == 0 and cols // 256 in (1, 2, 4, 8, 16)
+def softmax_dropout_supported(t, cols=None) -> bool:
+    """True when rows of `cols` (default: all) of the last dimension of `t` have a one-pass kernel: bf16, up to 4096 elements, at
+    a pitch of whole 16-byte pieces."""
+    ld = t.shape[-1]
+    return t.dtype == torch.bfloat16 and ld % 8 == 0 and (ld if cols is None else cols) <= 4096
+
+
+def softmax_pitch(cols: int) -> int:
+    """Pitch at which bf16 score rows of `cols` are laid out: a multiple of 16 bytes for rows the one-pass kernels take, so that
+    TMA reads and writes them where they lie."""
+    return (cols + 7) // 8 * 8 if cols <= 4096 else cols
+
+
+def softmax_last_error() -> int:
+    """Error word of the wide-row softmax kernel's bounded waits (0: none ran out)."""
+    return lib().ffk_softmax_last_error()
 
 
 def _decl_softmax_dropout(l):
     P, I, F, S = c_void_p, c_int, c_float, c_void_p
-    l.ffk_softmax_dropout_fwd.argtypes = [P, P, P, I, I, F, I, F, c_ulonglong, P, I, S]
+    l.ffk_softmax_dropout_fwd.argtypes = [P, P, P, I, I, I, F, I, F, c_ulonglong, P, I, S]
     l.ffk_softmax_dropout_fwd.restype = c_int
-    l.ffk_softmax_dropout_bwd.argtypes = [P, P, P, I, I, F, F, c_ulonglong, P, I, S]
+    l.ffk_softmax_dropout_bwd.argtypes = [P, P, P, I, I, I, F, F, c_ulonglong, P, I, S]
     l.ffk_softmax_dropout_bwd.restype = c_int
+    l.ffk_dropout_rows.argtypes = [P, P, c_longlong, I, I, F, c_ulonglong, P, S]
+    l.ffk_dropout_rows.restype = c_int
 
 
 _sd_declared = [False]
@@ -951,21 +966,32 @@ def _sdlib():
     return l
 
 
-def softmax_dropout_fwd(x, y, y_dropped, p, salt, seed_tensor=None, scale=1.0, causal_q=0):
-    """y = softmax(scale*x) and, in the same pass, y_dropped = dropout(y, p) (y_dropped may be None)."""
+def softmax_dropout_fwd(x, y, y_dropped, p, salt, seed_tensor=None, scale=1.0, causal_q=0, cols=None):
+    """y = softmax(scale*x) and, in the same pass, y_dropped = dropout(y, p) (y_dropped may be None).  `cols`: the rows' length
+    where it is less than the last dimension (their pitch)."""
     _cuda_contig(x, y, y_dropped, seed_tensor)
-    cols = x.shape[-1]
-    rows = x.numel() // cols
-    _check(_sdlib().ffk_softmax_dropout_fwd(x.data_ptr(), y.data_ptr(), _p(y_dropped), rows, cols, scale, causal_q, p,
+    ld = x.shape[-1]
+    rows = x.numel() // ld
+    _check(_sdlib().ffk_softmax_dropout_fwd(x.data_ptr(), y.data_ptr(), _p(y_dropped), rows, cols or ld, ld, scale, causal_q, p,
                                             salt & (2**64 - 1), _p(seed_tensor), _dt(x), _stream()), "ffk_softmax_dropout_fwd")
 
 
-def softmax_dropout_bwd(dy, y, dx, p, salt, seed_tensor=None, scale=1.0):
+def dropout_rows(x, out, cols, p, salt, seed_tensor=None):
+    """out = dropout(x) over bf16 rows of `cols` at the pitch of the last dimension, with the mask of softmax_dropout_fwd."""
+    _cuda_contig(x, out, seed_tensor)
+    ld = x.shape[-1]
+    if x.dtype != torch.bfloat16 or out.shape != x.shape or out.dtype != x.dtype:
+        raise KernelError("dropout_rows: bf16 tensors of one shape expected")
+    _check(_sdlib().ffk_dropout_rows(x.data_ptr(), out.data_ptr(), x.numel() // ld, cols, ld, p, salt & (2**64 - 1), _p(seed_tensor),
+                                     _stream()), "ffk_dropout_rows")
+
+
+def softmax_dropout_bwd(dy, y, dx, p, salt, seed_tensor=None, scale=1.0, cols=None):
     """dx = softmax backward of the gradient that first goes back through the same dropout mask."""
     _cuda_contig(dy, y, dx, seed_tensor)
-    cols = y.shape[-1]
-    rows = y.numel() // cols
-    _check(_sdlib().ffk_softmax_dropout_bwd(dy.data_ptr(), y.data_ptr(), dx.data_ptr(), rows, cols, scale, p,
+    ld = y.shape[-1]
+    rows = y.numel() // ld
+    _check(_sdlib().ffk_softmax_dropout_bwd(dy.data_ptr(), y.data_ptr(), dx.data_ptr(), rows, cols or ld, ld, scale, p,
                                             salt & (2**64 - 1), _p(seed_tensor), _dt(y), _stream()), "ffk_softmax_dropout_bwd")
 
 

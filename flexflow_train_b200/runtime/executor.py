@@ -432,7 +432,10 @@ class AttentionOp(OpImpl):
                 self.hb = max(1, min(H, (H * blk) // per_batch))
                 while H % self.hb:
                     self.hb -= 1
-        self.probs = torch.empty(self.B if not (self.cb or self.fused) else 0, H, self.Sq, self.Sk, dtype=cdt, device=dev)
+        # The score rows have a pitch of whole 16-byte pieces, so that TMA addresses them at any key count: at 500 keys (1000
+        # bytes per row) each of the products used to copy the scores to such a pitch first, 81 us a time for 128 x 500 x 500.
+        self.ldp = K.softmax_pitch(self.Sk) if ex.on_gpu else self.Sk
+        self.probs = torch.empty(self.B if not (self.cb or self.fused) else 0, H, self.Sq, self.ldp, dtype=cdt, device=dev)
         self.ctx = torch.empty(self.B * self.Sq, H * vd, dtype=dt, device=dev)
         if not self.core16:
             self.c_ctx = self.ctx
@@ -574,21 +577,24 @@ class AttentionOp(OpImpl):
             self._forward_core_blocked()
             return self._forward_out()
         # scores[b,h,sq,sk] = alpha * q . k^T
+        ldp = self.ldp
         self._bg(Sq, Sk, kd, self.c_q, self.ldq, kd, Sq * self.ldq, False, self.c_k, self.ldk, kd, Sk * self.ldk, False,
-                 self.probs, Sk, Sq * Sk, H * Sq * Sk, alpha=self.alpha)
+                 self.probs, ldp, Sq * ldp, H * Sq * ldp, alpha=self.alpha)
         causal_q = Sq if self.ex.cfg.causal_attention else 0
         p = self.probs
-        if self.p_drop > 0 and K.softmax_dropout_supported(self.probs):
-            # probabilities and their dropped copy in one pass
-            p = self.kept_p if self.kept_p is not None else self.ex.big_scratch(1, self.probs)
-            K.softmax_dropout_fwd(self.probs, self.probs, p, self.p_drop, self.salt, self.ex.seed_tensor, causal_q=causal_q)
+        if K.softmax_dropout_supported(self.probs, Sk):
+            # probabilities and, with dropout, their dropped copy in one pass
+            pd = None
+            if self.p_drop > 0:
+                p = pd = self.kept_p if self.kept_p is not None else self.ex.big_scratch(1, self.probs)
+            K.softmax_dropout_fwd(self.probs, self.probs, pd, self.p_drop, self.salt, self.ex.seed_tensor, causal_q=causal_q, cols=Sk)
         else:
             K.softmax_fwd(self.probs, out=self.probs, causal_q=causal_q)
             if self.p_drop > 0:
                 p = self.kept_p if self.kept_p is not None else self.ex.big_scratch(1, self.probs)
                 K.dropout(self.probs, self.p_drop, self.salt, out=p, seed_tensor=self.ex.seed_tensor)
         # ctx[b,sq,h,:] = p . v
-        self._bg(Sq, vd, Sk, p, Sk, Sq * Sk, H * Sq * Sk, False, self.c_v, self.ldv, vd, Sk * self.ldv, True,
+        self._bg(Sq, vd, Sk, p, ldp, Sq * ldp, H * Sq * ldp, False, self.c_v, self.ldv, vd, Sk * self.ldv, True,
                  self.c_ctx, H * vd, vd, Sq * H * vd)
         self._forward_out()
 
@@ -639,24 +645,28 @@ class AttentionOp(OpImpl):
             p = self.kept_p
         elif self.p_drop > 0:  # regenerate the dropped probabilities (mask is a function of the step seed)
             p = ex.big_scratch(1, self.probs)
-            K.dropout(self.probs, self.p_drop, self.salt, out=p, seed_tensor=ex.seed_tensor)
+            if self.ldp != Sk:
+                K.dropout_rows(self.probs, p, Sk, self.p_drop, self.salt, ex.seed_tensor)
+            else:
+                K.dropout(self.probs, self.p_drop, self.salt, out=p, seed_tensor=ex.seed_tensor)
+        ldp = self.ldp
         dP = ex.big_scratch(0, self.probs)
         # dP[b,h,sq,sk] = dctx[b,sq,h,:] . v[b,sk,h,:]^T
         self._bg(Sq, Sk, vd, self.c_dctx, H * vd, vd, Sq * H * vd, False, self.c_v, self.ldv, vd, Sk * self.ldv, False,
-                 dP, Sk, Sq * Sk, H * Sq * Sk)
+                 dP, ldp, Sq * ldp, H * Sq * ldp)
         # dV[b,sk,h,:] = p^T . dctx
-        self._bg(Sk, vd, Sq, p, Sk, Sq * Sk, H * Sq * Sk, True, self.c_dctx, H * vd, vd, Sq * H * vd, True,
+        self._bg(Sk, vd, Sq, p, ldp, Sq * ldp, H * Sq * ldp, True, self.c_dctx, H * vd, vd, Sq * H * vd, True,
                  self.c_dv, self.ldv, vd, Sk * self.ldv)
-        if K.softmax_dropout_supported(self.probs):
-            K.softmax_dropout_bwd(dP, self.probs, dP, self.p_drop, self.salt, ex.seed_tensor, scale=self.alpha)
+        if K.softmax_dropout_supported(self.probs, Sk):
+            K.softmax_dropout_bwd(dP, self.probs, dP, self.p_drop, self.salt, ex.seed_tensor, scale=self.alpha, cols=Sk)
         else:
             if self.p_drop > 0:
                 K.dropout(dP, self.p_drop, self.salt, out=dP, seed_tensor=ex.seed_tensor)
             K.softmax_bwd(dP, self.probs, dx=dP, scale=self.alpha)
         # dQ = dS . K ; dK = dS^T . Q
-        self._bg(Sq, kd, Sk, dP, Sk, Sq * Sk, H * Sq * Sk, False, self.c_k, self.ldk, kd, Sk * self.ldk, True,
+        self._bg(Sq, kd, Sk, dP, ldp, Sq * ldp, H * Sq * ldp, False, self.c_k, self.ldk, kd, Sk * self.ldk, True,
                  self.c_dq, self.ldq, kd, Sq * self.ldq)
-        self._bg(Sk, kd, Sq, dP, Sk, Sq * Sk, H * Sq * Sk, True, self.c_q, self.ldq, kd, Sq * self.ldq, True,
+        self._bg(Sk, kd, Sq, dP, ldp, Sq * ldp, H * Sq * ldp, True, self.c_q, self.ldq, kd, Sq * self.ldq, True,
                  self.c_dk, self.ldk, kd, Sk * self.ldk)
         self._backward_projections(wg, accw, n_q, n_k, n_v)
 

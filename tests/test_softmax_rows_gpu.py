@@ -1,0 +1,96 @@
+"""One-pass softmax, softmax + dropout and softmax + cross-entropy at the row lengths where their vectors end."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from flexflow_train_b200.ops import kernels as K  # noqa: E402
+
+# a bf16 result is within half an ulp (2^-9) of a value that carries the fp32 exponential's error (|x| * 2^-23 and 2 ulp)
+REL = 2.0 ** -8
+
+
+def _near(got, want, floor=1e-8):
+    want = want.double()
+    bad = (got.double() - want).abs() > REL * want.abs() + floor
+    assert not bad.any(), (int(bad.sum()), (got.double() - want).abs().max().item())
+
+
+@pytest.mark.parametrize("cols", [8, 248, 256, 264, 1000, 4088, 4096, 4104, 8192, 8200, 32000, 32776, 65536, 65544])
+@pytest.mark.parametrize("rows", [5, 700])  # 700: more rows than blocks, every ring stage is filled again
+def test_softmax_and_cross_entropy_rows(cols, rows):
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    x = (torch.randn(rows, cols, generator=gen, device="cuda") * 3).bfloat16()
+    x[1, 0], x[2, cols - 1] = float("-inf"), 40.0  # a masked logit, a row whose last element dominates
+    ref = torch.softmax(x.double(), -1)
+    _near(K.softmax_fwd(x), ref)
+    _near(K.softmax_fwd(x, scale=0.25), torch.softmax(x.double() * 0.25, -1))
+    for dt in (torch.int32, torch.int64):
+        labels = torch.randint(0, cols, (rows,), generator=gen, device="cuda", dtype=dt)
+        labels[:4] = torch.tensor([0, cols - 1, cols - 1, -1], device="cuda", dtype=dt)
+        loss, dl, probs = torch.empty(rows, device="cuda"), torch.empty_like(x), torch.empty_like(x)
+        K.softmax_ce(x, labels, loss, dl, probs, grad_scale=0.5)
+        _near(probs, ref)
+        want = ref.clone()
+        want[torch.arange(rows, device="cuda"), labels.long().clamp(min=0)] -= 1
+        want[3] = 0
+        _near(dl, want * 0.5, floor=2.0 ** -22)  # p - 1 cancels: fp32 ulps of 1
+        wl = torch.logsumexp(x.double(), -1) - x.double().gather(1, labels.long().clamp(min=0)[:, None])[:, 0]
+        wl[3] = 0
+        assert torch.allclose(loss.double(), wl, rtol=1e-5, atol=1e-5)
+    assert K.softmax_last_error() == 0
+
+
+@pytest.mark.parametrize("cols", [1, 7, 9, 250, 255, 257, 500, 1001, 4090])
+@pytest.mark.parametrize("causal", [False, True])
+def test_pitched_softmax_dropout(cols, causal):
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    rows, ld = 37, K.softmax_pitch(cols)
+    seed, salt, p = torch.tensor([1234567], device="cuda"), 99, 0.25
+    x = torch.full((rows, ld), float("nan"), device="cuda", dtype=torch.bfloat16)  # what the pitch's tail holds is nobody's
+    x[:, :cols] = torch.randn(rows, cols, generator=gen, device="cuda").bfloat16()
+    xd = x[:, :cols].double() * 0.5
+    if causal:
+        q = torch.arange(rows, device="cuda") % 10
+        xd = xd.masked_fill(torch.arange(cols, device="cuda")[None] > q[:, None], float("-inf"))
+    ref = torch.softmax(xd, -1)
+    keep = K.dropout(torch.ones(rows, cols, device="cuda"), p, salt, seed_tensor=seed)  # the flat mask, scaled
+    y, yd, again = torch.empty_like(x), torch.empty_like(x), torch.empty_like(x)
+    K.softmax_dropout_fwd(x, y, yd, p, salt, seed, scale=0.5, causal_q=10 if causal else 0, cols=cols)
+    _near(y[:, :cols], ref)
+    _near(yd[:, :cols], ref * keep)
+    assert not y[:, cols:].any() and not yd[:, cols:].any()
+    K.dropout_rows(y, again, cols, p, salt, seed)
+    _near(again[:, :cols], y[:, :cols].double() * keep)
+    dy = torch.full_like(x, float("nan"))
+    dy[:, :cols] = torch.randn(rows, cols, generator=gen, device="cuda").bfloat16()
+    dx = torch.empty_like(x)
+    K.softmax_dropout_bwd(dy, y, dx, p, salt, seed, scale=0.5, cols=cols)
+    g, yr = dy[:, :cols].double() * keep, y[:, :cols].double()
+    want = 0.5 * yr * (g - (g * yr).sum(-1, keepdim=True))
+    # the row sum is one of fp32: its error, up to cols ulps of the sum of magnitudes, times y
+    slack = 0.5 * yr * (g * yr).abs().sum(-1, keepdim=True) * cols * 2.0 ** -24
+    assert ((dx[:, :cols].double() - want).abs() <= REL * want.abs() + slack + 1e-9).all()
+
+
+def test_attention_core_with_odd_key_counts():
+    """Unfused attention at a key count whose score rows need a pitch, against the fused kernels; dropped probabilities kept and
+    formed again."""
+    from flexflow_train_b200 import _ffcore as core
+    from flexflow_train_b200.runtime.executor import ExecConfig, Executable, OptimizerConfig
+
+    def run(fused, drop, keep):
+        cfg = {"batch_size": 2, "sequence_length": 43, "num_heads": 2, "dim_feedforward": 64, "num_features": 128, "num_encoder_layers": 1,
+               "num_decoder_layers": 1, "vocab_size": 64, "dropout": drop}
+        g = core.build_model("transformer", cfg)
+        ex = Executable(g, ExecConfig(seed=3, fused_attention=fused, keep_dropped_probs=keep, optimizer=OptimizerConfig(kind="sgd", lr=0.1)))
+        gen = torch.Generator(device="cuda").manual_seed(0)
+        ins = {n["name"]: torch.randn(list(n["outputs"][0][1].sizes), generator=gen, device="cuda") for n in g.nodes() if n["type"] == "INPUT"}
+        labels = torch.randint(0, 64, (86,), generator=gen, device="cuda", dtype=torch.int32)
+        ex.train_step(ins, labels)
+        return ex.grads.float().clone()
+
+    a, b = run(False, 0.0, True), run(True, 0.0, True)
+    assert (a - b).norm() / b.norm() < 3e-2  # bf16 scores and probabilities against fp32 ones
+    a, b = run(False, 0.3, True), run(False, 0.3, False)  # kept and regenerated dropped probabilities: one rounding apart
+    assert (a - b).norm() / b.norm() < 1e-2
