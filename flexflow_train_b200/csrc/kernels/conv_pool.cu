@@ -553,65 +553,79 @@ __global__ void pool_bwd_vec_kernel(const bf16 *__restrict__ dy, const unsigned 
 // walks rows lane, lane + lanes, ... of the block's row chunk; consecutive threads read consecutive 16-byte
 // pieces of memory (the last group of a row is followed by the first group of the next row).  Per-lane sums go
 // through shared memory in a fixed order, so the result does not depend on scheduling.
+// Bound by HBM, or by L2 where the activation still lies there: four rows per trip keep 4 (backward: 8) loads in flight per
+// thread.  Backward used to walk one row at a time and to read the forward output for the ReLU mask; the mask is the sign of
+// x * scale + shift, the very value the forward pass rounded and clamped, so x gives it when the caller hands over the shift.
 constexpr int BNV_THREADS = 256;
-__global__ void bn_partial_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, const bf16 *__restrict__ relu_y,
-                                      float *__restrict__ part, const float *__restrict__ mean, const float *__restrict__ rstd, long long R,
-                                      int C, int rows_per_chunk, int mode) {
+// forward: y = relu(x * scale + shift)
+__device__ __forceinline__ void bn_scale_shift(const bf16 *gamma, const bf16 *beta, const float *mean, const float *rstd, int c, float (&sc)[8],
+                                               float (&sh)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    sc[i] = __fmul_rn(rstd[c + i], gamma ? bf2f(gamma[c + i]) : 1.f);
+    sh[i] = __fmaf_rn(-mean[c + i], sc[i], beta ? bf2f(beta[c + i]) : 0.f);
+  }
+}
+// mode 0: sums of a and a*a; mode 1: sums of dy' and dy' * xhat with a = dy, b = x, dy' = dy where the forward ReLU passed
+enum { BN_NO_RELU = 0, BN_RELU_Y = 1, BN_RELU_X = 2 };  // no ReLU; its mask from the forward output; from x, gamma and beta
+template <int MODE, int RELU>
+__global__ void __launch_bounds__(BNV_THREADS, 3)
+bn_partial_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, const bf16 *__restrict__ relu_y,
+                      const bf16 *__restrict__ gamma, const bf16 *__restrict__ beta,
+                      float *__restrict__ part, const float *__restrict__ mean, const float *__restrict__ rstd, long long R, int C,
+                      int rows_per_chunk) {
   extern __shared__ float sred[];  // [lanes][2][C]
   const int groups = C >> 3;
   const int lanes = BNV_THREADS / groups;
   const int gidx = threadIdx.x % groups, lane = threadIdx.x / groups;
-  long long r0 = (long long)blockIdx.x * rows_per_chunk;
-  long long r1 = r0 + rows_per_chunk < R ? r0 + rows_per_chunk : R;
-  float u[8], v[8], m[8], rs[8];
+  const long long r0 = (long long)blockIdx.x * rows_per_chunk;
+  const long long r1 = r0 + rows_per_chunk < R ? r0 + rows_per_chunk : R;
+  float u[8], v[8], m[8], sc[8], sh[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) { u[i] = 0.f; v[i] = 0.f; m[i] = 0.f; rs[i] = 0.f; }
+  for (int i = 0; i < 8; ++i) { u[i] = 0.f; v[i] = 0.f; m[i] = 0.f; sc[i] = 0.f; sh[i] = 0.f; }
   if (lane < lanes) {
-    if (mode) {
+    if (MODE) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { m[i] = mean[gidx * 8 + i]; rs[i] = rstd[gidx * 8 + i]; }
+      for (int i = 0; i < 8; ++i) m[i] = mean[gidx * 8 + i];
+      if (RELU == BN_RELU_X) bn_scale_shift(gamma, beta, mean, rstd, gidx * 8, sc, sh);
     }
-    long long r = r0 + lane;
-    if (mode == 0) {
-      // four rows per trip: four independent 16-byte loads in flight per thread
-      for (; r + 3LL * lanes < r1; r += 4LL * lanes) {
-        uint4 q0 = *reinterpret_cast<const uint4 *>(a + r * C + gidx * 8);
-        uint4 q1 = *reinterpret_cast<const uint4 *>(a + (r + lanes) * C + gidx * 8);
-        uint4 q2 = *reinterpret_cast<const uint4 *>(a + (r + 2LL * lanes) * C + gidx * 8);
-        uint4 q3 = *reinterpret_cast<const uint4 *>(a + (r + 3LL * lanes) * C + gidx * 8);
-        float f0[8], f1[8], f2[8], f3[8];
-        unpack8(q0, f0); unpack8(q1, f1); unpack8(q2, f2); unpack8(q3, f3);
+    auto add = [&](const uint4 &qa, const uint4 &qb, const uint4 &qy) {
+      float av[8], xv[8], yv[8];
+      unpack8(qa, av);
+      if (MODE) unpack8(qb, xv);
+      if (RELU == BN_RELU_Y) unpack8(qy, yv);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          u[i] += (f0[i] + f1[i]) + (f2[i] + f3[i]);
-          v[i] += (f0[i] * f0[i] + f1[i] * f1[i]) + (f2[i] * f2[i] + f3[i] * f3[i]);
+      for (int i = 0; i < 8; ++i) {
+        if (!MODE) { u[i] += av[i]; v[i] += av[i] * av[i]; }
+        else {
+          if (RELU == BN_RELU_X && !(__fmaf_rn(xv[i], sc[i], sh[i]) > 0.f)) av[i] = 0.f;
+          if (RELU == BN_RELU_Y && yv[i] <= 0.f) av[i] = 0.f;
+          u[i] += av[i];
+          v[i] += av[i] * (xv[i] - m[i]);
         }
       }
-    }
-    for (; r < r1; r += lanes) {
-      const long long off = r * C + gidx * 8;
-      float av[8];
-      unpack8(*reinterpret_cast<const uint4 *>(a + off), av);
-      if (mode == 0) {
+    };
+    const long long step = (long long)lanes * C;
+    const uint4 none = make_uint4(0, 0, 0, 0);
+    long long r = r0 + lane, off = r * C + gidx * 8;
+    for (; r + 3LL * lanes < r1; r += 4LL * lanes, off += 4 * step) {
+      uint4 qa[4], qb[4], qy[4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) { u[i] += av[i]; v[i] += av[i] * av[i]; }
-      } else {
-        float xv[8];
-        unpack8(*reinterpret_cast<const uint4 *>(b + off), xv);
-        if (relu_y) {
-          float yv[8];
-          unpack8(*reinterpret_cast<const uint4 *>(relu_y + off), yv);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) if (yv[i] <= 0.f) av[i] = 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { u[i] += av[i]; v[i] += av[i] * (xv[i] - m[i]) * rs[i]; }
+      for (int k = 0; k < 4; ++k) {
+        qa[k] = *reinterpret_cast<const uint4 *>(a + off + k * step);
+        qb[k] = MODE ? *reinterpret_cast<const uint4 *>(b + off + k * step) : none;
+        qy[k] = RELU == BN_RELU_Y ? *reinterpret_cast<const uint4 *>(relu_y + off + k * step) : none;
       }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) add(qa[k], qb[k], qy[k]);
     }
+    for (; r < r1; r += lanes, off += step)
+      add(*reinterpret_cast<const uint4 *>(a + off), MODE ? *reinterpret_cast<const uint4 *>(b + off) : none,
+          RELU == BN_RELU_Y ? *reinterpret_cast<const uint4 *>(relu_y + off) : none);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       sred[(lane * 2 + 0) * C + gidx * 8 + i] = u[i];
-      sred[(lane * 2 + 1) * C + gidx * 8 + i] = v[i];
+      sred[(lane * 2 + 1) * C + gidx * 8 + i] = MODE ? v[i] * rstd[gidx * 8 + i] : v[i];
     }
   }
   __syncthreads();
@@ -621,43 +635,48 @@ __global__ void bn_partial_vec_kernel(const bf16 *__restrict__ a, const bf16 *__
     part[(long long)blockIdx.x * 2 * C + c] = s;
   }
 }
-__global__ void bn_apply_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, const bf16 *__restrict__ gamma,
-                                    const bf16 *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd,
-                                    long long total8, int C, int relu) {
-  // the grid-stride step is a multiple of the number of channel groups, so a thread stays on one group and
-  // keeps that group's scale and shift in registers: y = x * scale + shift
+// Element-wise passes: the grid-stride step is a multiple of the number of channel groups, so a thread stays on one group and
+// keeps that group's constants in registers; two 16-byte pieces per operand and trip.
+__global__ void __launch_bounds__(256) bn_apply_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, const bf16 *__restrict__ gamma,
+                                                           const bf16 *__restrict__ beta, const float *__restrict__ mean,
+                                                           const float *__restrict__ rstd, long long total8, int C, int relu) {
   const int groups = C >> 3;
   const long long usable = ((long long)gridDim.x * blockDim.x / groups) * groups;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t0 >= usable) return;
-  const int c = (int)(t0 % groups) * 8;
   float sc[8], sh[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    sc[i] = rstd[c + i] * (gamma ? bf2f(gamma[c + i]) : 1.f);
-    sh[i] = (beta ? bf2f(beta[c + i]) : 0.f) - mean[c + i] * sc[i];
-  }
+  bn_scale_shift(gamma, beta, mean, rstd, (int)(t0 % groups) * 8, sc, sh);
   const float floor_ = relu ? 0.f : -INFINITY;
-  for (long long t = t0; t < total8; t += usable) {
+  auto one = [&](const uint4 &q) {
     float f[8];
-    unpack8(reinterpret_cast<const uint4 *>(x)[t], f);
+    unpack8(q, f);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = fmaxf(fmaf(f[i], sc[i], sh[i]), floor_);
-    reinterpret_cast<uint4 *>(y)[t] = pack8(f);
+    for (int i = 0; i < 8; ++i) f[i] = fmaxf(__fmaf_rn(f[i], sc[i], sh[i]), floor_);
+    return pack8(f);
+  };
+  const uint4 *xv = reinterpret_cast<const uint4 *>(x);
+  uint4 *yv = reinterpret_cast<uint4 *>(y);
+  long long t = t0;
+  for (; t + usable < total8; t += 2 * usable) {
+    const uint4 q0 = xv[t], q1 = xv[t + usable];
+    yv[t] = one(q0);
+    yv[t + usable] = one(q1);
   }
+  if (t < total8) yv[t] = one(xv[t]);
 }
-__global__ void bn_bwd_apply_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ relu_y,
-                                        const bf16 *__restrict__ gamma, const float *__restrict__ mean, const float *__restrict__ rstd,
-                                        const float *__restrict__ sums, bf16 *__restrict__ dx, long long total8, int C, float inv_r,
-                                        int accumulate) {
-  // dx = a * dy' + b * x + c per channel (constants kept in registers, see bn_apply_vec_kernel):
-  //   xh = (x - mean) * rstd;  dx = gamma * rstd * (dy' - s1/R - xh * s2/R)
+// dx = ka * dy' + kb * x + kc per channel, xh = (x - mean) * rstd:  dx = gamma * rstd * (dy' - s1/R - xh * s2/R)
+template <int RELU>
+__global__ void __launch_bounds__(256)
+bn_bwd_apply_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ relu_y, const bf16 *__restrict__ gamma,
+                        const bf16 *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd,
+                        const float *__restrict__ sums, bf16 *__restrict__ dx, long long total8, int C, float inv_r, int accumulate) {
   const int groups = C >> 3;
   const long long usable = ((long long)gridDim.x * blockDim.x / groups) * groups;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t0 >= usable) return;
   const int c = (int)(t0 % groups) * 8;
-  float ka[8], kb[8], kc[8];
+  float ka[8], kb[8], kc[8], sc[8], sh[8];
+  if (RELU == BN_RELU_X) bn_scale_shift(gamma, beta, mean, rstd, c, sc, sh);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float rs = rstd[c + i], g = gamma ? bf2f(gamma[c + i]) : 1.f;
@@ -666,24 +685,34 @@ __global__ void bn_bwd_apply_vec_kernel(const bf16 *__restrict__ dy, const bf16 
     kb[i] = -g * rs * rs * s2;
     kc[i] = g * rs * (mean[c + i] * rs * s2 - s1);
   }
-  for (long long t = t0; t < total8; t += usable) {
-    float g[8], xv[8], o[8];
-    unpack8(reinterpret_cast<const uint4 *>(dy)[t], g);
-    unpack8(reinterpret_cast<const uint4 *>(x)[t], xv);
-    if (relu_y) {
-      float yv[8];
-      unpack8(reinterpret_cast<const uint4 *>(relu_y)[t], yv);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) if (yv[i] <= 0.f) g[i] = 0.f;
-    }
-    if (accumulate) unpack8(reinterpret_cast<const uint4 *>(dx)[t], o);
+  auto one = [&](const uint4 &qg, const uint4 &qx, const uint4 &qy, const uint4 &qo) {
+    float g[8], xv[8], yv[8], o[8];
+    unpack8(qg, g);
+    unpack8(qx, xv);
+    if (RELU == BN_RELU_Y) unpack8(qy, yv);
+    if (accumulate) unpack8(qo, o);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
+      if (RELU == BN_RELU_X && !(__fmaf_rn(xv[i], sc[i], sh[i]) > 0.f)) g[i] = 0.f;
+      if (RELU == BN_RELU_Y && yv[i] <= 0.f) g[i] = 0.f;
       const float v = fmaf(ka[i], g[i], fmaf(kb[i], xv[i], kc[i]));
       o[i] = accumulate ? o[i] + v : v;
     }
-    reinterpret_cast<uint4 *>(dx)[t] = pack8(o);
+    return pack8(o);
+  };
+  const uint4 *gp = reinterpret_cast<const uint4 *>(dy), *xp = reinterpret_cast<const uint4 *>(x), *yp = reinterpret_cast<const uint4 *>(relu_y);
+  uint4 *op = reinterpret_cast<uint4 *>(dx);
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  long long t = t0;
+  for (; t + usable < total8; t += 2 * usable) {
+    const long long t2 = t + usable;
+    const uint4 g0 = gp[t], g1 = gp[t2], x0 = xp[t], x1 = xp[t2];
+    const uint4 y0 = RELU == BN_RELU_Y ? yp[t] : none, y1 = RELU == BN_RELU_Y ? yp[t2] : none;
+    const uint4 o0 = accumulate ? op[t] : none, o1 = accumulate ? op[t2] : none;
+    op[t] = one(g0, x0, y0, o0);
+    op[t2] = one(g1, x1, y1, o1);
   }
+  if (t < total8) op[t] = one(gp[t], xp[t], RELU == BN_RELU_Y ? yp[t] : none, accumulate ? op[t] : none);
 }
 
 inline FastDiv make_fd(int d_) {
@@ -820,7 +849,7 @@ static bool bn_vec_ok(int C, const void *a, const void *b, const void *c) {
 static int bn_chunks_vec(long long R, int C, int *rows_per_chunk) {
   const int lanes = BNV_THREADS / (C / 8);
   long long maxc = (R + 4LL * lanes - 1) / (4LL * lanes);  // at least ~4 rows per thread
-  long long chunks = maxc < 148 * 4 ? maxc : 148 * 4;
+  long long chunks = maxc < 148 * 3 ? maxc : 148 * 3;
   if (chunks < 1) chunks = 1;
   long long rpc = (R + chunks - 1) / chunks;
   chunks = (R + rpc - 1) / rpc;
@@ -850,10 +879,10 @@ FFK_API int ffk_batchnorm_fwd(const void *x, void *y, const void *gamma, const v
     int rv;
     int cv = bn_chunks_vec(R, C, &rv);
     const int lanes = BNV_THREADS / (C / 8);
-    bn_partial_vec_kernel<<<cv, BNV_THREADS, (size_t)lanes * 2 * C * sizeof(float), st>>>((const bf16 *)x, nullptr, nullptr, scratch, nullptr,
-                                                                                          nullptr, R, C, rv, 0);
+    bn_partial_vec_kernel<0, BN_NO_RELU><<<cv, BNV_THREADS, (size_t)lanes * 2 * C * sizeof(float), st>>>(
+        (const bf16 *)x, nullptr, nullptr, nullptr, nullptr, scratch, nullptr, nullptr, R, C, rv);
     bn_finalize_stats_kernel<<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, cv, C, R, eps, mean, rstd);
-    bn_apply_vec_kernel<<<ffk_blocks(total / 8, 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta, mean,
+    bn_apply_vec_kernel<<<ffk_blocks(total / 8, 512), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta, mean,
                                                                     rstd, total / 8, C, relu);
     return (int)cudaGetLastError();
   }
@@ -877,10 +906,11 @@ FFK_API int ffk_batchnorm_fwd(const void *x, void *y, const void *gamma, const v
   return (int)cudaGetLastError();
 }
 
-// relu_y: the forward output when a ReLU was fused (masks dy), else null.  dgamma/dbeta may be null.
-FFK_API int ffk_batchnorm_bwd(const void *dy, const void *x, const void *relu_y, const void *gamma, const float *mean, const float *rstd,
-                              void *dx, void *dgamma, void *dbeta, float *scratch, long long R, int C, int dt, int accumulate_dx,
-                              int accumulate_gamma, int accumulate_beta, cudaStream_t st) {
+// relu_y: the forward output when a ReLU was fused (masks dy), else null.  mask_from_x: gamma and beta are still those of the
+// forward pass, so the mask may be taken from x instead.  dgamma/dbeta may be null.
+FFK_API int ffk_batchnorm_bwd(const void *dy, const void *x, const void *relu_y, const void *gamma, const void *beta, int mask_from_x,
+                              const float *mean, const float *rstd, void *dx, void *dgamma, void *dbeta, float *scratch, long long R, int C,
+                              int dt, int accumulate_dx, int accumulate_gamma, int accumulate_beta, cudaStream_t st) {
   if (R <= 0 || C <= 0) return 0;
   int rpc;
   int chunks = bn_chunks(R, C, &rpc);
@@ -893,14 +923,25 @@ FFK_API int ffk_batchnorm_bwd(const void *dy, const void *x, const void *relu_y,
     int cv = bn_chunks_vec(R, C, &rv);
     const int lanes = BNV_THREADS / (C / 8);
     float *sums_v = scratch + (long long)cv * 2 * C;
-    bn_partial_vec_kernel<<<cv, BNV_THREADS, (size_t)lanes * 2 * C * sizeof(float), st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y,
-                                                                                          scratch, mean, rstd, R, C, rv, 1);
+    const size_t psm = (size_t)lanes * 2 * C * sizeof(float);
+    const int ag = ffk_blocks(total / 8, 512);
+    const int mask = !relu_y ? BN_NO_RELU : mask_from_x ? BN_RELU_X : BN_RELU_Y;
+#define BN_PART(M)                                                                                                                     \
+  bn_partial_vec_kernel<1, M><<<cv, BNV_THREADS, psm, st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, (const bf16 *)gamma, \
+                                                            (const bf16 *)beta, scratch, mean, rstd, R, C, rv)
+#define BN_APPLY(M)                                                                                                                   \
+  bn_bwd_apply_vec_kernel<M><<<ag, 256, 0, st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, (const bf16 *)gamma,          \
+                                                 (const bf16 *)beta, mean, rstd, sums_v, (bf16 *)dx, total / 8, C, inv_r, accumulate_dx)
+    if (mask == BN_RELU_X) BN_PART(BN_RELU_X);
+    else if (mask == BN_RELU_Y) BN_PART(BN_RELU_Y);
+    else BN_PART(BN_NO_RELU);
     bn_finalize_grads_kernel<bf16><<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, cv, C, sums_v, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_gamma,
                                                                      accumulate_beta);
-    if (dx)
-      bn_bwd_apply_vec_kernel<<<ffk_blocks(total / 8, 256), 256, 0, st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y,
-                                                                          (const bf16 *)gamma, mean, rstd, sums_v, (bf16 *)dx, total / 8, C,
-                                                                          inv_r, accumulate_dx);
+    if (dx && mask == BN_RELU_X) BN_APPLY(BN_RELU_X);
+    else if (dx && mask == BN_RELU_Y) BN_APPLY(BN_RELU_Y);
+    else if (dx) BN_APPLY(BN_NO_RELU);
+#undef BN_PART
+#undef BN_APPLY
     return (int)cudaGetLastError();
   }
   if (dt == 1) {

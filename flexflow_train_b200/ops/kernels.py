@@ -1008,7 +1008,7 @@ def _decl_conv(l):
         "ffk_pool2d_bwd": ([P, P, P, IP, LP, I, I, I, S], c_int),
         "ffk_batchnorm_scratch": ([L, I], c_longlong),
         "ffk_batchnorm_fwd": ([P, P, P, P, P, P, P, L, I, F, I, I, S], c_int),
-        "ffk_batchnorm_bwd": ([P, P, P, P, P, P, P, P, P, P, L, I, I, I, I, I, S], c_int),
+        "ffk_batchnorm_bwd": ([P, P, P, P, P, I, P, P, P, P, P, P, L, I, I, I, I, I, S], c_int),
     }
     for name, (args, res) in sig.items():
         fn = getattr(l, name)
@@ -1148,8 +1148,11 @@ def batchnorm_fwd(x, y, gamma, beta, mean, rstd, scratch, rows, cols, eps, relu=
 
 
 def batchnorm_bwd(dy, x, relu_y, gamma, mean, rstd, dx, dgamma, dbeta, scratch, rows, cols, accumulate_dx=False,
-                  accumulate_gamma=False, accumulate_beta=False):
-    _cuda_contig(dy, x, relu_y, gamma, mean, rstd, dx, dgamma, dbeta, scratch)
-    _check(_clib().ffk_batchnorm_bwd(dy.data_ptr(), x.data_ptr(), _p(relu_y), _p(gamma), mean.data_ptr(), rstd.data_ptr(), _p(dx),
+                  accumulate_gamma=False, accumulate_beta=False, beta=None, mask_from_x=False):
+    """mask_from_x: gamma and `beta` are those of the forward pass, so a fused ReLU's mask may be formed again from x instead of
+    read from relu_y."""
+    _cuda_contig(dy, x, relu_y, gamma, mean, rstd, dx, dgamma, dbeta, scratch, beta)
+    _check(_clib().ffk_batchnorm_bwd(dy.data_ptr(), x.data_ptr(), _p(relu_y), _p(gamma), _p(beta), int(mask_from_x),
+                                     mean.data_ptr(), rstd.data_ptr(), _p(dx),
                                      _p(dgamma), _p(dbeta), scratch.data_ptr(), rows, cols, _dt(dy), int(accumulate_dx),
                                      int(accumulate_gamma), int(accumulate_beta), _stream()), "ffk_batchnorm_bwd")

@@ -307,7 +307,8 @@ class BatchNormOp(OpImpl):
                         gb.grad if gb is not None and gb.requires_grad else None,
                         bb.grad if bb is not None and bb.requires_grad else None, self.ex.scratch_f32(), self.rows, self.cols,
                         accumulate_dx=self.acc.get("INPUT", False) and self.in_nhwc,
-                        accumulate_gamma=self.acc.get("GAMMA", False), accumulate_beta=self.acc.get("BETA", False))
+                        accumulate_gamma=self.acc.get("GAMMA", False), accumulate_beta=self.acc.get("BETA", False),
+                        beta=self.beta, mask_from_x=True)
         if dx is not None and not self.in_nhwc:
             n, c, h, w = self.shape
             K.permute(dx.view(n, h, w, c), (0, 3, 1, 2), out=xb.grad.view(n, c, h, w), accumulate=self.acc["INPUT"])

@@ -234,3 +234,25 @@ def test_inception_v3_trains_one_step():
         losses.append(ex.mean_loss())
     assert all(l == l and l < 1e4 for l in losses), losses
     assert K.gemm_last_error() == 0
+
+
+@pytest.mark.parametrize("cols", [8, 24, 192, 2048])
+@pytest.mark.parametrize("rows", [1, 37, 5000])
+@pytest.mark.parametrize("affine", [False, True])
+def test_batchnorm_relu_mask_from_x(rows, cols, affine):
+    """The ReLU mask formed again from x is the mask of the forward output, element for element."""
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, device="cuda", generator=g).bfloat16()
+    dy = torch.randn(rows, cols, device="cuda", generator=g).bfloat16()
+    gamma = torch.randn(cols, device="cuda", generator=g).bfloat16() if affine else None
+    beta = torch.randn(cols, device="cuda", generator=g).bfloat16() if affine else None
+    y, mean, rstd = torch.empty_like(x), torch.empty(cols, device="cuda"), torch.empty(cols, device="cuda")
+    scratch = torch.empty(K.batchnorm_scratch(rows, cols), device="cuda")
+    K.batchnorm_fwd(x, y, gamma, beta, mean, rstd, scratch, rows, cols, 1e-5, relu=True)
+    out = []
+    for from_x in (False, True):
+        dx, dg, db = torch.full_like(x, 0.5), torch.empty(cols, device="cuda").bfloat16(), torch.empty(cols, device="cuda").bfloat16()
+        K.batchnorm_bwd(dy, x, y, gamma, mean, rstd, dx, dg, db, scratch, rows, cols, accumulate_dx=True, beta=beta, mask_from_x=from_x)
+        out.append((dx, dg, db))
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
