@@ -155,67 +155,72 @@ conv_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {  // the whole warp runs the loop, one lane issues (see the GEMM kernel)
+      const bool leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (long long item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
         const ConvItem it = decode_item<MODE>(item, p);
         for (int kb = it.k0; kb < it.k1; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
+          ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
           if (!ok) break;
           const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
           const uint32_t sb = sa + Cfg::A_BYTES;
-          if constexpr (!WG) {
-            const int tap = kb / p.chunks, cc = kb - tap * p.chunks;
-            const int r = tap / p.KW, s = tap - r * p.KW;
-            mbar_expect_tx(&full_bar[stage], box_bytes + (uint32_t)Cfg::B_BYTES);
-            tma_load_4d(sa, &tmapA, &full_bar[stage], cc * 64, it.w0 + p.off_w + p.sgn * s, it.h0 + p.off_h + p.sgn * r, it.n0);
-            if constexpr (MODE == CONV_FPROP) {
-              // BN filter rows, 64 reduction columns of this tap and chunk (columns past the tap's C meet zero channels)
-              tma_load_4d(sb, &tmapB, &full_bar[stage], tap * p.Cf + cc * 64, it.nb * BN, 0, 0);
+          if (leader) {
+            if constexpr (!WG) {
+              const int tap = kb / p.chunks, cc = kb - tap * p.chunks;
+              const int r = tap / p.KW, s = tap - r * p.KW;
+              mbar_expect_tx(&full_bar[stage], box_bytes + (uint32_t)Cfg::B_BYTES);
+              tma_load_4d(sa, &tmapA, &full_bar[stage], cc * 64, it.w0 + p.off_w + p.sgn * s, it.h0 + p.off_h + p.sgn * r, it.n0);
+              if constexpr (MODE == CONV_FPROP) {
+                // BN filter rows, 64 reduction columns of this tap and chunk (columns past the tap's C meet zero channels)
+                tma_load_4d(sb, &tmapB, &full_bar[stage], tap * p.Cf + cc * 64, it.nb * BN, 0, 0);
+              } else {
+#pragma unroll
+                for (int c = 0; c < BN / 64; ++c)
+                  tma_load_4d(sb + c * 64 * 128, &tmapB, &full_bar[stage], tap * p.Cf + it.nb * BN + c * 64, cc * 64, 0, 0);
+              }
             } else {
+              int t = kb;
+              const int w0 = (t % p.tiles_w) * p.bw;
+              t /= p.tiles_w;
+              const int h0 = (t % p.tiles_h) * p.bh;
+              const int n0 = (t / p.tiles_h) * p.bn;
+              const int r = it.tap / p.KW, s = it.tap - r * p.KW;
+              mbar_expect_tx(&full_bar[stage], box_bytes * (uint32_t)(2 + BN / 64));
 #pragma unroll
-              for (int c = 0; c < BN / 64; ++c)
-                tma_load_4d(sb + c * 64 * 128, &tmapB, &full_bar[stage], tap * p.Cf + it.nb * BN + c * 64, cc * 64, 0, 0);
+              for (int c = 0; c < 2; ++c)
+                tma_load_4d(sa + c * 128 * 128, &tmapA, &full_bar[stage], it.mb * 128 + c * 64, w0 + p.off_w + s, h0 + p.off_h + r, n0);
+#pragma unroll
+              for (int c = 0; c < BN / 64; ++c) tma_load_4d(sb + c * 128 * 128, &tmapB, &full_bar[stage], it.nb * BN + c * 64, w0, h0, n0);
             }
-          } else {
-            int t = kb;
-            const int w0 = (t % p.tiles_w) * p.bw;
-            t /= p.tiles_w;
-            const int h0 = (t % p.tiles_h) * p.bh;
-            const int n0 = (t / p.tiles_h) * p.bn;
-            const int r = it.tap / p.KW, s = it.tap - r * p.KW;
-            mbar_expect_tx(&full_bar[stage], box_bytes * (uint32_t)(2 + BN / 64));
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-              tma_load_4d(sa + c * 128 * 128, &tmapA, &full_bar[stage], it.mb * 128 + c * 64, w0 + p.off_w + s, h0 + p.off_h + r, n0);
-#pragma unroll
-            for (int c = 0; c < BN / 64; ++c) tma_load_4d(sb + c * 128 * 128, &tmapB, &full_bar[stage], it.nb * BN + c * 64, w0, h0, n0);
           }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
       for (int s = 0; s < STAGES && ok; ++s) {   // every load issued has landed and been consumed before the CTA exits
-        ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
+      const bool leader = elect_one();
       int stage = 0, acc = 0;
       uint32_t phase = 0, acc_phase = 0;
       bool ok = true;
       const int wg_ksteps = (p.rows + 15) / 16;
       for (long long item = blockIdx.x; item < p.num_items && ok; item += gridDim.x) {
         const ConvItem it = decode_item<MODE>(item, p);
-        ok = mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+        ok = mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
         for (int kb = it.k0; kb < it.k1; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+          ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
           if (!ok) break;
           tc_fence_after();
           const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
@@ -226,14 +231,18 @@ conv_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
             const int left = p.CK - (kb % p.chunks) * 64;
             ksteps = left >= 64 ? 4 : (left + 15) / 16;
           }
-          for (int k = 0; k < ksteps; ++k)
-            tc_mma<false>(d_tmem, desc_advance(adesc, (uint32_t)k * Cfg::A_KADV), desc_advance(bdesc, (uint32_t)k * Cfg::B_KADV), Cfg::IDESC,
-                          ((kb - it.k0) | k) != 0 ? 1u : 0u);
-          tc_commit(&empty_bar[stage]);
+          if (leader) {
+            for (int k = 0; k < ksteps; ++k)
+              tc_mma<false>(d_tmem, desc_advance(adesc, (uint32_t)k * Cfg::A_KADV), desc_advance(bdesc, (uint32_t)k * Cfg::B_KADV), Cfg::IDESC,
+                            ((kb - it.k0) | k) != 0 ? 1u : 0u);
+            tc_commit(&empty_bar[stage]);
+          }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        tc_commit(&tmem_full[acc]);
+        if (leader) tc_commit(&tmem_full[acc]);
+        __syncwarp();
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }

@@ -15,10 +15,20 @@
 // without a transpose pass.  Two batch dimensions (inner `nh`, outer `nb`)
 // with independent strides cover attention's [batch, seq, head, dim] views.
 //
-// CTA layout (320 threads): warp 0 issues TMA loads, warp 1 allocates TMEM and
-// issues tcgen05.mma from one thread, warps 2..9 are the epilogue (TMEM ->
-// registers -> bias/activation/addend -> global).  Two TMEM accumulator stages
-// let the epilogue of tile i overlap the main loop of tile i+1.
+// CTA layout (384 threads): warp 0 issues TMA loads, warp 1 allocates TMEM and
+// issues tcgen05.mma, warps 2..9 are the epilogue (TMEM -> registers ->
+// bias/activation/addend -> global), warps 10 and 11 push a shard to the peers.
+// Two TMEM accumulator stages let the epilogue of tile i overlap the main loop
+// of tile i+1.
+//
+// The issuing warps run their loops as a whole, with one elected lane for the
+// TMA, MMA and commit instructions.  With the loop inside `if (lane == 0)` the
+// compiler keeps the addresses and descriptors in per-thread registers and moves
+// each into the uniform registers these instructions take: 0.28 us per k-block
+// whatever the tile (128 x 512 x 2048: 13.8 us, now 12.2; 128 x 64 tiles 13.4,
+// now 11.1), with MN-major operands, which take a TMA load per 64 columns, 0.31
+// (2048 x 2048 x 8000, both MN-major, 80 us, now 63; tf32 2048 x 2048 x 4096 84,
+// now 67).
 //
 // Every mbarrier wait is bounded: after ~2 s without progress the waiting thread
 // records an error code, raises a CTA-wide abort flag and every role leaves its
@@ -224,7 +234,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    {  // the whole warp runs the loop, one lane issues
+      const bool leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -255,6 +266,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
               }
               __nanosleep(100);
             }
+            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             gate_seen |= 1u << src;
             // the pushed rows were written by a peer through the generic proxy; order them before the
@@ -263,45 +275,48 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
           }
         }
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
+          ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
           if (!ok) break;
           uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
           uint32_t sb = sa + Cfg::A_BYTES;
           int k0 = kb * Cfg::BK;
-          if constexpr (CTA2) {
-            // both CTAs' loads are counted on the even CTA's barrier, which expects the bytes of the whole pair
-            if (pair_rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::STAGE_BYTES);
-            const uint32_t fb = mapa_u32(smem_u32(&full_bar[stage]), 0);
-            if constexpr (!A_MN) {
-              tma_load_4d_pair(sa, &tmapA, fb, k0, a_row, bh, bb);
-            } else {
+          if (leader) {
+            if constexpr (CTA2) {
+              // both CTAs' loads are counted on the even CTA's barrier, which expects the bytes of the whole pair
+              if (pair_rank == 0) mbar_expect_tx(&full_bar[stage], 2 * Cfg::STAGE_BYTES);
+              const uint32_t fb = mapa_u32(smem_u32(&full_bar[stage]), 0);
+              if constexpr (!A_MN) {
+                tma_load_4d_pair(sa, &tmapA, fb, k0, a_row, bh, bb);
+              } else {
 #pragma unroll
-              for (int c = 0; c < BM / Cfg::ROW_ELEMS; ++c) tma_load_4d_pair(sa + c * Cfg::BK * 128, &tmapA, fb, a_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
-            }
-            if constexpr (!B_MN) {
-              tma_load_4d_pair(sb, &tmapB, fb, k0, b_row, bh, bb);
-            } else {
+                for (int c = 0; c < BM / Cfg::ROW_ELEMS; ++c) tma_load_4d_pair(sa + c * Cfg::BK * 128, &tmapA, fb, a_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
+              }
+              if constexpr (!B_MN) {
+                tma_load_4d_pair(sb, &tmapB, fb, k0, b_row, bh, bb);
+              } else {
 #pragma unroll
-              for (int c = 0; c < Cfg::BN_CTA / Cfg::ROW_ELEMS; ++c)
-                tma_load_4d_pair(sb + c * Cfg::BK * 128, &tmapB, fb, b_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
-            }
-          } else {
-            mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
-            if constexpr (!A_MN) {
-              tma_load_4d(sa, &tmapA, &full_bar[stage], k0, a_row, bh, bb);
+                for (int c = 0; c < Cfg::BN_CTA / Cfg::ROW_ELEMS; ++c)
+                  tma_load_4d_pair(sb + c * Cfg::BK * 128, &tmapB, fb, b_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
+              }
             } else {
+              mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
+              if constexpr (!A_MN) {
+                tma_load_4d(sa, &tmapA, &full_bar[stage], k0, a_row, bh, bb);
+              } else {
 #pragma unroll
-              for (int c = 0; c < BM / Cfg::ROW_ELEMS; ++c)
-                tma_load_4d(sa + c * Cfg::BK * 128, &tmapA, &full_bar[stage], a_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
-            }
-            if constexpr (!B_MN) {
-              tma_load_4d(sb, &tmapB, &full_bar[stage], k0, b_row, bh, bb);
-            } else {
+                for (int c = 0; c < BM / Cfg::ROW_ELEMS; ++c)
+                  tma_load_4d(sa + c * Cfg::BK * 128, &tmapA, &full_bar[stage], a_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
+              }
+              if constexpr (!B_MN) {
+                tma_load_4d(sb, &tmapB, &full_bar[stage], k0, b_row, bh, bb);
+              } else {
 #pragma unroll
-              for (int c = 0; c < BN / Cfg::ROW_ELEMS; ++c)
-                tma_load_4d(sb + c * Cfg::BK * 128, &tmapB, &full_bar[stage], b_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
+                for (int c = 0; c < BN / Cfg::ROW_ELEMS; ++c)
+                  tma_load_4d(sb + c * Cfg::BK * 128, &tmapB, &full_bar[stage], b_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
+              }
             }
           }
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -309,13 +324,14 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
       // The consumer releases each stage only after using it, so waiting for all
       // stages to be empty again covers every load in flight.
       for (int s = 0; s < STAGES && ok; ++s) {
-        ok = mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && pair_rank == 0) {
+    if (pair_rank == 0) {  // the whole warp runs the loop, one lane issues
+      const bool leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -324,35 +340,41 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
       for (long long item = worker; item < num_items && ok; item += num_workers) {
         const int kb0 = (int)(item / p.num_tiles) * p.kb_per_split;
         const int kb1 = kb0 + p.kb_per_split < num_kb ? kb0 + p.kb_per_split : num_kb;
-        ok = mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+        ok = mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
         if (!ok) break;
         tc_fence_after();
         uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
         for (int kb = kb0; kb < kb1; ++kb) {
-          ok = mbar_wait(&full_bar[stage], phase, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+          ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
           if (!ok) break;
           tc_fence_after();
           uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
           uint32_t sb = sa + Cfg::A_BYTES;
           uint64_t adesc = make_smem_desc(sa, Cfg::A_LBO, Cfg::SBO);
           uint64_t bdesc = make_smem_desc(sb, Cfg::B_LBO, Cfg::SBO);
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < Cfg::BK / Cfg::UMMA_K; ++k) {
-            if constexpr (CTA2)
-              tc_mma_pair_bf16(d_tmem, adesc + (uint64_t)((k * Cfg::A_KADV) >> 4), bdesc + (uint64_t)((k * Cfg::B_KADV) >> 4), Cfg::IDESC,
-                               ((kb - kb0) | k) != 0 ? 1u : 0u);
-            else
-              tc_mma<ES == 4>(d_tmem, adesc + (uint64_t)((k * Cfg::A_KADV) >> 4), bdesc + (uint64_t)((k * Cfg::B_KADV) >> 4),
-                              Cfg::IDESC, ((kb - kb0) | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < Cfg::BK / Cfg::UMMA_K; ++k) {
+              if constexpr (CTA2)
+                tc_mma_pair_bf16(d_tmem, adesc + (uint64_t)((k * Cfg::A_KADV) >> 4), bdesc + (uint64_t)((k * Cfg::B_KADV) >> 4), Cfg::IDESC,
+                                 ((kb - kb0) | k) != 0 ? 1u : 0u);
+              else
+                tc_mma<ES == 4>(d_tmem, adesc + (uint64_t)((k * Cfg::A_KADV) >> 4), bdesc + (uint64_t)((k * Cfg::B_KADV) >> 4),
+                                Cfg::IDESC, ((kb - kb0) | k) != 0 ? 1u : 0u);
+            }
+            // frees the smem stage (in both CTAs of a pair) once these MMAs retire
+            if constexpr (CTA2) tc_commit_pair(&empty_bar[stage]);
+            else tc_commit(&empty_bar[stage]);
           }
-          // frees the smem stage (in both CTAs of a pair) once these MMAs retire
-          if constexpr (CTA2) tc_commit_pair(&empty_bar[stage]);
-          else tc_commit(&empty_bar[stage]);
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        if constexpr (CTA2) tc_commit_pair(&tmem_full[acc]);
-        else tc_commit(&tmem_full[acc]);
+        if (leader) {
+          if constexpr (CTA2) tc_commit_pair(&tmem_full[acc]);
+          else tc_commit(&tmem_full[acc]);
+        }
+        __syncwarp();
         if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       }
     }
