@@ -333,8 +333,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+    {  // the whole warp runs the loop, one lane issues: loop state in uniform registers (see gemm_sm100.cu)
+      const bool leader = elect_one();
+      bool ok = mbar_wait_warp(q_full, 0, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
       // descriptors are built once; an MMA then costs two adds
       const uint64_t dq = make_smem_desc(smem_u32(smem + C::OFF_Q), 16, 1024);
       const uint64_t dk0 = make_smem_desc(smem_u32(smem + C::OFF_K), 16, 1024);
@@ -344,21 +345,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       auto issue_s = [&](int j) -> bool {
         const int t = j % C::NS;
         const uint32_t ph = (uint32_t)(j / C::NS) & 1u;
-        if (!mbar_wait(&k_full[t], ph, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
-        if (!mbar_wait(&s_empty[t], ph ^ 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
+        if (!mbar_wait_warp(&k_full[t], ph, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
+        if (!mbar_wait_warp(&s_empty[t], ph ^ 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
         tc_fence_after();
         const uint64_t dk = desc_advance(dk0, (uint32_t)(t * C::KV_BYTES));
         const uint32_t d_tmem = tmem_base + (uint32_t)(C::TMEM_S + t * 128);
-        {
+        if (leader) {
           tc_mma_bf16<false>(d_tmem, dq, dk, C::IDESC_S);
 #pragma unroll
           for (int ks = 1; ks < D / 16; ++ks) {
             const uint32_t off = (uint32_t)((ks >> 2) * (BQ * 128) + (ks & 3) * 32);   // panel, then 32 bytes per k-step
             tc_mma_bf16<true>(d_tmem, desc_advance(dq, off), desc_advance(dk, off), C::IDESC_S);
           }
+          tc_commit(&s_full[t]);
+          tc_commit(&k_empty[t]);
         }
-        tc_commit(&s_full[t]);
-        tc_commit(&k_empty[t]);
+        __syncwarp();
         attn_trace(p, 20, j);
         return true;
       };
@@ -368,14 +370,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       for (int j = 0; j < n_tiles && ok; ++j) {
         if (j + 2 < n_tiles) { ok = issue_s(j + 2); if (!ok) break; }
         const int vt = j % C::NV;
-        ok = mbar_wait(&v_full[vt], (uint32_t)(j / C::NV) & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA) &&
-             mbar_wait(&p_full[j % C::NS], (uint32_t)(j / C::NS) & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+        ok = mbar_wait_warp(&v_full[vt], (uint32_t)(j / C::NV) & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA) &&
+             mbar_wait_warp(&p_full[j % C::NS], (uint32_t)(j / C::NS) & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
         if (!ok) break;
         attn_trace(p, 21, j);
         tc_fence_after();
         const uint64_t dv = desc_advance(dv0, (uint32_t)(vt * C::KV_BYTES));
         const uint32_t d_tmem = tmem_base + (uint32_t)C::TMEM_O;
-        {
+        if (leader) {
           // O += P V.  A = P (K-major, two panels of 64 keys); B = V (N = head dim contiguous: MN-major, 16 key rows per step)
           // P(j) lies in the first 64 columns of the tensor-memory buffer its scores came from (bf16 pairs, 8 columns per
           // step of 16 keys)
@@ -385,9 +387,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 #pragma unroll
           for (int ks = 1; ks < BKF / 16; ++ks)
             tc_mma_ts_bf16<true>(d_tmem, a_tmem + (uint32_t)(ks * 8), desc_advance(dv, (uint32_t)(ks * 16 * 128)), C::IDESC_PV);
+          tc_commit(&v_empty[vt]);
+          tc_commit(&pv_done[j % C::NS]);
         }
-        tc_commit(&v_empty[vt]);
-        tc_commit(&pv_done[j % C::NS]);
+        __syncwarp();
         attn_trace(p, 22, j);
       }
     }
@@ -1127,8 +1130,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      bool ok = mbar_wait(kv_full, 0, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+    {  // the whole warp runs the loop, one lane issues (see the forward kernel)
+      const bool leader = elect_one();
+      auto all_try = [](uint64_t *bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)); };
+      bool ok = mbar_wait_warp(kv_full, 0, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
       // descriptors are built once; "K-major" = the reduction runs along a row (16 / 1024), "M-major" or "N-major" = the
       // reduction runs down the rows of the two 64-column panels (panel stride / 1024, 2048 bytes per step of 16 rows)
       const uint64_t dK_kmaj = make_smem_desc(smem_u32(smem + C::OFF_K), 16, 1024);
@@ -1147,22 +1152,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       auto issue_s = [&](int it, bool try_only) -> int {      // 1 issued, 0 not yet (try_only), -1 a wait ran out
         const int s = it & 1;
         if (try_only) {
-          if (!mbar_try_wait(&q_full[s], (uint32_t)(it >> 1) & 1u) || !mbar_try_wait(s_empty, ((uint32_t)it & 1u) ^ 1u)) return 0;
+          if (!all_try(&q_full[s], (uint32_t)(it >> 1) & 1u) || !all_try(s_empty, ((uint32_t)it & 1u) ^ 1u)) return 0;
         } else {
-          if (!mbar_wait(&q_full[s], (uint32_t)(it >> 1) & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return -1;
-          if (!mbar_wait(s_empty, ((uint32_t)it & 1u) ^ 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return -1;
+          if (!mbar_wait_warp(&q_full[s], (uint32_t)(it >> 1) & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return -1;
+          if (!mbar_wait_warp(s_empty, ((uint32_t)it & 1u) ^ 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return -1;
         }
         tc_fence_after();
         const uint64_t a = desc_advance(dQ_kmaj0, (uint32_t)(s * C::TILE_BYTES));
         const uint32_t d = tmem_base + (uint32_t)C::TMEM_S;
-        tc_mma_bf16<false>(d, a, dK_kmaj, C::IDESC_SS);
+        if (leader) {
+          tc_mma_bf16<false>(d, a, dK_kmaj, C::IDESC_SS);
 #pragma unroll
-        for (int ks = 1; ks < D / 16; ++ks) tc_mma_bf16<true>(d, desc_advance(a, koff(ks)), desc_advance(dK_kmaj, koff(ks)), C::IDESC_SS);
-        tc_commit(s_full);
+          for (int ks = 1; ks < D / 16; ++ks) tc_mma_bf16<true>(d, desc_advance(a, koff(ks)), desc_advance(dK_kmaj, koff(ks)), C::IDESC_SS);
+          tc_commit(s_full);
+        }
+        __syncwarp();
         attn_trace(p, 23, it);
         return 1;
       };
-      // Waits for `bar` like mbar_wait; while it waits, the next step's S is issued as soon as it can be (pending_s is then
+      // Waits for `bar` like mbar_wait_warp; while it waits, the next step's S is issued as soon as it can be (pending_s is then
       // cleared): the probability warps can work on step it + 1 while the tensor core still runs the products of step it.
       bool pending_s = false;
       int next_it = 0;
@@ -1174,10 +1182,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             const int r = issue_s(next_it, true);
             if (r > 0) pending_s = false;
           }
-          if (mbar_try_wait(bar, parity)) return true;
+          if (all_try(bar, parity)) return true;
           if ((++spins & 63u) == 0) {
-            if (*abort_flag) return false;
-            if (ffk_globaltimer() - t0 > WAIT_LIMIT_NS) {
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) return false;
+            if (__any_sync(0xffffffffu, ffk_globaltimer() - t0 > WAIT_LIMIT_NS)) {
               *abort_flag = 1;
               if (p.err) atomicCAS(p.err, 0, (int)FFK_ERR_TIMEOUT_MMA);
               return false;
@@ -1186,14 +1194,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         }
       };
       auto issue_dp = [&](int it) -> bool {     // dP = dO_it V^T, into the columns the previous step's dQ^T has left
-        if (!mbar_wait(do_full, (uint32_t)it & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
-        if (!mbar_wait(dq_empty, ((uint32_t)it & 1u) ^ 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
+        if (!mbar_wait_warp(do_full, (uint32_t)it & 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
+        if (!mbar_wait_warp(dq_empty, ((uint32_t)it & 1u) ^ 1u, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA)) return false;
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)C::TMEM_DPQ;
-        tc_mma_bf16<false>(d, dDO_kmaj, dV_kmaj, C::IDESC_SS);
+        if (leader) {
+          tc_mma_bf16<false>(d, dDO_kmaj, dV_kmaj, C::IDESC_SS);
 #pragma unroll
-        for (int ks = 1; ks < D / 16; ++ks) tc_mma_bf16<true>(d, desc_advance(dDO_kmaj, koff(ks)), desc_advance(dV_kmaj, koff(ks)), C::IDESC_SS);
-        tc_commit(dp_full);
+          for (int ks = 1; ks < D / 16; ++ks) tc_mma_bf16<true>(d, desc_advance(dDO_kmaj, koff(ks)), desc_advance(dV_kmaj, koff(ks)), C::IDESC_SS);
+          tc_commit(dp_full);
+        }
+        __syncwarp();
         attn_trace(p, 24, it);
         return true;
       };
@@ -1206,22 +1217,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         ok = wait_issuing_s(p_full, ph);
         if (!ok) break;
         tc_fence_after();
-        {
+        if (leader) {
           const uint32_t d = tmem_base + (uint32_t)C::TMEM_DV;
           if (it == 0) tc_mma_bf16<false>(d, dP_mmaj, dDO_nmaj, C::IDESC_T);
           else tc_mma_bf16<true>(d, dP_mmaj, dDO_nmaj, C::IDESC_T);
 #pragma unroll
           for (int ks = 1; ks < BQ / 16; ++ks) tc_mma_bf16<true>(d, desc_advance(dP_mmaj, ks * 2048u), desc_advance(dDO_nmaj, ks * 2048u), C::IDESC_T);
+          tc_commit(p_empty);
+          tc_commit(do_empty);
         }
-        tc_commit(p_empty);
-        tc_commit(do_empty);
+        __syncwarp();
         attn_trace(p, 20, it);
         // dQ_it^T = K^T dS^T (the dS warps have read dP out of these columns before they wrote dS)
         ok = wait_issuing_s(ds_full, ph);
         if (!ok) break;
         attn_trace(p, 21, it);
         tc_fence_after();
-        {
+        if (leader) {
           const uint32_t d = tmem_base + (uint32_t)C::TMEM_DPQ;
           if constexpr (D == 128) {   // transposed: lanes = head-dim index
             tc_mma_bf16<false>(d, dK_mmaj, dDS_kmaj, C::IDESC_DQT);
@@ -1234,23 +1246,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             for (int ks = 1; ks < C::BK / 16; ++ks)
               tc_mma_bf16<true>(d, desc_advance(dDS_kmaj, koff(ks)), desc_advance(dK_mmaj, ks * 2048u), C::IDESC_DQ);
           }
+          tc_commit(dq_full);
         }
-        tc_commit(dq_full);
         // dK += dS^T Q_it
-        {
+        if (leader) {
           const uint32_t d = tmem_base + (uint32_t)C::TMEM_DK;
           const uint64_t bq = desc_advance(dQ_nmaj0, (uint32_t)((it & 1) * C::TILE_BYTES));
           if (it == 0) tc_mma_bf16<false>(d, dDS_mmaj, bq, C::IDESC_T);
           else tc_mma_bf16<true>(d, dDS_mmaj, bq, C::IDESC_T);
 #pragma unroll
           for (int ks = 1; ks < BQ / 16; ++ks) tc_mma_bf16<true>(d, desc_advance(dDS_mmaj, ks * 2048u), desc_advance(bq, ks * 2048u), C::IDESC_T);
+          tc_commit(ds_empty);
+          tc_commit(&q_empty[it & 1]);
         }
-        tc_commit(ds_empty);
-        tc_commit(&q_empty[it & 1]);
+        __syncwarp();
         attn_trace(p, 22, it);
         if (it + 1 < n_it) ok = (!pending_s || issue_s(it + 1, false) > 0) && issue_dp(it + 1);
       }
-      if (ok) tc_commit(dkv_full);
+      if (ok && leader) tc_commit(dkv_full);
     }
   } else if (warp < 10) {
     // ------------------------------------------------------------------ P and dS: thread = query row x 64 of the block's 128 keys
