@@ -62,6 +62,8 @@ struct GemmArgs {
   // items are (tile, split) pairs and every split adds its partial into the fp32 output with atomics.
   int split_k;
   int kb_per_split;
+  int cluster_k;       // cluster kernel: CTAs that share a tile's K range
+  int cluster_stages;  // and stages of its operand ring
   // Dropout fused into the epilogue (after the activation): element (row, col) is kept when the counter-based
   // generator says so for flat index row * ldc + col -- the same function of (seed, index) as the stand-alone
   // dropout kernel, so backward regenerates the mask.  drop_seed_ptr (device memory) holds the per-step seed.
@@ -164,6 +166,68 @@ __device__ __forceinline__ void tile_coords(long long tile, const GemmArgs &p, i
   mb = first_m + (r % gsize);
   nb_ = r / gsize;
   if (p.mb_rotate) mb = (mb + p.mb_rotate) % p.tiles_m;
+}
+
+// Pre-activation copy, activation, dropout, addend, accumulate and store of four neighbouring values of one row: `coff` / `aoff` are
+// their element offsets in C (and C2) / in the addend, `vec4` says that all four columns exist.
+__device__ __forceinline__ void gemm_store4(const GemmArgs &p, void *Cout, float (&v)[4], long long coff, long long aoff, int col, bool vec4) {
+  if (p.C2) {
+    if (!p.aux_fp32 && vec4 && (((uintptr_t)((bf16 *)p.C2 + coff)) & 7) == 0)
+      *reinterpret_cast<uint2 *>((bf16 *)p.C2 + coff) = make_uint2(pack_bf162(v[0], v[1]), pack_bf162(v[2], v[3]));
+    else
+      for (int j = 0; j < 4; ++j) if (col + j < p.N) st_aux(p.C2, coff + j, p.aux_fp32, v[j]);
+  }
+  if (p.act != ACT_NONE) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = act_fwd(v[j], p.act);
+  }
+  if (p.drop_p > 0.f) {
+    const unsigned long long seed = p.drop_seed_ptr ? p.drop_salt * 0x9E3779B97F4A7C15ull + *p.drop_seed_ptr : p.drop_salt;
+    const uint32_t thr = ffk_drop_threshold(p.drop_p);
+    if (vec4 && (coff & 3) == 0) {
+      const uint32_t keep = ffk_keep4(seed, (unsigned long long)(coff >> 2), thr);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = ((keep >> j) & 1u) ? v[j] * p.drop_scale : 0.f;
+    } else {
+      for (int j = 0; j < 4; ++j) v[j] = ffk_keep(seed, (unsigned long long)(coff + j), thr) ? v[j] * p.drop_scale : 0.f;
+    }
+  }
+  if (p.addend) {
+    if (!p.aux_fp32 && vec4 && (((uintptr_t)((const bf16 *)p.addend + aoff)) & 7) == 0) {
+      uint2 u = *reinterpret_cast<const uint2 *>((const bf16 *)p.addend + aoff);
+      float2 a0 = unpack_bf162(u.x), a1 = unpack_bf162(u.y);
+      v[0] += a0.x; v[1] += a0.y; v[2] += a1.x; v[3] += a1.y;
+    } else {
+      for (int j = 0; j < 4; ++j) if (col + j < p.N) v[j] += ld_aux(p.addend, aoff + j, p.aux_fp32);
+    }
+  }
+  if (p.out_fp32) {
+    float *c = (float *)Cout + coff;
+    if (p.split_k > 1) {  // partial sum of one K range: the output was cleared (or holds the accumuland)
+      for (int j = 0; j < 4; ++j) if (col + j < p.N) atomicAdd(c + j, v[j]);
+    } else if (vec4 && (((uintptr_t)c) & 15) == 0) {
+      float4 o = make_float4(v[0], v[1], v[2], v[3]);
+      if (p.accumulate) {
+        float4 old = *reinterpret_cast<float4 *>(c);
+        o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
+      }
+      *reinterpret_cast<float4 *>(c) = o;
+    } else {
+      for (int j = 0; j < 4; ++j) if (col + j < p.N) c[j] = p.accumulate ? c[j] + v[j] : v[j];
+    }
+  } else {
+    bf16 *c = (bf16 *)Cout + coff;
+    if (vec4 && (((uintptr_t)c) & 7) == 0) {
+      if (p.accumulate) {
+        uint2 u = *reinterpret_cast<uint2 *>(c);
+        float2 o0 = unpack_bf162(u.x), o1 = unpack_bf162(u.y);
+        v[0] += o0.x; v[1] += o0.y; v[2] += o1.x; v[3] += o1.y;
+      }
+      *reinterpret_cast<uint2 *>(c) = make_uint2(pack_bf162(v[0], v[1]), pack_bf162(v[2], v[3]));
+    } else {
+      for (int j = 0; j < 4; ++j) if (col + j < p.N) c[j] = f2bf(p.accumulate ? bf2f(c[j]) + v[j] : v[j]);
+    }
+  }
 }
 
 // Output maps of the scatter epilogue: one per owning rank's staging buffer (peer memory).
@@ -597,64 +661,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
             if (row >= p.M || !col_ok) continue;
             float v[4] = {f.x * p.alpha + b4[0], f.y * p.alpha + b4[1], f.z * p.alpha + b4[2], f.w * p.alpha + b4[3]};
             const long long coff = c_base + (long long)row * p.ldc + col;
-            if (p.C2) {
-              if (!p.aux_fp32 && vec4 && (((uintptr_t)((bf16 *)p.C2 + coff)) & 7) == 0)
-                *reinterpret_cast<uint2 *>((bf16 *)p.C2 + coff) = make_uint2(pack_bf162(v[0], v[1]), pack_bf162(v[2], v[3]));
-              else
-                for (int j = 0; j < 4; ++j) if (col + j < p.N) st_aux(p.C2, coff + j, p.aux_fp32, v[j]);
-            }
-            if (p.act != ACT_NONE) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) v[j] = act_fwd(v[j], p.act);
-            }
-            if (p.drop_p > 0.f) {
-              const unsigned long long seed = p.drop_seed_ptr ? p.drop_salt * 0x9E3779B97F4A7C15ull + *p.drop_seed_ptr : p.drop_salt;
-              const uint32_t thr = ffk_drop_threshold(p.drop_p);
-              if (vec4 && (coff & 3) == 0) {
-                const uint32_t keep = ffk_keep4(seed, (unsigned long long)(coff >> 2), thr);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] = ((keep >> j) & 1u) ? v[j] * p.drop_scale : 0.f;
-              } else {
-                for (int j = 0; j < 4; ++j) v[j] = ffk_keep(seed, (unsigned long long)(coff + j), thr) ? v[j] * p.drop_scale : 0.f;
-              }
-            }
-            if (p.addend) {
-              const long long aoff = a_base + (long long)row * p.ld_add + col;
-              if (!p.aux_fp32 && vec4 && (((uintptr_t)((const bf16 *)p.addend + aoff)) & 7) == 0) {
-                uint2 u = *reinterpret_cast<const uint2 *>((const bf16 *)p.addend + aoff);
-                float2 a0 = unpack_bf162(u.x), a1 = unpack_bf162(u.y);
-                v[0] += a0.x; v[1] += a0.y; v[2] += a1.x; v[3] += a1.y;
-              } else {
-                for (int j = 0; j < 4; ++j) if (col + j < p.N) v[j] += ld_aux(p.addend, aoff + j, p.aux_fp32);
-              }
-            }
-            if (p.out_fp32) {
-              float *c = (float *)Cout + coff;
-              if (p.split_k > 1) {  // partial sum of one K range: the output was cleared (or holds the accumuland)
-                for (int j = 0; j < 4; ++j) if (col + j < p.N) atomicAdd(c + j, v[j]);
-              } else if (vec4 && (((uintptr_t)c) & 15) == 0) {
-                float4 o = make_float4(v[0], v[1], v[2], v[3]);
-                if (p.accumulate) {
-                  float4 old = *reinterpret_cast<float4 *>(c);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *reinterpret_cast<float4 *>(c) = o;
-              } else {
-                for (int j = 0; j < 4; ++j) if (col + j < p.N) c[j] = p.accumulate ? c[j] + v[j] : v[j];
-              }
-            } else {
-              bf16 *c = (bf16 *)Cout + coff;
-              if (vec4 && (((uintptr_t)c) & 7) == 0) {
-                if (p.accumulate) {
-                  uint2 u = *reinterpret_cast<uint2 *>(c);
-                  float2 o0 = unpack_bf162(u.x), o1 = unpack_bf162(u.y);
-                  v[0] += o0.x; v[1] += o0.y; v[2] += o1.x; v[3] += o1.y;
-                }
-                *reinterpret_cast<uint2 *>(c) = make_uint2(pack_bf162(v[0], v[1]), pack_bf162(v[2], v[3]));
-              } else {
-                for (int j = 0; j < 4; ++j) if (col + j < p.N) c[j] = f2bf(p.accumulate ? bf2f(c[j]) + v[j] : v[j]);
-              }
-            }
+            gemm_store4(p, Cout, v, coff, a_base + (long long)row * p.ld_add + col, col, vec4);
           }
         }
         __syncwarp();
@@ -691,6 +698,219 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
       *done = 0;
     }
   }
+}
+
+// ----------------------------------------------------------------------------
+// Few output tiles: K split over a thread-block cluster
+// ----------------------------------------------------------------------------
+// A problem with fewer 128 x 128 tiles than SMs leaves most of the chip idle while a handful of SMs stream all of K one stage
+// after another (128 x 512 x 2048: four CTAs, 13.8 us).  Here a tile is 128 x BN and the S CTAs of a cluster share its K
+// range; each leaves its fp32 partial sum in its own shared memory, and after a cluster barrier CTA r adds the S partials
+// of rows [r, r + 1) * 128 / S over distributed shared memory, in a fixed order, and runs the epilogue on them: no workspace, no
+// atomics, no cleared output and one rounding, whatever the output type.  CTAs are not persistent and take at most
+// 96 KB of stages: clusters cannot fill every SM once, so the last ones share SMs with others (36 clusters of 4 with 192 KB each:
+// 27.8 us for 768 x 768 x 8192, with 96 KB 19.2), and the ring is no shorter for it (2048 x 512 x 2048: 11.3 and 11.2 us).
+constexpr int CK_THREADS = 256;
+template <int ES, int BN, bool A_MN, bool B_MN>
+struct ClusterCfg : GemmCfg<ES, BN, A_MN, B_MN> {
+  using Base = GemmCfg<ES, BN, A_MN, B_MN>;
+  static constexpr int MAX_STAGES = BN == 64 ? 4 : 3;             // 96 KB
+  static constexpr int PART_BYTES = BM * BN * 4;                  // the partial tile takes the place of the stages
+  __host__ __device__ static constexpr int region(int stages) {
+    return stages * Base::STAGE_BYTES > PART_BYTES ? stages * Base::STAGE_BYTES : PART_BYTES;
+  }
+  __host__ __device__ static constexpr int smem_bytes(int stages) { return region(stages) + 1024 + 256; }
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 f;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(f.x), "=f"(f.y), "=f"(f.z), "=f"(f.w) : "r"(addr) : "memory");
+  return f;
+}
+
+template <int ES, int BN, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(CK_THREADS, 2)
+gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_constant__ CUtensorMap tmapB, const GemmArgs p) {
+  using Cfg = ClusterCfg<ES, BN, A_MN, B_MN>;
+  const int STAGES = p.cluster_stages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *tiles = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t *full_bar = (uint64_t *)(tiles + Cfg::region(STAGES));  // [STAGES]
+  uint64_t *empty_bar = full_bar + STAGES;                 // [STAGES]
+  uint64_t *acc_full = full_bar + 2 * STAGES;
+  uint32_t *tmem_slot = (uint32_t *)(acc_full + 1);
+  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = p.cluster_k;
+  const int rank = (int)(blockIdx.x % (unsigned)S);
+  const int num_kb = (p.K + Cfg::BK - 1) / Cfg::BK;
+  const int kb0 = (int)((long long)num_kb * rank / S), kb1 = (int)((long long)num_kb * (rank + 1) / S);  // never empty: S <= num_kb
+  int mb, nb_, bh, bb;
+  tile_coords(blockIdx.x / (unsigned)S, p, mb, nb_, bh, bb);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"((uint32_t)BN) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    {  // TMA producer: the whole warp runs the loop, one lane issues
+      const bool leader = elect_one();
+      int stage = 0;
+      uint32_t phase = 0;
+      const int a_row = mb * BM, b_row = nb_ * BN;
+      bool ok = true;
+      int issued = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(&empty_bar[stage], phase ^ 1, abort_flag, p.err, FFK_ERR_TIMEOUT_PRODUCER);
+        if (!ok) break;
+        const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES), sb = sa + Cfg::A_BYTES;
+        const int k0 = kb * Cfg::BK;
+        if (leader) {
+          mbar_expect_tx(&full_bar[stage], Cfg::STAGE_BYTES);
+          if constexpr (!A_MN) {
+            tma_load_4d(sa, &tmapA, &full_bar[stage], k0, a_row, bh, bb);
+          } else {
+#pragma unroll
+            for (int c = 0; c < BM / Cfg::ROW_ELEMS; ++c)
+              tma_load_4d(sa + c * Cfg::BK * 128, &tmapA, &full_bar[stage], a_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
+          }
+          if constexpr (!B_MN) {
+            tma_load_4d(sb, &tmapB, &full_bar[stage], k0, b_row, bh, bb);
+          } else {
+#pragma unroll
+            for (int c = 0; c < BN / Cfg::ROW_ELEMS; ++c)
+              tma_load_4d(sb + c * Cfg::BK * 128, &tmapB, &full_bar[stage], b_row + c * Cfg::ROW_ELEMS, k0, bh, bb);
+          }
+        }
+        __syncwarp();
+        ++issued;
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      // given up: the loads in flight land (or a second limit runs out) before the CTA goes on to its exit
+      for (int s = 0; !ok && s < STAGES && s < issued; ++s) {
+        stage = stage == 0 ? STAGES - 1 : stage - 1;
+        if (stage == STAGES - 1) phase ^= 1;
+        const uint64_t t0 = ffk_globaltimer();
+        while (!mbar_try_wait(&full_bar[stage], phase) && ffk_globaltimer() - t0 < WAIT_LIMIT_NS) {}
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    {  // MMA issuer: the whole warp runs the loop, one lane issues
+      const bool leader = elect_one();
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        ok = mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.err, FFK_ERR_TIMEOUT_MMA);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES), sb = sa + Cfg::A_BYTES;
+        const uint64_t adesc = make_smem_desc(sa, Cfg::A_LBO, Cfg::SBO), bdesc = make_smem_desc(sb, Cfg::B_LBO, Cfg::SBO);
+        if (leader) {
+#pragma unroll
+          for (int k = 0; k < Cfg::BK / Cfg::UMMA_K; ++k)
+            tc_mma<ES == 4>(tmem_base, adesc + (uint64_t)((k * Cfg::A_KADV) >> 4), bdesc + (uint64_t)((k * Cfg::B_KADV) >> 4), Cfg::IDESC,
+                            ((kb - kb0) | k) != 0 ? 1u : 0u);
+          tc_commit(&empty_bar[stage]);
+        }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (ok && leader) tc_commit(acc_full);
+    }
+    __syncwarp();
+  }
+
+  // accumulator -> this CTA's partial tile [128][BN] (fp32, 16-byte units XORed with the row against bank conflicts)
+  bool ok = mbar_wait(acc_full, 0, abort_flag, p.err, FFK_ERR_TIMEOUT_EPILOGUE);
+  ok = __all_sync(0xffffffffu, ok);
+  tc_fence_after();
+  const uint32_t part = smem_u32(tiles);
+  if (ok) {
+    const int q = warp & 3;  // the tensor-memory lanes this warp can read
+    const uint32_t my_row = (uint32_t)(q * 32 + lane);
+#pragma unroll
+    for (int c0 = (warp >> 2) * 32; c0 < BN; c0 += 64) {
+      uint32_t r[32];
+      tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(part + my_row * (BN * 4) + ((((uint32_t)c0 >> 2) + u) ^ (my_row & 7)) * 16),
+                     "r"(r[4 * u]), "r"(r[4 * u + 1]), "r"(r[4 * u + 2]), "r"(r[4 * u + 3])
+                     : "memory");
+    }
+  }
+  tc_fence_before();
+  cluster_sync_all();
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)BN) : "memory");
+  }
+
+  // rows [rank, rank + 1) * 128 / S of the tile: sum over the cluster, epilogue
+  constexpr int UNITS = BN / 4, ROWS_PER_PASS = CK_THREADS / UNITS;
+  const int unit = threadIdx.x % UNITS;
+  const int col = nb_ * BN + unit * 4;
+  if (ok && col < p.N) {
+    const bool vec4 = col + 4 <= p.N;
+    float b4[4] = {0.f, 0.f, 0.f, 0.f};
+    if (p.bias) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (col + j < p.N) b4[j] = ld_aux(p.bias, col + j, p.aux_fp32);
+    }
+    const long long c_base = (long long)bh * p.c_sh + (long long)bb * p.c_sb, a_base = (long long)bh * p.add_sh + (long long)bb * p.add_sb;
+    const bool simple = vec4 && !p.out_fp32 && !p.accumulate && !p.C2 && !p.addend && (p.act == ACT_NONE || p.act == ACT_RELU) &&
+                        p.ldc % 4 == 0 && (((uintptr_t)((bf16 *)p.C + c_base)) & 7) == 0;
+    const float relu_floor = p.act == ACT_RELU ? 0.f : -INFINITY;
+    const int rows = BM / S;
+    // two rows at a time, all partials of both requested before the first is used: a remote read takes a few hundred cycles
+    for (int rl = threadIdx.x / UNITS; rl < rows; rl += 2 * ROWS_PER_PASS) {
+      float4 x[2][8];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int rt = rank * rows + rl + h * ROWS_PER_PASS;
+        const uint32_t addr = part + (uint32_t)rt * (BN * 4) + (uint32_t)((unit ^ (rt & 7)) * 16);
+#pragma unroll
+        for (int s = 0; s < 8; ++s)
+          if (s < S && rl + h * ROWS_PER_PASS < rows) x[h][s] = ld_cluster_f4(mapa_u32(addr, (uint32_t)s));
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int row = mb * BM + rank * rows + rl + h * ROWS_PER_PASS;
+        if (rl + h * ROWS_PER_PASS >= rows || row >= p.M) break;
+        float4 f = x[h][0];
+#pragma unroll
+        for (int s = 1; s < 8; ++s)
+          if (s < S) { f.x += x[h][s].x; f.y += x[h][s].y; f.z += x[h][s].z; f.w += x[h][s].w; }
+        float v[4] = {f.x * p.alpha + b4[0], f.y * p.alpha + b4[1], f.z * p.alpha + b4[2], f.w * p.alpha + b4[3]};
+        const long long coff = c_base + (long long)row * p.ldc + col;
+        if (simple)
+          *reinterpret_cast<uint2 *>((bf16 *)p.C + coff) = make_uint2(pack_bf162(fmaxf(v[0], relu_floor), fmaxf(v[1], relu_floor)),
+                                                                      pack_bf162(fmaxf(v[2], relu_floor), fmaxf(v[3], relu_floor)));
+        else
+          gemm_store4(p, p.C, v, coff, a_base + (long long)row * p.ld_add + col, col, vec4);
+      }
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();  // a CTA's partial tile stays until every CTA of the cluster has read it
 }
 
 // ----------------------------------------------------------------------------
@@ -1032,6 +1252,48 @@ int launch_pair_major(bool a_mn, bool b_mn, const CUtensorMap &ta, const CUtenso
   return launch_pair<256, true, true>(ta, tb, tc, sm, args, max_ctas, stream);
 }
 
+template <int ES, int BN, bool A_MN, bool B_MN>
+int launch_cluster(const CUtensorMap &ta, const CUtensorMap &tb, GemmArgs &args, int split, cudaStream_t stream) {
+  using Cfg = ClusterCfg<ES, BN, A_MN, B_MN>;
+  auto kern = gemm_cluster_kernel<ES, BN, A_MN, B_MN>;
+  static bool attr_done = false;
+  if (!attr_done) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::smem_bytes(Cfg::MAX_STAGES));
+    if (e != cudaSuccess) return (int)e;
+    attr_done = true;
+  }
+  args.tiles_m = (args.M + BM - 1) / BM;
+  args.tiles_n = (args.N + BN - 1) / BN;
+  args.num_tiles = (long long)args.tiles_m * args.tiles_n * args.nh * args.nb;
+  args.split_k = 1;
+  args.cluster_k = split;
+  const int kb_per = ((args.K + Cfg::BK - 1) / Cfg::BK + split - 1) / split;
+  args.cluster_stages = kb_per < Cfg::MAX_STAGES ? kb_per : Cfg::MAX_STAGES;
+  args.tma_store = 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(args.num_tiles * split));
+  cfg.blockDim = dim3(CK_THREADS);
+  cfg.dynamicSmemBytes = Cfg::smem_bytes(args.cluster_stages);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, args);
+}
+template <int BN>
+int launch_cluster_major(int es, bool a_mn, bool b_mn, const CUtensorMap &ta, const CUtensorMap &tb, GemmArgs &args, int split,
+                         cudaStream_t stream) {
+  if (es == 4) return launch_cluster<4, BN, false, false>(ta, tb, args, split, stream);
+  if (!a_mn && !b_mn) return launch_cluster<2, BN, false, false>(ta, tb, args, split, stream);
+  if (!a_mn && b_mn) return launch_cluster<2, BN, false, true>(ta, tb, args, split, stream);
+  if (a_mn && !b_mn) return launch_cluster<2, BN, true, false>(ta, tb, args, split, stream);
+  return launch_cluster<2, BN, true, true>(ta, tb, args, split, stream);
+}
+
 int sm_count() {
   static int n = 0;
   if (!n) {
@@ -1088,9 +1350,67 @@ struct FfkGemmDesc {
   float drop_p;
   unsigned long long drop_salt;
   const void *drop_seed_ptr;
+  // cluster kernel: CTAs that share a tile's K range (2, 4 or 8; with bn 64 or 128); 0 = choose, -1 = persistent kernel
+  int split;
 };
 
 static int g_pair_mode = 1;  // 1: CTA pairs where they apply, 0: never
+// Tile width and kernel of a plain problem, by estimated time in us.  The constants are fits to runs of both kernels on 55 shapes
+// (M 37 to 8192, N 64 to 5272, K 64 to 8192, all operand orders): a launch with prologue and epilogue, then per k-block and
+// wave what one CTA takes, more where the CTAs together reach what L2 delivers (about 20 TB/s to six
+// stages per CTA, 15 to the cluster kernel's three or four).  Examples, persistent / cluster:
+// 128 x 512 x 2048 12.3 / 6.7 us (64 wide, 8 CTAs per tile), 512 x 512 x 4096 both MN-major 22.7 / 10.9, 2048 x 512 x 4096
+// 19.8 / 15.1, 2304 x 768 x 8192 34.4 / 32.5 (left to the persistent kernel: the estimate does not see it),
+// 2048 x 2048 x 8000 63.1 at 128 columns, 50.4 at 256.
+static void gemm_plan(const FfkGemmDesc *d, long long nbatch, int *bn, int *split) {
+  const int es = d->es, sms = sm_count();
+  const int num_kb = (int)(((long long)d->K * es + 127) / 128);
+  const long long tm = (d->M + BM - 1) / BM;
+  auto tiles = [&](int w) { return tm * ((d->N + w - 1) / w) * nbatch; };
+  auto l2_us = [](long long ctas, int w, float tbs) { return (float)ctas * (128.f + (float)w) * 128.f / (tbs * 1e6f); };  // a k-block of all
+  float best = 1e30f;
+  const bool plain32 = d->out_fp32 && !d->C2 && !d->addend && d->act == ACT_NONE && nbatch == 1 && d->alpha == 1.f;
+  for (int w = 64; w <= (es == 4 ? 128 : 256); w *= 2) {
+    if (w > 64 && d->N <= w / 2) break;
+    const long long t = tiles(w);
+    float us;
+    if (w == 256 && g_pair_mode && d->M >= 256 && (long long)((d->M + 255) / 256) * ((d->N + 255) / 256) * nbatch >= sms / 2) {
+      const long long pt = (long long)((d->M + 255) / 256) * ((d->N + 255) / 256) * nbatch;
+      const float waves = (float)((pt + sms / 2 - 1) / (sms / 2));
+      us = 6.7f + waves * (float)num_kb * 0.32f + 1.2f * (waves - 1.f);
+    } else {
+      const float waves = (float)((t + sms - 1) / sms);
+      const long long ctas = t < sms ? t : sms;
+      const float rate = w == 256 ? 0.3f : 0.22f, l2 = l2_us(ctas, w, 20.f);
+      us = (w == 64 ? 4.3f : w == 128 ? 5.4f : 6.7f) + waves * (float)num_kb * (l2 > rate ? l2 : rate) + 0.8f * (waves - 1.f);
+      if (plain32 && w <= 128 && t * 2 <= sms && num_kb >= 16) {  // split over all SMs with atomics onto a cleared output
+        const float sk = 10.f + (float)num_kb * (float)t / (float)sms * 0.3f;
+        if (sk < us) us = sk;
+      }
+    }
+    if (us < best) {
+      best = us;
+      *bn = w;
+      *split = -1;
+    }
+  }
+  for (int w = 64; w <= 128; w *= 2) {
+    if (w > 64 && d->N <= w / 2) break;
+    for (int sp = 2; sp <= 8; sp *= 2) {
+      const long long ctas = tiles(w) * sp;
+      if (sp > num_kb || ctas > sms - 4) break;
+      const float l2 = l2_us(ctas, w, 15.f);
+      float us = (w == 64 ? 5.8f : 6.9f) + (float)((num_kb + sp - 1) / sp) * (l2 > 0.22f ? l2 : 0.22f);
+      if (sp == 8 && ctas > 96) us += 1.5f;  // more clusters of 8 than the GPCs place at once
+      if (us < best - 0.2f) {
+        best = us;
+        *bn = w;
+        *split = sp;
+      }
+    }
+  }
+}
+
 // CTA-pair (tcgen05 cta_group::2) kernel on (1) or off (0) process-wide; for A/B measurements.
 FFK_API void ffk_gemm_set_cta_pairs(int enabled) { g_pair_mode = enabled ? 1 : 0; }
 static int g_disable_tma_store = 0;
@@ -1159,7 +1479,10 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
     else gemm_simt_kernel<float><<<grid, block, SIMT_SMEM_BYTES, stream>>>(o, a);
     return (int)cudaGetLastError();
   }
-  int bn = d->bn;
+  int bn = d->bn, split = d->split;
+  if (split == 0 && bn == 0 && !fused && d->max_ctas <= 0) gemm_plan(d, nbatch, &bn, &split);
+  if (split > 0 && (fused || (bn != 64 && bn != 128) || (split != 2 && split != 4 && split != 8) || split > (d->K + 128 / es - 1) / (128 / es)))
+    return -2;
   if (bn == 0) {
     // Prefer the widest tile that still gives every SM work.
     long long t256 = (long long)((d->M + 127) / 128) * ((d->N + 255) / 256) * d->nh * d->nb;
@@ -1171,7 +1494,7 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
   // A CTA pair per 256 x 256 tile when the problem has at least one such tile per pair of SMs and none of the fused-collective
   // or split-K machinery is involved (those stay on the single-CTA kernel).
   bool pair = false;
-  if (g_pair_mode && es == 2 && bn == 256 && !fused && d->M >= 256) {
+  if (g_pair_mode && split <= 0 && es == 2 && bn == 256 && !fused && d->M >= 256) {
     const long long t = (long long)((d->M + 255) / 256) * ((d->N + 255) / 256) * nbatch;
     pair = t >= sm_count() / 2;
   }
@@ -1210,6 +1533,9 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
   cudaGetSymbolAddress(&errp, g_gemm_err);
   a.err = (int *)errp;
   int max_ctas = d->max_ctas > 0 ? d->max_ctas : sm_count();
+  if (split > 0)
+    return bn == 64 ? launch_cluster_major<64>(es, d->a_mn, d->b_mn, ta, tb, a, split, stream)
+                    : launch_cluster_major<128>(es, d->a_mn, d->b_mn, ta, tb, a, split, stream);
   // TMA-store epilogue for the plain bf16 case (bias + ReLU/none) when the output can be described by a tensor map
   CUtensorMap tc = ta;
   a.tma_store = 0;

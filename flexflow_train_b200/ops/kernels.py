@@ -60,6 +60,7 @@ class GemmDesc(ctypes.Structure):
         ("push_flag", c_void_p * 8), ("push_sync", c_void_p), ("push_world", c_int), ("push_rank", c_int),
         # dropout applied by the epilogue after the activation
         ("drop_p", c_float), ("drop_salt", c_ulonglong), ("drop_seed_ptr", c_void_p),
+        ("split", c_int),
     ]
 
 
@@ -241,12 +242,13 @@ def gemm_raw(*, M, N, K, A, lda, B, ldb, C, ldc, a_mn=False, b_mn=False, es=2, n
              a_sh=0, a_sb=0, b_sh=0, b_sb=0, c_sh=0, c_sb=0, C2=None, bias=None, addend=None,
              ld_add=0, add_sh=0, add_sb=0, alpha=1.0, act=0, out_fp32=False, accumulate=False,
              bn=0, max_ctas=0, scatter=None, scatter_rows=0, scatter_src=0, gate_flags=None, gate_sync=None,
-             gate_rows=0, mb_rotate=0, push=None, dropout=None):
+             gate_rows=0, mb_rotate=0, push=None, dropout=None, split=0):
     """D = epilogue(alpha * A[M,K] . B[N,K]^T) on raw pointers; see gemm_sm100.cu.
 
     scatter / scatter_rows / scatter_src: write each output tile into the owning rank's staging buffer
     (GEMM -> reduce-scatter).  gate_flags / gate_sync / gate_rows / mb_rotate: wait for pushed row blocks of A
-    (all-gather -> GEMM)."""
+    (all-gather -> GEMM).  bn / split: tile width and, for the cluster kernel, the CTAs that share a tile's K range (0: chosen by
+    size, split -1: the persistent kernel)."""
     plain = not scatter and gate_flags is None and push is None and dropout is None
     # (batches of small problems have a kernel of their own that reads any layout: same condition as in ffk_gemm)
     small_batched = max(nh, 1) * max(nb, 1) >= 32 and M * N <= 1024 and (M + N) * (K + 1) <= 2304
@@ -264,6 +266,7 @@ def gemm_raw(*, M, N, K, A, lda, B, ldb, C, ldc, a_mn=False, b_mn=False, es=2, n
                  C, ldc, c_sh, c_sb, C2, bias, addend, ld_add, add_sh, add_sb, alpha, act, int(out_fp32),
                  int(accumulate), bn, max_ctas, sc, scatter_rows, scatter_src, gate_flags, gate_sync, gate_rows,
                  mb_rotate)
+    d.split = split
     if dropout is not None:  # (p, salt, seed tensor or None)
         d.drop_p, d.drop_salt = float(dropout[0]), int(dropout[1]) & (2**64 - 1)
         d.drop_seed_ptr = None if dropout[2] is None else dropout[2].data_ptr()

@@ -270,9 +270,7 @@ class LinearOp(OpImpl):
         rows, cols = self.x2d.shape[0], self.w.shape[0]
         self.pre = torch.empty(rows, cols, dtype=x.dtype, device=x.device) if (self.act == "gelu" and self.ex.cfg.training) else None
         self.ex.need_scratch(4 * K.bias_act_bwd_scratch(rows, cols) if K.available() and self.ex.on_gpu else 0)
-        # A small layer under a large batch: the weight gradient has a handful of output tiles and a reduction over
-        # thousands of rows.  Computed into an fp32 scratch, the GEMM splits that reduction over all SMs (one CTA
-        # streaming 4096 rows takes ~25 us; 148 CTAs sharing them a few); a cast then adds it into the bf16 gradient.
+        # weight gradient by way of an fp32 scratch (see wgrad_splits)
         if self.ex.cfg.training and self.ex.wgrad_splits(rows, cols, self.w.shape[1], x.dtype):
             self.ex.need_scratch(4 * cols * self.w.shape[1])
 
@@ -1151,12 +1149,14 @@ class Executable:
         return self._big[slot][:n].view(like.dtype).view(like.shape)
 
     # A small layer under a large batch: its weight gradient has a handful of output tiles and a reduction over
-    # thousands of rows, so a direct GEMM keeps a few CTAs streaming all rows while the other SMs idle.  Computed into
-    # an fp32 scratch instead, the GEMM splits the reduction over all SMs; a cast then adds it into the bf16 gradient.
+    # thousands of rows, so one CTA per tile would stream all rows while the other SMs idle.  Up to 16384 rows the GEMM shares
+    # a tile's reduction among the 8 CTAs of a cluster (64 x 256 x 4096: 7.5 us; scratch, its clearing and the cast 16).  Beyond that
+    # 8 CTAs per tile are too few: computed into an fp32 scratch, the GEMM splits the reduction over all SMs, and a cast
+    # adds it into the bf16 gradient.
     @staticmethod
     def wgrad_splits(rows: int, n_out: int, k_in: int, dtype) -> bool:
         tiles = ((n_out + 127) // 128) * ((k_in + 127) // 128)
-        return dtype == torch.bfloat16 and tiles * 2 <= 148 and rows >= 1024
+        return dtype == torch.bfloat16 and tiles * 2 <= 148 and rows > 16384
 
     def wgrad_gemm(self, dy: torch.Tensor, x: torch.Tensor, out: torch.Tensor, accumulate: bool):
         """out[n_out, k_in] (+)= dy[rows, n_out]^T . x[rows, k_in]"""
