@@ -290,6 +290,26 @@ __global__ void cast_f32_bf16_kernel(const float *__restrict__ s, bf16 *__restri
   for (long long i = nv * 8 + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) d[i] = f2bf(s[i]);
 }
 
+// bf16 -> fp32 (written or added): the projections of fp32 attention around its bf16 core.  Through the general cast, which goes by
+// way of double one element at a time, 4096 x 2048 took 30 us.
+__global__ void cast_bf16_f32_kernel(const bf16 *__restrict__ s, float *__restrict__ d, long long n, int accumulate) {
+  const long long nv = n / 8, stride = (long long)gridDim.x * blockDim.x, t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  for (long long i = t0; i < nv; i += stride) {
+    const uint4 u = *reinterpret_cast<const uint4 *>(s + i * 8);
+    const float2 a = unpack_bf162(u.x), b = unpack_bf162(u.y), c = unpack_bf162(u.z), e = unpack_bf162(u.w);
+    float4 lo = make_float4(a.x, a.y, b.x, b.y), hi = make_float4(c.x, c.y, e.x, e.y);
+    float4 *p = reinterpret_cast<float4 *>(d + i * 8);
+    if (accumulate) {
+      const float4 x = p[0], y = p[1];
+      lo.x += x.x; lo.y += x.y; lo.z += x.z; lo.w += x.w;
+      hi.x += y.x; hi.y += y.y; hi.z += y.z; hi.w += y.w;
+    }
+    p[0] = lo;
+    p[1] = hi;
+  }
+  for (long long i = nv * 8 + t0; i < n; i += stride) d[i] = bf2f(s[i]) + (accumulate ? d[i] : 0.f);
+}
+
 // dz = dy * act'(saved) ; per-column partial sums of dz go to `partial`
 // ([gridDim.y, cols] floats) for the bias gradient.  One block handles a
 // 32-column strip over a slab of rows.
@@ -384,13 +404,16 @@ FFK_API int ffk_cast(const void *src, int sdt, void *dst, int ddt, long long n, 
   if (n <= 0) return 0;
   if (sdt == DT_F32 && ddt == DT_BF16 && !accumulate && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0)
     cast_f32_bf16_kernel<<<ffk_blocks(n / 8 + 1, 256), 256, 0, st>>>((const float *)src, (bf16 *)dst, n);
+  else if (sdt == DT_BF16 && ddt == DT_F32 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0)
+    cast_bf16_f32_kernel<<<ffk_blocks(n / 8 + 1, 256), 256, 0, st>>>((const bf16 *)src, (float *)dst, n, accumulate);
   else
     cast_kernel<<<ffk_blocks(n, 256), 256, 0, st>>>(src, sdt, dst, ddt, n, accumulate);
   return (int)cudaGetLastError();
 }
 // Number of float slots `partial` must hold for ffk_bias_act_bwd.
-// Row chunks of the column reduction: at least 64 rows each, and enough chunks that a narrow matrix (768 columns =
-// three column blocks) still fills the GPU.
+// Row chunks of the column reduction: 64 rows each and enough chunks that a narrow matrix (768 columns = three column blocks)
+// still fills the GPU; fewer rows, down to one per thread, where 64 would leave fewer than two blocks per SM (64 x 1024: 4 blocks,
+// 7.5 us of one load after another).
 static int bias_act_row_chunks(int rows, int cols) {
   const int col_blocks = (cols + 255) / 256;
   int cap = (148 * 4 + col_blocks - 1) / col_blocks;
@@ -398,6 +421,8 @@ static int bias_act_row_chunks(int rows, int cols) {
   int gy = rows / 64;
   if (gy < 1) gy = 1;
   if (gy > cap) gy = cap;
+  const int fill = (148 * 2 + col_blocks - 1) / col_blocks, most = (rows + 7) / 8;
+  if (gy < fill) gy = fill < most ? fill : most;
   return gy;
 }
 FFK_API long long ffk_bias_act_bwd_scratch(int rows, int cols) { return (long long)bias_act_row_chunks(rows, cols) * cols; }

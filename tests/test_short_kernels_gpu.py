@@ -1,0 +1,80 @@
+"""Copies, casts and thin products at the sizes where their vectors, tiles and index splits end."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from flexflow_train_b200.ops import kernels as K  # noqa: E402
+
+
+def _randn(*shape, dtype=torch.bfloat16, seed=0):
+    return torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda").to(dtype)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 4099, 1 << 20])
+@pytest.mark.parametrize("accumulate", [False, True])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_cast_up(n, accumulate, offset):
+    s = _randn(n + offset)[offset:]
+    d = _randn(n + offset, dtype=torch.float32, seed=1)[offset:]
+    want = s.float() + d if accumulate else s.float()
+    K.cast(s, d, accumulate=accumulate)
+    assert torch.equal(d, want)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (7, 1024), (64, 1024), (65, 264), (300, 256), (2048, 512), (64, 10), (4096, 1)])
+def test_bias_gradient_of_few_rows(rows, cols):
+    dy, y = _randn(rows, cols), _randn(rows, cols, seed=1)
+    dz, db = torch.empty_like(dy), torch.empty(cols, device="cuda").bfloat16()
+    scratch = torch.empty(K.bias_act_bwd_scratch(rows, cols), device="cuda")
+    K.bias_act_bwd(dy, y, dz, db, scratch, "relu")
+    want = dy * (y > 0)
+    assert torch.equal(dz, want)
+    ref = want.double().sum(0)
+    # fp32 sums of `rows` terms, one bf16 rounding
+    assert ((db.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + want.double().abs().sum(0) * rows * 2.0 ** -24 + 1e-7).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.int64])
+@pytest.mark.parametrize("outer,block,src_ld,dst_ld,offset", [(1, 1, 1, 1, 0), (64, 5270, 5270, 5272, 0), (9, 13, 13, 16, 1), (257, 6, 9, 8, 2),
+                                                              (5000, 942, 1000, 944, 3)])
+def test_block_copy(dtype, outer, block, src_ld, dst_ld, offset):
+    src = (torch.rand(outer * src_ld + offset, device="cuda") * 200).to(dtype)
+    dst = torch.zeros(outer * dst_ld + offset, device="cuda", dtype=dtype)
+    want = dst.clone()
+    want[offset:].view(outer, dst_ld)[:, :block] = src[offset:].view(outer, src_ld)[:, :block]
+    K.block_copy(src, offset, src_ld, dst, offset, dst_ld, outer, block)
+    assert torch.equal(dst, want)
+
+
+@pytest.mark.parametrize("shape,perm", [((4096, 9, 64), (0, 2, 1)), ((3, 5, 7, 11), (3, 1, 0, 2)), ((1, 1), (1, 0)), ((2, 3, 2, 3, 2, 3), (5, 3, 1, 4, 2, 0)),
+                                        ((70000,), (0,))])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32, torch.int64])
+def test_permute(shape, perm, dtype):
+    x = (_randn(*shape, dtype=torch.float32) * 100).to(dtype)
+    assert torch.equal(K.permute(x, perm), x.permute(perm).contiguous())
+    if dtype != torch.int64:
+        out = torch.ones_like(x.permute(perm).contiguous())
+        K.permute(x, perm, out=out, accumulate=True)
+        assert torch.equal(out, 1 + x.permute(perm))
+
+
+@pytest.mark.parametrize("M,N,Kd", [(1, 1, 1), (64, 512, 10), (10, 512, 64), (17, 65, 33), (33, 7, 128), (100, 30, 129), (64, 2048, 3)])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float32])
+def test_thin_products(M, N, Kd, dt):
+    """Row pitches that TMA cannot address; K on both sides of the thin kernel's limit, with epilogue and batches."""
+    a, b = _randn(2, M, Kd, dtype=dt), _randn(2, N, Kd, dtype=dt, seed=1)
+    bias, old = _randn(N, dtype=dt, seed=2), _randn(2, M, N, dtype=dt, seed=3)
+    ref = a.double() @ b.double().transpose(1, 2)
+    tol = lambda w: Kd * 2.0 ** -20 + w.abs() * (2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -20) + 1e-6  # noqa: E731  fp32 sums, one rounding
+    for a_mn in (False, True):
+        for b_mn in (False, True):
+            x, w = (a.transpose(1, 2).contiguous() if a_mn else a), (b.transpose(1, 2).contiguous() if b_mn else b)
+            if a.element_size() * x.shape[2] % 16 == 0 and b.element_size() * w.shape[2] % 16 == 0 and Kd > 8:
+                continue  # both addressable: the tensor cores' case
+            C = old.clone()
+            K.gemm_raw(M=M, N=N, K=Kd, A=x.data_ptr(), lda=x.shape[2], a_sb=M * Kd, a_mn=a_mn, B=w.data_ptr(), ldb=w.shape[2], b_sb=N * Kd,
+                       b_mn=b_mn, C=C.data_ptr(), ldc=N, c_sb=M * N, nb=2, es=a.element_size(), out_fp32=dt == torch.float32,
+                       bias=bias.data_ptr(), act=K.ACT_CODES["relu"], accumulate=True)
+            want = torch.relu(ref + bias.double()) + old.double()
+            assert ((C.double() - want).abs() <= tol(want)).all(), (a_mn, b_mn, (C.double() - want).abs().max().item())
