@@ -251,6 +251,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t *tmem_slot = (uint32_t *)(bars + 25);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   if ((uintptr_t)(smem - smem_raw) > (uintptr_t)C::SLACK) {  // the launch did not leave room to align the tiles: refuse
+    pdl_entry();
     if (threadIdx.x == 0 && p.err) atomicCAS(p.err, 0, (int)FFK_ERR_BAD_ARG);
     return;
   }
@@ -284,6 +285,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_entry();  // the set-up above ran under the previous kernel's tail
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -602,6 +604,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint32_t *tmem_slot = (uint32_t *)(bars + 17);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   if ((uintptr_t)(smem - smem_raw) > (uintptr_t)C::SLACK) {
+    pdl_entry();
     if (threadIdx.x == 0 && p.err) atomicCAS(p.err, 0, (int)FFK_ERR_BAD_ARG);
     return;
   }
@@ -639,6 +642,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_entry();  // the set-up above ran under the previous kernel's tail
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -940,6 +944,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 template <int D>
 __global__ void attn_delta_kernel(const bf16 *__restrict__ dO, long long lddo, const bf16 *__restrict__ O, long long ldo,
                                   float *__restrict__ delta, int B, int H, int Sq) {
+  pdl_entry();
   const int lane = threadIdx.x & 31;
   const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const long long total = (long long)B * Sq * H;
@@ -968,6 +973,7 @@ __global__ void attn_delta_kernel(const bf16 *__restrict__ dO, long long lddo, c
 // fp32 accumulators [B, H, Sk, D] -> bf16 [B*Sk, ld] (head h at columns h*D)
 template <int D>
 __global__ void attn_acc_to_bf16_kernel(const float *__restrict__ acc, bf16 *__restrict__ out, long long ld, int B, int H, int Sk) {
+  pdl_entry();
   const long long total = (long long)B * H * Sk * (D / 4);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int c4 = (int)(i % (D / 4));
@@ -1048,6 +1054,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   uint32_t *tmem_slot = (uint32_t *)(bars + 17);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   if ((uintptr_t)(smem - smem_raw) > (uintptr_t)C::SLACK) {  // the launch did not leave room to align the tiles: refuse
+    pdl_entry();
     if (threadIdx.x == 0 && p.err) atomicCAS(p.err, 0, (int)FFK_ERR_BAD_ARG);
     return;
   }
@@ -1080,6 +1087,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_entry();  // the set-up above ran under the previous kernel's tail
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -1505,7 +1513,7 @@ int launch_fwd2(const CUtensorMap &tq, const CUtensorMap &tk, const CUtensorMap 
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  attn_fwd2_kernel<D, P_TMEM><<<(unsigned)grid, FWD2_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, a);
+  ffk_launch(attn_fwd2_kernel<D, P_TMEM>, (unsigned)grid, FWD2_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, a);
   return (int)cudaGetLastError();
 }
 
@@ -1555,7 +1563,7 @@ static int launch_fwd1(const CUtensorMap &tq, const CUtensorMap &tk, const CUten
     if (e != cudaSuccess) return (int)e;
     attr = true;
   }
-  attn_fwd_kernel<D, DROP><<<(unsigned)grid, ATT_THREADS, FwdCfg<D>::SMEM_BYTES, stream>>>(tq, tk, tv, a);
+  ffk_launch(attn_fwd_kernel<D, DROP>, (unsigned)grid, ATT_THREADS, FwdCfg<D>::SMEM_BYTES, stream, tq, tk, tv, a);
   return (int)cudaGetLastError();
 }
 
@@ -1610,7 +1618,7 @@ static int launch_bwd(const FfkAttnDesc *d, AttnArgs &a, cudaStream_t stream) {
   if (e != cudaSuccess) return (int)e;
   {
     const long long warps = (long long)d->B * d->Sq * d->H;
-    attn_delta_kernel<D><<<(unsigned)((warps + 7) / 8), 256, 0, stream>>>((const bf16 *)d->dO, d->lddo, (const bf16 *)d->O, d->ldo,
+    ffk_launch(attn_delta_kernel<D>, (unsigned)((warps + 7) / 8), 256, 0, stream, (const bf16 *)d->dO, d->lddo, (const bf16 *)d->O, d->ldo,
                                                                            (float *)d->delta, d->B, d->H, d->Sq);
   }
   static bool attr = false;
@@ -1621,8 +1629,8 @@ static int launch_bwd(const FfkAttnDesc *d, AttnArgs &a, cudaStream_t stream) {
   }
   const long long grid = (long long)((d->Sk + C::BK - 1) / C::BK) * d->H * d->B;
   if (grid > 0x7fffffffll) return -2;
-  attn_bwd_kernel<D><<<(unsigned)grid, BWD_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, tdo, a);
-  attn_acc_to_bf16_kernel<D><<<ffk_blocks(n_acc / 4, 256), 256, 0, stream>>>(a.dQ_acc, (bf16 *)d->dQ, d->lddq, d->B, d->H, d->Sq);
+  ffk_launch(attn_bwd_kernel<D>, (unsigned)grid, BWD_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, tdo, a);
+  ffk_launch(attn_acc_to_bf16_kernel<D>, ffk_blocks(n_acc / 4, 256), 256, 0, stream, a.dQ_acc, (bf16 *)d->dQ, d->lddq, d->B, d->H, d->Sq);
   return (int)cudaGetLastError();
 }
 

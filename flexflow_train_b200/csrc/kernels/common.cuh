@@ -38,6 +38,31 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
 
+// Programmatic dependent launch.  Kernels are launched while their predecessor in the stream still runs and wait for it here,
+// before their first access to global memory; then they let their own successor be launched.  A step of short kernels spends as
+// much time between kernels as in them: launch, block scheduling and, in the tensor-core kernels (which call this after
+// their set-up), barrier initialisation and tensor-memory allocation now run under the previous kernel's tail.  Every block waits,
+// also one without work: a kernel that ended before its predecessor would release its successor too early.
+__device__ __forceinline__ void pdl_entry() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename T> struct FfkSame { typedef T type; };
+template <typename... P>
+static inline int ffk_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, typename FfkSame<P>::type... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 __device__ __forceinline__ float bf2f(bf16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ bf16 f2bf(float v) { return __float2bfloat16_rn(v); }
 

@@ -61,6 +61,7 @@ __device__ __forceinline__ void split3(long long t, const FastDiv &f_c8, const F
 // ------------------------------------------------------------------------------------------- im2col
 // vector path: bf16 channels-last, C % 8 == 0; one thread moves 8 channels (16 bytes)
 __global__ void im2col_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ col, ConvGeom g, long long total) {
+  pdl_entry();
   const int c8n = g.C >> 3, kk_n = g.KH * g.KW;
   const bool small = total < (1ll << 31);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -96,6 +97,7 @@ __global__ void im2col_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__
 // generic path: any strides / dtype; one thread per (row, k) including the zero padding columns
 template <typename T>
 __global__ void im2col_kernel(const T *__restrict__ x, bf16 *__restrict__ col, ConvGeom g, long long total) {
+  pdl_entry();
   const int K = g.KH * g.KW * g.C;
   const bool small = total < (1ll << 31);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -138,6 +140,7 @@ __global__ void im2col_kernel(const T *__restrict__ x, bf16 *__restrict__ col, C
 // dx[n, ih, iw, c] (+)= sum over (kh, kw) with (ih + PH - kh) % SH == 0 ... of dcol[(n, oh, ow), (kh, kw, c)]
 template <typename T>
 __global__ void col2im_kernel(const bf16 *__restrict__ dcol, T *__restrict__ dx, ConvGeom g, long long total, int accumulate) {
+  pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % g.C);
     long long r = t / g.C;
@@ -167,6 +170,7 @@ __global__ void col2im_kernel(const bf16 *__restrict__ dcol, T *__restrict__ dx,
 }
 // vector form: bf16 channels-last output, C % 8 == 0
 __global__ void col2im_vec_kernel(const bf16 *__restrict__ dcol, bf16 *__restrict__ dx, ConvGeom g, long long total, int accumulate) {
+  pdl_entry();
   const int c8n = g.C >> 3;
   const bool small = total < (1ll << 31);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -210,6 +214,7 @@ __global__ void col2im_vec_kernel(const bf16 *__restrict__ dcol, bf16 *__restric
 // w [OC, C, KH, KW] -> wp [OC, Kp] with k = (kh*KW + kw)*C + c (zero padding columns)
 template <typename T>
 __global__ void filter_pack_kernel(const T *__restrict__ w, bf16 *__restrict__ wp, int OC, int C, int KH, int KW, int Kp) {
+  pdl_entry();
   long long total = (long long)OC * Kp;
   int K = C * KH * KW;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -227,6 +232,7 @@ __global__ void filter_pack_kernel(const T *__restrict__ w, bf16 *__restrict__ w
 template <typename T>
 __global__ void filter_unpack_kernel(const float *__restrict__ dwp, T *__restrict__ dw, int OC, int C, int KH, int KW, int Kp,
                                      int accumulate) {
+  pdl_entry();
   long long total = (long long)OC * C * KH * KW;
   int KK = KH * KW;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -246,6 +252,7 @@ __global__ void filter_unpack_kernel(const float *__restrict__ dwp, T *__restric
 template <typename T>
 __global__ void pool_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, unsigned char *__restrict__ arg, ConvGeom g, int mode,
                                 long long total) {
+  pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % g.C);
     long long r = t / g.C;
@@ -280,6 +287,7 @@ __global__ void pool_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, unsi
 template <typename T>
 __global__ void pool_bwd_kernel(const T *__restrict__ dy, const unsigned char *__restrict__ arg, T *__restrict__ dx, ConvGeom g, int mode,
                                 long long total, int accumulate) {
+  pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % g.C);
     long long r = t / g.C;
@@ -323,6 +331,7 @@ template <typename T>
 __global__ void bn_partial_kernel(const T *__restrict__ a, const T *__restrict__ b, const T *__restrict__ relu_y, float *__restrict__ part,
                                   const float *__restrict__ mean, const float *__restrict__ rstd, long long R, int C, int rows_per_chunk,
                                   int mode) {
+  pdl_entry();
   // mode 0: sums of a and a*a (forward statistics)
   // mode 1: sums of dy and dy * xhat with a = dy, b = x (backward); dy is masked where relu_y <= 0
   __shared__ float s0[BN_TY][BN_TX + 1], s1[BN_TY][BN_TX + 1];
@@ -374,6 +383,7 @@ __device__ __forceinline__ void bn_fold(const float *__restrict__ part, int chun
 }
 __global__ void bn_finalize_stats_kernel(const float *__restrict__ part, int chunks, int C, long long R, float eps, float *__restrict__ mean,
                                          float *__restrict__ rstd) {
+  pdl_entry();
   int c = blockIdx.x * 32 + threadIdx.x;
   float s, q;
   bn_fold(part, chunks, C, c, s, q);
@@ -388,6 +398,7 @@ __global__ void bn_finalize_stats_kernel(const float *__restrict__ part, int chu
 template <typename T>
 __global__ void bn_finalize_grads_kernel(const float *__restrict__ part, int chunks, int C, float *__restrict__ sums, T *__restrict__ dgamma,
                                          T *__restrict__ dbeta, int acc_gamma, int acc_beta) {
+  pdl_entry();
   int c = blockIdx.x * 32 + threadIdx.x;
   float s, q;
   bn_fold(part, chunks, C, c, s, q);
@@ -400,6 +411,7 @@ __global__ void bn_finalize_grads_kernel(const float *__restrict__ part, int chu
 template <typename T>
 __global__ void bn_apply_kernel(const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ gamma, const T *__restrict__ beta,
                                 const float *__restrict__ mean, const float *__restrict__ rstd, long long total, int C, int relu) {
+  pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % C);
     float v = (ldf(x + t) - mean[c]) * rstd[c];
@@ -413,6 +425,7 @@ __global__ void bn_apply_kernel(const T *__restrict__ x, T *__restrict__ y, cons
 __global__ void bn_apply_bf16x2_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, const bf16 *__restrict__ gamma,
                                        const bf16 *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd,
                                        long long pairs, int C, int relu) {
+  pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < pairs; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)((t * 2) % C);
     float2 v = unpack_bf162(reinterpret_cast<const uint32_t *>(x)[t]);
@@ -429,6 +442,7 @@ template <typename T>
 __global__ void bn_bwd_apply_kernel(const T *__restrict__ dy, const T *__restrict__ x, const T *__restrict__ relu_y, const T *__restrict__ gamma,
                                     const float *__restrict__ mean, const float *__restrict__ rstd, const float *__restrict__ sums,
                                     T *__restrict__ dx, long long total, int C, float inv_r, int accumulate) {
+  pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % C);
     float g = ldf(dy + t);
@@ -455,6 +469,7 @@ __device__ __forceinline__ uint4 pack8(const float *f) {
 
 __global__ void pool_fwd_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, unsigned char *__restrict__ arg, ConvGeom g, int mode,
                                     long long total) {
+  pdl_entry();
   const int c8n = g.C >> 3;
   const bool small = total < (1ll << 31);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -500,6 +515,7 @@ __global__ void pool_fwd_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict
 
 __global__ void pool_bwd_vec_kernel(const bf16 *__restrict__ dy, const unsigned char *__restrict__ arg, bf16 *__restrict__ dx, ConvGeom g,
                                     int mode, long long total, int accumulate) {
+  pdl_entry();
   const int c8n = g.C >> 3;
   const bool small = total < (1ll << 31);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -574,6 +590,7 @@ bn_partial_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, co
                       const bf16 *__restrict__ gamma, const bf16 *__restrict__ beta,
                       float *__restrict__ part, const float *__restrict__ mean, const float *__restrict__ rstd, long long R, int C,
                       int rows_per_chunk) {
+  pdl_entry();
   extern __shared__ float sred[];  // [lanes][2][C]
   const int groups = C >> 3;
   const int lanes = BNV_THREADS / groups;
@@ -640,6 +657,7 @@ bn_partial_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, co
 __global__ void __launch_bounds__(256) bn_apply_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, const bf16 *__restrict__ gamma,
                                                            const bf16 *__restrict__ beta, const float *__restrict__ mean,
                                                            const float *__restrict__ rstd, long long total8, int C, int relu) {
+  pdl_entry();
   const int groups = C >> 3;
   const long long usable = ((long long)gridDim.x * blockDim.x / groups) * groups;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -670,6 +688,7 @@ __global__ void __launch_bounds__(256)
 bn_bwd_apply_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ relu_y, const bf16 *__restrict__ gamma,
                         const bf16 *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd,
                         const float *__restrict__ sums, bf16 *__restrict__ dx, long long total8, int C, float inv_r, int accumulate) {
+  pdl_entry();
   const int groups = C >> 3;
   const long long usable = ((long long)gridDim.x * blockDim.x / groups) * groups;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -752,11 +771,11 @@ FFK_API int ffk_im2col(const void *x, void *col, const int *geom, const long lon
   if (g.Kp < K || (g.Kp % 8) != 0) return -2;
   if (dt == 1 && vec_ok(g, x) && g.Kp == K) {
     long long total = rows * g.KH * g.KW * (g.C / 8);
-    im2col_vec_kernel<<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)col, g, total);
+    ffk_launch(im2col_vec_kernel, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)x, (bf16 *)col, g, total);
   } else {
     long long total = rows * g.Kp;
-    if (dt == 1) im2col_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)col, g, total);
-    else if (dt == 0) im2col_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>((const float *)x, (bf16 *)col, g, total);
+    if (dt == 1) ffk_launch(im2col_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)x, (bf16 *)col, g, total);
+    else if (dt == 0) ffk_launch(im2col_kernel<float>, ffk_blocks(total, 256), 256, 0, st, (const float *)x, (bf16 *)col, g, total);
     else return -2;
   }
   return (int)cudaGetLastError();
@@ -768,11 +787,11 @@ FFK_API int ffk_col2im(const void *dcol, void *dx, const int *geom, const long l
   if (total <= 0) return 0;
   if (dt == 1 && vec_ok(g, dx)) {
     long long tv = total / 8;
-    col2im_vec_kernel<<<ffk_blocks(tv, 256), 256, 0, st>>>((const bf16 *)dcol, (bf16 *)dx, g, tv, accumulate);
+    ffk_launch(col2im_vec_kernel, ffk_blocks(tv, 256), 256, 0, st, (const bf16 *)dcol, (bf16 *)dx, g, tv, accumulate);
   } else if (dt == 1) {
-    col2im_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)dcol, (bf16 *)dx, g, total, accumulate);
+    ffk_launch(col2im_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)dcol, (bf16 *)dx, g, total, accumulate);
   } else if (dt == 0) {
-    col2im_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)dcol, (float *)dx, g, total, accumulate);
+    ffk_launch(col2im_kernel<float>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)dcol, (float *)dx, g, total, accumulate);
   } else {
     return -2;
   }
@@ -782,8 +801,8 @@ FFK_API int ffk_col2im(const void *dcol, void *dx, const int *geom, const long l
 FFK_API int ffk_filter_pack(const void *w, void *wp, int OC, int C, int KH, int KW, int Kp, int dt, cudaStream_t st) {
   long long total = (long long)OC * Kp;
   if (total <= 0) return 0;
-  if (dt == 1) filter_pack_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)w, (bf16 *)wp, OC, C, KH, KW, Kp);
-  else if (dt == 0) filter_pack_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>((const float *)w, (bf16 *)wp, OC, C, KH, KW, Kp);
+  if (dt == 1) ffk_launch(filter_pack_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)w, (bf16 *)wp, OC, C, KH, KW, Kp);
+  else if (dt == 0) ffk_launch(filter_pack_kernel<float>, ffk_blocks(total, 256), 256, 0, st, (const float *)w, (bf16 *)wp, OC, C, KH, KW, Kp);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -791,8 +810,8 @@ FFK_API int ffk_filter_pack(const void *w, void *wp, int OC, int C, int KH, int 
 FFK_API int ffk_filter_unpack(const float *dwp, void *dw, int OC, int C, int KH, int KW, int Kp, int dt, int accumulate, cudaStream_t st) {
   long long total = (long long)OC * C * KH * KW;
   if (total <= 0) return 0;
-  if (dt == 1) filter_unpack_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>(dwp, (bf16 *)dw, OC, C, KH, KW, Kp, accumulate);
-  else if (dt == 0) filter_unpack_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>(dwp, (float *)dw, OC, C, KH, KW, Kp, accumulate);
+  if (dt == 1) ffk_launch(filter_unpack_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, dwp, (bf16 *)dw, OC, C, KH, KW, Kp, accumulate);
+  else if (dt == 0) ffk_launch(filter_unpack_kernel<float>, ffk_blocks(total, 256), 256, 0, st, dwp, (float *)dw, OC, C, KH, KW, Kp, accumulate);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -805,11 +824,11 @@ FFK_API int ffk_pool2d_fwd(const void *x, void *y, void *arg, const int *geom, c
   if (g.KH * g.KW > 255) return -2;
   if (dt == 1 && vec_ok(g, x) && ((uintptr_t)y % 16) == 0 && ((uintptr_t)arg % 8) == 0) {
     long long tv = total / 8;
-    pool_fwd_vec_kernel<<<ffk_blocks(tv, 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (unsigned char *)arg, g, mode, tv);
+    ffk_launch(pool_fwd_vec_kernel, ffk_blocks(tv, 256), 256, 0, st, (const bf16 *)x, (bf16 *)y, (unsigned char *)arg, g, mode, tv);
     return (int)cudaGetLastError();
   }
-  if (dt == 1) pool_fwd_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (unsigned char *)arg, g, mode, total);
-  else if (dt == 0) pool_fwd_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>((const float *)x, (float *)y, (unsigned char *)arg, g, mode, total);
+  if (dt == 1) ffk_launch(pool_fwd_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)x, (bf16 *)y, (unsigned char *)arg, g, mode, total);
+  else if (dt == 0) ffk_launch(pool_fwd_kernel<float>, ffk_blocks(total, 256), 256, 0, st, (const float *)x, (float *)y, (unsigned char *)arg, g, mode, total);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -822,12 +841,12 @@ FFK_API int ffk_pool2d_bwd(const void *dy, const void *arg, void *dx, const int 
   if (mode == 0 && !arg) return -2;
   if (dt == 1 && vec_ok(g, dx) && ((uintptr_t)dy % 16) == 0 && ((uintptr_t)arg % 8) == 0) {
     long long tv = total / 8;
-    pool_bwd_vec_kernel<<<ffk_blocks(tv, 256), 256, 0, st>>>((const bf16 *)dy, (const unsigned char *)arg, (bf16 *)dx, g, mode, tv,
+    ffk_launch(pool_bwd_vec_kernel, ffk_blocks(tv, 256), 256, 0, st, (const bf16 *)dy, (const unsigned char *)arg, (bf16 *)dx, g, mode, tv,
                                                              accumulate);
     return (int)cudaGetLastError();
   }
-  if (dt == 1) pool_bwd_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)dy, (const unsigned char *)arg, (bf16 *)dx, g, mode, total, accumulate);
-  else if (dt == 0) pool_bwd_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>((const float *)dy, (const unsigned char *)arg, (float *)dx, g, mode, total, accumulate);
+  if (dt == 1) ffk_launch(pool_bwd_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)dy, (const unsigned char *)arg, (bf16 *)dx, g, mode, total, accumulate);
+  else if (dt == 0) ffk_launch(pool_bwd_kernel<float>, ffk_blocks(total, 256), 256, 0, st, (const float *)dy, (const unsigned char *)arg, (float *)dx, g, mode, total, accumulate);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -879,26 +898,26 @@ FFK_API int ffk_batchnorm_fwd(const void *x, void *y, const void *gamma, const v
     int rv;
     int cv = bn_chunks_vec(R, C, &rv);
     const int lanes = BNV_THREADS / (C / 8);
-    bn_partial_vec_kernel<0, BN_NO_RELU><<<cv, BNV_THREADS, (size_t)lanes * 2 * C * sizeof(float), st>>>(
+    ffk_launch(bn_partial_vec_kernel<0, BN_NO_RELU>, cv, BNV_THREADS, (size_t)lanes * 2 * C * sizeof(float), st, 
         (const bf16 *)x, nullptr, nullptr, nullptr, nullptr, scratch, nullptr, nullptr, R, C, rv);
-    bn_finalize_stats_kernel<<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, cv, C, R, eps, mean, rstd);
-    bn_apply_vec_kernel<<<ffk_blocks(total / 8, 512), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta, mean,
+    ffk_launch(bn_finalize_stats_kernel, (C + 31) / 32, dim3(32, BN_FOLD), 0, st, scratch, cv, C, R, eps, mean, rstd);
+    ffk_launch(bn_apply_vec_kernel, ffk_blocks(total / 8, 512), 256, 0, st, (const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta, mean,
                                                                     rstd, total / 8, C, relu);
     return (int)cudaGetLastError();
   }
   if (dt == 1) {
-    bn_partial_kernel<bf16><<<grid, block, 0, st>>>((const bf16 *)x, nullptr, nullptr, scratch, nullptr, nullptr, R, C, rpc, 0);
-    bn_finalize_stats_kernel<<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, chunks, C, R, eps, mean, rstd);
+    ffk_launch(bn_partial_kernel<bf16>, grid, block, 0, st, (const bf16 *)x, nullptr, nullptr, scratch, nullptr, nullptr, R, C, rpc, 0);
+    ffk_launch(bn_finalize_stats_kernel, (C + 31) / 32, dim3(32, BN_FOLD), 0, st, scratch, chunks, C, R, eps, mean, rstd);
     if ((C % 2) == 0 && ((uintptr_t)x % 4) == 0 && ((uintptr_t)y % 4) == 0)
-      bn_apply_bf16x2_kernel<<<ffk_blocks(total / 2, 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta,
+      ffk_launch(bn_apply_bf16x2_kernel, ffk_blocks(total / 2, 256), 256, 0, st, (const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta,
                                                                          mean, rstd, total / 2, C, relu);
     else
-      bn_apply_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta, mean,
+      ffk_launch(bn_apply_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)x, (bf16 *)y, (const bf16 *)gamma, (const bf16 *)beta, mean,
                                                                     rstd, total, C, relu);
   } else if (dt == 0) {
-    bn_partial_kernel<float><<<grid, block, 0, st>>>((const float *)x, nullptr, nullptr, scratch, nullptr, nullptr, R, C, rpc, 0);
-    bn_finalize_stats_kernel<<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, chunks, C, R, eps, mean, rstd);
-    bn_apply_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>((const float *)x, (float *)y, (const float *)gamma, (const float *)beta,
+    ffk_launch(bn_partial_kernel<float>, grid, block, 0, st, (const float *)x, nullptr, nullptr, scratch, nullptr, nullptr, R, C, rpc, 0);
+    ffk_launch(bn_finalize_stats_kernel, (C + 31) / 32, dim3(32, BN_FOLD), 0, st, scratch, chunks, C, R, eps, mean, rstd);
+    ffk_launch(bn_apply_kernel<float>, ffk_blocks(total, 256), 256, 0, st, (const float *)x, (float *)y, (const float *)gamma, (const float *)beta,
                                                                    mean, rstd, total, C, relu);
   } else {
     return -2;
@@ -927,15 +946,15 @@ FFK_API int ffk_batchnorm_bwd(const void *dy, const void *x, const void *relu_y,
     const int ag = ffk_blocks(total / 8, 512);
     const int mask = !relu_y ? BN_NO_RELU : mask_from_x ? BN_RELU_X : BN_RELU_Y;
 #define BN_PART(M)                                                                                                                     \
-  bn_partial_vec_kernel<1, M><<<cv, BNV_THREADS, psm, st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, (const bf16 *)gamma, \
+  ffk_launch(bn_partial_vec_kernel<1, M>, cv, BNV_THREADS, psm, st, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, (const bf16 *)gamma, \
                                                             (const bf16 *)beta, scratch, mean, rstd, R, C, rv)
 #define BN_APPLY(M)                                                                                                                   \
-  bn_bwd_apply_vec_kernel<M><<<ag, 256, 0, st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, (const bf16 *)gamma,          \
+  ffk_launch(bn_bwd_apply_vec_kernel<M>, ag, 256, 0, st, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, (const bf16 *)gamma,          \
                                                  (const bf16 *)beta, mean, rstd, sums_v, (bf16 *)dx, total / 8, C, inv_r, accumulate_dx)
     if (mask == BN_RELU_X) BN_PART(BN_RELU_X);
     else if (mask == BN_RELU_Y) BN_PART(BN_RELU_Y);
     else BN_PART(BN_NO_RELU);
-    bn_finalize_grads_kernel<bf16><<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, cv, C, sums_v, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_gamma,
+    ffk_launch(bn_finalize_grads_kernel<bf16>, (C + 31) / 32, dim3(32, BN_FOLD), 0, st, scratch, cv, C, sums_v, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_gamma,
                                                                      accumulate_beta);
     if (dx && mask == BN_RELU_X) BN_APPLY(BN_RELU_X);
     else if (dx && mask == BN_RELU_Y) BN_APPLY(BN_RELU_Y);
@@ -945,19 +964,19 @@ FFK_API int ffk_batchnorm_bwd(const void *dy, const void *x, const void *relu_y,
     return (int)cudaGetLastError();
   }
   if (dt == 1) {
-    bn_partial_kernel<bf16><<<grid, block, 0, st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, scratch, mean, rstd, R, C, rpc, 1);
-    bn_finalize_grads_kernel<bf16><<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, chunks, C, sums, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_gamma,
+    ffk_launch(bn_partial_kernel<bf16>, grid, block, 0, st, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y, scratch, mean, rstd, R, C, rpc, 1);
+    ffk_launch(bn_finalize_grads_kernel<bf16>, (C + 31) / 32, dim3(32, BN_FOLD), 0, st, scratch, chunks, C, sums, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_gamma,
                                                                      accumulate_beta);
     if (dx)
-      bn_bwd_apply_kernel<bf16><<<ffk_blocks(total, 256), 256, 0, st>>>((const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y,
+      ffk_launch(bn_bwd_apply_kernel<bf16>, ffk_blocks(total, 256), 256, 0, st, (const bf16 *)dy, (const bf16 *)x, (const bf16 *)relu_y,
                                                                         (const bf16 *)gamma, mean, rstd, sums, (bf16 *)dx, total, C, inv_r,
                                                                         accumulate_dx);
   } else if (dt == 0) {
-    bn_partial_kernel<float><<<grid, block, 0, st>>>((const float *)dy, (const float *)x, (const float *)relu_y, scratch, mean, rstd, R, C, rpc, 1);
-    bn_finalize_grads_kernel<float><<<(C + 31) / 32, dim3(32, BN_FOLD), 0, st>>>(scratch, chunks, C, sums, (float *)dgamma, (float *)dbeta,
+    ffk_launch(bn_partial_kernel<float>, grid, block, 0, st, (const float *)dy, (const float *)x, (const float *)relu_y, scratch, mean, rstd, R, C, rpc, 1);
+    ffk_launch(bn_finalize_grads_kernel<float>, (C + 31) / 32, dim3(32, BN_FOLD), 0, st, scratch, chunks, C, sums, (float *)dgamma, (float *)dbeta,
                                                                       accumulate_gamma, accumulate_beta);
     if (dx)
-      bn_bwd_apply_kernel<float><<<ffk_blocks(total, 256), 256, 0, st>>>((const float *)dy, (const float *)x, (const float *)relu_y,
+      ffk_launch(bn_bwd_apply_kernel<float>, ffk_blocks(total, 256), 256, 0, st, (const float *)dy, (const float *)x, (const float *)relu_y,
                                                                          (const float *)gamma, mean, rstd, sums, (float *)dx, total, C, inv_r,
                                                                          accumulate_dx);
   } else {

@@ -151,6 +151,7 @@ conv_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_entry();  // the set-up above ran under the previous kernel's tail
   const uint32_t box_bytes = (uint32_t)p.rows * 128u;   // one 64-channel box of the pixel tile
 
   if (warp == 0) {
@@ -411,7 +412,7 @@ int launch_conv(const CUtensorMap &ta, const CUtensorMap &tb, const ConvArgs &a,
     attr = true;
   }
   const long long grid = a.num_items < conv_sm_count() ? a.num_items : conv_sm_count();
-  conv_sm100_kernel<BN, MODE><<<(unsigned)grid, CONV_THREADS, Cfg::SMEM_BYTES, st>>>(ta, tb, a);
+  ffk_launch(conv_sm100_kernel<BN, MODE>, (unsigned)grid, CONV_THREADS, Cfg::SMEM_BYTES, st, ta, tb, a);
   return (int)cudaGetLastError();
 }
 

@@ -9,6 +9,7 @@ namespace {
 // dst[i, :] = src[idx[i], :] for rows of `vec_per_row` 16-byte vectors; idx == nullptr: rows first .. first + n - 1
 __global__ void load_rows_vec_kernel(const uint4 *__restrict__ src, const long long *__restrict__ idx, uint4 *__restrict__ dst, long long n,
                                      long long vec_per_row, long long first, long long num_samples) {
+  pdl_entry();
   const long long total = n * vec_per_row;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const long long i = t / vec_per_row, v = t - i * vec_per_row;
@@ -19,6 +20,7 @@ __global__ void load_rows_vec_kernel(const uint4 *__restrict__ src, const long l
 }
 __global__ void load_rows_byte_kernel(const unsigned char *__restrict__ src, const long long *__restrict__ idx, unsigned char *__restrict__ dst,
                                       long long n, long long row_bytes, long long first, long long num_samples) {
+  pdl_entry();
   const long long total = n * row_bytes;
   for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     const long long i = t / row_bytes, v = t - i * row_bytes;
@@ -39,11 +41,11 @@ FFK_API int ffk_load_rows(const void *src, const void *idx, void *dst, long long
   const bool vec = row_bytes % 16 == 0 && (((uintptr_t)src) & 15) == 0 && (((uintptr_t)dst) & 15) == 0;
   if (vec) {
     const long long total = n * (row_bytes / 16);
-    load_rows_vec_kernel<<<ffk_blocks(total, 256), 256, 0, st>>>((const uint4 *)src, (const long long *)idx, (uint4 *)dst, n, row_bytes / 16, first,
+    ffk_launch(load_rows_vec_kernel, ffk_blocks(total, 256), 256, 0, st, (const uint4 *)src, (const long long *)idx, (uint4 *)dst, n, row_bytes / 16, first,
                                                                  num_samples);
   } else {
     const long long total = n * row_bytes;
-    load_rows_byte_kernel<<<ffk_blocks(total, 256), 256, 0, st>>>((const unsigned char *)src, (const long long *)idx, (unsigned char *)dst, n,
+    ffk_launch(load_rows_byte_kernel, ffk_blocks(total, 256), 256, 0, st, (const unsigned char *)src, (const long long *)idx, (unsigned char *)dst, n,
                                                                   row_bytes, first, num_samples);
   }
   return (int)cudaGetLastError();

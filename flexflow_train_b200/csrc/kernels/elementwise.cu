@@ -98,6 +98,7 @@ template <> struct V16<bf16> {
 
 template <typename T>
 __global__ void unary_fwd_kernel(int op, const T *__restrict__ x, T *__restrict__ y, long long n, float s) {
+  pdl_entry();
   constexpr int N = V16<T>::N;
   long long nv = n / N;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -115,6 +116,7 @@ __global__ void unary_fwd_kernel(int op, const T *__restrict__ x, T *__restrict_
 template <typename T>
 __global__ void unary_bwd_kernel(int op, const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ dy,
                                  T *__restrict__ dx, long long n, float s, int accumulate) {
+  pdl_entry();
   constexpr int N = V16<T>::N;
   long long nv = n / N;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -153,6 +155,7 @@ __device__ __forceinline__ float binary_apply(int op, float a, float b) {
 template <typename T>
 __global__ void binary_fwd_kernel(int op, const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ y,
                                   long long n, long long bn) {
+  pdl_entry();
   constexpr int N = V16<T>::N;
   long long stride = (long long)gridDim.x * blockDim.x;
   if (bn == n) {
@@ -177,6 +180,7 @@ __global__ void binary_fwd_kernel(int op, const T *__restrict__ a, const T *__re
 template <typename T>
 __global__ void binary_bwd_kernel(int op, const T *__restrict__ a, const T *__restrict__ b, const T *__restrict__ dy,
                                   T *da, T *db, long long n, int accumulate) {
+  pdl_entry();
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     float g = V16<T>::ld1(dy + i);
@@ -199,6 +203,7 @@ __global__ void binary_bwd_kernel(int op, const T *__restrict__ a, const T *__re
 template <typename T>
 __global__ void dropout_kernel(const T *__restrict__ x, const T *__restrict__ r, T *__restrict__ y, long long n,
                                float p, float scale, unsigned long long seed, const unsigned long long *seed_ptr) {
+  pdl_entry();
   // seed_ptr (optional) points at a per-step seed in device memory, so a captured CUDA graph draws a new
   // mask on every replay; `seed` then acts as the per-operator salt.
   if (seed_ptr) seed = seed * 0x9E3779B97F4A7C15ull + *seed_ptr;
@@ -226,6 +231,7 @@ __global__ void dropout_kernel(const T *__restrict__ x, const T *__restrict__ r,
 
 template <typename T>
 __global__ void axpby_kernel(const T *__restrict__ x, T *__restrict__ y, long long n, float a, float b) {
+  pdl_entry();
   constexpr int N = V16<T>::N;
   long long nv = n / N;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -243,6 +249,7 @@ __global__ void axpby_kernel(const T *__restrict__ x, T *__restrict__ y, long lo
 
 template <typename T>
 __global__ void fill_kernel(T *y, long long n, float v) {
+  pdl_entry();
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) V16<T>::st1(y + i, v);
 }
@@ -272,6 +279,7 @@ __device__ __forceinline__ void store_any(void *p, long long i, int dt, double v
 }
 // dst = cast(src)  (accumulate: dst += cast(src), the backward of a cast)
 __global__ void cast_kernel(const void *src, int sdt, void *dst, int ddt, long long n, int accumulate) {
+  pdl_entry();
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     double v = load_any(src, i, sdt);
@@ -281,6 +289,7 @@ __global__ void cast_kernel(const void *src, int sdt, void *dst, int ddt, long l
 }
 // fast paths for the two casts on the training hot path
 __global__ void cast_f32_bf16_kernel(const float *__restrict__ s, bf16 *__restrict__ d, long long n) {
+  pdl_entry();
   long long nv = n / 8, stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride) {
     float4 a = *reinterpret_cast<const float4 *>(s + i * 8), b = *reinterpret_cast<const float4 *>(s + i * 8 + 4);
@@ -293,6 +302,7 @@ __global__ void cast_f32_bf16_kernel(const float *__restrict__ s, bf16 *__restri
 // bf16 -> fp32 (written or added): the projections of fp32 attention around its bf16 core.  Through the general cast, which goes by
 // way of double one element at a time, 4096 x 2048 took 30 us.
 __global__ void cast_bf16_f32_kernel(const bf16 *__restrict__ s, float *__restrict__ d, long long n, int accumulate) {
+  pdl_entry();
   const long long nv = n / 8, stride = (long long)gridDim.x * blockDim.x, t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = t0; i < nv; i += stride) {
     const uint4 u = *reinterpret_cast<const uint4 *>(s + i * 8);
@@ -316,6 +326,7 @@ __global__ void cast_bf16_f32_kernel(const bf16 *__restrict__ s, float *__restri
 template <typename T>
 __global__ void bias_act_bwd_kernel(const T *__restrict__ dy, const T *__restrict__ saved, T *__restrict__ dz,
                                     float *__restrict__ partial, int rows, int cols, int act) {
+  pdl_entry();
   __shared__ float red[8][33];
   int col = blockIdx.x * 32 + threadIdx.x;  // blockDim = (32, 8)
   float acc = 0.f;
@@ -339,6 +350,7 @@ __global__ void bias_act_bwd_kernel(const T *__restrict__ dy, const T *__restric
 }
 template <typename T>
 __global__ void colsum_finish_kernel(const float *__restrict__ partial, int nparts, int cols, T *out, int accumulate) {
+  pdl_entry();
   int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= cols) return;
   float s = 0.f;
@@ -355,27 +367,27 @@ __global__ void colsum_finish_kernel(const float *__restrict__ partial, int npar
 
 FFK_API int ffk_unary_fwd(int op, const void *x, void *y, long long n, float s, int dt, cudaStream_t st) {
   if (n <= 0) return 0;
-  DISPATCH_FLOAT(dt, (unary_fwd_kernel<T><<<ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st>>>(op, (const T *)x, (T *)y, n, s)));
+  DISPATCH_FLOAT(dt, (ffk_launch(unary_fwd_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, op, (const T *)x, (T *)y, n, s)));
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_unary_bwd(int op, const void *x, const void *y, const void *dy, void *dx, long long n, float s, int dt,
                           int accumulate, cudaStream_t st) {
   if (n <= 0) return 0;
-  DISPATCH_FLOAT(dt, (unary_bwd_kernel<T><<<ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st>>>(
+  DISPATCH_FLOAT(dt, (ffk_launch(unary_bwd_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, 
                          op, (const T *)x, (const T *)y, (const T *)dy, (T *)dx, n, s, accumulate)));
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_binary_fwd(int op, const void *a, const void *b, void *y, long long n, long long bn, int dt,
                            cudaStream_t st) {
   if (n <= 0) return 0;
-  DISPATCH_FLOAT(dt, (binary_fwd_kernel<T><<<ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st>>>(
+  DISPATCH_FLOAT(dt, (ffk_launch(binary_fwd_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, 
                          op, (const T *)a, (const T *)b, (T *)y, n, bn)));
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_binary_bwd(int op, const void *a, const void *b, const void *dy, void *da, void *db, long long n,
                            int dt, int accumulate, cudaStream_t st) {
   if (n <= 0) return 0;
-  DISPATCH_FLOAT(dt, (binary_bwd_kernel<T><<<ffk_blocks(n, 256), 256, 0, st>>>(op, (const T *)a, (const T *)b,
+  DISPATCH_FLOAT(dt, (ffk_launch(binary_bwd_kernel<T>, ffk_blocks(n, 256), 256, 0, st, op, (const T *)a, (const T *)b,
                                                                                 (const T *)dy, (T *)da, (T *)db, n,
                                                                                 accumulate)));
   return (int)cudaGetLastError();
@@ -385,29 +397,29 @@ FFK_API int ffk_dropout(const void *x, const void *r, void *y, long long n, floa
                         const unsigned long long *seed_ptr, int dt, cudaStream_t st) {
   if (n <= 0) return 0;
   float scale = p < 1.f ? 1.f / (1.f - p) : 0.f;
-  DISPATCH_FLOAT(dt, (dropout_kernel<T><<<ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st>>>(
+  DISPATCH_FLOAT(dt, (ffk_launch(dropout_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, 
                          (const T *)x, (const T *)r, (T *)y, n, p, scale, seed, seed_ptr)));
   return (int)cudaGetLastError();
 }
 // y = a*x + b*y
 FFK_API int ffk_axpby(const void *x, void *y, long long n, float a, float b, int dt, cudaStream_t st) {
   if (n <= 0) return 0;
-  DISPATCH_FLOAT(dt, (axpby_kernel<T><<<ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st>>>((const T *)x, (T *)y, n, a, b)));
+  DISPATCH_FLOAT(dt, (ffk_launch(axpby_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, (const T *)x, (T *)y, n, a, b)));
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_fill(void *y, long long n, float v, int dt, cudaStream_t st) {
   if (n <= 0) return 0;
-  DISPATCH_FLOAT(dt, (fill_kernel<T><<<ffk_blocks(n, 256), 256, 0, st>>>((T *)y, n, v)));
+  DISPATCH_FLOAT(dt, (ffk_launch(fill_kernel<T>, ffk_blocks(n, 256), 256, 0, st, (T *)y, n, v)));
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_cast(const void *src, int sdt, void *dst, int ddt, long long n, int accumulate, cudaStream_t st) {
   if (n <= 0) return 0;
   if (sdt == DT_F32 && ddt == DT_BF16 && !accumulate && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0)
-    cast_f32_bf16_kernel<<<ffk_blocks(n / 8 + 1, 256), 256, 0, st>>>((const float *)src, (bf16 *)dst, n);
+    ffk_launch(cast_f32_bf16_kernel, ffk_blocks(n / 8 + 1, 256), 256, 0, st, (const float *)src, (bf16 *)dst, n);
   else if (sdt == DT_BF16 && ddt == DT_F32 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0)
-    cast_bf16_f32_kernel<<<ffk_blocks(n / 8 + 1, 256), 256, 0, st>>>((const bf16 *)src, (float *)dst, n, accumulate);
+    ffk_launch(cast_bf16_f32_kernel, ffk_blocks(n / 8 + 1, 256), 256, 0, st, (const bf16 *)src, (float *)dst, n, accumulate);
   else
-    cast_kernel<<<ffk_blocks(n, 256), 256, 0, st>>>(src, sdt, dst, ddt, n, accumulate);
+    ffk_launch(cast_kernel, ffk_blocks(n, 256), 256, 0, st, src, sdt, dst, ddt, n, accumulate);
   return (int)cudaGetLastError();
 }
 // Number of float slots `partial` must hold for ffk_bias_act_bwd.
@@ -434,17 +446,17 @@ static int bias_act_bwd_impl(const void *dy, const void *saved, void *dz, void *
   const int gy = bias_act_row_chunks(rows, cols);
   if (dt == DT_BF16 && cols % 8 == 0 && (((uintptr_t)dy | (uintptr_t)saved | (uintptr_t)dz) & 15) == 0) {
     dim3 vgrid((cols + 255) / 256, gy), vblock(32, 8);
-    vec::bias_act_bwd_vec_kernel<<<vgrid, vblock, 0, st>>>((const bf16 *)dy, (const bf16 *)saved, (bf16 *)dz, dbias ? partial : nullptr, rows,
+    ffk_launch(vec::bias_act_bwd_vec_kernel, vgrid, vblock, 0, st, (const bf16 *)dy, (const bf16 *)saved, (bf16 *)dz, dbias ? partial : nullptr, rows,
                                                           cols, act, drop_p, drop_salt, (const unsigned long long *)drop_seed_ptr);
-    if (dbias) vec::fold_partials_kernel<bf16><<<(cols + 31) / 32, dim3(32, 32), 0, st>>>(partial, gy, cols, (bf16 *)dbias, (bf16 *)nullptr, accumulate);
+    if (dbias) ffk_launch(vec::fold_partials_kernel<bf16>, (cols + 31) / 32, dim3(32, 32), 0, st, partial, gy, cols, (bf16 *)dbias, (bf16 *)nullptr, accumulate);
     return (int)cudaGetLastError();
   }
   if (drop_p > 0.f) return -2;  // the fused-dropout form exists for the 16-byte vector path only
   dim3 grid((cols + 31) / 32, gy), block(32, 8);
   DISPATCH_FLOAT(dt, {
-    bias_act_bwd_kernel<T><<<grid, block, 0, st>>>((const T *)dy, (const T *)saved, (T *)dz, dbias ? partial : nullptr,
+    ffk_launch(bias_act_bwd_kernel<T>, grid, block, 0, st, (const T *)dy, (const T *)saved, (T *)dz, dbias ? partial : nullptr,
                                                     rows, cols, act);
-    if (dbias) colsum_finish_kernel<T><<<(cols + 255) / 256, 256, 0, st>>>(partial, gy, cols, (T *)dbias, accumulate);
+    if (dbias) ffk_launch(colsum_finish_kernel<T>, (cols + 255) / 256, 256, 0, st, partial, gy, cols, (T *)dbias, accumulate);
   });
   return (int)cudaGetLastError();
 }

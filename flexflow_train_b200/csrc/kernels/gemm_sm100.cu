@@ -295,6 +295,7 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
   if constexpr (CTA2) cluster_sync_all();  // the partner's barriers exist before anything is signalled across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_entry();  // the set-up above ran under the previous kernel's tail
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -765,6 +766,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_entry();  // the set-up above ran under the previous kernel's tail
 
   if (warp == 0) {
     {  // TMA producer: the whole warp runs the loop, one lane issues
@@ -989,6 +991,7 @@ __device__ __forceinline__ void simt_stage(float *s, const float (&r)[ST], int m
 
 template <typename T>
 __global__ void __launch_bounds__(SIMT_WARPS * 32, 2) gemm_simt_kernel(SimtOperands o, GemmArgs p) {
+  pdl_entry();
   extern __shared__ __align__(16) float simt_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float *sa = simt_smem + warp * SIMT_WARP_FLOATS, *sb = sa + ST * SA_LD;
@@ -1059,6 +1062,7 @@ __global__ void __launch_bounds__(SIMT_WARPS * 32, 2) gemm_simt_kernel(SimtOpera
 constexpr int TH_M = 16, TH_N = 64, TH_K = 32, TH_MAX_K = 128;
 template <typename T>
 __global__ void __launch_bounds__(256) gemm_thin_kernel(SimtOperands o, GemmArgs p) {
+  pdl_entry();
   __shared__ float sa[TH_M][TH_K + 1], sb[TH_N][TH_K + 1];
   const int batch = blockIdx.z, bh = batch % p.nh, bb = batch / p.nh;
   const int m0 = blockIdx.y * TH_M, n0 = blockIdx.x * TH_N;
@@ -1150,6 +1154,7 @@ __device__ __forceinline__ void small_stage(float *s, const T *X, int rows, int 
 
 template <typename T>
 __global__ void __launch_bounds__(SB_WARPS * 32) gemm_small_batched_kernel(SimtOperands o, GemmArgs p) {
+  pdl_entry();
   extern __shared__ __align__(16) float simt_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int batch = blockIdx.x * SB_WARPS + warp;
@@ -1242,13 +1247,15 @@ int launch_pair(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap 
   cfg.blockDim = dim3(GEMM_THREADS);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, sm, args);
   return (int)e;
 }
@@ -1288,7 +1295,9 @@ int launch_cfg(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &
   long long grid = items < max_ctas ? items : max_ctas;
   if (grid < 1) return 0;
   if (args.split_k > 1) args.tma_store = 0;
-  kern<<<(unsigned)grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, sm, args);
+  // a fused collective waits for its peers: nothing is launched ahead of its end, and it is not launched ahead itself
+  if (args.scatter_rows || args.gate_flags || args.push_src) kern<<<(unsigned)grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, sm, args);
+  else ffk_launch(kern, (unsigned)grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, ta, tb, tc, sm, args);
   return (int)cudaGetLastError();
 }
 
@@ -1332,13 +1341,15 @@ int launch_cluster(const CUtensorMap &ta, const CUtensorMap &tb, GemmArgs &args,
   cfg.blockDim = dim3(CK_THREADS);
   cfg.dynamicSmemBytes = Cfg::smem_bytes(args.cluster_stages);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)split;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, args);
 }
 template <int BN>
@@ -1512,8 +1523,8 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
       const int blocks = (int)((nbatch + SB_WARPS - 1) / SB_WARPS);
       // only the panels' own size: more resident warps per SM hide the staging loads
       const int smem = SB_WARPS * (d->M + d->N) * (d->K + 1) * 4;
-      if (es == 2) gemm_small_batched_kernel<bf16><<<blocks, SB_WARPS * 32, smem, stream>>>(so, a);
-      else gemm_small_batched_kernel<float><<<blocks, SB_WARPS * 32, smem, stream>>>(so, a);
+      if (es == 2) ffk_launch(gemm_small_batched_kernel<bf16>, blocks, SB_WARPS * 32, smem, stream, so, a);
+      else ffk_launch(gemm_small_batched_kernel<float>, blocks, SB_WARPS * 32, smem, stream, so, a);
       return (int)cudaGetLastError();
     }
     // K up to 128 and few enough tiles for one wave or two: with more, the 32 x 32 tiles' reuse of their operands pays
@@ -1522,8 +1533,8 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
       if (ty <= 65535 && tx * ty * nbatch <= 148 * 8) {
         SimtOperands to{d->A, d->B, d->lda, d->a_sh, d->a_sb, d->ldb, d->b_sh, d->b_sb, d->a_mn, d->b_mn, 1, 0};
         dim3 tg((unsigned)tx, (unsigned)ty, (unsigned)nbatch);
-        if (es == 2) gemm_thin_kernel<bf16><<<tg, 256, 0, stream>>>(to, a);
-        else gemm_thin_kernel<float><<<tg, 256, 0, stream>>>(to, a);
+        if (es == 2) ffk_launch(gemm_thin_kernel<bf16>, tg, 256, 0, stream, to, a);
+        else ffk_launch(gemm_thin_kernel<float>, tg, 256, 0, stream, to, a);
         return (int)cudaGetLastError();
       }
     }
@@ -1543,8 +1554,8 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
     const int gy = group_batch ? tiles_m : (tiles_m + tpb - 1) / tpb, gz = group_batch ? (nbatch + tpb - 1) / tpb : nbatch;
     if (gy > 65535 || gz > 65535) return -2;
     dim3 grid((d->N + ST - 1) / ST, gy, gz), block(SIMT_WARPS * 32);
-    if (es == 2) gemm_simt_kernel<bf16><<<grid, block, SIMT_SMEM_BYTES, stream>>>(o, a);
-    else gemm_simt_kernel<float><<<grid, block, SIMT_SMEM_BYTES, stream>>>(o, a);
+    if (es == 2) ffk_launch(gemm_simt_kernel<bf16>, grid, block, SIMT_SMEM_BYTES, stream, o, a);
+    else ffk_launch(gemm_simt_kernel<float>, grid, block, SIMT_SMEM_BYTES, stream, o, a);
     return (int)cudaGetLastError();
   }
   int bn = d->bn, split = d->split;

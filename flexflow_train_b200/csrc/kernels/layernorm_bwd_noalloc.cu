@@ -58,6 +58,7 @@ template <typename T>
 __global__ void ln_bwd_noalloc_kernel(const T *__restrict__ dy, const T *__restrict__ x, const T *__restrict__ gamma,
                                       const float *__restrict__ mean, const float *__restrict__ rstd, T *__restrict__ dx,
                                       float *__restrict__ partial, int rows, int cols) {
+  pdl_entry();
   __shared__ float red[32];
   float *pg = partial + (long long)blockIdx.x * cols;
   float *pb = partial + ((long long)gridDim.x + blockIdx.x) * cols;
@@ -87,6 +88,7 @@ __global__ void ln_bwd_noalloc_kernel(const T *__restrict__ dy, const T *__restr
 }
 template <typename T>
 __global__ void ln_bwd_noalloc_finish_kernel(const float *__restrict__ partial, int nparts, int cols, T *dgamma, T *dbeta) {
+  pdl_entry();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
   float g = 0.f, b = 0.f;
@@ -102,11 +104,11 @@ template <typename T>
 int launch(const void *dy, const void *x, const void *gamma, const float *mean, const float *rstd, void *dx, void *dgamma, void *dbeta,
            float *scratch, int rows, int cols, cudaStream_t stream) {
   int grid = rows < NOALLOC_MAX_BLOCKS ? rows : NOALLOC_MAX_BLOCKS;
-  ln_bwd_noalloc_kernel<T><<<grid, 256, 0, stream>>>((const T *)dy, (const T *)x, (const T *)gamma, mean, rstd, (T *)dx, scratch, rows, cols);
+  ffk_launch(ln_bwd_noalloc_kernel<T>, grid, 256, 0, stream, (const T *)dy, (const T *)x, (const T *)gamma, mean, rstd, (T *)dx, scratch, rows, cols);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return (int)e;
   if (dgamma || dbeta) {
-    ln_bwd_noalloc_finish_kernel<T><<<(cols + 255) / 256, 256, 0, stream>>>(scratch, grid, cols, (T *)dgamma, (T *)dbeta);
+    ffk_launch(ln_bwd_noalloc_finish_kernel<T>, (cols + 255) / 256, 256, 0, stream, scratch, grid, cols, (T *)dgamma, (T *)dbeta);
     e = cudaGetLastError();
   }
   return (int)e;

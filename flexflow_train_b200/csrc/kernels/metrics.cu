@@ -26,6 +26,7 @@ template <> __device__ __forceinline__ float ldm<bf16>(const bf16 *p, long long 
 template <typename T>
 __global__ void metrics_kernel(const T *__restrict__ pred, const void *__restrict__ label_i, const T *__restrict__ label_d, int label64,
                                long long n, int c, int flags, double *__restrict__ acc) {
+  pdl_entry();
   __shared__ float part[M_SLOTS][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   float sums[M_SLOTS];
@@ -107,9 +108,9 @@ FFK_API int ffk_metrics_update(const void *pred, const void *label_sparse, const
   long long want = (n + 7) / 8;
   const int grid = (int)(want < 148 * 8 ? want : 148 * 8);
   if (pred_dt == 0)
-    metrics_kernel<float><<<grid, 256, 0, st>>>((const float *)pred, label_sparse, (const float *)label_dense, label_dt == 3, n, c, flags, acc);
+    ffk_launch(metrics_kernel<float>, grid, 256, 0, st, (const float *)pred, label_sparse, (const float *)label_dense, label_dt == 3, n, c, flags, acc);
   else if (pred_dt == 1)
-    metrics_kernel<bf16><<<grid, 256, 0, st>>>((const bf16 *)pred, label_sparse, (const bf16 *)label_dense, label_dt == 3, n, c, flags, acc);
+    ffk_launch(metrics_kernel<bf16>, grid, 256, 0, st, (const bf16 *)pred, label_sparse, (const bf16 *)label_dense, label_dt == 3, n, c, flags, acc);
   else
     return -2;
   return (int)cudaGetLastError();

@@ -27,6 +27,7 @@ __global__ void layernorm_fwd_kernel(const T *__restrict__ a, const T *__restric
                                      const T *__restrict__ beta, T *__restrict__ xsum, T *__restrict__ y,
                                      float *__restrict__ mean, float *__restrict__ rstd, int rows, int cols,
                                      float eps) {
+  pdl_entry();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T *pa = a + (long long)row * cols;
@@ -68,6 +69,7 @@ __global__ void layernorm_bwd_kernel(const T *__restrict__ dy, const T *__restri
                                      const float *__restrict__ mean, const float *__restrict__ rstd,
                                      T *__restrict__ dx, T *__restrict__ dx2, float *__restrict__ partial, int rows,
                                      int cols, int accumulate_dx, int accumulate_dx2) {
+  pdl_entry();
   __shared__ float red[32];
   float dg[KMAX], db[KMAX];
 #pragma unroll
@@ -127,6 +129,7 @@ __global__ void layernorm_bwd_kernel(const T *__restrict__ dy, const T *__restri
 template <typename T>
 __global__ void softmax_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, int rows, int cols, float scale,
                                    int causal_q) {
+  pdl_entry();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T *px = x + (long long)row * cols;
@@ -147,6 +150,7 @@ __global__ void softmax_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, i
 template <typename T>
 __global__ void softmax_bwd_kernel(const T *__restrict__ dy, const T *__restrict__ y, T *__restrict__ dx, int rows,
                                    int cols, float scale) {
+  pdl_entry();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T *pdy = dy + (long long)row * cols;
@@ -166,6 +170,7 @@ template <typename T, typename L>
 __global__ void softmax_ce_kernel(const T *__restrict__ logits, const L *__restrict__ labels, T *__restrict__ probs,
                                   T *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols,
                                   float grad_scale) {
+  pdl_entry();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T *px = logits + (long long)row * cols;
@@ -193,6 +198,7 @@ template <int VPT, typename L>
 __global__ void __launch_bounds__(512, 2) softmax_ce_row_kernel(const bf16 *__restrict__ logits, const L *__restrict__ labels,
                                                                 bf16 *__restrict__ probs, bf16 *__restrict__ dlogits,
                                                                 float *__restrict__ loss, int cols, float grad_scale) {
+  pdl_entry();
   __shared__ float red[64];
   const int nvec = cols >> 3;
   const long long base = (long long)blockIdx.x * cols;
@@ -238,6 +244,7 @@ template <bool CE, typename L>
 __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__restrict__ x, const L *__restrict__ labels, bf16 *__restrict__ probs,
                                                                bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols,
                                                                float scale, float grad_scale, int depth) {
+  pdl_entry();
   extern __shared__ __align__(128) uint8_t wide_smem[];
   __shared__ float red[64];
   __shared__ uint64_t full[4];
@@ -345,6 +352,7 @@ enum { LOSS_SPARSE_CCE = 0, LOSS_CCE = 1, LOSS_MSE_AVG = 2, LOSS_IDENTITY = 3, L
 template <typename T, typename L>
 __global__ void loss_bwd_kernel(int kind, const T *__restrict__ pred, const void *__restrict__ target,
                                 T *__restrict__ dpred, long long rows, int cols, float scale) {
+  pdl_entry();
   long long n = rows * cols;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -366,6 +374,7 @@ __global__ void loss_bwd_kernel(int kind, const T *__restrict__ pred, const void
 template <typename T, typename L>
 __global__ void loss_fwd_kernel(int kind, const T *__restrict__ pred, const void *__restrict__ target,
                                 float *__restrict__ loss, int rows, int cols) {
+  pdl_entry();
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const T *pp = pred + (long long)row * cols;
@@ -420,7 +429,7 @@ FFK_API int ffk_layernorm_fwd(const void *a, const void *b, const void *gamma, c
       const int wv = cols / 256;
       long long want = ((long long)rows + 7) / 8;
       const int grid = (int)(want < 148 * 2 ? want : 148 * 2);
-#define LN_WARP(V) vec::layernorm_fwd_warp_kernel<V><<<grid, 256, 0, st>>>(A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, eps)
+#define LN_WARP(V) ffk_launch(vec::layernorm_fwd_warp_kernel<V>, grid, 256, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, eps)
       switch (wv) {
         case 1: LN_WARP(1); break;
         case 2: LN_WARP(2); break;
@@ -434,13 +443,13 @@ FFK_API int ffk_layernorm_fwd(const void *a, const void *b, const void *gamma, c
 #undef LN_WARP
       return (int)cudaGetLastError();
     }
-    if (vpt == 1) vec::layernorm_fwd_vec_kernel<1><<<rows_grid(rows), threads, 0, st>>>(A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
-    else if (vpt == 2) vec::layernorm_fwd_vec_kernel<2><<<rows_grid(rows), threads, 0, st>>>(A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
-    else vec::layernorm_fwd_vec_kernel<4><<<rows_grid(rows), threads, 0, st>>>(A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
+    if (vpt == 1) ffk_launch(vec::layernorm_fwd_vec_kernel<1>, rows_grid(rows), threads, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
+    else if (vpt == 2) ffk_launch(vec::layernorm_fwd_vec_kernel<2>, rows_grid(rows), threads, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
+    else ffk_launch(vec::layernorm_fwd_vec_kernel<4>, rows_grid(rows), threads, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
     return (int)cudaGetLastError();
   }
   int threads = cols >= 2048 ? 512 : 256;
-  DISPATCH_FLOAT(dt, (layernorm_fwd_kernel<T><<<rows_grid(rows), threads, 0, st>>>(
+  DISPATCH_FLOAT(dt, (ffk_launch(layernorm_fwd_kernel<T>, rows_grid(rows), threads, 0, st, 
                          (const T *)a, (const T *)b, (const T *)gamma, (const T *)beta, (T *)xsum, (T *)y, mean, rstd,
                          rows, cols, eps)));
   return (int)cudaGetLastError();
@@ -479,25 +488,25 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
   if (vec) {
     int vpt = ln_vpt(cols), threads = cols / 8 / vpt;
     const bf16 *DY = (const bf16 *)dy, *X = (const bf16 *)x, *G = (const bf16 *)gamma;
-    if (vpt == 1) vec::layernorm_bwd_vec_kernel<1><<<grid, threads, 0, st>>>(DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
-    else if (vpt == 2) vec::layernorm_bwd_vec_kernel<2><<<grid, threads, 0, st>>>(DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
-    else vec::layernorm_bwd_vec_kernel<4><<<grid, threads, 0, st>>>(DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
+    if (vpt == 1) ffk_launch(vec::layernorm_bwd_vec_kernel<1>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
+    else if (vpt == 2) ffk_launch(vec::layernorm_bwd_vec_kernel<2>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
+    else ffk_launch(vec::layernorm_bwd_vec_kernel<4>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     if (part)
-      vec::fold_partials_kernel<bf16><<<(cols + 31) / 32, dim3(32, 32), 0, st>>>(part, grid, cols, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_params);
+      ffk_launch(vec::fold_partials_kernel<bf16>, (cols + 31) / 32, dim3(32, 32), 0, st, part, grid, cols, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_params);
     return (int)cudaGetLastError();
   }
   DISPATCH_FLOAT(dt, {
     if (cols <= 512 * 4)
-      layernorm_bwd_kernel<T, 4><<<grid, 512, 0, st>>>((const T *)dy, (const T *)x, (const T *)gamma, mean, rstd,
+      ffk_launch(layernorm_bwd_kernel<T, 4>, grid, 512, 0, st, (const T *)dy, (const T *)x, (const T *)gamma, mean, rstd,
                                                         (T *)dx, (T *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     else if (cols <= 512 * 16)
-      layernorm_bwd_kernel<T, 16><<<grid, 512, 0, st>>>((const T *)dy, (const T *)x, (const T *)gamma, mean, rstd,
+      ffk_launch(layernorm_bwd_kernel<T, 16>, grid, 512, 0, st, (const T *)dy, (const T *)x, (const T *)gamma, mean, rstd,
                                                          (T *)dx, (T *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     else
-      layernorm_bwd_kernel<T, 32><<<grid, 512, 0, st>>>((const T *)dy, (const T *)x, (const T *)gamma, mean, rstd,
+      ffk_launch(layernorm_bwd_kernel<T, 32>, grid, 512, 0, st, (const T *)dy, (const T *)x, (const T *)gamma, mean, rstd,
                                                          (T *)dx, (T *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     if (part)
-      vec::fold_partials_kernel<T><<<(cols + 31) / 32, dim3(32, 32), 0, st>>>(part, grid, cols, (T *)dgamma, (T *)dbeta, accumulate_params);
+      ffk_launch(vec::fold_partials_kernel<T>, (cols + 31) / 32, dim3(32, 32), 0, st, part, grid, cols, (T *)dgamma, (T *)dbeta, accumulate_params);
   });
   return (int)cudaGetLastError();
 }
@@ -521,10 +530,10 @@ FFK_API int ffk_softmax_dropout_fwd(const void *x, void *y, void *yd, int rows, 
 #define SM_FWD(V)                                                                                                                        \
   case V:                                                                                                                                \
     if (cols == 256 * V && ld == cols)                                                                                                   \
-      vec::softmax_fwd_warp_kernel<V, true><<<grid, 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (bf16 *)yd, rows, cols, ld, scale, causal_q, \
+      ffk_launch(vec::softmax_fwd_warp_kernel<V, true>, grid, 256, 0, st, (const bf16 *)x, (bf16 *)y, (bf16 *)yd, rows, cols, ld, scale, causal_q, \
                                                                   p, salt, seed_ptr);                                                    \
     else                                                                                                                                 \
-      vec::softmax_fwd_warp_kernel<V, false><<<grid, 256, 0, st>>>((const bf16 *)x, (bf16 *)y, (bf16 *)yd, rows, cols, ld, scale, causal_q, \
+      ffk_launch(vec::softmax_fwd_warp_kernel<V, false>, grid, 256, 0, st, (const bf16 *)x, (bf16 *)y, (bf16 *)yd, rows, cols, ld, scale, causal_q, \
                                                                    p, salt, seed_ptr);                                                   \
     break;
   switch (softmax_vpt(cols)) { SM_FWD(1) SM_FWD(2) SM_FWD(3) SM_FWD(4) SM_FWD(6) SM_FWD(8) SM_FWD(16) }
@@ -540,10 +549,10 @@ FFK_API int ffk_softmax_dropout_bwd(const void *dy, const void *y, void *dx, int
 #define SM_BWD(V)                                                                                                                       \
   case V:                                                                                                                               \
     if (cols == 256 * V && ld == cols)                                                                                                  \
-      vec::softmax_bwd_warp_kernel<V, true><<<grid, 256, 0, st>>>((const bf16 *)dy, (const bf16 *)y, (bf16 *)dx, rows, cols, ld, scale, p, \
+      ffk_launch(vec::softmax_bwd_warp_kernel<V, true>, grid, 256, 0, st, (const bf16 *)dy, (const bf16 *)y, (bf16 *)dx, rows, cols, ld, scale, p, \
                                                                   salt, seed_ptr);                                                      \
     else                                                                                                                                \
-      vec::softmax_bwd_warp_kernel<V, false><<<grid, 256, 0, st>>>((const bf16 *)dy, (const bf16 *)y, (bf16 *)dx, rows, cols, ld, scale, p, \
+      ffk_launch(vec::softmax_bwd_warp_kernel<V, false>, grid, 256, 0, st, (const bf16 *)dy, (const bf16 *)y, (bf16 *)dx, rows, cols, ld, scale, p, \
                                                                    salt, seed_ptr);                                                     \
     break;
   switch (softmax_vpt(cols)) { SM_BWD(1) SM_BWD(2) SM_BWD(3) SM_BWD(4) SM_BWD(6) SM_BWD(8) SM_BWD(16) }
@@ -555,7 +564,7 @@ FFK_API int ffk_dropout_rows(const void *x, void *y, long long rows, int cols, i
                              const unsigned long long *seed_ptr, cudaStream_t st) {
   if (rows <= 0) return 0;
   if (!softmax_warp_ok(cols, ld, 1, x, y, nullptr)) return -3;
-  vec::dropout_rows_kernel<<<ffk_blocks(rows * (ld / 8), 256), 256, 0, st>>>((const bf16 *)x, (bf16 *)y, rows, cols, ld, p, salt, seed_ptr);
+  ffk_launch(vec::dropout_rows_kernel, ffk_blocks(rows * (ld / 8), 256), 256, 0, st, (const bf16 *)x, (bf16 *)y, rows, cols, ld, p, salt, seed_ptr);
   return (int)cudaGetLastError();
 }
 
@@ -584,7 +593,7 @@ static int launch_softmax_wide(const void *x, const void *labels, void *probs, v
   int depth = WIDE_SMEM / per_sm / (cols * 2);
   if (depth > 4) depth = 4;
   const int grid = rows < 148 * per_sm ? rows : 148 * per_sm;
-  kern<<<grid, threads, (size_t)depth * cols * 2, st>>>((const bf16 *)x, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss, rows, cols,
+  ffk_launch(kern, grid, threads, (size_t)depth * cols * 2, st, (const bf16 *)x, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss, rows, cols,
                                                         scale, grad_scale, depth);
   return (int)cudaGetLastError();
 }
@@ -607,12 +616,12 @@ FFK_API int ffk_softmax_fwd(const void *x, void *y, int rows, int cols, float sc
   int threads, vpt;
   if (dt == 1 && cols % 8 == 0 && causal_q <= 0 && aligned16(x) && aligned16(y) && (vpt = row_block(cols, threads)) != 0) {
     // only rows beyond the wide kernel's come here (the shorter ones took the warp kernel)
-    if (vpt <= 8) vec::softmax_fwd_row_kernel<8><<<rows, threads, 0, st>>>((const bf16 *)x, (bf16 *)y, cols, scale);
-    else vec::softmax_fwd_row_kernel<16><<<rows, threads, 0, st>>>((const bf16 *)x, (bf16 *)y, cols, scale);
+    if (vpt <= 8) ffk_launch(vec::softmax_fwd_row_kernel<8>, rows, threads, 0, st, (const bf16 *)x, (bf16 *)y, cols, scale);
+    else ffk_launch(vec::softmax_fwd_row_kernel<16>, rows, threads, 0, st, (const bf16 *)x, (bf16 *)y, cols, scale);
     return (int)cudaGetLastError();
   }
   threads = cols >= 1024 ? 256 : 128;
-  DISPATCH_FLOAT(dt, (softmax_fwd_kernel<T><<<rows < 148 * 16 ? rows : 148 * 16, threads, 0, st>>>(
+  DISPATCH_FLOAT(dt, (ffk_launch(softmax_fwd_kernel<T>, rows < 148 * 16 ? rows : 148 * 16, threads, 0, st, 
                          (const T *)x, (T *)y, rows, cols, scale, causal_q)));
   return (int)cudaGetLastError();
 }
@@ -622,7 +631,7 @@ FFK_API int ffk_softmax_bwd(const void *dy, const void *y, void *dx, int rows, i
   if (softmax_warp_ok(cols, cols, dt, dy, y, dx))
     return ffk_softmax_dropout_bwd(dy, y, dx, rows, cols, cols, scale, 0.f, 0, nullptr, dt, st);
   int threads = cols >= 1024 ? 256 : 128;
-  DISPATCH_FLOAT(dt, (softmax_bwd_kernel<T><<<rows < 148 * 16 ? rows : 148 * 16, threads, 0, st>>>(
+  DISPATCH_FLOAT(dt, (ffk_launch(softmax_bwd_kernel<T>, rows < 148 * 16 ? rows : 148 * 16, threads, 0, st, 
                          (const T *)dy, (const T *)y, (T *)dx, rows, cols, scale)));
   return (int)cudaGetLastError();
 }
@@ -630,10 +639,10 @@ template <int VPT>
 static void launch_softmax_ce_row(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols,
                                   float grad_scale, int label_dt, int threads, cudaStream_t st) {
   if (label_dt == 3)
-    softmax_ce_row_kernel<VPT, long long><<<rows, threads, 0, st>>>((const bf16 *)logits, (const long long *)labels, (bf16 *)probs,
+    ffk_launch(softmax_ce_row_kernel<VPT, long long>, rows, threads, 0, st, (const bf16 *)logits, (const long long *)labels, (bf16 *)probs,
                                                                     (bf16 *)dlogits, loss, cols, grad_scale);
   else
-    softmax_ce_row_kernel<VPT, int><<<rows, threads, 0, st>>>((const bf16 *)logits, (const int *)labels, (bf16 *)probs, (bf16 *)dlogits, loss,
+    ffk_launch(softmax_ce_row_kernel<VPT, int>, rows, threads, 0, st, (const bf16 *)logits, (const int *)labels, (bf16 *)probs, (bf16 *)dlogits, loss,
                                                               cols, grad_scale);
 }
 // label_dt: 2 = int32, 3 = int64
@@ -658,10 +667,10 @@ FFK_API int ffk_softmax_ce(const void *logits, const void *labels, void *probs, 
   const int grid = rows < 148 * 4 ? rows : 148 * 4;
   DISPATCH_FLOAT(dt, {
     if (label_dt == 3)
-      softmax_ce_kernel<T, long long><<<grid, threads, 0, st>>>((const T *)logits, (const long long *)labels,
+      ffk_launch(softmax_ce_kernel<T, long long>, grid, threads, 0, st, (const T *)logits, (const long long *)labels,
                                                                  (T *)probs, (T *)dlogits, loss, rows, cols, grad_scale);
     else
-      softmax_ce_kernel<T, int><<<grid, threads, 0, st>>>((const T *)logits, (const int *)labels, (T *)probs,
+      ffk_launch(softmax_ce_kernel<T, int>, grid, threads, 0, st, (const T *)logits, (const int *)labels, (T *)probs,
                                                            (T *)dlogits, loss, rows, cols, grad_scale);
   });
   return (int)cudaGetLastError();
@@ -671,10 +680,10 @@ FFK_API int ffk_loss_bwd(int kind, const void *pred, const void *target, void *d
   if (rows <= 0) return 0;
   DISPATCH_FLOAT(dt, {
     if (label_dt == 3)
-      loss_bwd_kernel<T, long long><<<ffk_blocks(rows * cols, 256), 256, 0, st>>>(kind, (const T *)pred, target,
+      ffk_launch(loss_bwd_kernel<T, long long>, ffk_blocks(rows * cols, 256), 256, 0, st, kind, (const T *)pred, target,
                                                                                    (T *)dpred, rows, cols, scale);
     else
-      loss_bwd_kernel<T, int><<<ffk_blocks(rows * cols, 256), 256, 0, st>>>(kind, (const T *)pred, target, (T *)dpred,
+      ffk_launch(loss_bwd_kernel<T, int>, ffk_blocks(rows * cols, 256), 256, 0, st, kind, (const T *)pred, target, (T *)dpred,
                                                                              rows, cols, scale);
   });
   return (int)cudaGetLastError();
@@ -684,10 +693,10 @@ FFK_API int ffk_loss_fwd(int kind, const void *pred, const void *target, float *
   if (rows <= 0) return 0;
   DISPATCH_FLOAT(dt, {
     if (label_dt == 3)
-      loss_fwd_kernel<T, long long><<<rows < 2368 ? rows : 2368, 128, 0, st>>>(kind, (const T *)pred, target, loss,
+      ffk_launch(loss_fwd_kernel<T, long long>, rows < 2368 ? rows : 2368, 128, 0, st, kind, (const T *)pred, target, loss,
                                                                                 rows, cols);
     else
-      loss_fwd_kernel<T, int><<<rows < 2368 ? rows : 2368, 128, 0, st>>>(kind, (const T *)pred, target, loss, rows,
+      ffk_launch(loss_fwd_kernel<T, int>, rows < 2368 ? rows : 2368, 128, 0, st, kind, (const T *)pred, target, loss, rows,
                                                                           cols);
   });
   return (int)cudaGetLastError();

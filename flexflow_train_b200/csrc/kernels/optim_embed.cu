@@ -21,6 +21,7 @@ __global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float 
                             const G *__restrict__ g, bf16 *__restrict__ shadow, long long n, float alpha_t,
                             float beta1, float beta2, float eps, float wd, float gscale,
                             const float *__restrict__ alpha_ptr) {
+  pdl_entry();
   // alpha_ptr (optional): bias-corrected step size kept in device memory so that a captured CUDA graph
   // sees the value of the current step.
   if (alpha_ptr) alpha_t = *alpha_ptr;
@@ -62,6 +63,7 @@ template <typename G>
 __global__ void sgd_kernel(float *__restrict__ w, float *__restrict__ mom, const G *__restrict__ g,
                            bf16 *__restrict__ shadow, long long n, float lr, float momentum, int nesterov, float wd,
                            float gscale) {
+  pdl_entry();
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
     float wk = w[i];
@@ -82,6 +84,7 @@ __global__ void sgd_kernel(float *__restrict__ w, float *__restrict__ mom, const
 template <typename W, typename I, typename O>
 __global__ void embedding_fwd_kernel(const I *__restrict__ idx, const W *__restrict__ table, O *__restrict__ out,
                                      long long tokens, int bag, int dim, long long entries, int avg) {
+  pdl_entry();
   long long total = tokens * dim;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -102,6 +105,7 @@ __device__ __forceinline__ void atomic_add_any(bf16 *p, float v) { atomicAdd(p, 
 template <typename W, typename I, typename O>
 __global__ void embedding_bwd_kernel(const I *__restrict__ idx, const O *__restrict__ dout, W *__restrict__ dtable,
                                      long long tokens, int bag, int dim, long long entries, int avg) {
+  pdl_entry();
   long long total = tokens * dim;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -121,6 +125,7 @@ __global__ void embedding_bwd_kernel(const I *__restrict__ idx, const O *__restr
 template <typename I, typename O>
 __global__ void embedding_sgd_kernel(const I *__restrict__ idx, const O *__restrict__ dout, float *__restrict__ table,
                                      long long tokens, int bag, int dim, long long entries, float lr) {
+  pdl_entry();
   long long total = tokens * dim;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -143,9 +148,9 @@ FFK_API int ffk_adam_update(float *w, float *m, float *v, const void *g, void *s
   if (n <= 0) return 0;
   int grid = ffk_blocks(n / 4 + 1, 256, 148 * 8);
   if (grad_dt == 1)
-    adam_kernel<bf16><<<grid, 256, 0, st>>>(w, m, v, (const bf16 *)g, (bf16 *)shadow, n, alpha_t, beta1, beta2, eps, wd, gscale, alpha_ptr);
+    ffk_launch(adam_kernel<bf16>, grid, 256, 0, st, w, m, v, (const bf16 *)g, (bf16 *)shadow, n, alpha_t, beta1, beta2, eps, wd, gscale, alpha_ptr);
   else
-    adam_kernel<float><<<grid, 256, 0, st>>>(w, m, v, (const float *)g, (bf16 *)shadow, n, alpha_t, beta1, beta2, eps, wd, gscale, alpha_ptr);
+    ffk_launch(adam_kernel<float>, grid, 256, 0, st, w, m, v, (const float *)g, (bf16 *)shadow, n, alpha_t, beta1, beta2, eps, wd, gscale, alpha_ptr);
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_sgd_update(float *w, float *mom, const void *g, void *shadow, long long n, float lr, float momentum,
@@ -153,9 +158,9 @@ FFK_API int ffk_sgd_update(float *w, float *mom, const void *g, void *shadow, lo
   if (n <= 0) return 0;
   int grid = ffk_blocks(n, 256, 148 * 8);
   if (grad_dt == 1)
-    sgd_kernel<bf16><<<grid, 256, 0, st>>>(w, mom, (const bf16 *)g, (bf16 *)shadow, n, lr, momentum, nesterov, wd, gscale);
+    ffk_launch(sgd_kernel<bf16>, grid, 256, 0, st, w, mom, (const bf16 *)g, (bf16 *)shadow, n, lr, momentum, nesterov, wd, gscale);
   else
-    sgd_kernel<float><<<grid, 256, 0, st>>>(w, mom, (const float *)g, (bf16 *)shadow, n, lr, momentum, nesterov, wd, gscale);
+    ffk_launch(sgd_kernel<float>, grid, 256, 0, st, w, mom, (const float *)g, (bf16 *)shadow, n, lr, momentum, nesterov, wd, gscale);
   return (int)cudaGetLastError();
 }
 
@@ -164,10 +169,10 @@ static int emb_launch(int which, const void *idx, const void *table_or_dtable, c
                       int bag, int dim, long long entries, int avg, cudaStream_t st) {
   int grid = ffk_blocks(tokens * dim, 256);
   if (which == 0)
-    embedding_fwd_kernel<W, I, O><<<grid, 256, 0, st>>>((const I *)idx, (const W *)table_or_dtable, (O *)out_or_dout,
+    ffk_launch(embedding_fwd_kernel<W, I, O>, grid, 256, 0, st, (const I *)idx, (const W *)table_or_dtable, (O *)out_or_dout,
                                                          tokens, bag, dim, entries, avg);
   else
-    embedding_bwd_kernel<W, I, O><<<grid, 256, 0, st>>>((const I *)idx, (const O *)out_or_dout, (W *)table_or_dtable,
+    ffk_launch(embedding_bwd_kernel<W, I, O>, grid, 256, 0, st, (const I *)idx, (const O *)out_or_dout, (W *)table_or_dtable,
                                                          tokens, bag, dim, entries, avg);
   return (int)cudaGetLastError();
 }
@@ -201,10 +206,10 @@ FFK_API int ffk_embedding_sgd(const void *idx, const void *dout, float *table, l
                               long long entries, float lr, int idx_dt, int out_dt, cudaStream_t st) {
   if (tokens <= 0) return 0;
   int grid = ffk_blocks(tokens * dim, 256);
-  if (idx_dt == 3 && out_dt == 1) embedding_sgd_kernel<long long, bf16><<<grid, 256, 0, st>>>((const long long *)idx, (const bf16 *)dout, table, tokens, bag, dim, entries, lr);
-  else if (idx_dt == 2 && out_dt == 1) embedding_sgd_kernel<int, bf16><<<grid, 256, 0, st>>>((const int *)idx, (const bf16 *)dout, table, tokens, bag, dim, entries, lr);
-  else if (idx_dt == 3 && out_dt == 0) embedding_sgd_kernel<long long, float><<<grid, 256, 0, st>>>((const long long *)idx, (const float *)dout, table, tokens, bag, dim, entries, lr);
-  else if (idx_dt == 2 && out_dt == 0) embedding_sgd_kernel<int, float><<<grid, 256, 0, st>>>((const int *)idx, (const float *)dout, table, tokens, bag, dim, entries, lr);
+  if (idx_dt == 3 && out_dt == 1) ffk_launch(embedding_sgd_kernel<long long, bf16>, grid, 256, 0, st, (const long long *)idx, (const bf16 *)dout, table, tokens, bag, dim, entries, lr);
+  else if (idx_dt == 2 && out_dt == 1) ffk_launch(embedding_sgd_kernel<int, bf16>, grid, 256, 0, st, (const int *)idx, (const bf16 *)dout, table, tokens, bag, dim, entries, lr);
+  else if (idx_dt == 3 && out_dt == 0) ffk_launch(embedding_sgd_kernel<long long, float>, grid, 256, 0, st, (const long long *)idx, (const float *)dout, table, tokens, bag, dim, entries, lr);
+  else if (idx_dt == 2 && out_dt == 0) ffk_launch(embedding_sgd_kernel<int, float>, grid, 256, 0, st, (const int *)idx, (const float *)dout, table, tokens, bag, dim, entries, lr);
   else return -2;
   return (int)cudaGetLastError();
 }

@@ -41,6 +41,7 @@ __device__ __forceinline__ uint32_t keep8(unsigned long long seed, unsigned long
 template <int VPT, bool FULL>
 __global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, bf16 *__restrict__ yd, int rows, int cols, int ld,
                                         float scale, int causal_q, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
+  pdl_entry();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   unsigned long long seed = salt;
   if (seed_ptr) seed = salt * 0x9E3779B97F4A7C15ull + *seed_ptr;
@@ -95,6 +96,7 @@ __global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__rest
 template <int VPT, bool FULL>
 __global__ void softmax_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ y, bf16 *__restrict__ dx, int rows, int cols,
                                         int ld, float scale, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
+  pdl_entry();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   unsigned long long seed = salt;
   if (seed_ptr) seed = salt * 0x9E3779B97F4A7C15ull + *seed_ptr;
@@ -138,6 +140,7 @@ __global__ void softmax_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 
 // y = dropout(x) over rows of `cols` at pitch `ld`, the mask of softmax_fwd_warp_kernel's yd; a thread per 8 elements
 static __global__ void dropout_rows_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, long long rows, int cols, int ld, float p_drop,
                                            unsigned long long salt, const unsigned long long *seed_ptr) {
+  pdl_entry();
   const unsigned long long seed = seed_ptr ? salt * 0x9E3779B97F4A7C15ull + *seed_ptr : salt;
   const float keep_scale = p_drop < 1.f ? 1.f / (1.f - p_drop) : 0.f;
   const uint32_t thr = ffk_drop_threshold(p_drop);
@@ -205,6 +208,7 @@ __device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, flo
 }
 template <int VPT>
 __global__ void __launch_bounds__(512, 2) softmax_fwd_row_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, int cols, float scale) {
+  pdl_entry();
   __shared__ float red[64];
   const int nvec = cols >> 3;
   const long long base = (long long)blockIdx.x * cols;
@@ -232,6 +236,7 @@ template <int VPT>
 __global__ void layernorm_fwd_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, const bf16 *__restrict__ gamma,
                                          const bf16 *__restrict__ beta, bf16 *__restrict__ xsum, bf16 *__restrict__ y,
                                          float *__restrict__ mean, float *__restrict__ rstd, int rows, int cols, float eps) {
+  pdl_entry();
   // two block reductions per row (mean, then centred variance), each through its own double-buffered slot so
   // that one barrier per reduction suffices
   __shared__ float red_a[2][32], red_b[2][32];
@@ -328,6 +333,7 @@ __global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const bf16 *
                                                                     const bf16 *__restrict__ gamma, const bf16 *__restrict__ beta,
                                                                     bf16 *__restrict__ xsum, bf16 *__restrict__ y, float *__restrict__ mean,
                                                                     float *__restrict__ rstd, int rows, float eps) {
+  pdl_entry();
   constexpr int COLS = 256 * VPT, NV = 32 * VPT;
   __shared__ uint4 g_s[NV], b_s[NV];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -396,6 +402,7 @@ template <int VPT>
 __global__ void layernorm_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ gamma,
                                          const float *__restrict__ mean, const float *__restrict__ rstd, bf16 *__restrict__ dx,
                                          bf16 *__restrict__ dx2, float *__restrict__ partial, int rows, int cols, int acc1, int acc2) {
+  pdl_entry();
   // the two row sums are reduced together through a double-buffered slot: one barrier per row
   __shared__ float2 red2[2][32];
   int parity = 0;
@@ -501,6 +508,7 @@ __global__ void layernorm_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16
 static __global__ void bias_act_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ saved, bf16 *__restrict__ dz,
                                         float *__restrict__ partial, int rows, int cols, int act, float drop_p,
                                         unsigned long long drop_salt, const unsigned long long *drop_seed_ptr) {
+  pdl_entry();
   const unsigned long long dseed = drop_seed_ptr ? drop_salt * 0x9E3779B97F4A7C15ull + *drop_seed_ptr : drop_salt;
   const uint32_t dthr = ffk_drop_threshold(drop_p);
   const float dscale = drop_p > 0.f ? 1.f / (1.f - drop_p) : 1.f;
@@ -554,6 +562,7 @@ static __global__ void bias_act_bwd_vec_kernel(const bf16 *__restrict__ dy, cons
 // form took 60 us for 1184 parts of 768 columns: three blocks, each thread a chain of 1184 dependent additions.
 template <typename T>
 __global__ void fold_partials_kernel(const float *__restrict__ partial, int nparts, int cols, T *out, T *out2, int accumulate) {
+  pdl_entry();
   __shared__ float s1[32][33], s2[32][33];
   const int tx = threadIdx.x, ty = threadIdx.y, c = blockIdx.x * 32 + tx;
   float a = 0.f, b = 0.f;

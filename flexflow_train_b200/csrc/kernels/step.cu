@@ -29,6 +29,7 @@ constexpr int STAGE_THREADS = 256;
 constexpr int STAGE_UNITS = STAGE_THREADS * 4;  // 16-byte units of a segment's source that one block moves: 4 loads in flight per thread
 
 __global__ void __launch_bounds__(STAGE_THREADS) stage_batch_kernel(const __grid_constant__ FfkStageArgs a) {
+  pdl_entry();
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     if (a.alpha_ptr) *a.alpha_ptr = a.alpha;
     if (a.seed_ptr) *a.seed_ptr = a.seed;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) stage_batch_kernel(const __grid
 // Mean of the per-row losses, written straight into page-locked host memory: one launch in the place of a reduction and a
 // device-to-host copy (5.8 us on the device at the end of every step that reports its loss, and one more launch).
 __global__ void __launch_bounds__(1024) loss_mean_kernel(const float *__restrict__ rows, long long n, float *out) {
+  pdl_entry();
   __shared__ float red[32];
   float s = 0.f;
   const bool aligned = (((uintptr_t)rows) & 15) == 0;
@@ -104,11 +106,11 @@ FFK_API int ffk_stage_batch(const FfkStageArgs *in, cudaStream_t st) {
     blocks += (int)b;
   }
   if (blocks == 0) blocks = 1;
-  stage_batch_kernel<<<blocks, STAGE_THREADS, 0, st>>>(a);
+  ffk_launch(stage_batch_kernel, blocks, STAGE_THREADS, 0, st, a);
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_loss_mean(const float *rows, long long n, float *out_host, cudaStream_t st) {
   if (n <= 0) return -2;
-  loss_mean_kernel<<<1, 1024, 0, st>>>(rows, n, out_host);
+  ffk_launch(loss_mean_kernel, 1, 1024, 0, st, rows, n, out_host);
   return (int)cudaGetLastError();
 }

@@ -34,6 +34,7 @@ struct Dims {
 template <typename W>
 __global__ void permute_kernel(const W *__restrict__ src, W *__restrict__ dst, Dims d, long long total, int accumulate_f32,
                                int accumulate_bf16) {
+  pdl_entry();
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     long long rem = i, off = 0;
@@ -61,6 +62,7 @@ struct Dims32 {
 template <typename W>
 __global__ void permute32_kernel(const W *__restrict__ src, W *__restrict__ dst, Dims32 d, unsigned total, int accumulate_f32,
                                  int accumulate_bf16) {
+  pdl_entry();
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * stride) {
     W v[4];
@@ -96,6 +98,7 @@ __global__ void permute32_kernel(const W *__restrict__ src, W *__restrict__ dst,
 // dst[b][c][r] = src[b][r][c], 32x32 tiles through shared memory
 template <typename W>
 __global__ void transpose2d_kernel(const W *__restrict__ src, W *__restrict__ dst, int rows, int cols) {
+  pdl_entry();
   __shared__ W tile[32][33];
   long long base = (long long)blockIdx.z * rows * cols;
   int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
@@ -115,6 +118,7 @@ __global__ void transpose2d_kernel(const W *__restrict__ src, W *__restrict__ ds
 template <typename T>
 __global__ void block_copy_kernel(const T *__restrict__ src, long long src_ld, T *__restrict__ dst, long long dst_ld,
                                   long long outer, long long block, int accumulate) {
+  pdl_entry();
   long long total = outer * block;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -129,6 +133,7 @@ __global__ void block_copy_kernel(const T *__restrict__ src, long long src_ld, T
 // Plain copy of fewer than 2^31 elements: the row / column split by multiply-high, four elements in flight per thread.
 template <typename T>
 __global__ void block_copy32_kernel(const T *__restrict__ src, long long src_ld, T *__restrict__ dst, long long dst_ld, unsigned total, CopyDiv f) {
+  pdl_entry();
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * stride) {
     T v[4];
@@ -156,6 +161,7 @@ __global__ void block_copy32_kernel(const T *__restrict__ src, long long src_ld,
 // (channel concatenation of channels-last activations is this case).
 __global__ void block_copy_vec_kernel(const uint4 *__restrict__ src, long long src_ld, uint4 *__restrict__ dst, long long dst_ld,
                                       unsigned total, CopyDiv f, int accumulate_bf16) {
+  pdl_entry();
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     const unsigned o = cdiv(i, f), b = i - o * f.d;
@@ -180,6 +186,7 @@ enum { RED_SUM = 0, RED_MEAN = 1, RED_MAX = 2, RED_MIN = 3, RED_PROD = 4 };
 // x viewed as [outer, red, inner] -> y [outer, inner]
 template <typename T>
 __global__ void reduce_kernel(const T *__restrict__ x, T *__restrict__ y, long long outer, long long red, long long inner, int op) {
+  pdl_entry();
   long long total = outer * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -198,6 +205,7 @@ __global__ void reduce_kernel(const T *__restrict__ x, T *__restrict__ y, long l
 template <typename T>
 __global__ void reduce_bwd_kernel(const T *__restrict__ dy, T *__restrict__ dx, long long outer, long long red, long long inner,
                                   float scale, int accumulate) {
+  pdl_entry();
   long long total = outer * red * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -214,6 +222,7 @@ __global__ void reduce_bwd_kernel(const T *__restrict__ dy, T *__restrict__ dx, 
 template <typename T>
 __global__ void reduce_select_bwd_kernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ dy, T *__restrict__ dx,
                                          long long outer, long long red, long long inner, int op, int accumulate) {
+  pdl_entry();
   long long total = outer * red * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -240,6 +249,7 @@ __global__ void reduce_select_bwd_kernel(const T *__restrict__ x, const T *__res
 template <typename T, typename I>
 __global__ void gather_kernel(const T *__restrict__ x, const I *__restrict__ idx, T *__restrict__ y, long long outer, long long xd,
                               long long id, long long inner) {
+  pdl_entry();
   long long total = outer * id * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -251,6 +261,7 @@ __global__ void gather_kernel(const T *__restrict__ x, const I *__restrict__ idx
 template <typename I>
 __global__ void gather_bwd_kernel(const float *__restrict__ dy_f, const bf16 *__restrict__ dy_b, const I *__restrict__ idx,
                                   float *dx_f, bf16 *dx_b, long long outer, long long xd, long long id, long long inner) {
+  pdl_entry();
   long long total = outer * id * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -267,6 +278,7 @@ __global__ void gather_bwd_kernel(const float *__restrict__ dy_f, const bf16 *__
 // (<= a few thousand columns) and small k are the use case; the cost is O(k * cols / 32) per row.
 template <typename T>
 __global__ void topk_kernel(const T *__restrict__ x, T *__restrict__ vals, int *__restrict__ idxs, int rows, int cols, int k) {
+  pdl_entry();
   int warps_per_block = blockDim.x >> 5, lane = threadIdx.x & 31;
   for (int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps_per_block) {
     const T *p = x + (long long)row * cols;
@@ -299,6 +311,7 @@ __global__ void topk_kernel(const T *__restrict__ x, T *__restrict__ vals, int *
 template <typename T>
 __global__ void topk_bwd_kernel(const T *__restrict__ dvals, const int *__restrict__ idxs, T *__restrict__ dx, int rows, int cols, int k,
                                 int accumulate) {
+  pdl_entry();
   long long total = (long long)rows * k;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -311,6 +324,7 @@ __global__ void topk_bwd_kernel(const T *__restrict__ dvals, const int *__restri
 // x [outer, n, inner] -> y[o, j, :] = x[o, n-1-j, :]
 template <typename W>
 __global__ void reverse_kernel(const W *__restrict__ x, W *__restrict__ y, long long outer, long long n, long long inner) {
+  pdl_entry();
   long long total = outer * n * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -346,7 +360,7 @@ FFK_API int ffk_permute(const void *src, void *dst, int ndim, const long long *s
     for (int i = 0; i < ndim; ++i) { q.size[i] = make_cdiv((unsigned)sizes[i]); q.stride[i] = src_strides[i]; }
     const int r = by_elem_size(es, [&](auto *tag) {
       typedef typename std::remove_pointer<decltype(tag)>::type W;
-      permute32_kernel<W><<<ffk_blocks(total, 512), 256, 0, st>>>((const W *)src, (W *)dst, q, (unsigned)total, accumulate == 1, accumulate == 2);
+      ffk_launch(permute32_kernel<W>, ffk_blocks(total, 512), 256, 0, st, (const W *)src, (W *)dst, q, (unsigned)total, accumulate == 1, accumulate == 2);
       return 0;
     });
     return r ? r : (int)cudaGetLastError();
@@ -354,7 +368,7 @@ FFK_API int ffk_permute(const void *src, void *dst, int ndim, const long long *s
   int grid = ffk_blocks(total, 256);
   int r = by_elem_size(es, [&](auto *tag) {
     typedef typename std::remove_pointer<decltype(tag)>::type W;
-    permute_kernel<W><<<grid, 256, 0, st>>>((const W *)src, (W *)dst, d, total, accumulate == 1, accumulate == 2);
+    ffk_launch(permute_kernel<W>, grid, 256, 0, st, (const W *)src, (W *)dst, d, total, accumulate == 1, accumulate == 2);
     return 0;
   });
   return r ? r : (int)cudaGetLastError();
@@ -364,7 +378,7 @@ FFK_API int ffk_transpose2d(const void *src, void *dst, int batch, int rows, int
   dim3 grid((cols + 31) / 32, (rows + 31) / 32, batch), block(32, 8);
   int r = by_elem_size(es, [&](auto *tag) {
     typedef typename std::remove_pointer<decltype(tag)>::type W;
-    transpose2d_kernel<W><<<grid, block, 0, st>>>((const W *)src, (W *)dst, rows, cols);
+    ffk_launch(transpose2d_kernel<W>, grid, block, 0, st, (const W *)src, (W *)dst, rows, cols);
     return 0;
   });
   return r ? r : (int)cudaGetLastError();
@@ -379,7 +393,7 @@ FFK_API int ffk_block_copy(const void *src, long long src_ld, void *dst, long lo
                      pieces < (1ll << 31) && (!accumulate || dt == 1);
     if (vec) {
       const CopyDiv f = make_cdiv((unsigned)(bytes / 16));
-      block_copy_vec_kernel<<<ffk_blocks(pieces, 256), 256, 0, st>>>((const uint4 *)src, sp / 16, (uint4 *)dst, dp / 16, (unsigned)pieces, f,
+      ffk_launch(block_copy_vec_kernel, ffk_blocks(pieces, 256), 256, 0, st, (const uint4 *)src, sp / 16, (uint4 *)dst, dp / 16, (unsigned)pieces, f,
                                                                      accumulate);
       return (int)cudaGetLastError();
     }
@@ -395,30 +409,30 @@ FFK_API int ffk_block_copy(const void *src, long long src_ld, void *dst, long lo
     const CopyDiv f = make_cdiv((unsigned)block);
     const int r = by_elem_size(es, [&](auto *tag) {
       typedef typename std::remove_pointer<decltype(tag)>::type W;
-      block_copy32_kernel<W><<<ffk_blocks(total, 512), 256, 0, st>>>((const W *)src, src_ld, (W *)dst, dst_ld, total, f);
+      ffk_launch(block_copy32_kernel<W>, ffk_blocks(total, 512), 256, 0, st, (const W *)src, src_ld, (W *)dst, dst_ld, total, f);
       return 0;
     });
     return r ? r : (int)cudaGetLastError();
   }
   int grid = ffk_blocks(outer * block, 256);
   if (accumulate) {
-    if (dt == 0) block_copy_kernel<float><<<grid, 256, 0, st>>>((const float *)src, src_ld, (float *)dst, dst_ld, outer, block, 1);
-    else if (dt == 1) block_copy_kernel<bf16><<<grid, 256, 0, st>>>((const bf16 *)src, src_ld, (bf16 *)dst, dst_ld, outer, block, 1);
+    if (dt == 0) ffk_launch(block_copy_kernel<float>, grid, 256, 0, st, (const float *)src, src_ld, (float *)dst, dst_ld, outer, block, 1);
+    else if (dt == 1) ffk_launch(block_copy_kernel<bf16>, grid, 256, 0, st, (const bf16 *)src, src_ld, (bf16 *)dst, dst_ld, outer, block, 1);
     else return -2;
     return (int)cudaGetLastError();
   }
-  if (es == 2) block_copy_kernel<unsigned short><<<grid, 256, 0, st>>>((const unsigned short *)src, src_ld, (unsigned short *)dst, dst_ld, outer, block, 0);
-  else if (es == 4) block_copy_kernel<float><<<grid, 256, 0, st>>>((const float *)src, src_ld, (float *)dst, dst_ld, outer, block, 0);
-  else if (es == 8) block_copy_kernel<double><<<grid, 256, 0, st>>>((const double *)src, src_ld, (double *)dst, dst_ld, outer, block, 0);
-  else if (es == 1) block_copy_kernel<unsigned char><<<grid, 256, 0, st>>>((const unsigned char *)src, src_ld, (unsigned char *)dst, dst_ld, outer, block, 0);
+  if (es == 2) ffk_launch(block_copy_kernel<unsigned short>, grid, 256, 0, st, (const unsigned short *)src, src_ld, (unsigned short *)dst, dst_ld, outer, block, 0);
+  else if (es == 4) ffk_launch(block_copy_kernel<float>, grid, 256, 0, st, (const float *)src, src_ld, (float *)dst, dst_ld, outer, block, 0);
+  else if (es == 8) ffk_launch(block_copy_kernel<double>, grid, 256, 0, st, (const double *)src, src_ld, (double *)dst, dst_ld, outer, block, 0);
+  else if (es == 1) ffk_launch(block_copy_kernel<unsigned char>, grid, 256, 0, st, (const unsigned char *)src, src_ld, (unsigned char *)dst, dst_ld, outer, block, 0);
   else return -2;
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_reduce(const void *x, void *y, long long outer, long long red, long long inner, int op, int dt, cudaStream_t st) {
   if (outer * inner <= 0) return 0;
   int grid = ffk_blocks(outer * inner, 256);
-  if (dt == 0) reduce_kernel<float><<<grid, 256, 0, st>>>((const float *)x, (float *)y, outer, red, inner, op);
-  else if (dt == 1) reduce_kernel<bf16><<<grid, 256, 0, st>>>((const bf16 *)x, (bf16 *)y, outer, red, inner, op);
+  if (dt == 0) ffk_launch(reduce_kernel<float>, grid, 256, 0, st, (const float *)x, (float *)y, outer, red, inner, op);
+  else if (dt == 1) ffk_launch(reduce_kernel<bf16>, grid, 256, 0, st, (const bf16 *)x, (bf16 *)y, outer, red, inner, op);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -426,8 +440,8 @@ FFK_API int ffk_reduce_bwd(const void *dy, void *dx, long long outer, long long 
                            int accumulate, cudaStream_t st) {
   if (outer * red * inner <= 0) return 0;
   int grid = ffk_blocks(outer * red * inner, 256);
-  if (dt == 0) reduce_bwd_kernel<float><<<grid, 256, 0, st>>>((const float *)dy, (float *)dx, outer, red, inner, scale, accumulate);
-  else if (dt == 1) reduce_bwd_kernel<bf16><<<grid, 256, 0, st>>>((const bf16 *)dy, (bf16 *)dx, outer, red, inner, scale, accumulate);
+  if (dt == 0) ffk_launch(reduce_bwd_kernel<float>, grid, 256, 0, st, (const float *)dy, (float *)dx, outer, red, inner, scale, accumulate);
+  else if (dt == 1) ffk_launch(reduce_bwd_kernel<bf16>, grid, 256, 0, st, (const bf16 *)dy, (bf16 *)dx, outer, red, inner, scale, accumulate);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -437,8 +451,8 @@ FFK_API int ffk_reduce_select_bwd(const void *x, const void *y, const void *dy, 
   if (outer * red * inner <= 0) return 0;
   if (op < 2 || op > 4) return -2;
   int grid = ffk_blocks(outer * red * inner, 256);
-  if (dt == 0) reduce_select_bwd_kernel<float><<<grid, 256, 0, st>>>((const float *)x, (const float *)y, (const float *)dy, (float *)dx, outer, red, inner, op, accumulate);
-  else if (dt == 1) reduce_select_bwd_kernel<bf16><<<grid, 256, 0, st>>>((const bf16 *)x, (const bf16 *)y, (const bf16 *)dy, (bf16 *)dx, outer, red, inner, op, accumulate);
+  if (dt == 0) ffk_launch(reduce_select_bwd_kernel<float>, grid, 256, 0, st, (const float *)x, (const float *)y, (const float *)dy, (float *)dx, outer, red, inner, op, accumulate);
+  else if (dt == 1) ffk_launch(reduce_select_bwd_kernel<bf16>, grid, 256, 0, st, (const bf16 *)x, (const bf16 *)y, (const bf16 *)dy, (bf16 *)dx, outer, red, inner, op, accumulate);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -446,10 +460,10 @@ FFK_API int ffk_gather(const void *x, const void *idx, void *y, long long outer,
                        int idx_dt, cudaStream_t st) {
   if (outer * id * inner <= 0) return 0;
   int grid = ffk_blocks(outer * id * inner, 256);
-  if (es == 4 && idx_dt == 3) gather_kernel<float, long long><<<grid, 256, 0, st>>>((const float *)x, (const long long *)idx, (float *)y, outer, xd, id, inner);
-  else if (es == 4) gather_kernel<float, int><<<grid, 256, 0, st>>>((const float *)x, (const int *)idx, (float *)y, outer, xd, id, inner);
-  else if (es == 2 && idx_dt == 3) gather_kernel<unsigned short, long long><<<grid, 256, 0, st>>>((const unsigned short *)x, (const long long *)idx, (unsigned short *)y, outer, xd, id, inner);
-  else if (es == 2) gather_kernel<unsigned short, int><<<grid, 256, 0, st>>>((const unsigned short *)x, (const int *)idx, (unsigned short *)y, outer, xd, id, inner);
+  if (es == 4 && idx_dt == 3) ffk_launch(gather_kernel<float, long long>, grid, 256, 0, st, (const float *)x, (const long long *)idx, (float *)y, outer, xd, id, inner);
+  else if (es == 4) ffk_launch(gather_kernel<float, int>, grid, 256, 0, st, (const float *)x, (const int *)idx, (float *)y, outer, xd, id, inner);
+  else if (es == 2 && idx_dt == 3) ffk_launch(gather_kernel<unsigned short, long long>, grid, 256, 0, st, (const unsigned short *)x, (const long long *)idx, (unsigned short *)y, outer, xd, id, inner);
+  else if (es == 2) ffk_launch(gather_kernel<unsigned short, int>, grid, 256, 0, st, (const unsigned short *)x, (const int *)idx, (unsigned short *)y, outer, xd, id, inner);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -463,16 +477,16 @@ FFK_API int ffk_gather_bwd(const void *dy, const void *idx, void *dx, long long 
   float *dxf = dt == 0 ? (float *)dx : nullptr;
   bf16 *dxb = dt == 1 ? (bf16 *)dx : nullptr;
   if (dt != 0 && dt != 1) return -2;
-  if (idx_dt == 3) gather_bwd_kernel<long long><<<grid, 256, 0, st>>>(dyf, dyb, (const long long *)idx, dxf, dxb, outer, xd, id, inner);
-  else gather_bwd_kernel<int><<<grid, 256, 0, st>>>(dyf, dyb, (const int *)idx, dxf, dxb, outer, xd, id, inner);
+  if (idx_dt == 3) ffk_launch(gather_bwd_kernel<long long>, grid, 256, 0, st, dyf, dyb, (const long long *)idx, dxf, dxb, outer, xd, id, inner);
+  else ffk_launch(gather_bwd_kernel<int>, grid, 256, 0, st, dyf, dyb, (const int *)idx, dxf, dxb, outer, xd, id, inner);
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_topk(const void *x, void *vals, int *idxs, int rows, int cols, int k, int dt, cudaStream_t st) {
   if (rows <= 0) return 0;
   int grid = (rows + 7) / 8;
   if (grid > 148 * 8) grid = 148 * 8;
-  if (dt == 0) topk_kernel<float><<<grid, 256, 0, st>>>((const float *)x, (float *)vals, idxs, rows, cols, k);
-  else if (dt == 1) topk_kernel<bf16><<<grid, 256, 0, st>>>((const bf16 *)x, (bf16 *)vals, idxs, rows, cols, k);
+  if (dt == 0) ffk_launch(topk_kernel<float>, grid, 256, 0, st, (const float *)x, (float *)vals, idxs, rows, cols, k);
+  else if (dt == 1) ffk_launch(topk_kernel<bf16>, grid, 256, 0, st, (const bf16 *)x, (bf16 *)vals, idxs, rows, cols, k);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -480,8 +494,8 @@ FFK_API int ffk_topk(const void *x, void *vals, int *idxs, int rows, int cols, i
 FFK_API int ffk_topk_bwd(const void *dvals, const int *idxs, void *dx, int rows, int cols, int k, int dt, int accumulate, cudaStream_t st) {
   if (rows <= 0) return 0;
   int grid = ffk_blocks((long long)rows * k, 256);
-  if (dt == 0) topk_bwd_kernel<float><<<grid, 256, 0, st>>>((const float *)dvals, idxs, (float *)dx, rows, cols, k, accumulate);
-  else if (dt == 1) topk_bwd_kernel<bf16><<<grid, 256, 0, st>>>((const bf16 *)dvals, idxs, (bf16 *)dx, rows, cols, k, accumulate);
+  if (dt == 0) ffk_launch(topk_bwd_kernel<float>, grid, 256, 0, st, (const float *)dvals, idxs, (float *)dx, rows, cols, k, accumulate);
+  else if (dt == 1) ffk_launch(topk_bwd_kernel<bf16>, grid, 256, 0, st, (const bf16 *)dvals, idxs, (bf16 *)dx, rows, cols, k, accumulate);
   else return -2;
   return (int)cudaGetLastError();
 }
@@ -490,7 +504,7 @@ FFK_API int ffk_reverse(const void *x, void *y, long long outer, long long n, lo
   int grid = ffk_blocks(outer * n * inner, 256);
   int r = by_elem_size(es, [&](auto *tag) {
     typedef typename std::remove_pointer<decltype(tag)>::type W;
-    reverse_kernel<W><<<grid, 256, 0, st>>>((const W *)x, (W *)y, outer, n, inner);
+    ffk_launch(reverse_kernel<W>, grid, 256, 0, st, (const W *)x, (W *)y, outer, n, inner);
     return 0;
   });
   return r ? r : (int)cudaGetLastError();
