@@ -78,3 +78,66 @@ def test_thin_products(M, N, Kd, dt):
                        bias=bias.data_ptr(), act=K.ACT_CODES["relu"], accumulate=True)
             want = torch.relu(ref + bias.double()) + old.double()
             assert ((C.double() - want).abs() <= tol(want)).all(), (a_mn, b_mn, (C.double() - want).abs().max().item())
+
+
+@pytest.mark.parametrize("cols", [256, 512, 768, 1024, 1280])
+@pytest.mark.parametrize("rows", [63, 64, 65, 2401])
+@pytest.mark.parametrize("acc", [False, True])
+def test_layernorm_backward_rows(rows, cols, acc):
+    """Row counts around the blocks of the one-warp-per-row kernel (1280 columns take the block-per-row one)."""
+    x, dy, g = _randn(rows, cols), _randn(rows, cols, seed=1), _randn(cols, seed=2)
+    mean, rstd, y = torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda"), torch.empty_like(x)
+    K.layernorm_fwd(x, g, g, 1e-5, out=y, mean=mean, rstd=rstd)
+    old, old2 = _randn(rows, cols, seed=3), _randn(rows, cols, seed=4)
+    dx, dx2, dg, db = old.clone(), old2.clone(), _randn(cols, seed=5), _randn(cols, seed=6)
+    og, ob = dg.clone(), db.clone()
+    K.layernorm_bwd(dy, x, g, mean, rstd, dx, dg, db, torch.empty(K.layernorm_bwd_scratch(rows, cols), device="cuda"), accumulate_dx=acc,
+                    accumulate_params=acc, dx2=dx2, accumulate_dx2=not acc)
+    xd = x.double().requires_grad_(True)
+    gd, bd = g.double().requires_grad_(True), g.double().requires_grad_(True)
+    torch.nn.functional.layer_norm(xd, (cols,), gd, bd, 1e-5).backward(dy.double())
+
+    def near(got, want, slack):
+        assert ((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + slack).all(), (got.double() - want).abs().max().item()
+
+    # fp32 statistics and row sums against fp64: a few ulps of values of order |dy| * |gamma| * rstd
+    near(dx, xd.grad + (old.double() if acc else 0), 1e-4)
+    near(dx2, xd.grad + (0 if acc else old2.double()), 1e-4)
+    sums = rows * 2.0 ** -24 * 16
+    near(dg, gd.grad + (og.double() if acc else 0), sums * rows ** 0.5 + 1e-3)
+    near(db, bd.grad + (ob.double() if acc else 0), sums * rows ** 0.5 + 1e-3)
+
+
+@pytest.mark.parametrize("dim", [8, 64, 2048, 12])
+@pytest.mark.parametrize("bag,aggr", [(1, "sum"), (3, "sum"), (4, "avg")])
+@pytest.mark.parametrize("table_dt,out_dt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16), (torch.float32, torch.float32)])
+@pytest.mark.parametrize("idx_dt", [torch.int32, torch.int64])
+def test_embedding_pieces(dim, bag, aggr, table_dt, out_dt, idx_dt):
+    """Lookup, scatter and sparse step in 16-byte pieces (12 columns: element by element); indexes out of range count as nothing."""
+    tokens, entries = 301, 1000
+    table = _randn(entries, dim, dtype=torch.float32).to(table_dt)
+    idx = torch.randperm(tokens * bag + 50, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))[:tokens * bag] % (entries + 1)
+    idx = torch.where(idx == entries, -1, idx).to(idx_dt).view(tokens, bag)
+    if bag > 1:
+        out = torch.empty(tokens, dim, device="cuda", dtype=out_dt)
+    else:
+        out = torch.empty(tokens, 1, dim, device="cuda", dtype=out_dt).view(tokens, dim)
+    K.embedding_fwd(idx, table, out, aggr=aggr)
+    ok = (idx >= 0).double()[..., None]
+    rows = table.double()[idx.long().clamp(min=0)] * ok
+    want = rows.sum(1) / (bag if aggr == "avg" else 1)
+    ulp = lambda dt: 2.0 ** -8 if dt == torch.bfloat16 else 2.0 ** -22  # noqa: E731
+    assert ((out.double() - want).abs() <= want.abs() * ulp(out_dt) + rows.abs().sum(1) * 2.0 ** -22).all()
+    dout = _randn(tokens, dim, dtype=torch.float32, seed=2).to(out_dt)
+    dt = torch.zeros_like(table)
+    K.embedding_bwd(idx, dout, dt, aggr=aggr)
+    ref = torch.zeros(entries, dim, device="cuda", dtype=torch.float64)
+    mag = torch.zeros_like(ref)
+    g = (dout.double() / (bag if aggr == "avg" else 1))[:, None].expand(-1, bag, -1) * ok
+    ref.index_put_((idx.long().clamp(min=0).view(-1),), g.reshape(-1, dim), accumulate=True)
+    mag.index_put_((idx.long().clamp(min=0).view(-1),), g.abs().reshape(-1, dim), accumulate=True)
+    assert ((dt.double() - ref).abs() <= mag * 4 * ulp(table_dt)).all()  # at most a few additions per row, one rounding each
+    if table_dt == torch.float32:
+        t2 = table.clone()
+        K.embedding_sgd(idx, dout, t2, 0.5, aggr=aggr)
+        assert ((t2.double() - (table.double() - 0.5 * ref)).abs() <= (mag + table.double().abs()) * 2.0 ** -20).all()
