@@ -469,7 +469,13 @@ static int ln_bwd_grid(int rows, int cols, bool vec) {
   const int g = 148 * per_sm;
   return rows < g ? rows : g;
 }
-// floats of scratch needed by ffk_layernorm_bwd (the larger of the two kernel forms' needs)
+// The one-warp-per-row backward kernel takes rows of 256, 512, 768 or 1024; from 64 rows on its blocks of 8 warps are filled.
+static bool ln_bwd_warp_ok(int rows, int cols) { return cols % 256 == 0 && cols <= 1024 && rows >= 64; }
+static int ln_bwd_warp_grid(int rows, int cols) {
+  const int most = cols <= 512 ? 148 * 2 : 148, want = (rows + 7) / 8;
+  return want < most ? want : most;
+}
+// floats of scratch needed by ffk_layernorm_bwd (the larger of the kernel forms' needs)
 FFK_API long long ffk_layernorm_bwd_scratch(int rows, int cols) {
   const int a = ln_bwd_grid(rows, cols, true), b = ln_bwd_grid(rows, cols, false);
   return 2ll * (a > b ? a : b) * cols;
@@ -488,7 +494,19 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
   if (vec) {
     int vpt = ln_vpt(cols), threads = cols / 8 / vpt;
     const bf16 *DY = (const bf16 *)dy, *X = (const bf16 *)x, *G = (const bf16 *)gamma;
-    if (vpt == 1) ffk_launch(vec::layernorm_bwd_vec_kernel<1>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
+    if (ln_bwd_warp_ok(rows, cols)) {
+      grid = ln_bwd_warp_grid(rows, cols);
+#define LN_BWD(V)                                                                                                                            \
+  ffk_launch(vec::layernorm_bwd_warp_kernel<V>, grid, 256, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, accumulate_dx, \
+             accumulate_dx2)
+      switch (cols / 256) {
+        case 1: LN_BWD(1); break;
+        case 2: LN_BWD(2); break;
+        case 3: LN_BWD(3); break;
+        default: LN_BWD(4); break;
+      }
+#undef LN_BWD
+    } else if (vpt == 1) ffk_launch(vec::layernorm_bwd_vec_kernel<1>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     else if (vpt == 2) ffk_launch(vec::layernorm_bwd_vec_kernel<2>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     else ffk_launch(vec::layernorm_bwd_vec_kernel<4>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     if (part)
