@@ -256,3 +256,29 @@ def test_batchnorm_relu_mask_from_x(rows, cols, affine):
         out.append((dx, dg, db))
     for a, b in zip(*out):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("mode,s,p", [("avg", 1, 1), ("max", 2, 0), ("max", 2, 1)])
+@pytest.mark.parametrize("h,w", [(3, 3), (4, 6), (7, 5), (8, 12), (17, 13)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_pool_3x3(mode, s, p, h, w, accumulate):
+    """The 3 x 3 kernels of the channels-last path at widths on both sides of a run, borders included."""
+    n, c = 2, 24
+    gen = torch.Generator(device="cuda").manual_seed(h * 100 + w)
+    x = torch.randn(n, h, w, c, device="cuda", generator=gen).bfloat16()
+    g = K.ConvGeometry(n, c, h, w, 3, 3, s, s, p, p, K.nhwc_strides(n, c, h, w), kp=0)
+    y = torch.empty(n, g.oh, g.ow, c, device="cuda", dtype=torch.bfloat16)
+    arg = torch.empty(y.numel(), device="cuda", dtype=torch.uint8) if mode == "max" else None
+    K.pool2d_fwd(x, y, arg, g, mode)
+    # (a contiguous oracle: torch's channels-last average-pool backward is wrong at the borders without count_include_pad)
+    xr = x.double().permute(0, 3, 1, 2).contiguous().requires_grad_(True)
+    yr = F.max_pool2d(xr, 3, s, p) if mode == "max" else F.avg_pool2d(xr, 3, s, p, count_include_pad=False)
+    ref = yr.permute(0, 2, 3, 1)
+    assert ((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 9 * 2.0 ** -22).all()  # nine fp32 terms, one rounding
+    dy = torch.randn(y.shape, device="cuda", generator=gen).bfloat16()
+    old = torch.randn(x.shape, device="cuda", generator=gen).bfloat16()
+    dx = old.clone()
+    K.pool2d_bwd(dy.view(-1), arg, dx, g, mode, accumulate=accumulate)
+    yr.backward(dy.double().permute(0, 3, 1, 2).contiguous())
+    want = xr.grad.permute(0, 2, 3, 1) + (old.double() if accumulate else 0)
+    assert ((dx.double() - want).abs() <= want.abs() * 2.0 ** -8 + 9 * 2.0 ** -21).all()
