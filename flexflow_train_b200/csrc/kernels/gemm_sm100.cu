@@ -133,7 +133,10 @@ struct GemmCfg {
   // 1024 B apart (SBO) and the next MN chunk starts BK*128 B later (LBO).
   static constexpr uint32_t A_LBO = A_MN ? BK * 128 : 16;
   static constexpr uint32_t B_LBO = B_MN ? BK * 128 : 16;
-  static constexpr uint32_t SBO = 1024;
+  // 32-bit elements transposed by the MMA swizzle in 32-byte atoms, whose pattern repeats every 4 rows of 128 bytes: groups of
+  // 4 k-rows are 512 B apart.
+  static constexpr uint32_t A_SBO = ES == 4 && A_MN ? 512 : 1024, B_SBO = ES == 4 && B_MN ? 512 : 1024;
+  static constexpr uint32_t A_TYPE = ES == 4 && A_MN ? 1 : 2, B_TYPE = ES == 4 && B_MN ? 1 : 2;
   static constexpr uint32_t A_KADV = A_MN ? UMMA_K * 128 : UMMA_K * ES;  // bytes per UMMA k-step
   static constexpr uint32_t B_KADV = B_MN ? UMMA_K * 128 : UMMA_K * ES;
   static constexpr uint32_t IDESC = (1u << 4)                                  // D = f32
@@ -415,8 +418,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
           tc_fence_after();
           uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES);
           uint32_t sb = sa + Cfg::A_BYTES;
-          uint64_t adesc = make_smem_desc(sa, Cfg::A_LBO, Cfg::SBO);
-          uint64_t bdesc = make_smem_desc(sb, Cfg::B_LBO, Cfg::SBO);
+          uint64_t adesc = make_smem_desc(sa, Cfg::A_LBO, Cfg::A_SBO, Cfg::A_TYPE);
+          uint64_t bdesc = make_smem_desc(sb, Cfg::B_LBO, Cfg::B_SBO, Cfg::B_TYPE);
           if (leader) {
 #pragma unroll
             for (int k = 0; k < Cfg::BK / Cfg::UMMA_K; ++k) {
@@ -822,7 +825,7 @@ gemm_cluster_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_cons
         if (!ok) break;
         tc_fence_after();
         const uint32_t sa = smem_u32(tiles + stage * Cfg::STAGE_BYTES), sb = sa + Cfg::A_BYTES;
-        const uint64_t adesc = make_smem_desc(sa, Cfg::A_LBO, Cfg::SBO), bdesc = make_smem_desc(sb, Cfg::B_LBO, Cfg::SBO);
+        const uint64_t adesc = make_smem_desc(sa, Cfg::A_LBO, Cfg::A_SBO, Cfg::A_TYPE), bdesc = make_smem_desc(sb, Cfg::B_LBO, Cfg::B_SBO, Cfg::B_TYPE);
         if (leader) {
 #pragma unroll
           for (int k = 0; k < Cfg::BK / Cfg::UMMA_K; ++k)
@@ -1187,7 +1190,7 @@ __global__ void __launch_bounds__(SB_WARPS * 32) gemm_small_batched_kernel(SimtO
 // K-major operand: contiguous = k, rows = m|n, box {128/ES, box_rows}.
 // MN-major operand: contiguous = m|n, rows = k, box {128/ES, BK}.
 int make_operand_map(CUtensorMap *map, const void *ptr, int es, long long contiguous, long long rows, long long ld,
-                     int nh, long long sh, int nb, long long sb, int box_rows) {
+                     int nh, long long sh, int nb, long long sb, int box_rows, bool mn = false) {
   EncodeTiledFn enc = get_encode_fn();
   if (!enc) return -1;
   cuuint64_t dims[4] = {(cuuint64_t)contiguous, (cuuint64_t)rows, (cuuint64_t)nh, (cuuint64_t)nb};
@@ -1199,7 +1202,8 @@ int make_operand_map(CUtensorMap *map, const void *ptr, int es, long long contig
   cuuint32_t box[4] = {(cuuint32_t)(128 / es), (cuuint32_t)box_rows, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult r = enc(map, es == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (void *)ptr,
-                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   es == 4 && mn ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
@@ -1355,7 +1359,12 @@ int launch_cluster(const CUtensorMap &ta, const CUtensorMap &tb, GemmArgs &args,
 template <int BN>
 int launch_cluster_major(int es, bool a_mn, bool b_mn, const CUtensorMap &ta, const CUtensorMap &tb, GemmArgs &args, int split,
                          cudaStream_t stream) {
-  if (es == 4) return launch_cluster<4, BN, false, false>(ta, tb, args, split, stream);
+  if (es == 4) {
+    if (!a_mn && !b_mn) return launch_cluster<4, BN, false, false>(ta, tb, args, split, stream);
+    if (!a_mn && b_mn) return launch_cluster<4, BN, false, true>(ta, tb, args, split, stream);
+    if (a_mn && !b_mn) return launch_cluster<4, BN, true, false>(ta, tb, args, split, stream);
+    return launch_cluster<4, BN, true, true>(ta, tb, args, split, stream);
+  }
   if (!a_mn && !b_mn) return launch_cluster<2, BN, false, false>(ta, tb, args, split, stream);
   if (!a_mn && b_mn) return launch_cluster<2, BN, false, true>(ta, tb, args, split, stream);
   if (a_mn && !b_mn) return launch_cluster<2, BN, true, false>(ta, tb, args, split, stream);
@@ -1420,6 +1429,8 @@ struct FfkGemmDesc {
   const void *drop_seed_ptr;
   // cluster kernel: CTAs that share a tile's K range (2, 4 or 8; with bn 64 or 128); 0 = choose, -1 = persistent kernel
   int split;
+  // MN-major fp32 operands: 1 = tf32 on the tensor cores like K-major ones, 0 = fp32 products in the general kernel
+  int tf32_mn;
 };
 
 static int g_pair_mode = 1;  // 1: CTA pairs where they apply, 0: never
@@ -1496,7 +1507,7 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
   if (d->M <= 0 || d->N <= 0 || d->K <= 0) return 0;
   bool tma_ok = !(((uintptr_t)d->A & 15) || ((uintptr_t)d->B & 15)) && !((d->lda * es) % 16 || (d->ldb * es) % 16) &&
                 !((d->nh > 1 && ((d->a_sh * es) % 16 || (d->b_sh * es) % 16)) || (d->nb > 1 && ((d->a_sb * es) % 16 || (d->b_sb * es) % 16))) &&
-                !(es == 4 && (d->a_mn || d->b_mn));  // tf32 operands must be K-major
+                !(es == 4 && (d->a_mn || d->b_mn) && !d->tf32_mn);
   const bool fused = d->scatter_rows || d->gate_flags || d->push_src || d->drop_p > 0.f;
   // many small problems: one warp each on the CUDA cores beats one mostly empty 128-row tensor-core tile each
   const long long nbatch = (long long)(d->nh < 1 ? 1 : d->nh) * (d->nb < 1 ? 1 : d->nb);
@@ -1581,10 +1592,10 @@ FFK_API int ffk_gemm(const FfkGemmDesc *d, cudaStream_t stream) {
   CUtensorMap ta, tb;
   int r;
   if (!d->a_mn) r = make_operand_map(&ta, d->A, es, d->K, d->M, d->lda, d->nh, d->a_sh, d->nb, d->a_sb, BM);
-  else r = make_operand_map(&ta, d->A, es, d->M, d->K, d->lda, d->nh, d->a_sh, d->nb, d->a_sb, BK);
+  else r = make_operand_map(&ta, d->A, es, d->M, d->K, d->lda, d->nh, d->a_sh, d->nb, d->a_sb, BK, true);
   if (r) return r;
   if (!d->b_mn) r = make_operand_map(&tb, d->B, es, d->K, d->N, d->ldb, d->nh, d->b_sh, d->nb, d->b_sb, pair ? bn / 2 : bn);
-  else r = make_operand_map(&tb, d->B, es, d->N, d->K, d->ldb, d->nh, d->b_sh, d->nb, d->b_sb, BK);
+  else r = make_operand_map(&tb, d->B, es, d->N, d->K, d->ldb, d->nh, d->b_sh, d->nb, d->b_sb, BK, true);
   if (r) return r;
 
   GemmArgs a;

@@ -60,7 +60,7 @@ class GemmDesc(ctypes.Structure):
         ("push_flag", c_void_p * 8), ("push_sync", c_void_p), ("push_world", c_int), ("push_rank", c_int),
         # dropout applied by the epilogue after the activation
         ("drop_p", c_float), ("drop_salt", c_ulonglong), ("drop_seed_ptr", c_void_p),
-        ("split", c_int),
+        ("split", c_int), ("tf32_mn", c_int),
     ]
 
 
@@ -242,13 +242,14 @@ def gemm_raw(*, M, N, K, A, lda, B, ldb, C, ldc, a_mn=False, b_mn=False, es=2, n
              a_sh=0, a_sb=0, b_sh=0, b_sb=0, c_sh=0, c_sb=0, C2=None, bias=None, addend=None,
              ld_add=0, add_sh=0, add_sb=0, alpha=1.0, act=0, out_fp32=False, accumulate=False,
              bn=0, max_ctas=0, scatter=None, scatter_rows=0, scatter_src=0, gate_flags=None, gate_sync=None,
-             gate_rows=0, mb_rotate=0, push=None, dropout=None, split=0):
+             gate_rows=0, mb_rotate=0, push=None, dropout=None, split=0, tf32_mn=False):
     """D = epilogue(alpha * A[M,K] . B[N,K]^T) on raw pointers; see gemm_sm100.cu.
 
     scatter / scatter_rows / scatter_src: write each output tile into the owning rank's staging buffer
     (GEMM -> reduce-scatter).  gate_flags / gate_sync / gate_rows / mb_rotate: wait for pushed row blocks of A
     (all-gather -> GEMM).  bn / split: tile width and, for the cluster kernel, the CTAs that share a tile's K range (0: chosen by
-    size, split -1: the persistent kernel)."""
+    size, split -1: the persistent kernel).  tf32_mn: fp32 operands that are MN-major run as tf32 on the tensor cores, as K-major ones
+    do; without it they are multiplied in fp32 by the general kernel."""
     plain = not scatter and gate_flags is None and push is None and dropout is None
     # (batches of small problems have a kernel of their own that reads any layout: same condition as in ffk_gemm)
     small_batched = max(nh, 1) * max(nb, 1) >= 32 and M * N <= 1024 and (M + N) * (K + 1) <= 2304
@@ -266,7 +267,7 @@ def gemm_raw(*, M, N, K, A, lda, B, ldb, C, ldc, a_mn=False, b_mn=False, es=2, n
                  C, ldc, c_sh, c_sb, C2, bias, addend, ld_add, add_sh, add_sb, alpha, act, int(out_fp32),
                  int(accumulate), bn, max_ctas, sc, scatter_rows, scatter_src, gate_flags, gate_sync, gate_rows,
                  mb_rotate)
-    d.split = split
+    d.split, d.tf32_mn = split, int(tf32_mn)
     if dropout is not None:  # (p, salt, seed tensor or None)
         d.drop_p, d.drop_salt = float(dropout[0]), int(dropout[1]) & (2**64 - 1)
         d.drop_seed_ptr = None if dropout[2] is None else dropout[2].data_ptr()
@@ -399,17 +400,20 @@ def matmul_nt(a, b, out=None, *, bias=None, act=None, addend=None, pre_act_out=N
     return out
 
 
+def _tf32_mn(M, N, K) -> bool:
+    """Whether an fp32 product with MN-major operands runs as tf32: where it did by way of transposed copies, whose pitch is K (small
+    products at an odd K stay fp32)."""
+    return K % 4 == 0 or 2.0 * M * N * K >= _REPACK_MIN_FLOPS
+
+
 def matmul_nn(a, b, out=None, *, alpha=1.0, accumulate=False, out_dtype=None, bn=0):
     """out[M,N] = a[M,K] @ b[K,N].  Linear dgrad (a = dY, b = W[out,in])."""
     M, K = a.shape
     N = b.shape[1]
     out = _gemm_out(out, M, N, a, out_dtype)
     _cuda_contig(a, b, out)
-    if a.dtype == torch.float32:
-        # fp32 storage runs on the tf32 path, whose operands must be K-major: transpose b once
-        return matmul_nt(a, transpose2d(b), out=out, alpha=alpha, accumulate=accumulate, bn=bn)
     gemm_raw(M=M, N=N, K=K, A=a.data_ptr(), lda=K, B=b.data_ptr(), ldb=N, b_mn=True, C=out.data_ptr(), ldc=N,
-             es=_es(a), alpha=alpha, out_fp32=out.dtype == torch.float32, accumulate=accumulate, bn=bn)
+             es=_es(a), alpha=alpha, out_fp32=out.dtype == torch.float32, accumulate=accumulate, bn=bn, tf32_mn=_tf32_mn(M, N, K))
     return out
 
 
@@ -419,11 +423,9 @@ def matmul_tn(a, b, out=None, *, alpha=1.0, accumulate=False, out_dtype=None, bn
     N = b.shape[1]
     out = _gemm_out(out, M, N, a, out_dtype)
     _cuda_contig(a, b, out)
-    if a.dtype == torch.float32:
-        return matmul_nt(transpose2d(a), transpose2d(b), out=out, alpha=alpha, accumulate=accumulate, bn=bn)
     gemm_raw(M=M, N=N, K=K, A=a.data_ptr(), lda=M, a_mn=True, B=b.data_ptr(), ldb=N, b_mn=True,
              C=out.data_ptr(), ldc=N, es=_es(a), alpha=alpha, out_fp32=out.dtype == torch.float32,
-             accumulate=accumulate, bn=bn)
+             accumulate=accumulate, bn=bn, tf32_mn=_tf32_mn(M, N, K))
     return out
 
 

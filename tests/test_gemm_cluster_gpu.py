@@ -86,3 +86,22 @@ def test_chosen_kernel(M, N, Kd, accumulate):
     _run(a, b, M, N, Kd, False, True, C, ldc=N, accumulate=accumulate)
     _close(C, ref[0] + (old.double() if accumulate else 0), Kd, torch.bfloat16)
     assert K.gemm_last_error() == 0
+
+
+@pytest.mark.parametrize("M,N,Kd", [(4, 8, 4), (64, 96, 36), (128, 64, 512), (130, 132, 200), (300, 260, 1000), (2048, 512, 4096), (512, 512, 37), (20, 24, 7)])
+def test_fp32_transposed_operands(M, N, Kd):
+    """tf32 products that read their operands as they lie give what they give on transposed copies."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + Kd)
+    a, b = torch.randn(M, Kd, generator=g, device="cuda"), torch.randn(N, Kd, generator=g, device="cuda")
+    ref = a.double() @ b.double().t()
+    at, bt = a.t().contiguous(), b.t().contiguous()
+    for got in (K.matmul_nt(a, b), K.matmul_nn(a, bt), K.matmul_tn(at, bt)):
+        # operands cut to 11 bits (2^-10 relative each), errors of random sign: far below Kd^0.5 * 6 of them
+        assert (got.double() - ref).abs().max() <= 6 * Kd ** 0.5 * 2.0 ** -9
+    old = torch.randn(M, N, generator=g, device="cuda")
+    c = old.clone()
+    K.matmul_tn(at, bt, out=c, accumulate=True)
+    assert (c.double() - old.double() - ref).abs().max() <= 6 * Kd ** 0.5 * 2.0 ** -9
+    if Kd % 4:  # small or repacked: no further from fp64 than the transposed copies were
+        assert (K.matmul_tn(at, bt).double() - ref).norm() <= 1.01 * (K.matmul_nt(a, b).double() - ref).norm() + 1e-6
+    assert K.gemm_last_error() == 0
