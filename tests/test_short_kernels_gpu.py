@@ -141,3 +141,36 @@ def test_embedding_pieces(dim, bag, aggr, table_dt, out_dt, idx_dt):
         t2 = table.clone()
         K.embedding_sgd(idx, dout, t2, 0.5, aggr=aggr)
         assert ((t2.double() - (table.double() - 0.5 * ref)).abs() <= (mag + table.double().abs()) * 2.0 ** -20).all()
+
+
+@pytest.mark.parametrize("cols", [256, 512, 768, 1024, 1280])
+@pytest.mark.parametrize("rows", [7, 64, 1201])
+def test_layernorm_fp32_rows(rows, cols):
+    x, r, dy, g, b = (_randn(*s, dtype=torch.float32, seed=i) for i, s in enumerate([(rows, cols), (rows, cols), (rows, cols), (cols,), (cols,)]))
+    mean, rstd, y, xsum = torch.empty(rows, device="cuda"), torch.empty(rows, device="cuda"), torch.empty_like(x), torch.empty_like(x)
+    K.layernorm_fwd(x, g, b, 1e-5, residual=r, xsum=xsum, out=y, mean=mean, rstd=rstd)
+    assert torch.equal(xsum, x + r)
+    xd, gd, bd = xsum.double().requires_grad_(True), g.double().requires_grad_(True), b.double().requires_grad_(True)
+    ref = torch.nn.functional.layer_norm(xd, (cols,), gd, bd, 1e-5)
+    # fp32 row sums of `cols` terms of order one, combined in a tree of depth log2(cols) + 8
+    eps = 2.0 ** -24 * 32
+    assert (y.double() - ref).abs().max() <= 8 * eps * ref.abs().max()
+    ref.backward(dy.double())
+    dx, dg, db = torch.empty_like(x), torch.empty_like(g), torch.empty_like(b)
+    K.layernorm_bwd(dy, xsum, g, mean, rstd, dx, dg, db, torch.empty(K.layernorm_bwd_scratch(rows, cols), device="cuda"))
+    assert (dx.double() - xd.grad).abs().max() <= 8 * eps * xd.grad.abs().max()
+    for got, want in ((dg, gd.grad), (db, bd.grad)):
+        assert (got.double() - want).abs().max() <= 8 * eps * max(want.abs().max().item(), rows ** 0.5)
+
+
+@pytest.mark.parametrize("M,N,Kd", [(9, 9, 64), (9, 64, 9), (64, 9, 9), (1, 1, 5), (5, 33, 20)])
+@pytest.mark.parametrize("out_dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_small_batched_products(M, N, Kd, out_dt, accumulate):
+    a, b, old = _randn(70, M, Kd), _randn(70, N, Kd, seed=1), _randn(70, M, N, dtype=torch.float32, seed=2).to(out_dt)
+    C = old.clone()
+    K.gemm_raw(M=M, N=N, K=Kd, A=a.data_ptr(), lda=Kd, a_sb=M * Kd, B=b.data_ptr(), ldb=Kd, b_sb=N * Kd, C=C.data_ptr(), ldc=N, c_sb=M * N,
+               nb=70, alpha=0.5, out_fp32=out_dt == torch.float32, accumulate=accumulate)
+    want = 0.5 * (a.double() @ b.double().transpose(1, 2)) + (old.double() if accumulate else 0)
+    ulp = 2.0 ** -8 if out_dt == torch.bfloat16 else 0
+    assert ((C.double() - want).abs() <= want.abs() * ulp + Kd * 2.0 ** -20).all()  # fp32 sums of Kd terms, one rounding
