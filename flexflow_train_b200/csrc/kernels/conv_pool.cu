@@ -886,6 +886,7 @@ FFK_API int ffk_im2col(const void *x, void *col, const int *geom, const long lon
   ConvGeom g = make_geom(geom, strides);
   long long rows = (long long)g.N * g.OH * g.OW;
   if (rows <= 0) return 0;
+  FfkTraffic traffic((rows * g.Kp + (long long)g.N * g.H * g.W * g.C) * 2);
   int K = g.KH * g.KW * g.C;
   if (g.Kp < K || (g.Kp % 8) != 0) return -2;
   if (dt == 1 && vec_ok(g, x) && g.Kp == K) {
@@ -904,6 +905,7 @@ FFK_API int ffk_col2im(const void *dcol, void *dx, const int *geom, const long l
   ConvGeom g = make_geom(geom, strides);
   long long total = (long long)g.N * g.H * g.W * g.C;
   if (total <= 0) return 0;
+  FfkTraffic traffic(((long long)g.N * g.OH * g.OW * g.Kp + total) * 2);
   if (dt == 1 && vec_ok(g, dx)) {
     long long tv = total / 8;
     ffk_launch(col2im_vec_kernel, ffk_blocks(tv, 256), 256, 0, st, (const bf16 *)dcol, (bf16 *)dx, g, tv, accumulate);
@@ -940,6 +942,7 @@ FFK_API int ffk_pool2d_fwd(const void *x, void *y, void *arg, const int *geom, c
   ConvGeom g = make_geom(geom, strides);
   long long total = (long long)g.N * g.OH * g.OW * g.C;
   if (total <= 0) return 0;
+  FfkTraffic traffic((total + (long long)g.N * g.H * g.W * g.C) * (dt == 1 ? 2 : 4));
   if (g.KH * g.KW > 255) return -2;
   if (dt == 1 && vec_ok(g, x) && ((uintptr_t)y % 16) == 0 && ((uintptr_t)arg % 8) == 0) {
     long long tv = total / 8;
@@ -963,6 +966,7 @@ FFK_API int ffk_pool2d_bwd(const void *dy, const void *arg, void *dx, const int 
   ConvGeom g = make_geom(geom, strides);
   long long total = (long long)g.N * g.H * g.W * g.C;
   if (total <= 0) return 0;
+  FfkTraffic traffic((total + (long long)g.N * g.OH * g.OW * g.C) * (dt == 1 ? 2 : 4));
   if (mode == 0 && !arg) return -2;
   if (dt == 1 && vec_ok(g, dx) && ((uintptr_t)dy % 16) == 0 && ((uintptr_t)arg % 8) == 0) {
     long long tv = total / 8;
@@ -1026,6 +1030,7 @@ FFK_API long long ffk_batchnorm_scratch(long long R, int C) {
 FFK_API int ffk_batchnorm_fwd(const void *x, void *y, const void *gamma, const void *beta, float *mean, float *rstd, float *scratch,
                               long long R, int C, float eps, int relu, int dt, cudaStream_t st) {
   if (R <= 0 || C <= 0) return 0;
+  FfkTraffic traffic(R * C * (dt == 1 ? 2 : 4) * 2);
   int rpc;
   int chunks = bn_chunks(R, C, &rpc);
   dim3 grid((C + BN_TX - 1) / BN_TX, chunks), block(BN_TX, BN_TY);
@@ -1067,6 +1072,7 @@ FFK_API int ffk_batchnorm_bwd(const void *dy, const void *x, const void *relu_y,
                               const float *mean, const float *rstd, void *dx, void *dgamma, void *dbeta, float *scratch, long long R, int C,
                               int dt, int accumulate_dx, int accumulate_gamma, int accumulate_beta, cudaStream_t st) {
   if (R <= 0 || C <= 0) return 0;
+  FfkTraffic traffic(R * C * (dt == 1 ? 2 : 4) * 3);
   int rpc;
   int chunks = bn_chunks(R, C, &rpc);
   dim3 grid((C + BN_TX - 1) / BN_TX, chunks), block(BN_TX, BN_TY);

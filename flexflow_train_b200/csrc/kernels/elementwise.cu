@@ -367,12 +367,14 @@ __global__ void colsum_finish_kernel(const float *__restrict__ partial, int npar
 
 FFK_API int ffk_unary_fwd(int op, const void *x, void *y, long long n, float s, int dt, cudaStream_t st) {
   if (n <= 0) return 0;
+  FfkTraffic traffic(n * (dt == DT_BF16 ? 2 : 4) * 2);
   DISPATCH_FLOAT(dt, (ffk_launch(unary_fwd_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, op, (const T *)x, (T *)y, n, s)));
   return (int)cudaGetLastError();
 }
 FFK_API int ffk_unary_bwd(int op, const void *x, const void *y, const void *dy, void *dx, long long n, float s, int dt,
                           int accumulate, cudaStream_t st) {
   if (n <= 0) return 0;
+  FfkTraffic traffic(n * (dt == DT_BF16 ? 2 : 4) * 3);
   DISPATCH_FLOAT(dt, (ffk_launch(unary_bwd_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, 
                          op, (const T *)x, (const T *)y, (const T *)dy, (T *)dx, n, s, accumulate)));
   return (int)cudaGetLastError();
@@ -396,6 +398,7 @@ FFK_API int ffk_binary_bwd(int op, const void *a, const void *b, const void *dy,
 FFK_API int ffk_dropout(const void *x, const void *r, void *y, long long n, float p, unsigned long long seed,
                         const unsigned long long *seed_ptr, int dt, cudaStream_t st) {
   if (n <= 0) return 0;
+  FfkTraffic traffic(n * (dt == DT_BF16 ? 2 : 4) * 2);
   float scale = p < 1.f ? 1.f / (1.f - p) : 0.f;
   DISPATCH_FLOAT(dt, (ffk_launch(dropout_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, 
                          (const T *)x, (const T *)r, (T *)y, n, p, scale, seed, seed_ptr)));
@@ -404,6 +407,7 @@ FFK_API int ffk_dropout(const void *x, const void *r, void *y, long long n, floa
 // y = a*x + b*y
 FFK_API int ffk_axpby(const void *x, void *y, long long n, float a, float b, int dt, cudaStream_t st) {
   if (n <= 0) return 0;
+  FfkTraffic traffic(n * (dt == DT_BF16 ? 2 : 4) * 3);
   DISPATCH_FLOAT(dt, (ffk_launch(axpby_kernel<T>, ffk_blocks(n / V16<T>::N + 1, 256), 256, 0, st, (const T *)x, (T *)y, n, a, b)));
   return (int)cudaGetLastError();
 }
@@ -414,6 +418,7 @@ FFK_API int ffk_fill(void *y, long long n, float v, int dt, cudaStream_t st) {
 }
 FFK_API int ffk_cast(const void *src, int sdt, void *dst, int ddt, long long n, int accumulate, cudaStream_t st) {
   if (n <= 0) return 0;
+  FfkTraffic traffic(n * 6);
   if (sdt == DT_F32 && ddt == DT_BF16 && !accumulate && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0)
     ffk_launch(cast_f32_bf16_kernel, ffk_blocks(n / 8 + 1, 256), 256, 0, st, (const float *)src, (bf16 *)dst, n);
   else if (sdt == DT_BF16 && ddt == DT_F32 && (((uintptr_t)src | (uintptr_t)dst) & 15) == 0)
@@ -443,11 +448,13 @@ FFK_API long long ffk_bias_act_bwd_scratch(int rows, int cols) { return (long lo
 static int bias_act_bwd_impl(const void *dy, const void *saved, void *dz, void *dbias, float *partial, int rows, int cols, int act, int dt,
                              int accumulate, float drop_p, unsigned long long drop_salt, const void *drop_seed_ptr, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * (dt == DT_BF16 ? 2 : 4) * (1 + (act != ACT_NONE) + (dz != nullptr)));
   const int gy = bias_act_row_chunks(rows, cols);
   if (dt == DT_BF16 && cols % 8 == 0 && (((uintptr_t)dy | (uintptr_t)saved | (uintptr_t)dz) & 15) == 0) {
     dim3 vgrid((cols + 255) / 256, gy), vblock(32, 8);
     ffk_launch(vec::bias_act_bwd_vec_kernel, vgrid, vblock, 0, st, (const bf16 *)dy, (const bf16 *)saved, (bf16 *)dz, dbias ? partial : nullptr, rows,
                                                           cols, act, drop_p, drop_salt, (const unsigned long long *)drop_seed_ptr);
+    traffic.done();
     if (dbias) ffk_launch(vec::fold_partials_kernel<bf16>, (cols + 31) / 32, dim3(32, 32), 0, st, partial, gy, cols, (bf16 *)dbias, (bf16 *)nullptr, accumulate);
     return (int)cudaGetLastError();
   }
@@ -456,6 +463,7 @@ static int bias_act_bwd_impl(const void *dy, const void *saved, void *dz, void *
   DISPATCH_FLOAT(dt, {
     ffk_launch(bias_act_bwd_kernel<T>, grid, block, 0, st, (const T *)dy, (const T *)saved, (T *)dz, dbias ? partial : nullptr,
                                                     rows, cols, act);
+    traffic.done();
     if (dbias) ffk_launch(colsum_finish_kernel<T>, (cols + 255) / 256, 256, 0, st, partial, gy, cols, (T *)dbias, accumulate);
   });
   return (int)cudaGetLastError();

@@ -421,6 +421,7 @@ static bool ln_vec_ok(int cols, const void *a, const void *b, const void *c, con
 FFK_API int ffk_layernorm_fwd(const void *a, const void *b, const void *gamma, const void *beta, void *xsum, void *y,
                               float *mean, float *rstd, int rows, int cols, float eps, int dt, cudaStream_t st) {
   if (rows <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * (dt == 1 ? 2 : 4) * (b ? 4 : 2));
   if (dt == 1 && ln_vec_ok(cols, a, b, gamma, beta, xsum, y)) {
     int vpt = ln_vpt(cols), threads = cols / 8 / vpt;
     const bf16 *A = (const bf16 *)a, *B = (const bf16 *)b, *G = (const bf16 *)gamma, *Bt = (const bf16 *)beta;
@@ -504,6 +505,7 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
                               void *dx, void *dx2, void *dgamma, void *dbeta, float *partial, int rows, int cols, int dt,
                               int accumulate_dx, int accumulate_dx2, int accumulate_params, cudaStream_t st) {
   if (rows <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * (dt == 1 ? 2 : 4) * (dx2 ? 4 : 3));
   if (cols > 16384) return -2;
   const bool vec = dt == 1 && ln_vec_ok(cols, dy, x, gamma, dx, dx2, nullptr);
   int grid = ln_bwd_grid(rows, cols, vec);
@@ -526,6 +528,7 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
     } else if (vpt == 1) ffk_launch(vec::layernorm_bwd_vec_kernel<1>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     else if (vpt == 2) ffk_launch(vec::layernorm_bwd_vec_kernel<2>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
     else ffk_launch(vec::layernorm_bwd_vec_kernel<4>, grid, threads, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
+    traffic.done();
     if (part)
       ffk_launch(vec::fold_partials_kernel<bf16>, (cols + 31) / 32, dim3(32, 32), 0, st, part, grid, cols, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_params);
     return (int)cudaGetLastError();
@@ -542,6 +545,7 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
       default: LN_BWD(4); break;
     }
 #undef LN_BWD
+    traffic.done();
     if (part)
       ffk_launch(vec::fold_partials_kernel<float>, (cols + 31) / 32, dim3(32, 32), 0, st, part, grid, cols, (float *)dgamma, (float *)dbeta,
                  accumulate_params);
@@ -557,6 +561,7 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
     else
       ffk_launch(layernorm_bwd_kernel<T, 32>, grid, 512, 0, st, (const T *)dy, (const T *)x, (const T *)gamma, mean, rstd,
                                                          (T *)dx, (T *)dx2, part, rows, cols, accumulate_dx, accumulate_dx2);
+    traffic.done();
     if (part)
       ffk_launch(vec::fold_partials_kernel<T>, (cols + 31) / 32, dim3(32, 32), 0, st, part, grid, cols, (T *)dgamma, (T *)dbeta, accumulate_params);
   });
@@ -577,6 +582,7 @@ static int softmax_vpt(int cols) {
 FFK_API int ffk_softmax_dropout_fwd(const void *x, void *y, void *yd, int rows, int cols, int ld, float scale, int causal_q, float p,
                                     unsigned long long salt, const unsigned long long *seed_ptr, int dt, cudaStream_t st) {
   if (rows <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * 2 * (yd ? 3 : 2));
   if (!softmax_warp_ok(cols, ld, dt, x, y, yd)) return -3;
   const int grid = ffk_blocks(rows, 8);
 #define SM_FWD(V)                                                                                                                        \
@@ -596,6 +602,7 @@ FFK_API int ffk_softmax_dropout_fwd(const void *x, void *y, void *yd, int rows, 
 FFK_API int ffk_softmax_dropout_bwd(const void *dy, const void *y, void *dx, int rows, int cols, int ld, float scale, float p,
                                     unsigned long long salt, const unsigned long long *seed_ptr, int dt, cudaStream_t st) {
   if (rows <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * 2 * 3);
   if (!softmax_warp_ok(cols, ld, dt, dy, y, dx)) return -3;
   const int grid = ffk_blocks(rows, 8);
 #define SM_BWD(V)                                                                                                                       \
@@ -661,6 +668,7 @@ FFK_API int ffk_softmax_last_error() {
 FFK_API int ffk_softmax_fwd(const void *x, void *y, int rows, int cols, float scale, int causal_q, int dt,
                             cudaStream_t st) {
   if (rows <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * (dt == 1 ? 2 : 4) * 2);
   if (softmax_warp_ok(cols, cols, dt, x, y, nullptr))
     return ffk_softmax_dropout_fwd(x, y, nullptr, rows, cols, cols, scale, causal_q, 0.f, 0, nullptr, dt, st);
   if (softmax_wide_ok(cols, dt) && causal_q <= 0 && aligned16(x) && aligned16(y))
@@ -680,6 +688,7 @@ FFK_API int ffk_softmax_fwd(const void *x, void *y, int rows, int cols, float sc
 FFK_API int ffk_softmax_bwd(const void *dy, const void *y, void *dx, int rows, int cols, float scale, int dt,
                             cudaStream_t st) {
   if (rows <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * (dt == 1 ? 2 : 4) * 3);
   if (softmax_warp_ok(cols, cols, dt, dy, y, dx))
     return ffk_softmax_dropout_bwd(dy, y, dx, rows, cols, cols, scale, 0.f, 0, nullptr, dt, st);
   int threads = cols >= 1024 ? 256 : 128;
@@ -701,6 +710,7 @@ static void launch_softmax_ce_row(const void *logits, const void *labels, void *
 FFK_API int ffk_softmax_ce(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows,
                            int cols, float grad_scale, int dt, int label_dt, cudaStream_t st) {
   if (rows <= 0) return 0;
+  FfkTraffic traffic((long long)rows * cols * (dt == 1 ? 2 : 4) * 2);
   if (softmax_wide_ok(cols, dt) && aligned16(logits) && aligned16(probs) && aligned16(dlogits))
     return label_dt == 3 ? launch_softmax_wide<true, long long>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st)
                          : launch_softmax_wide<true, int>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st);

@@ -1,6 +1,7 @@
-// rowwise_vec.cuh -- 128-bit vectorised fast paths of the row-wise kernels for bf16 rows whose length
-// is a multiple of 8: softmax fwd/bwd (optionally fused with dropout of the probabilities), LayerNorm
-// fwd/bwd (fused residual add) and the bias/activation backward with its column reduction.
+// rowwise_vec.cuh -- 128-bit vectorised fast paths of the row-wise kernels: softmax fwd/bwd (optionally fused
+// with dropout of the probabilities; bf16 rows of any length at a pitch of a multiple of 8), LayerNorm fwd/bwd
+// (fused residual add; bf16 and, one warp per row, fp32) and the bias/activation backward with its column
+// reduction (bf16 rows whose length is a multiple of 8).
 //
 // Each thread owns whole 8-element vectors of a row and keeps them in registers, so a row is read once
 // and written once; HBM traffic is the algorithmic minimum.  The scalar kernels in norm_softmax.cu and

@@ -354,6 +354,7 @@ FFK_API int ffk_permute(const void *src, void *dst, int ndim, const long long *s
   long long total = 1;
   for (int i = 0; i < ndim; ++i) { d.size[i] = sizes[i]; d.stride[i] = src_strides[i]; total *= sizes[i]; }
   if (total <= 0) return 0;
+  FfkTraffic traffic(total * es * 2);
   if (total < (1ll << 31) - 4ll * 148 * 16 * 256) {  // the last trip's indexes stay below 2^31
     Dims32 q;
     q.n = ndim;
@@ -387,6 +388,7 @@ FFK_API int ffk_transpose2d(const void *src, void *dst, int batch, int rows, int
 FFK_API int ffk_block_copy(const void *src, long long src_ld, void *dst, long long dst_ld, long long outer, long long block, int es,
                            int dt, int accumulate, cudaStream_t st) {
   if (outer * block <= 0) return 0;
+  FfkTraffic traffic(outer * block * es * 2);
   {
     const long long bytes = block * es, sp = src_ld * es, dp = dst_ld * es, pieces = outer * (bytes / 16);
     const bool vec = bytes % 16 == 0 && sp % 16 == 0 && dp % 16 == 0 && ((uintptr_t)src % 16) == 0 && ((uintptr_t)dst % 16) == 0 &&
