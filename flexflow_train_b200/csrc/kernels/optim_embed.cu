@@ -60,22 +60,113 @@ __global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float 
 }
 
 template <typename G>
-__global__ void sgd_kernel(float *__restrict__ w, float *__restrict__ mom, const G *__restrict__ g,
-                           bf16 *__restrict__ shadow, long long n, float lr, float momentum, int nesterov, float wd,
-                           float gscale) {
+__global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
+                            const G *__restrict__ g, bf16 *__restrict__ shadow, long long n, float alpha_t,
+                            float beta1, float beta2, float eps, float wd, float gscale,
+                            const float *__restrict__ alpha_ptr) {
   pdl_entry();
-  long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    float wk = w[i];
-    float gt = ldg(g, i) * gscale + wd * wk;
-    if (momentum > 0.f) {
-      float vk = mom[i] * momentum + gt;
-      mom[i] = vk;
-      gt = nesterov ? gt + momentum * vk : vk;
+  // alpha_ptr (optional): bias-corrected step size kept in device memory so that a captured CUDA graph
+  // sees the value of the current step.
+  if (alpha_ptr) alpha_t = *alpha_ptr;
+  long long stride = (long long)gridDim.x * blockDim.x * 4;
+  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += stride) {
+    if (i + 4 <= n) {
+      float4 w4 = *reinterpret_cast<float4 *>(w + i), m4 = *reinterpret_cast<float4 *>(m + i),
+             v4 = *reinterpret_cast<float4 *>(v + i);
+      float gg[4] = {ldg(g, i) * gscale, ldg(g, i + 1) * gscale, ldg(g, i + 2) * gscale, ldg(g, i + 3) * gscale};
+      float ww[4] = {w4.x, w4.y, w4.z, w4.w}, mm[4] = {m4.x, m4.y, m4.z, m4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float gt = gg[j] + wd * ww[j];
+        mm[j] = beta1 * mm[j] + (1.f - beta1) * gt;
+        vv[j] = beta2 * vv[j] + (1.f - beta2) * gt * gt;
+        ww[j] -= alpha_t * mm[j] / (sqrtf(vv[j]) + eps);
+      }
+      *reinterpret_cast<float4 *>(w + i) = make_float4(ww[0], ww[1], ww[2], ww[3]);
+      *reinterpret_cast<float4 *>(m + i) = make_float4(mm[0], mm[1], mm[2], mm[3]);
+      *reinterpret_cast<float4 *>(v + i) = make_float4(vv[0], vv[1], vv[2], vv[3]);
+      if (shadow) {
+        uint2 s = make_uint2(pack_bf162(ww[0], ww[1]), pack_bf162(ww[2], ww[3]));
+        *reinterpret_cast<uint2 *>(shadow + i) = s;
+      }
+    } else {
+      for (long long k = i; k < n; ++k) {
+        float gt = ldg(g, k) * gscale + wd * w[k];
+        float mk = beta1 * m[k] + (1.f - beta1) * gt;
+        float vk = beta2 * v[k] + (1.f - beta2) * gt * gt;
+        float wk = w[k] - alpha_t * mk / (sqrtf(vk) + eps);
+        w[k] = wk; m[k] = mk; v[k] = vk;
+        if (shadow) shadow[k] = f2bf(wk);
+      }
     }
-    wk -= lr * gt;
-    w[i] = wk;
-    if (shadow) shadow[i] = f2bf(wk);
+  }
+}
+
+// four gradients from an address of a whole piece
+__device__ __forceinline__ void ldg4(const float *p, float (&v)[4]) {
+  const float4 u = __ldcs(reinterpret_cast<const float4 *>(p));
+  v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w;
+}
+__device__ __forceinline__ void ldg4(const bf16 *p, float (&v)[4]) {
+  const uint2 u = __ldcs(reinterpret_cast<const uint2 *>(p));
+  const float2 a = unpack_bf162(u.x), b = unpack_bf162(u.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void to4(const float4 &q, float (&v)[4]) { v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w; }
+
+
+
+// SGD is bound by HBM (20 bytes per parameter with momentum, bf16 gradients and a shadow).  A thread takes two groups of four
+// parameters per trip and asks for all their state before it computes; what the step does not read again is streamed past L2.
+// Element by element it ran at 4.8 TB/s (33.6 million parameters 139 us, now 115); the same form gave Adam, whose state already
+// came in 16-byte pieces, nothing (163 us both).
+__device__ __forceinline__ float sgd_step(float wk, float gk, float *mom, float lr, float momentum, int nesterov, float wd, float gscale) {
+  float gt = gk * gscale + wd * wk;
+  if (momentum > 0.f) {
+    const float vk = *mom * momentum + gt;
+    *mom = vk;
+    gt = nesterov ? gt + momentum * vk : vk;
+  }
+  return wk - lr * gt;
+}
+template <typename G>
+__global__ void __launch_bounds__(256) sgd_kernel(float *__restrict__ w, float *__restrict__ mom, const G *__restrict__ g,
+                                                  bf16 *__restrict__ shadow, long long n, float lr, float momentum, int nesterov, float wd,
+                                                  float gscale) {
+  pdl_entry();
+  // groups of four where the arenas' addresses allow it (a slice may start anywhere)
+  const bool vec = (((uintptr_t)w | (uintptr_t)(momentum > 0.f ? mom : w)) & 15) == 0 && ((uintptr_t)g & (4 * sizeof(G) - 1)) == 0 &&
+                   ((uintptr_t)shadow & 7) == 0;
+  const long long half = (long long)gridDim.x * blockDim.x * 4, n4 = vec ? n & ~3ll : 0;
+  for (long long i0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i0 < n4; i0 += 2 * half) {
+    float ww[2][4], mm[2][4] = {}, gg[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const long long i = i0 + u * half;
+      if (i < n4) {
+        to4(__ldcs(reinterpret_cast<const float4 *>(w + i)), ww[u]);
+        if (momentum > 0.f) to4(__ldcs(reinterpret_cast<const float4 *>(mom + i)), mm[u]);
+        ldg4(g + i, gg[u]);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const long long i = i0 + u * half;
+      if (i < n4) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ww[u][j] = sgd_step(ww[u][j], gg[u][j], &mm[u][j], lr, momentum, nesterov, wd, gscale);
+        __stcs(reinterpret_cast<float4 *>(w + i), make_float4(ww[u][0], ww[u][1], ww[u][2], ww[u][3]));
+        if (momentum > 0.f) __stcs(reinterpret_cast<float4 *>(mom + i), make_float4(mm[u][0], mm[u][1], mm[u][2], mm[u][3]));
+        if (shadow) *reinterpret_cast<uint2 *>(shadow + i) = make_uint2(pack_bf162(ww[u][0], ww[u][1]), pack_bf162(ww[u][2], ww[u][3]));
+      }
+    }
+  }
+  for (long long k = n4 + (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+    float mk = momentum > 0.f ? mom[k] : 0.f;
+    const float wk = sgd_step(w[k], ldg(g, k), &mk, lr, momentum, nesterov, wd, gscale);
+    w[k] = wk;
+    if (momentum > 0.f) mom[k] = mk;
+    if (shadow) shadow[k] = f2bf(wk);
   }
 }
 
@@ -226,6 +317,7 @@ FFK_API int ffk_adam_update(float *w, float *m, float *v, const void *g, void *s
                             float beta1, float beta2, float eps, float wd, float gscale, const float *alpha_ptr,
                             int grad_dt, cudaStream_t st) {
   if (n <= 0) return 0;
+  FfkTraffic traffic(n * 28);
   int grid = ffk_blocks(n / 4 + 1, 256, 148 * 8);
   if (grad_dt == 1)
     ffk_launch(adam_kernel<bf16>, grid, 256, 0, st, w, m, v, (const bf16 *)g, (bf16 *)shadow, n, alpha_t, beta1, beta2, eps, wd, gscale, alpha_ptr);
@@ -236,7 +328,8 @@ FFK_API int ffk_adam_update(float *w, float *m, float *v, const void *g, void *s
 FFK_API int ffk_sgd_update(float *w, float *mom, const void *g, void *shadow, long long n, float lr, float momentum,
                            int nesterov, float wd, float gscale, int grad_dt, cudaStream_t st) {
   if (n <= 0) return 0;
-  int grid = ffk_blocks(n, 256, 148 * 8);
+  FfkTraffic traffic(n * 20);
+  int grid = ffk_blocks(n / 4 + 1, 256, 148 * 8);
   if (grad_dt == 1)
     ffk_launch(sgd_kernel<bf16>, grid, 256, 0, st, w, mom, (const bf16 *)g, (bf16 *)shadow, n, lr, momentum, nesterov, wd, gscale);
   else
@@ -247,6 +340,7 @@ FFK_API int ffk_sgd_update(float *w, float *mom, const void *g, void *shadow, lo
 template <typename W, typename I, typename O>
 static int emb_launch(int which, const void *idx, const void *table_or_dtable, const void *out_or_dout, long long tokens,
                       int bag, int dim, long long entries, int avg, cudaStream_t st) {
+  FfkTraffic traffic(tokens * dim * 4);
   if (emb_vec_ok(tokens, dim, table_or_dtable, out_or_dout)) {
     const unsigned per_row = (unsigned)(dim / 8), pieces = (unsigned)(tokens * per_row);
     const int vgrid = ffk_blocks(pieces, 256);

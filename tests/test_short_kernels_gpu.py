@@ -174,3 +174,35 @@ def test_small_batched_products(M, N, Kd, out_dt, accumulate):
     want = 0.5 * (a.double() @ b.double().transpose(1, 2)) + (old.double() if accumulate else 0)
     ulp = 2.0 ** -8 if out_dt == torch.bfloat16 else 0
     assert ((C.double() - want).abs() <= want.abs() * ulp + Kd * 2.0 ** -20).all()  # fp32 sums of Kd terms, one rounding
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 1021, 4096, 148 * 8 * 256 * 8 + 6])
+@pytest.mark.parametrize("grad_dt", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 1])  # 1: gradients that no 8- or 16-byte load takes (SGD: no array is aligned)
+def test_optimizer_steps(n, grad_dt, offset):
+    g = _randn(n + offset, dtype=torch.float32).to(grad_dt)[offset:]
+    w, m, v = _randn(n, dtype=torch.float32, seed=1), _randn(n, dtype=torch.float32, seed=2), _randn(n, dtype=torch.float32, seed=3).abs()
+    wd, md, vd, gd = w.double(), m.double(), v.double(), g.double()
+    shadow = torch.zeros(n, device="cuda").bfloat16()
+    K.adam_update(w, m, v, g, shadow, 1e-2, 0.9, 0.99, 1e-8, weight_decay=0.1)
+    gt = gd + 0.1 * wd
+    md = 0.9 * md + (1 - 0.9) * gt
+    vd = 0.99 * vd + (1 - 0.99) * gt * gt
+    want = wd - 1e-2 * md / (vd.sqrt() + 1e-8)
+    # single-precision steps with approximate division and square root (2 ulp each) of values of order one
+    for got, ref in ((m, md), (v, vd), (w, want)):
+        assert ((got.double() - ref).abs() <= 2.0 ** -20 * (1 + ref.abs())).all()
+    assert torch.equal(shadow, w.bfloat16())
+    for momentum, nesterov in ((0.0, False), (0.9, False), (0.9, True)):
+        w = _randn(n + offset, dtype=torch.float32, seed=4)[offset:]
+        mom = _randn(n + offset, dtype=torch.float32, seed=5)[offset:] if momentum else None
+        shadow = torch.zeros(n + offset, device="cuda").bfloat16()[offset:]
+        gt = gd + 0.1 * w.double()
+        ref_m = mom.double() * momentum + gt if momentum else None
+        step = gt if not momentum else gt + momentum * ref_m if nesterov else ref_m
+        want = w.double() - 0.05 * step
+        K.sgd_update(w, mom, g, shadow, 0.05, momentum=momentum, nesterov=nesterov, weight_decay=0.1)
+        assert ((w.double() - want).abs() <= 2.0 ** -20 * (1 + want.abs())).all()
+        if momentum:
+            assert ((mom.double() - ref_m).abs() <= 2.0 ** -20 * (1 + ref_m.abs())).all()
+        assert torch.equal(shadow, w.bfloat16())
