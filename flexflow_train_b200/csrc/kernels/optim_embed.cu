@@ -59,49 +59,6 @@ __global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float 
   }
 }
 
-template <typename G>
-__global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
-                            const G *__restrict__ g, bf16 *__restrict__ shadow, long long n, float alpha_t,
-                            float beta1, float beta2, float eps, float wd, float gscale,
-                            const float *__restrict__ alpha_ptr) {
-  pdl_entry();
-  // alpha_ptr (optional): bias-corrected step size kept in device memory so that a captured CUDA graph
-  // sees the value of the current step.
-  if (alpha_ptr) alpha_t = *alpha_ptr;
-  long long stride = (long long)gridDim.x * blockDim.x * 4;
-  for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += stride) {
-    if (i + 4 <= n) {
-      float4 w4 = *reinterpret_cast<float4 *>(w + i), m4 = *reinterpret_cast<float4 *>(m + i),
-             v4 = *reinterpret_cast<float4 *>(v + i);
-      float gg[4] = {ldg(g, i) * gscale, ldg(g, i + 1) * gscale, ldg(g, i + 2) * gscale, ldg(g, i + 3) * gscale};
-      float ww[4] = {w4.x, w4.y, w4.z, w4.w}, mm[4] = {m4.x, m4.y, m4.z, m4.w}, vv[4] = {v4.x, v4.y, v4.z, v4.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float gt = gg[j] + wd * ww[j];
-        mm[j] = beta1 * mm[j] + (1.f - beta1) * gt;
-        vv[j] = beta2 * vv[j] + (1.f - beta2) * gt * gt;
-        ww[j] -= alpha_t * mm[j] / (sqrtf(vv[j]) + eps);
-      }
-      *reinterpret_cast<float4 *>(w + i) = make_float4(ww[0], ww[1], ww[2], ww[3]);
-      *reinterpret_cast<float4 *>(m + i) = make_float4(mm[0], mm[1], mm[2], mm[3]);
-      *reinterpret_cast<float4 *>(v + i) = make_float4(vv[0], vv[1], vv[2], vv[3]);
-      if (shadow) {
-        uint2 s = make_uint2(pack_bf162(ww[0], ww[1]), pack_bf162(ww[2], ww[3]));
-        *reinterpret_cast<uint2 *>(shadow + i) = s;
-      }
-    } else {
-      for (long long k = i; k < n; ++k) {
-        float gt = ldg(g, k) * gscale + wd * w[k];
-        float mk = beta1 * m[k] + (1.f - beta1) * gt;
-        float vk = beta2 * v[k] + (1.f - beta2) * gt * gt;
-        float wk = w[k] - alpha_t * mk / (sqrtf(vk) + eps);
-        w[k] = wk; m[k] = mk; v[k] = vk;
-        if (shadow) shadow[k] = f2bf(wk);
-      }
-    }
-  }
-}
-
 // four gradients from an address of a whole piece
 __device__ __forceinline__ void ldg4(const float *p, float (&v)[4]) {
   const float4 u = __ldcs(reinterpret_cast<const float4 *>(p));
@@ -113,8 +70,6 @@ __device__ __forceinline__ void ldg4(const bf16 *p, float (&v)[4]) {
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
 __device__ __forceinline__ void to4(const float4 &q, float (&v)[4]) { v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w; }
-
-
 
 // SGD is bound by HBM (20 bytes per parameter with momentum, bf16 gradients and a shadow).  A thread takes two groups of four
 // parameters per trip and asks for all their state before it computes; what the step does not read again is streamed past L2.
