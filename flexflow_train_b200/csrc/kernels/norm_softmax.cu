@@ -430,7 +430,7 @@ FFK_API int ffk_layernorm_fwd(const void *a, const void *b, const void *gamma, c
       const int wv = cols / 256;
       long long want = ((long long)rows + 7) / 8;
       const int grid = (int)(want < 148 * 2 ? want : 148 * 2);
-#define LN_WARP(V) ffk_launch(vec::layernorm_fwd_warp_kernel<bf16, V>, grid, 256, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, eps)
+#define LN_WARP(V) ffk_launch(vec::layernorm_fwd_warp_kernel<V>, grid, 256, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, eps)
       switch (wv) {
         case 1: LN_WARP(1); break;
         case 2: LN_WARP(2); break;
@@ -447,23 +447,6 @@ FFK_API int ffk_layernorm_fwd(const void *a, const void *b, const void *gamma, c
     if (vpt == 1) ffk_launch(vec::layernorm_fwd_vec_kernel<1>, rows_grid(rows), threads, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
     else if (vpt == 2) ffk_launch(vec::layernorm_fwd_vec_kernel<2>, rows_grid(rows), threads, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
     else ffk_launch(vec::layernorm_fwd_vec_kernel<4>, rows_grid(rows), threads, 0, st, A, B, G, Bt, (bf16 *)xsum, (bf16 *)y, mean, rstd, rows, cols, eps);
-    return (int)cudaGetLastError();
-  }
-  // fp32 rows of up to 1024 (twice the registers per element): the same one warp per row
-  if (dt == 0 && cols % 256 == 0 && cols <= 1024 && rows >= 8 && aligned16(a) && aligned16(b) && aligned16(gamma) && aligned16(beta) &&
-      aligned16(xsum) && aligned16(y)) {
-    const long long want = ((long long)rows + 7) / 8;
-    const int grid = (int)(want < 148 * 2 ? want : 148 * 2);
-#define LN_WARP(V)                                                                                                                        \
-  ffk_launch(vec::layernorm_fwd_warp_kernel<float, V>, grid, 256, 0, st, (const float *)a, (const float *)b, (const float *)gamma,         \
-             (const float *)beta, (float *)xsum, (float *)y, mean, rstd, rows, eps)
-    switch (cols / 256) {
-      case 1: LN_WARP(1); break;
-      case 2: LN_WARP(2); break;
-      case 3: LN_WARP(3); break;
-      default: LN_WARP(4); break;
-    }
-#undef LN_WARP
     return (int)cudaGetLastError();
   }
   int threads = cols >= 2048 ? 512 : 256;
@@ -516,7 +499,7 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
     if (ln_bwd_warp_ok(rows, cols)) {
       grid = ln_bwd_warp_grid(rows, cols);
 #define LN_BWD(V)                                                                                                                            \
-  ffk_launch(vec::layernorm_bwd_warp_kernel<bf16, V>, grid, 256, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, accumulate_dx, \
+  ffk_launch(vec::layernorm_bwd_warp_kernel<V>, grid, 256, 0, st, DY, X, G, mean, rstd, (bf16 *)dx, (bf16 *)dx2, part, rows, accumulate_dx, \
              accumulate_dx2)
       switch (cols / 256) {
         case 1: LN_BWD(1); break;
@@ -531,24 +514,6 @@ FFK_API int ffk_layernorm_bwd(const void *dy, const void *x, const void *gamma, 
     traffic.done();
     if (part)
       ffk_launch(vec::fold_partials_kernel<bf16>, (cols + 31) / 32, dim3(32, 32), 0, st, part, grid, cols, (bf16 *)dgamma, (bf16 *)dbeta, accumulate_params);
-    return (int)cudaGetLastError();
-  }
-  if (dt == 0 && ln_bwd_warp_ok(rows, cols) && aligned16(dy) && aligned16(x) && aligned16(dx) && aligned16(dx2)) {
-    grid = ln_bwd_warp_grid(rows, cols);
-#define LN_BWD(V)                                                                                                                           \
-  ffk_launch(vec::layernorm_bwd_warp_kernel<float, V>, grid, 256, 0, st, (const float *)dy, (const float *)x, (const float *)gamma, mean, rstd, \
-             (float *)dx, (float *)dx2, part, rows, accumulate_dx, accumulate_dx2)
-    switch (cols / 256) {
-      case 1: LN_BWD(1); break;
-      case 2: LN_BWD(2); break;
-      case 3: LN_BWD(3); break;
-      default: LN_BWD(4); break;
-    }
-#undef LN_BWD
-    traffic.done();
-    if (part)
-      ffk_launch(vec::fold_partials_kernel<float>, (cols + 31) / 32, dim3(32, 32), 0, st, part, grid, cols, (float *)dgamma, (float *)dbeta,
-                 accumulate_params);
     return (int)cudaGetLastError();
   }
   DISPATCH_FLOAT(dt, {

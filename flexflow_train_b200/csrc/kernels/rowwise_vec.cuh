@@ -1,6 +1,6 @@
 // rowwise_vec.cuh -- 128-bit vectorised fast paths of the row-wise kernels: softmax fwd/bwd (optionally fused
 // with dropout of the probabilities; bf16 rows of any length at a pitch of a multiple of 8), LayerNorm fwd/bwd
-// (fused residual add; bf16 and, one warp per row, fp32) and the bias/activation backward with its column
+// (fused residual add; bf16) and the bias/activation backward with its column
 // reduction (bf16 rows whose length is a multiple of 8).
 //
 // Each thread owns whole 8-element vectors of a row and keeps them in registers, so a row is read once
@@ -23,28 +23,6 @@ __device__ __forceinline__ void unpack8(const uint4 &u, float *v) {
 __device__ __forceinline__ void st8(bf16 *p, const float *v) {
   *reinterpret_cast<uint4 *>(p) = make_uint4(pack_bf162(v[0], v[1]), pack_bf162(v[2], v[3]), pack_bf162(v[4], v[5]), pack_bf162(v[6], v[7]));
 }
-
-// Eight neighbouring elements of a row as they lie in memory: 16 bytes of bf16, 32 of fp32
-template <typename T> struct Piece;
-template <> struct Piece<bf16> {
-  typedef uint4 raw;
-  static __device__ __forceinline__ void unpack(const raw &u, float *v) { unpack8(u, v); }
-  static __device__ __forceinline__ void ld(const bf16 *p, float *v) { ld8(p, v); }
-  static __device__ __forceinline__ void st(bf16 *p, const float *v) { st8(p, v); }
-  static __device__ __forceinline__ float round(float v) { return bf2f(f2bf(v)); }
-};
-template <> struct Piece<float> {
-  struct __align__(16) raw { float4 a, b; };
-  static __device__ __forceinline__ void unpack(const raw &u, float *v) {
-    v[0] = u.a.x; v[1] = u.a.y; v[2] = u.a.z; v[3] = u.a.w; v[4] = u.b.x; v[5] = u.b.y; v[6] = u.b.z; v[7] = u.b.w;
-  }
-  static __device__ __forceinline__ void ld(const float *p, float *v) { unpack(*reinterpret_cast<const raw *>(p), v); }
-  static __device__ __forceinline__ void st(float *p, const float *v) {
-    reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4 *>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
-  }
-  static __device__ __forceinline__ float round(float v) { return v; }
-};
 
 // ---------------------------------------------------------------- softmax: one warp per row
 // Keep flags of the 8 elements from flat index e on (two group words where the row length is a multiple of 4, and e with it;
@@ -351,28 +329,28 @@ __global__ void layernorm_fwd_vec_kernel(const bf16 *__restrict__ a, const bf16 
 // (piece i of lane l = elements [(i * 32 + l) * 8, +8): coalesced), all loaded before anything is computed, so a
 // warp has VPT (2 VPT with a fused add) loads in flight and the two row reductions are warp shuffles: no
 // block-wide barrier after the one that stages gamma / beta in shared memory.
-template <typename T, int VPT>
-__global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const T *__restrict__ a, const T *__restrict__ b,
-                                                                    const T *__restrict__ gamma, const T *__restrict__ beta,
-                                                                    T *__restrict__ xsum, T *__restrict__ y, float *__restrict__ mean,
+template <int VPT>
+__global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b,
+                                                                    const bf16 *__restrict__ gamma, const bf16 *__restrict__ beta,
+                                                                    bf16 *__restrict__ xsum, bf16 *__restrict__ y, float *__restrict__ mean,
                                                                     float *__restrict__ rstd, int rows, float eps) {
   pdl_entry();
   constexpr int COLS = 256 * VPT, NV = 32 * VPT;
-  __shared__ typename Piece<T>::raw g_s[NV], b_s[NV];
+  __shared__ uint4 g_s[NV], b_s[NV];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   for (int i = threadIdx.x; i < NV; i += blockDim.x) {
-    if (gamma) g_s[i] = reinterpret_cast<const typename Piece<T>::raw *>(gamma)[i];
-    if (beta) b_s[i] = reinterpret_cast<const typename Piece<T>::raw *>(beta)[i];
+    if (gamma) g_s[i] = reinterpret_cast<const uint4 *>(gamma)[i];
+    if (beta) b_s[i] = reinterpret_cast<const uint4 *>(beta)[i];
   }
   __syncthreads();
   for (int row = blockIdx.x * wpb + wid; row < rows; row += gridDim.x * wpb) {
     const long long base = (long long)row * COLS;
-    const typename Piece<T>::raw *ar = reinterpret_cast<const typename Piece<T>::raw *>(a + base);
-    typename Piece<T>::raw ua[VPT], ub[VPT];
+    const uint4 *ar = reinterpret_cast<const uint4 *>(a + base);
+    uint4 ua[VPT], ub[VPT];
 #pragma unroll
     for (int i = 0; i < VPT; ++i) ua[i] = ar[i * 32 + lane];
     if (b) {
-      const typename Piece<T>::raw *br = reinterpret_cast<const typename Piece<T>::raw *>(b + base);
+      const uint4 *br = reinterpret_cast<const uint4 *>(b + base);
 #pragma unroll
       for (int i = 0; i < VPT; ++i) ub[i] = br[i * 32 + lane];
     }
@@ -380,16 +358,16 @@ __global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const T *__r
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-      Piece<T>::unpack(ua[i], v[i]);
+      unpack8(ua[i], v[i]);
       if (b) {
         float w[8];
-        Piece<T>::unpack(ub[i], w);
+        unpack8(ub[i], w);
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[i][j] += w[j];
         if (xsum) {
-          Piece<T>::st(xsum + base + (i * 32 + lane) * 8, v[i]);
+          st8(xsum + base + (i * 32 + lane) * 8, v[i]);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[i][j] = Piece<T>::round(v[i][j]);  // statistics of the value backward will read
+          for (int j = 0; j < 8; ++j) v[i][j] = bf2f(f2bf(v[i][j]));  // statistics of the value backward will read
         }
       }
 #pragma unroll
@@ -409,14 +387,14 @@ __global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const T *__r
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       float g8[8], b8[8];
-      if (gamma) Piece<T>::unpack(g_s[i * 32 + lane], g8);
-      if (beta) Piece<T>::unpack(b_s[i * 32 + lane], b8);
+      if (gamma) unpack8(g_s[i * 32 + lane], g8);
+      if (beta) unpack8(b_s[i * 32 + lane], b8);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         float o = (v[i][j] - mu) * rs;
         v[i][j] = gamma ? o * g8[j] + (beta ? b8[j] : 0.f) : o;
       }
-      Piece<T>::st(y + base + (i * 32 + lane) * 8, v[i]);
+      st8(y + base + (i * 32 + lane) * 8, v[i]);
     }
   }
 }
@@ -524,32 +502,31 @@ __global__ void layernorm_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16
 }
 
 // LayerNorm backward, one warp per row: cols = 256 * VPT, VPT <= 4 (the column sums of a lane's 8 * VPT columns stay in registers
-// over all its rows), bf16 or fp32.  No block-wide barrier per row, the next row's pieces in flight while this one is reduced, and one partial
+// over all its rows).  No block-wide barrier per row, the next row's pieces in flight while this one is reduced, and one partial
 // row of dgamma / dbeta per block of 8 warps instead of one per row group: at 2048 x 512 the block-per-row form spent as many
-// bytes on 1184 partial rows as on the data (8.7 us and 4.5 us to fold them).  fp32 rows took the scalar kernel (4096 x 512: 24 us).
-template <typename T, int VPT>
+// bytes on 1184 partial rows as on the data (8.7 us and 4.5 us to fold them).
+template <int VPT>
 __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1)
-layernorm_bwd_warp_kernel(const T *__restrict__ dy, const T *__restrict__ x, const T *__restrict__ gamma, const float *__restrict__ mean,
-                          const float *__restrict__ rstd, T *__restrict__ dx, T *__restrict__ dx2, float *__restrict__ partial, int rows,
+layernorm_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ gamma, const float *__restrict__ mean,
+                          const float *__restrict__ rstd, bf16 *__restrict__ dx, bf16 *__restrict__ dx2, float *__restrict__ partial, int rows,
                           int acc1, int acc2) {
   pdl_entry();
   constexpr int COLS = 256 * VPT;
   __shared__ float red[8][COLS];
   __shared__ float g_s[COLS];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < COLS; i += 256) g_s[i] = gamma ? (float)gamma[i] : 1.f;
+  for (int i = threadIdx.x; i < COLS; i += 256) g_s[i] = gamma ? bf2f(gamma[i]) : 1.f;
   __syncthreads();
   float dg[VPT][8], db[VPT][8];
 #pragma unroll
   for (int i = 0; i < VPT; ++i)
 #pragma unroll
     for (int j = 0; j < 8; ++j) { dg[i][j] = 0.f; db[i][j] = 0.f; }
-  typename Piece<T>::raw ng[VPT], nx[VPT];
+  uint4 ng[VPT], nx[VPT];
   const int first = blockIdx.x * 8 + wid, step = gridDim.x * 8;
   float nmu = 0.f, nrs = 0.f;
   auto fetch = [&](int row) {
-    typedef typename Piece<T>::raw Raw;
-    const Raw *pg = reinterpret_cast<const Raw *>(dy + (long long)row * COLS), *px = reinterpret_cast<const Raw *>(x + (long long)row * COLS);
+    const uint4 *pg = reinterpret_cast<const uint4 *>(dy + (long long)row * COLS), *px = reinterpret_cast<const uint4 *>(x + (long long)row * COLS);
 #pragma unroll
     for (int i = 0; i < VPT; ++i) { ng[i] = pg[i * 32 + lane]; nx[i] = px[i * 32 + lane]; }
     nmu = mean[row];
@@ -561,7 +538,7 @@ layernorm_bwd_warp_kernel(const T *__restrict__ dy, const T *__restrict__ x, con
     const float mu = nmu, rs = nrs;
     float s1 = 0.f, s2 = 0.f;
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) { Piece<T>::unpack(ng[i], g[i]); Piece<T>::unpack(nx[i], xh[i]); }
+    for (int i = 0; i < VPT; ++i) { unpack8(ng[i], g[i]); unpack8(nx[i], xh[i]); }
     if (row + step < rows) fetch(row + step);
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -589,19 +566,19 @@ layernorm_bwd_warp_kernel(const T *__restrict__ dy, const T *__restrict__ x, con
       if (dx2) {
         float t[8];
         if (acc2) {
-          Piece<T>::ld(dx2 + off, t);
+          ld8(dx2 + off, t);
 #pragma unroll
           for (int j = 0; j < 8; ++j) t[j] += o[j];
-          Piece<T>::st(dx2 + off, t);
-        } else Piece<T>::st(dx2 + off, o);
+          st8(dx2 + off, t);
+        } else st8(dx2 + off, o);
       }
       if (acc1) {
         float t[8];
-        Piece<T>::ld(dx + off, t);
+        ld8(dx + off, t);
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] += t[j];
       }
-      Piece<T>::st(dx + off, o);
+      st8(dx + off, o);
     }
   }
   if (!partial) return;
