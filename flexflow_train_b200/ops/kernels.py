@@ -500,6 +500,7 @@ def cast(src, dst, accumulate=False):
 
 
 def bias_act_bwd_scratch(rows, cols) -> int:
+    """fp32 elements of scratch `bias_act_bwd` needs for [rows, cols]; not monotonic in cols."""
     return lib().ffk_bias_act_bwd_scratch(rows, cols)
 
 
@@ -508,6 +509,8 @@ def bias_act_bwd(dy, saved, dz, dbias, scratch, act, accumulate=False, dropout=N
     through the dropout that the forward GEMM epilogue applied after the activation."""
     rows, cols = dy.shape
     _cuda_contig(dy, saved, dz, dbias, scratch)
+    if dbias is not None and (scratch is None or scratch.numel() * scratch.element_size() < 4 * bias_act_bwd_scratch(rows, cols)):
+        raise KernelError("bias_act_bwd: scratch smaller than bias_act_bwd_scratch(rows, cols)")
     if dropout is not None and dropout[0] > 0:
         l = lib()
         if not getattr(l, "_bad_declared", False):

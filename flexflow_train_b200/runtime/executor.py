@@ -458,7 +458,9 @@ class AttentionOp(OpImpl):
                 self.kept_p = torch.empty_like(self.probs)
         if not self.cb and not self.fused:
             ex.need_big_scratch(nbytes, 2 if (self.p_drop > 0 and self.kept_p is None) else 1)
-        ex.need_scratch(4 * K.bias_act_bwd_scratch(self.B * self.Sq, max(self.ldqkv, self.embed)) if ex.on_gpu else 0)
+        if ex.on_gpu:
+            # column sums of the two bias gradients; the need does not grow with the width (wide matrices take fewer row chunks)
+            ex.need_scratch(4 * max(K.bias_act_bwd_scratch(self.B * self.Sq, c) for c in (self.ldqkv, self.embed)))
         if ex.cfg.training and ex.wgrad_splits(self.B * self.Sq, self.embed, self.H * self.vd, torch.bfloat16):
             ex.need_scratch(4 * self.embed * self.H * self.vd)
         self.salt = ex.next_salt()

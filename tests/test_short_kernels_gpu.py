@@ -35,6 +35,15 @@ def test_bias_gradient_of_few_rows(rows, cols):
     assert ((db.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + want.double().abs().sum(0) * rows * 2.0 ** -24 + 1e-7).all()
 
 
+def test_bias_gradient_refuses_a_short_scratch():
+    dy, db = _randn(800, 768), torch.zeros(768, device="cuda").bfloat16()
+    short = torch.empty(K.bias_act_bwd_scratch(800, 768) - 1, device="cuda")
+    for scratch in (short, None):
+        with pytest.raises(K.KernelError, match="scratch"):
+            K.bias_act_bwd(dy, None, None, db, scratch, None)
+    K.bias_act_bwd(dy, _randn(800, 768, seed=1), torch.empty_like(dy), None, None, "relu")  # without a bias gradient none is needed
+
+
 @pytest.mark.parametrize("dtype", [torch.uint8, torch.bfloat16, torch.float32, torch.int64])
 @pytest.mark.parametrize("outer,block,src_ld,dst_ld,offset", [(1, 1, 1, 1, 0), (64, 5270, 5270, 5272, 0), (9, 13, 13, 16, 1), (257, 6, 9, 8, 2),
                                                               (5000, 942, 1000, 944, 3)])
