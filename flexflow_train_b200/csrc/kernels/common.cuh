@@ -42,10 +42,14 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 // before their first access to global memory; then they let their own successor be launched.  A step of short kernels spends as
 // much time between kernels as in them: launch, block scheduling and, in the tensor-core kernels (which call this after
 // their set-up), barrier initialisation and tensor-memory allocation now run under the previous kernel's tail.  Every block waits,
-// also one without work: a kernel that ended before its predecessor would release its successor too early.
+// also one without work: a kernel that ended before its predecessor would release its successor too early.  A kernel that waits
+// for another GPU does not release: its successor's idle blocks would hold slots that kernels of a side stream, which the
+// peer may be waiting for, need meanwhile.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_entry() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_wait();
+  pdl_release();
 }
 // Kernels that move much data are not launched ahead: their blocks would be placed one by one where the predecessor's leave, three on
 // one SM and one on another, for their whole run (LayerNorm of 8192 x 768: 10.4 us against 8.0; bias gradient of 2048 x 2048: 7.0

@@ -298,7 +298,8 @@ gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmapA, const __grid_consta
   if constexpr (CTA2) cluster_sync_all();  // the partner's barriers exist before anything is signalled across the pair
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_entry();  // the set-up above ran under the previous kernel's tail
+  pdl_wait();  // the set-up above ran under the previous kernel's tail
+  if (!(p.scatter_rows || p.gate_flags || p.push_src)) pdl_release();  // a fused collective waits for its peers: see pdl_wait
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -1299,7 +1300,7 @@ int launch_cfg(const CUtensorMap &ta, const CUtensorMap &tb, const CUtensorMap &
   long long grid = items < max_ctas ? items : max_ctas;
   if (grid < 1) return 0;
   if (args.split_k > 1) args.tma_store = 0;
-  // a fused collective waits for its peers: nothing is launched ahead of its end, and it is not launched ahead itself
+  // a fused collective waits for its peers: it is not launched ahead, and in the kernel it does not release its successor early
   if (args.scatter_rows || args.gate_flags || args.push_src) kern<<<(unsigned)grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, tc, sm, args);
   else ffk_launch(kern, (unsigned)grid, GEMM_THREADS, Cfg::SMEM_BYTES, stream, ta, tb, tc, sm, args);
   return (int)cudaGetLastError();
