@@ -192,10 +192,11 @@ __global__ void softmax_ce_kernel(const T *__restrict__ logits, const L *__restr
   }
 }
 
-// bf16 rows with cols % 8 == 0: the row stays in registers between the loss and the gradient (one block per row, see
-// rowwise_vec.cuh).
+// bf16 rows of up to 4096 with cols % 8 == 0: the row stays in registers between the loss and the gradient (one block per row,
+// see rowwise_vec.cuh).
+constexpr int ROW_THREADS = 128;
 template <int VPT, typename L>
-__global__ void __launch_bounds__(512, 2) softmax_ce_row_kernel(const bf16 *__restrict__ logits, const L *__restrict__ labels,
+__global__ void __launch_bounds__(ROW_THREADS) softmax_ce_row_kernel(const bf16 *__restrict__ logits, const L *__restrict__ labels,
                                                                 bf16 *__restrict__ probs, bf16 *__restrict__ dlogits,
                                                                 float *__restrict__ loss, int cols, float grad_scale) {
   pdl_entry();
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(512, 2) softmax_ce_row_kernel(const bf16 *__re
   const bool valid = label >= 0 && label < cols;
   const float at_label = valid ? bf2f(logits[base + label]) : 0.f;  // before dlogits is written: it may be the same buffer
   float m, s;
-  vec::row_max_sum<VPT>(u, nvec, 1.f, red, m, s);
+  vec::row_max_sum<VPT>(u, nvec, red, m, s);
   const float inv = 1.f / s;
   if (threadIdx.x == 0 && loss) loss[blockIdx.x] = valid ? (__logf(s) + m - at_label) : 0.f;
   if (!probs && !dlogits) return;
@@ -343,6 +344,74 @@ __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__res
       }
     }
     if (++stage == depth) { stage = 0; phase ^= 1; }
+  }
+}
+
+// Rows that the ring does not hold twice (more than 32768, cols % 8 == 0): one pass finds the row's maximum and the sum of exponentials
+// together, a second one over the row, which L2 still holds, writes the results; 16-byte accesses.  Softmax (labels null) or its
+// cross-entropy.  Bound by HBM and the second exponential: 1024 x 128256 takes 145 us (3.6 TB/s) for the loss and 141 for the softmax;
+// the scalar kernels take 584 and 747, the row in registers (64 of them for 16 pieces alone, so it spills) 365 for 2048 x 50304,
+// this one 111.
+template <typename L>
+__global__ void __launch_bounds__(512) softmax_long_kernel(const bf16 *__restrict__ x, const L *__restrict__ labels, bf16 *__restrict__ probs,
+                                                           bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols, float scale,
+                                                           float grad_scale) {
+  pdl_entry();
+  __shared__ float2 red[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int nvec = cols >> 3;
+  for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    const bf16 *px = x + (long long)row * cols;
+    const long long label = labels ? (long long)labels[row] : -1;
+    const bool valid = label >= 0 && label < cols;
+    float m = -INFINITY, s = 0.f;
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+      float v[8];
+      vec::ld8(px + (long long)i * 8, v);
+      float nm = m;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] *= scale;
+        nm = fmaxf(nm, v[j]);
+      }
+      const float sub = nm == -INFINITY ? 0.f : nm;  // nothing but masked elements so far: their exponentials are 0
+      float acc = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc += __expf(v[j] - sub);
+      s = s * __expf(m - sub) + acc;
+      m = nm;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const float om = __shfl_xor_sync(0xffffffffu, m, o), os = __shfl_xor_sync(0xffffffffu, s, o);
+      const float nm = fmaxf(m, om), sub = nm == -INFINITY ? 0.f : nm;
+      s = s * __expf(m - sub) + os * __expf(om - sub);
+      m = nm;
+    }
+    const float at_label = valid && threadIdx.x == 0 ? bf2f(px[label]) : 0.f;  // dlogits may be the same buffer
+    __syncthreads();  // the previous row's readers are done with `red`
+    if (lane == 0) red[wid] = make_float2(m, s);
+    __syncthreads();
+    float M = -INFINITY, S = 0.f;
+    for (int k = 0; k < nw; ++k) M = fmaxf(M, red[k].x);
+    for (int k = 0; k < nw; ++k) S += (red[k].x == -INFINITY && red[k].y == 0.f) ? 0.f : red[k].y * __expf(red[k].x - M);
+    const float inv = 1.f / S;
+    if (threadIdx.x == 0 && loss) loss[row] = valid ? (__logf(S) + M - at_label) : 0.f;
+    if (!probs && !dlogits) continue;
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+      const long long at = (long long)row * cols + (long long)i * 8;
+      float v[8];
+      vec::ld8(px + (long long)i * 8, v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = __expf(v[j] * scale - M) * inv;
+      if (probs) vec::st8(probs + at, v);
+      if (dlogits) {
+        const int hit = valid ? (int)label - i * 8 : -1;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = valid ? (v[j] - (j == hit ? 1.f : 0.f)) * grad_scale : 0.f;
+        vec::st8(dlogits + at, v);
+      }
+    }
   }
 }
 
@@ -592,16 +661,10 @@ FFK_API int ffk_dropout_rows(const void *x, void *y, long long rows, int cols, i
   return (int)cudaGetLastError();
 }
 
-// Block size and vectors per thread of the one-block-per-row kernels: at most 512 threads, the fewest that hold the row in
-// four vectors each (several small blocks per SM overlap one's loads with another's stores).  0 = the row is too long.
-static int row_block(int cols, int &threads) {
-  const int nvec = cols / 8;
-  threads = nvec <= 512 ? 128 : nvec <= 1024 ? 256 : 512;
-  const int v = (nvec + threads - 1) / threads;
-  return v <= 1 ? 1 : v <= 2 ? 2 : v <= 4 ? 4 : v <= 8 ? 8 : v <= 16 ? 16 : 0;
-}
 // The wide-row kernel takes rows of whole 16-byte pieces that fill its threads at least to half and its ring at least twice.
 static bool softmax_wide_ok(int cols, int dt) { return dt == 1 && cols % 8 == 0 && cols > 4096 && cols <= 32768; }
+static bool softmax_long_ok(int cols, int dt) { return dt == 1 && cols % 8 == 0 && cols > 32768; }
+static int long_grid(int rows) { return rows < 148 * 8 ? rows : 148 * 8; }
 template <bool CE, typename L>
 static int launch_softmax_wide(const void *x, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols, float scale,
                                float grad_scale, cudaStream_t st) {
@@ -638,14 +701,11 @@ FFK_API int ffk_softmax_fwd(const void *x, void *y, int rows, int cols, float sc
     return ffk_softmax_dropout_fwd(x, y, nullptr, rows, cols, cols, scale, causal_q, 0.f, 0, nullptr, dt, st);
   if (softmax_wide_ok(cols, dt) && causal_q <= 0 && aligned16(x) && aligned16(y))
     return launch_softmax_wide<false, int>(x, nullptr, y, nullptr, nullptr, rows, cols, scale, 1.f, st);
-  int threads, vpt;
-  if (dt == 1 && cols % 8 == 0 && causal_q <= 0 && aligned16(x) && aligned16(y) && (vpt = row_block(cols, threads)) != 0) {
-    // only rows beyond the wide kernel's come here (the shorter ones took the warp kernel)
-    if (vpt <= 8) ffk_launch(vec::softmax_fwd_row_kernel<8>, rows, threads, 0, st, (const bf16 *)x, (bf16 *)y, cols, scale);
-    else ffk_launch(vec::softmax_fwd_row_kernel<16>, rows, threads, 0, st, (const bf16 *)x, (bf16 *)y, cols, scale);
+  if (softmax_long_ok(cols, dt) && causal_q <= 0 && aligned16(x) && aligned16(y)) {
+    ffk_launch(softmax_long_kernel<int>, long_grid(rows), 512, 0, st, (const bf16 *)x, nullptr, (bf16 *)y, nullptr, nullptr, rows, cols, scale, 1.f);
     return (int)cudaGetLastError();
   }
-  threads = cols >= 1024 ? 256 : 128;
+  const int threads = cols >= 1024 ? 256 : 128;
   DISPATCH_FLOAT(dt, (ffk_launch(softmax_fwd_kernel<T>, rows < 148 * 16 ? rows : 148 * 16, threads, 0, st, 
                          (const T *)x, (T *)y, rows, cols, scale, causal_q)));
   return (int)cudaGetLastError();
@@ -661,36 +721,34 @@ FFK_API int ffk_softmax_bwd(const void *dy, const void *y, void *dx, int rows, i
                          (const T *)dy, (const T *)y, (T *)dx, rows, cols, scale)));
   return (int)cudaGetLastError();
 }
-template <int VPT>
+template <int VPT, typename L>
 static void launch_softmax_ce_row(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols,
-                                  float grad_scale, int label_dt, int threads, cudaStream_t st) {
-  if (label_dt == 3)
-    ffk_launch(softmax_ce_row_kernel<VPT, long long>, rows, threads, 0, st, (const bf16 *)logits, (const long long *)labels, (bf16 *)probs,
-                                                                    (bf16 *)dlogits, loss, cols, grad_scale);
-  else
-    ffk_launch(softmax_ce_row_kernel<VPT, int>, rows, threads, 0, st, (const bf16 *)logits, (const int *)labels, (bf16 *)probs, (bf16 *)dlogits, loss,
-                                                              cols, grad_scale);
+                                  float grad_scale, cudaStream_t st) {
+  ffk_launch(softmax_ce_row_kernel<VPT, L>, rows, ROW_THREADS, 0, st, (const bf16 *)logits, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss,
+             cols, grad_scale);
+}
+// bf16 rows of whole 16-byte pieces: in registers up to 4096, through the ring up to 32768, in two passes beyond
+template <typename L>
+static int launch_softmax_ce(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols, float grad_scale,
+                             cudaStream_t st) {
+  if (softmax_wide_ok(cols, 1)) return launch_softmax_wide<true, L>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st);
+  if (softmax_long_ok(cols, 1))
+    ffk_launch(softmax_long_kernel<L>, long_grid(rows), 512, 0, st, (const bf16 *)logits, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss, rows,
+               cols, 1.f, grad_scale);
+  else if (cols <= 8 * ROW_THREADS) launch_softmax_ce_row<1, L>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, st);
+  else if (cols <= 16 * ROW_THREADS) launch_softmax_ce_row<2, L>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, st);
+  else launch_softmax_ce_row<4, L>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, st);
+  return (int)cudaGetLastError();
 }
 // label_dt: 2 = int32, 3 = int64
 FFK_API int ffk_softmax_ce(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows,
                            int cols, float grad_scale, int dt, int label_dt, cudaStream_t st) {
   if (rows <= 0) return 0;
   FfkTraffic traffic((long long)rows * cols * (dt == 1 ? 2 : 4) * 2);
-  if (softmax_wide_ok(cols, dt) && aligned16(logits) && aligned16(probs) && aligned16(dlogits))
-    return label_dt == 3 ? launch_softmax_wide<true, long long>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st)
-                         : launch_softmax_wide<true, int>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st);
-  int threads, vpt;
-  if (dt == 1 && cols % 8 == 0 && aligned16(logits) && aligned16(probs) && aligned16(dlogits) && (vpt = row_block(cols, threads)) != 0) {
-    switch (vpt) {
-      case 1: launch_softmax_ce_row<1>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
-      case 2: launch_softmax_ce_row<2>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
-      case 4: launch_softmax_ce_row<4>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
-      case 8: launch_softmax_ce_row<8>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
-      default: launch_softmax_ce_row<16>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, label_dt, threads, st); break;
-    }
-    return (int)cudaGetLastError();
-  }
-  threads = cols >= 4096 ? 1024 : 256;
+  if (dt == 1 && cols % 8 == 0 && aligned16(logits) && aligned16(probs) && aligned16(dlogits))
+    return label_dt == 3 ? launch_softmax_ce<long long>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, st)
+                         : launch_softmax_ce<int>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, st);
+  const int threads = cols >= 4096 ? 1024 : 256;
   const int grid = rows < 148 * 4 ? rows : 148 * 4;
   DISPATCH_FLOAT(dt, {
     if (label_dt == 3)

@@ -159,7 +159,7 @@ static __global__ void dropout_rows_kernel(const bf16 *__restrict__ x, bf16 *__r
   }
 }
 
-// ---------------------------------------------------------------- softmax over rows of one block each
+// ---------------------------------------------------------------- rows of one block each
 // The row (cols % 8 == 0, up to 8 * VPT * blockDim.x) stays packed in registers between the maximum, the sum and the result, so
 // HBM sees one read and one write.
 template <int VPT>
@@ -170,9 +170,9 @@ __device__ __forceinline__ void row_load(const bf16 *p, int nvec, uint4 (&u)[VPT
     if (c < nvec) u[i] = reinterpret_cast<const uint4 *>(p)[c];
   }
 }
-// maximum of the row's values times scale, and the sum of exp(value * scale - maximum); `red`: 64 floats of shared memory
+// maximum of the row's values and the sum of exp(value - maximum); `red`: 64 floats of shared memory
 template <int VPT>
-__device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, float scale, float *red, float &mx, float &sum) {
+__device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, float *red, float &mx, float &sum) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float m = -INFINITY;
 #pragma unroll
@@ -181,7 +181,7 @@ __device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, flo
       float v[8];
       unpack8(u[i], v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) m = fmaxf(m, v[j] * scale);
+      for (int j = 0; j < 8; ++j) m = fmaxf(m, v[j]);
     }
   m = warp_max(m);
   if (lane == 0) red[wid] = m;
@@ -196,7 +196,7 @@ __device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, flo
       unpack8(u[i], v);
       float a = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) a += __expf(v[j] * scale - m);
+      for (int j = 0; j < 8; ++j) a += __expf(v[j] - m);
       s += a;
     }
   s = warp_sum(s);
@@ -207,30 +207,6 @@ __device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, flo
   mx = m;
   sum = s;
 }
-template <int VPT>
-__global__ void __launch_bounds__(512, 2) softmax_fwd_row_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, int cols, float scale) {
-  pdl_entry();
-  __shared__ float red[64];
-  const int nvec = cols >> 3;
-  const long long base = (long long)blockIdx.x * cols;
-  uint4 u[VPT];
-  row_load<VPT>(x + base, nvec, u);
-  float m, s;
-  row_max_sum<VPT>(u, nvec, scale, red, m, s);
-  const float inv = 1.f / s;
-#pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int c = i * blockDim.x + threadIdx.x;
-    if (c < nvec) {
-      float v[8];
-      unpack8(u[i], v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = __expf(v[j] * scale - m) * inv;
-      st8(y + base + c * 8, v);
-    }
-  }
-}
-
 // ---------------------------------------------------------------- LayerNorm: one block per row
 // cols = 8 * blockDim.x * VPT.  y = LN(a + b) * gamma + beta, xsum = a + b (when b is given).
 template <int VPT>

@@ -41,6 +41,42 @@ def test_softmax_and_cross_entropy_rows(cols, rows):
     assert K.softmax_last_error() == 0
 
 
+@pytest.mark.parametrize("cols", [4096, 8192, 32776, 65544, 131072])
+def test_rows_with_masked_pieces(cols):
+    """Whole pieces, and a thread's and a warp's whole share of the row, masked out."""
+    x = torch.randn(6, cols, generator=torch.Generator(device="cuda").manual_seed(cols), device="cuda").bfloat16()
+    x[0, :8], x[1, 8:], x[2, :cols - 8], x[3, : cols // 2] = (float("-inf"),) * 4
+    ref = torch.softmax(x.double(), -1)
+    _near(K.softmax_fwd(x), ref)
+    labels = torch.tensor([9, 3, cols - 1, cols - 2, 0, -1], device="cuda")
+    loss, probs = torch.empty(6, device="cuda"), torch.empty_like(x)
+    K.softmax_ce(x, labels, loss, x, probs)  # the gradient in the place of the logits
+    _near(probs, ref)
+    want = -torch.log(ref.gather(1, labels.clamp(min=0)[:, None]))[:, 0]
+    want[5] = 0
+    assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5)
+
+
+def test_vocabularies_beyond_the_ring_keep_its_rate():
+    """The same number of elements in rows of 131072 as in rows of 32768: a scalar form of the long rows takes several times as long."""
+    def us(rows, cols, fn):
+        x = torch.randn(rows, cols, device="cuda").bfloat16()
+        labels = torch.zeros(rows, device="cuda", dtype=torch.int32)
+        loss, dl = torch.empty(rows, device="cuda"), torch.empty_like(x)
+        got = []
+        for _ in range(8):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            K.softmax_ce(x, labels, loss, dl) if fn == "ce" else K.softmax_fwd(x, out=dl)
+            e1.record()
+            e1.synchronize()
+            got.append(e0.elapsed_time(e1))
+        return sorted(got)[3]
+
+    for fn in ("ce", "softmax"):
+        assert us(1024, 131072, fn) < 2.5 * us(4096, 32768, fn), fn
+
+
 @pytest.mark.parametrize("cols", [1, 7, 9, 250, 255, 257, 500, 1001, 4090])
 @pytest.mark.parametrize("causal", [False, True])
 def test_pitched_softmax_dropout(cols, causal):
