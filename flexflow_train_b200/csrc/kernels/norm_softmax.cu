@@ -244,7 +244,7 @@ __device__ int g_rows_err = 0;
 template <bool CE, typename L>
 __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__restrict__ x, const L *__restrict__ labels, bf16 *__restrict__ probs,
                                                                bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols,
-                                                               float scale, float grad_scale, int depth) {
+                                                               float scale, float grad_scale, int depth, unsigned long long wait_ns) {
   pdl_entry();
   extern __shared__ __align__(128) uint8_t wide_smem[];
   __shared__ float red[64];
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__res
   int stage = 0;
   uint32_t phase = 0;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
-    const bool ok = mbar_wait(&full[stage], phase, &abort_flag, &g_rows_err, FFK_ERR_TIMEOUT_PRODUCER);
+    const bool ok = mbar_wait(&full[stage], phase, &abort_flag, &g_rows_err, FFK_ERR_TIMEOUT_PRODUCER, wait_ns);
     const uint4 *src = reinterpret_cast<const uint4 *>(wide_smem + (size_t)stage * row_bytes);
     float v[WIDE_VPT][8];
     float m = -INFINITY;
@@ -297,14 +297,24 @@ __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__res
     }
     m = warp_max(m);
     if (lane == 0) red[wid] = m;
-    // past this barrier the row's stage is free; a copy that never came (ok is false) ends the block here
+    // past this barrier the row's stage is free; a copy that did not come (ok is false) ends the block here
     if (__syncthreads_or(!ok)) {
-      if (threadIdx.x == 0)   // the other stages' copies land, or a second limit runs out, before the shared memory goes away
-        for (int k = 0; k < depth; ++k) {
+      if (threadIdx.x == 0)   // the copies in flight land, or a second limit runs out, before the shared memory goes away
+        for (int a = 0; a < depth && row + (long long)a * gridDim.x < rows; ++a) {
+          const int k = stage + a < depth ? stage + a : stage + a - depth;
           const uint64_t t0 = ffk_globaltimer();
           while (!mbar_try_wait(&full[k], k >= stage ? phase : phase ^ 1) && ffk_globaltimer() - t0 < WAIT_LIMIT_NS) {}
         }
       __syncthreads();
+      // the rows this block leaves undone are no numbers, so that what an earlier call left there does not pass for results
+      const uint4 nan8 = make_uint4(0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu, 0x7FFF7FFFu);
+      for (long long r = row; r < rows; r += gridDim.x) {
+        if (CE && threadIdx.x == 0 && loss) loss[r] = __int_as_float(0x7FFFFFFF);
+        for (int c = threadIdx.x; c < nvec; c += blockDim.x) {
+          if (probs) reinterpret_cast<uint4 *>(probs + r * cols)[c] = nan8;
+          if (CE && dlogits) reinterpret_cast<uint4 *>(dlogits + r * cols)[c] = nan8;
+        }
+      }
       return;
     }
     if (threadIdx.x == 0 && row + (long long)depth * gridDim.x < rows) fetch((int)(row + (long long)depth * gridDim.x), stage);
@@ -667,7 +677,7 @@ static bool softmax_long_ok(int cols, int dt) { return dt == 1 && cols % 8 == 0 
 static int long_grid(int rows) { return rows < 148 * 8 ? rows : 148 * 8; }
 template <bool CE, typename L>
 static int launch_softmax_wide(const void *x, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols, float scale,
-                               float grad_scale, cudaStream_t st) {
+                               float grad_scale, cudaStream_t st, unsigned long long wait_ns = WAIT_LIMIT_NS) {
   auto kern = softmax_wide_kernel<CE, L>;
   static bool attr_done = false;
   if (!attr_done) {
@@ -681,7 +691,7 @@ static int launch_softmax_wide(const void *x, const void *labels, void *probs, v
   if (depth > 4) depth = 4;
   const int grid = rows < 148 * per_sm ? rows : 148 * per_sm;
   ffk_launch(kern, grid, threads, (size_t)depth * cols * 2, st, (const bf16 *)x, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss, rows, cols,
-                                                        scale, grad_scale, depth);
+                                                        scale, grad_scale, depth, wait_ns);
   return (int)cudaGetLastError();
 }
 // Error word of the wide-row kernel's bounded waits (read and cleared; synchronises the device).
@@ -759,6 +769,12 @@ FFK_API int ffk_softmax_ce(const void *logits, const void *labels, void *probs, 
                                                            (T *)dlogits, loss, rows, cols, grad_scale);
   });
   return (int)cudaGetLastError();
+}
+// The wide-row cross-entropy with another limit of its waits: 0 lets the first one run out, so that a test sees what then comes back.
+FFK_API int ffk_softmax_ce_wait(const void *logits, const int *labels, void *probs, void *dlogits, float *loss, int rows, int cols,
+                                unsigned long long wait_ns, cudaStream_t st) {
+  if (rows <= 0 || !softmax_wide_ok(cols, 1) || !aligned16(logits) || !aligned16(probs) || !aligned16(dlogits)) return -2;
+  return launch_softmax_wide<true, int>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, 1.f, st, wait_ns);
 }
 FFK_API int ffk_loss_bwd(int kind, const void *pred, const void *target, void *dpred, long long rows, int cols,
                          float scale, int dt, int label_dt, cudaStream_t st) {

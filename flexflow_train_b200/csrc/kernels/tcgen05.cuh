@@ -34,17 +34,17 @@ static __device__ __forceinline__ uint32_t mbar_try_wait(uint64_t *bar, uint32_t
       : "memory");
   return ok;
 }
-// Bounded wait.  Returns false when the limit ran out or another role aborted.
+// Bounded wait.  Returns false when the limit ran out (0: it has, whatever the barrier's state) or another role aborted.
 static __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
-                                          int *err, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
+                                          int *err, int code, uint64_t limit_ns = WAIT_LIMIT_NS) {
+  if (limit_ns != 0 && mbar_try_wait(bar, parity)) return true;
   uint64_t t0 = ffk_globaltimer();
   uint32_t spins = 0;
   while (true) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (limit_ns != 0 && mbar_try_wait(bar, parity)) return true;
     if ((++spins & 63u) == 0) {
       if (*abort_flag) return false;
-      if (ffk_globaltimer() - t0 > WAIT_LIMIT_NS) {
+      if (ffk_globaltimer() - t0 > limit_ns) {
         *abort_flag = 1;
         if (err) atomicCAS(err, 0, code);
         return false;

@@ -949,8 +949,19 @@ def softmax_pitch(cols: int) -> int:
 
 
 def softmax_last_error() -> int:
-    """Error word of the wide-row softmax kernel's bounded waits (0: none ran out)."""
+    """Error word of the wide-row softmax kernel's bounded waits (0: none ran out).  Rows left undone hold NaN."""
     return lib().ffk_softmax_last_error()
+
+
+def softmax_ce_wait(logits, labels, loss, dlogits, probs, wait_ns: int):
+    """`softmax_ce` of wide bf16 rows with int32 labels, whose kernel waits `wait_ns` nanoseconds for a row (0: gives up at once)."""
+    _cuda_contig(logits, labels, loss, dlogits, probs)
+    rows, cols = logits.shape
+    if logits.dtype != torch.bfloat16 or labels.dtype != torch.int32 or labels.numel() < rows or loss.numel() < rows:
+        raise KernelError("softmax_ce_wait: bf16 rows, one int32 label and one loss each expected")
+    l = _sdlib()
+    _check(l.ffk_softmax_ce_wait(logits.data_ptr(), labels.data_ptr(), _p(probs), _p(dlogits), loss.data_ptr(), rows, cols, wait_ns, _stream()),
+           "ffk_softmax_ce_wait")
 
 
 def _decl_softmax_dropout(l):
@@ -961,6 +972,8 @@ def _decl_softmax_dropout(l):
     l.ffk_softmax_dropout_bwd.restype = c_int
     l.ffk_dropout_rows.argtypes = [P, P, c_longlong, I, I, F, c_ulonglong, P, S]
     l.ffk_dropout_rows.restype = c_int
+    l.ffk_softmax_ce_wait.argtypes = [P, P, P, P, P, I, I, c_ulonglong, S]
+    l.ffk_softmax_ce_wait.restype = c_int
 
 
 _sd_declared = [False]

@@ -57,6 +57,20 @@ def test_rows_with_masked_pieces(cols):
     assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5)
 
 
+@pytest.mark.parametrize("rows,cols", [(5, 4104), (700, 8192), (300, 32768)])
+def test_rows_given_up_hold_no_numbers(rows, cols):
+    """A wait that runs out must not leave an earlier call's values in the place of results."""
+    x = torch.randn(rows, cols, device="cuda").bfloat16()
+    labels = torch.zeros(rows, device="cuda", dtype=torch.int32)
+    loss, dl, probs = torch.ones(rows, device="cuda"), torch.ones_like(x), torch.ones_like(x)
+    K.softmax_ce_wait(x, labels, loss, dl, probs, 0)
+    assert K.softmax_last_error() != 0 and K.softmax_last_error() == 0  # read and cleared
+    assert loss.isnan().all() and dl.isnan().all() and probs.isnan().all()
+    K.softmax_ce_wait(x, labels, loss, dl, probs, 10**9)
+    _near(probs, torch.softmax(x.double(), -1))
+    assert K.softmax_last_error() == 0 and loss.isfinite().all() and dl.isfinite().all()
+
+
 def test_vocabularies_beyond_the_ring_keep_its_rate():
     """The same number of elements in rows of 131072 as in rows of 32768: a scalar form of the long rows takes several times as long."""
     def us(rows, cols, fn):
