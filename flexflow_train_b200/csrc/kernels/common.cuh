@@ -78,6 +78,17 @@ static inline int ffk_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t
   return (int)cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// Lets `kernel` take `bytes` of dynamic shared memory on the current device; `done` (one bit per device) remembers where it may.
+template <typename K>
+static inline cudaError_t ffk_allow_smem(K kernel, int bytes, unsigned long long &done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (done >> (dev & 63) & 1)) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done |= 1ull << (dev & 63);
+  return e;
+}
+
 __device__ __forceinline__ float bf2f(bf16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ bf16 f2bf(float v) { return __float2bfloat16_rn(v); }
 

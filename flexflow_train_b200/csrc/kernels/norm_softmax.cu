@@ -679,12 +679,8 @@ template <bool CE, typename L>
 static int launch_softmax_wide(const void *x, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols, float scale,
                                float grad_scale, cudaStream_t st, unsigned long long wait_ns = WAIT_LIMIT_NS) {
   auto kern = softmax_wide_kernel<CE, L>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, WIDE_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
+  static unsigned long long done = 0;
+  if (cudaError_t e = ffk_allow_smem(kern, WIDE_SMEM, done)) return (int)e;
   const int threads = cols <= 8192 ? 256 : cols <= 16384 ? 512 : 1024;   // at most four pieces of 8 per thread
   const int per_sm = 1024 / threads;
   int depth = WIDE_SMEM / per_sm / (cols * 2);

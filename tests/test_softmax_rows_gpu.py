@@ -71,6 +71,14 @@ def test_rows_given_up_hold_no_numbers(rows, cols):
     assert K.softmax_last_error() == 0 and loss.isfinite().all() and dl.isfinite().all()
 
 
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_wide_rows_on_every_device_of_a_process():
+    for dev in range(2):
+        with torch.cuda.device(dev):
+            x = torch.randn(3, 8192, device="cuda").bfloat16()
+            _near(K.softmax_fwd(x), torch.softmax(x.double(), -1))
+
+
 def test_vocabularies_beyond_the_ring_keep_its_rate():
     """The same number of elements in rows of 131072 as in rows of 32768: a scalar form of the long rows takes several times as long."""
     def us(rows, cols, fn):
