@@ -17,6 +17,7 @@ Differences from the reference that matter for speed:
 """
 from __future__ import annotations
 
+import gc
 import math
 from dataclasses import dataclass, field
 from typing import Callable, Dict, List, Optional, Tuple
@@ -1736,19 +1737,39 @@ class Executable:
         if not (self.cfg.use_cuda_graph and self.on_gpu and self.dist is None) or self.cfg.profile_layers \
                 or torch.cuda.is_current_stream_capturing():
             return self.forward()
+        if not self._fwd_warmed:  # lazy library initialisation must not happen during capture
+            self._fwd_warmed = True
+            return self.forward()
         if self._fwd_graph is None:
-            if not self._fwd_warmed:  # lazy library initialisation must not happen during capture
-                self._fwd_warmed = True
-                return self.forward()
-            graph = torch.cuda.CUDAGraph()
-            cap_stream = torch.cuda.Stream()
-            cap_stream.wait_stream(torch.cuda.current_stream())
-            # thread_local: other threads of the process may allocate while this one captures
-            with torch.cuda.graph(graph, stream=cap_stream, capture_error_mode="thread_local"):
-                self.forward()
-            torch.cuda.current_stream().wait_stream(cap_stream)
-            self._fwd_graph = graph
+            self._fwd_graph = self._capture_forward() or False
+        if self._fwd_graph is False:
+            return self.forward()
         self._fwd_graph.replay()
+
+    def _capture_forward(self):
+        """The forward pass as a CUDA graph; None where the graph's own pool finds no memory for what operators allocate as they go, which
+        leaves the forward eager.  Captured without what `torch.cuda.graph` does before a capture: other threads' work and cached
+        memory stay as they are (no device synchronisation, no emptied cache)."""
+        graph, complete = torch.cuda.CUDAGraph(), True
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        collecting = gc.isenabled()
+        gc.disable()  # a graph or stream that a collection frees must not be destroyed during the capture
+        try:
+            with torch.cuda.stream(side):
+                # thread_local: other threads of the process may allocate while this one captures
+                graph.capture_begin(capture_error_mode="thread_local")
+                try:
+                    self.forward()
+                except torch.cuda.OutOfMemoryError:
+                    complete = False
+                finally:
+                    graph.capture_end()
+        finally:
+            if collecting:
+                gc.enable()
+        torch.cuda.current_stream().wait_stream(side)
+        return graph if complete else None
 
     def infer(self, inputs: Dict[str, torch.Tensor]):
         self.set_inputs(inputs)

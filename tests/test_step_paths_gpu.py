@@ -40,6 +40,39 @@ def test_forward_inside_a_callers_capture():
     assert torch.equal(y, want)
 
 
+def test_capturing_the_forward_leaves_the_process_alone(monkeypatch):
+    """The call that captures neither synchronises the device nor empties the allocator's cache under other threads."""
+    m = api.compile("mlp", {"batch_size": 4, "input_dim": 16}, training=False)
+    x = torch.randn(4, 16, device="cuda")
+    want, calls = m.forward({"input": x}).clone(), []
+    for name in ("synchronize", "empty_cache"):
+        monkeypatch.setattr(torch.cuda, name, lambda *a, name=name, **k: calls.append(name))
+    got = m.forward({"input": x}).clone()
+    monkeypatch.undo()
+    assert not calls and torch.equal(got, want) and torch.equal(m.forward({"input": x}), want)
+    assert m.executable._fwd_graph
+
+
+def test_forward_stays_eager_without_memory_for_a_graph(monkeypatch):
+    """Operators that allocate as they go find their memory in the cache; a graph's pool, which has to have its own, may not."""
+    m = api.compile("mlp", {"batch_size": 4, "input_dim": 16}, training=False)
+    eager = Executable(m.graph, ExecConfig(training=False, use_cuda_graph=False))
+    eager.load_state_dict(m.state_dict())
+    op = next(o for o in m.executable.ops.values() if o.type == "LINEAR")
+    plain = op.forward
+
+    def allocates():
+        plain()
+        if torch.cuda.is_current_stream_capturing():
+            raise torch.cuda.OutOfMemoryError("no memory left")
+
+    monkeypatch.setattr(op, "forward", allocates)
+    for _ in range(3):
+        x = torch.randn(4, 16, device="cuda")
+        assert torch.equal(m.forward({"input": x}), eager.infer({"input": x}))
+    assert torch.randn(3, device="cuda").isfinite().all()  # the generator is not left inside a capture
+
+
 @pytest.mark.parametrize("n", [1, 7, 4096, 4099, 16384 * 3 + 5])
 @pytest.mark.parametrize("offset", [0, 1])  # 1: no 16-byte alignment
 def test_stage_batch_copies_and_casts_like_copy(n, offset):
