@@ -942,7 +942,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // ================================================================================================ backward
 // delta[b, h, q] = sum_c dO[b, q, h, c] * O[b, q, h, c]; one warp per (row, head)
 template <int D>
-__global__ void attn_delta_kernel(const bf16 *__restrict__ dO, long long lddo, const bf16 *__restrict__ O, long long ldo,
+__global__ void attn_delta_kernel(const bf16 *dO, long long lddo, const bf16 *O, long long ldo,
                                   float *__restrict__ delta, int B, int H, int Sq) {
   pdl_entry();
   const int lane = threadIdx.x & 31;
@@ -972,7 +972,7 @@ __global__ void attn_delta_kernel(const bf16 *__restrict__ dO, long long lddo, c
 
 // fp32 accumulators [B, H, Sk, D] -> bf16 [B*Sk, ld] (head h at columns h*D)
 template <int D>
-__global__ void attn_acc_to_bf16_kernel(const float *__restrict__ acc, bf16 *__restrict__ out, long long ld, int B, int H, int Sk) {
+__global__ void attn_acc_to_bf16_kernel(const float *acc, bf16 *__restrict__ out, long long ld, int B, int H, int Sk) {
   pdl_entry();
   const long long total = (long long)B * H * Sk * (D / 4);
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {

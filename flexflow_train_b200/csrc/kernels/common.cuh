@@ -45,9 +45,16 @@ __device__ __forceinline__ uint32_t smem_u32(const void *p) {
 // also one without work: a kernel that ended before its predecessor would release its successor too early.  A kernel that waits
 // for another GPU does not release: its successor's idle blocks would hold slots that kernels of a side stream, which the
 // peer may be waiting for, need meanwhile.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_entry() {
+//
+// What a kernel reads may be written by its predecessor while it is already running.  So a pointer it only reads through is not
+// __restrict__ (that would let the compiler take it for constant during the whole kernel, fetch it through the non-coherent path or
+// ahead of the wait); outputs keep theirs, and the ones that are also read (an accumulated gradient, a weight) are handed to
+// pdl_entry, which keeps their loads behind it.
+__device__ __forceinline__ void pdl_wait() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void pdl_release() { cudaTriggerProgrammaticLaunchCompletion(); }
+template <typename... P>
+__device__ __forceinline__ void pdl_entry(P *...io) {
+  (..., [](const void *p) { asm volatile("" ::"l"(p) : "memory"); }(io));
   pdl_wait();
   pdl_release();
 }

@@ -60,7 +60,7 @@ __device__ __forceinline__ void split3(long long t, const FastDiv &f_c8, const F
 
 // ------------------------------------------------------------------------------------------- im2col
 // vector path: bf16 channels-last, C % 8 == 0; one thread moves 8 channels (16 bytes)
-__global__ void im2col_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ col, ConvGeom g, long long total) {
+__global__ void im2col_vec_kernel(const bf16 *x, bf16 *__restrict__ col, ConvGeom g, long long total) {
   pdl_entry();
   const int c8n = g.C >> 3, kk_n = g.KH * g.KW;
   const bool small = total < (1ll << 31);
@@ -96,7 +96,7 @@ __global__ void im2col_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__
 }
 // generic path: any strides / dtype; one thread per (row, k) including the zero padding columns
 template <typename T>
-__global__ void im2col_kernel(const T *__restrict__ x, bf16 *__restrict__ col, ConvGeom g, long long total) {
+__global__ void im2col_kernel(const T *x, bf16 *__restrict__ col, ConvGeom g, long long total) {
   pdl_entry();
   const int K = g.KH * g.KW * g.C;
   const bool small = total < (1ll << 31);
@@ -139,8 +139,8 @@ __global__ void im2col_kernel(const T *__restrict__ x, bf16 *__restrict__ col, C
 // ------------------------------------------------------------------------------------------- col2im (gather form)
 // dx[n, ih, iw, c] (+)= sum over (kh, kw) with (ih + PH - kh) % SH == 0 ... of dcol[(n, oh, ow), (kh, kw, c)]
 template <typename T>
-__global__ void col2im_kernel(const bf16 *__restrict__ dcol, T *__restrict__ dx, ConvGeom g, long long total, int accumulate) {
-  pdl_entry();
+__global__ void col2im_kernel(const bf16 *dcol, T *__restrict__ dx, ConvGeom g, long long total, int accumulate) {
+  pdl_entry(dx);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % g.C);
     long long r = t / g.C;
@@ -169,8 +169,8 @@ __global__ void col2im_kernel(const bf16 *__restrict__ dcol, T *__restrict__ dx,
   }
 }
 // vector form: bf16 channels-last output, C % 8 == 0
-__global__ void col2im_vec_kernel(const bf16 *__restrict__ dcol, bf16 *__restrict__ dx, ConvGeom g, long long total, int accumulate) {
-  pdl_entry();
+__global__ void col2im_vec_kernel(const bf16 *dcol, bf16 *__restrict__ dx, ConvGeom g, long long total, int accumulate) {
+  pdl_entry(dx);
   const int c8n = g.C >> 3;
   const bool small = total < (1ll << 31);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -213,7 +213,7 @@ __global__ void col2im_vec_kernel(const bf16 *__restrict__ dcol, bf16 *__restric
 // ------------------------------------------------------------------------------------------- filter repacking
 // w [OC, C, KH, KW] -> wp [OC, Kp] with k = (kh*KW + kw)*C + c (zero padding columns)
 template <typename T>
-__global__ void filter_pack_kernel(const T *__restrict__ w, bf16 *__restrict__ wp, int OC, int C, int KH, int KW, int Kp) {
+__global__ void filter_pack_kernel(const T *w, bf16 *__restrict__ wp, int OC, int C, int KH, int KW, int Kp) {
   pdl_entry();
   long long total = (long long)OC * Kp;
   int K = C * KH * KW;
@@ -230,9 +230,9 @@ __global__ void filter_pack_kernel(const T *__restrict__ w, bf16 *__restrict__ w
 }
 // dwp [OC, Kp] (fp32) -> dw [OC, C, KH, KW] (+)=
 template <typename T>
-__global__ void filter_unpack_kernel(const float *__restrict__ dwp, T *__restrict__ dw, int OC, int C, int KH, int KW, int Kp,
+__global__ void filter_unpack_kernel(const float *dwp, T *__restrict__ dw, int OC, int C, int KH, int KW, int Kp,
                                      int accumulate) {
-  pdl_entry();
+  pdl_entry(dw);
   long long total = (long long)OC * C * KH * KW;
   int KK = KH * KW;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -250,7 +250,7 @@ __global__ void filter_unpack_kernel(const float *__restrict__ dwp, T *__restric
 // output channels-last [N, OH, OW, C]; input with arbitrary strides.  mode 0 = max (argmax window offset saved),
 // 1 = average over the valid (unpadded) window elements.
 template <typename T>
-__global__ void pool_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, unsigned char *__restrict__ arg, ConvGeom g, int mode,
+__global__ void pool_fwd_kernel(const T *x, T *__restrict__ y, unsigned char *__restrict__ arg, ConvGeom g, int mode,
                                 long long total) {
   pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -285,9 +285,9 @@ __global__ void pool_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, unsi
 }
 // gather-form backward: one thread per input element
 template <typename T>
-__global__ void pool_bwd_kernel(const T *__restrict__ dy, const unsigned char *__restrict__ arg, T *__restrict__ dx, ConvGeom g, int mode,
+__global__ void pool_bwd_kernel(const T *dy, const unsigned char *arg, T *__restrict__ dx, ConvGeom g, int mode,
                                 long long total, int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % g.C);
     long long r = t / g.C;
@@ -328,8 +328,8 @@ __global__ void pool_bwd_kernel(const T *__restrict__ dy, const unsigned char *_
 constexpr int BN_TX = 32, BN_TY = 8;
 
 template <typename T>
-__global__ void bn_partial_kernel(const T *__restrict__ a, const T *__restrict__ b, const T *__restrict__ relu_y, float *__restrict__ part,
-                                  const float *__restrict__ mean, const float *__restrict__ rstd, long long R, int C, int rows_per_chunk,
+__global__ void bn_partial_kernel(const T *a, const T *b, const T *relu_y, float *__restrict__ part,
+                                  const float *mean, const float *rstd, long long R, int C, int rows_per_chunk,
                                   int mode) {
   pdl_entry();
   // mode 0: sums of a and a*a (forward statistics)
@@ -366,7 +366,7 @@ __global__ void bn_partial_kernel(const T *__restrict__ a, const T *__restrict__
 }
 // Fold the per-chunk partial sums: block = 32 columns x BN_FOLD chunk lanes, fixed summation order.
 constexpr int BN_FOLD = 32;
-__device__ __forceinline__ void bn_fold(const float *__restrict__ part, int chunks, int C, int c, float &s, float &q) {
+__device__ __forceinline__ void bn_fold(const float *part, int chunks, int C, int c, float &s, float &q) {
   __shared__ float fs[BN_FOLD][33], fq[BN_FOLD][33];
   float a = 0.f, b = 0.f;
   if (c < C)
@@ -381,7 +381,7 @@ __device__ __forceinline__ void bn_fold(const float *__restrict__ part, int chun
   if (threadIdx.y == 0)
     for (int i = 0; i < BN_FOLD; ++i) { s += fs[i][threadIdx.x]; q += fq[i][threadIdx.x]; }
 }
-__global__ void bn_finalize_stats_kernel(const float *__restrict__ part, int chunks, int C, long long R, float eps, float *__restrict__ mean,
+__global__ void bn_finalize_stats_kernel(const float *part, int chunks, int C, long long R, float eps, float *__restrict__ mean,
                                          float *__restrict__ rstd) {
   pdl_entry();
   int c = blockIdx.x * 32 + threadIdx.x;
@@ -396,9 +396,9 @@ __global__ void bn_finalize_stats_kernel(const float *__restrict__ part, int chu
 }
 // sums[0][c] = sum dy, sums[1][c] = sum dy*xhat; also writes dgamma/dbeta (+)= when given
 template <typename T>
-__global__ void bn_finalize_grads_kernel(const float *__restrict__ part, int chunks, int C, float *__restrict__ sums, T *__restrict__ dgamma,
+__global__ void bn_finalize_grads_kernel(const float *part, int chunks, int C, float *__restrict__ sums, T *__restrict__ dgamma,
                                          T *__restrict__ dbeta, int acc_gamma, int acc_beta) {
-  pdl_entry();
+  pdl_entry(dgamma, dbeta);
   int c = blockIdx.x * 32 + threadIdx.x;
   float s, q;
   bn_fold(part, chunks, C, c, s, q);
@@ -409,8 +409,8 @@ __global__ void bn_finalize_grads_kernel(const float *__restrict__ part, int chu
   if (dgamma) stf(dgamma + c, q + (acc_gamma ? ldf(dgamma + c) : 0.f));
 }
 template <typename T>
-__global__ void bn_apply_kernel(const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ gamma, const T *__restrict__ beta,
-                                const float *__restrict__ mean, const float *__restrict__ rstd, long long total, int C, int relu) {
+__global__ void bn_apply_kernel(const T *x, T *__restrict__ y, const T *gamma, const T *beta,
+                                const float *mean, const float *rstd, long long total, int C, int relu) {
   pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % C);
@@ -422,8 +422,8 @@ __global__ void bn_apply_kernel(const T *__restrict__ x, T *__restrict__ y, cons
   }
 }
 // two elements per thread for bf16 with even C
-__global__ void bn_apply_bf16x2_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, const bf16 *__restrict__ gamma,
-                                       const bf16 *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd,
+__global__ void bn_apply_bf16x2_kernel(const bf16 *x, bf16 *__restrict__ y, const bf16 *gamma,
+                                       const bf16 *beta, const float *mean, const float *rstd,
                                        long long pairs, int C, int relu) {
   pdl_entry();
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < pairs; t += (long long)gridDim.x * blockDim.x) {
@@ -439,10 +439,10 @@ __global__ void bn_apply_bf16x2_kernel(const bf16 *__restrict__ x, bf16 *__restr
 }
 // dx = gamma * rstd * (dy' - sum_dy / R - xhat * sum_dy_xhat / R)
 template <typename T>
-__global__ void bn_bwd_apply_kernel(const T *__restrict__ dy, const T *__restrict__ x, const T *__restrict__ relu_y, const T *__restrict__ gamma,
-                                    const float *__restrict__ mean, const float *__restrict__ rstd, const float *__restrict__ sums,
+__global__ void bn_bwd_apply_kernel(const T *dy, const T *x, const T *relu_y, const T *gamma,
+                                    const float *mean, const float *rstd, const float *sums,
                                     T *__restrict__ dx, long long total, int C, float inv_r, int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
     int c = (int)(t % C);
     float g = ldf(dy + t);
@@ -467,7 +467,7 @@ __device__ __forceinline__ uint4 pack8(const float *f) {
   return o;
 }
 
-__global__ void pool_fwd_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, unsigned char *__restrict__ arg, ConvGeom g, int mode,
+__global__ void pool_fwd_vec_kernel(const bf16 *x, bf16 *__restrict__ y, unsigned char *__restrict__ arg, ConvGeom g, int mode,
                                     long long total) {
   pdl_entry();
   const int c8n = g.C >> 3;
@@ -513,9 +513,9 @@ __global__ void pool_fwd_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict
   }
 }
 
-__global__ void pool_bwd_vec_kernel(const bf16 *__restrict__ dy, const unsigned char *__restrict__ arg, bf16 *__restrict__ dx, ConvGeom g,
+__global__ void pool_bwd_vec_kernel(const bf16 *dy, const unsigned char *arg, bf16 *__restrict__ dx, ConvGeom g,
                                     int mode, long long total, int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   const int c8n = g.C >> 3;
   const bool small = total < (1ll << 31);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
@@ -572,9 +572,9 @@ __global__ void pool_bwd_vec_kernel(const bf16 *__restrict__ dy, const unsigned 
 // (64 x 17 x 17 x 768 backward: 66 us, 28 MB each way).
 constexpr int AVG3_RUN = 6;
 template <bool BWD>
-__global__ void __launch_bounds__(256) pool_avg3_kernel(const bf16 *__restrict__ in, bf16 *__restrict__ out, ConvGeom g, FastDiv f_runs, int runs,
+__global__ void __launch_bounds__(256) pool_avg3_kernel(const bf16 *in, bf16 *__restrict__ out, ConvGeom g, FastDiv f_runs, int runs,
                                                         unsigned total, int accumulate) {
-  pdl_entry();
+  pdl_entry(out);
   // forward: `in` has the geometry's strides and `out` is dense; backward: the other way round
   const long long dense_w = g.C, dense_h = (long long)g.W * g.C, dense_n = (long long)g.H * dense_h;
   const long long in_w = BWD ? dense_w : g.sw, in_h = BWD ? dense_h : g.sh, in_n = BWD ? dense_n : g.sn;
@@ -634,9 +634,9 @@ __global__ void __launch_bounds__(256) pool_avg3_kernel(const bf16 *__restrict__
   }
 }
 // 3 x 3 maximum pooling with stride 2, backward: an input position lies in at most two windows per direction
-__global__ void __launch_bounds__(256) pool_max3s2_bwd_kernel(const bf16 *__restrict__ dy, const unsigned char *__restrict__ arg,
+__global__ void __launch_bounds__(256) pool_max3s2_bwd_kernel(const bf16 *dy, const unsigned char *arg,
                                                               bf16 *__restrict__ dx, ConvGeom g, unsigned total, int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   const int c8n = g.C >> 3;
   for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     unsigned r, c8, r2, iw, n, ih;
@@ -700,9 +700,9 @@ __device__ __forceinline__ void bn_scale_shift(const bf16 *gamma, const bf16 *be
 enum { BN_NO_RELU = 0, BN_RELU_Y = 1, BN_RELU_X = 2 };  // no ReLU; its mask from the forward output; from x, gamma and beta
 template <int MODE, int RELU>
 __global__ void __launch_bounds__(BNV_THREADS, 3)
-bn_partial_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, const bf16 *__restrict__ relu_y,
-                      const bf16 *__restrict__ gamma, const bf16 *__restrict__ beta,
-                      float *__restrict__ part, const float *__restrict__ mean, const float *__restrict__ rstd, long long R, int C,
+bn_partial_vec_kernel(const bf16 *a, const bf16 *b, const bf16 *relu_y,
+                      const bf16 *gamma, const bf16 *beta,
+                      float *__restrict__ part, const float *mean, const float *rstd, long long R, int C,
                       int rows_per_chunk) {
   pdl_entry();
   extern __shared__ float sred[];  // [lanes][2][C]
@@ -768,9 +768,9 @@ bn_partial_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, co
 }
 // Element-wise passes: the grid-stride step is a multiple of the number of channel groups, so a thread stays on one group and
 // keeps that group's constants in registers; two 16-byte pieces per operand and trip.
-__global__ void __launch_bounds__(256) bn_apply_vec_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, const bf16 *__restrict__ gamma,
-                                                           const bf16 *__restrict__ beta, const float *__restrict__ mean,
-                                                           const float *__restrict__ rstd, long long total8, int C, int relu) {
+__global__ void __launch_bounds__(256) bn_apply_vec_kernel(const bf16 *x, bf16 *__restrict__ y, const bf16 *gamma,
+                                                           const bf16 *beta, const float *mean,
+                                                           const float *rstd, long long total8, int C, int relu) {
   pdl_entry();
   const int groups = C >> 3;
   const long long usable = ((long long)gridDim.x * blockDim.x / groups) * groups;
@@ -799,10 +799,10 @@ __global__ void __launch_bounds__(256) bn_apply_vec_kernel(const bf16 *__restric
 // dx = ka * dy' + kb * x + kc per channel, xh = (x - mean) * rstd:  dx = gamma * rstd * (dy' - s1/R - xh * s2/R)
 template <int RELU>
 __global__ void __launch_bounds__(256)
-bn_bwd_apply_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ relu_y, const bf16 *__restrict__ gamma,
-                        const bf16 *__restrict__ beta, const float *__restrict__ mean, const float *__restrict__ rstd,
-                        const float *__restrict__ sums, bf16 *__restrict__ dx, long long total8, int C, float inv_r, int accumulate) {
-  pdl_entry();
+bn_bwd_apply_vec_kernel(const bf16 *dy, const bf16 *x, const bf16 *relu_y, const bf16 *gamma,
+                        const bf16 *beta, const float *mean, const float *rstd,
+                        const float *sums, bf16 *__restrict__ dx, long long total8, int C, float inv_r, int accumulate) {
+  pdl_entry(dx);
   const int groups = C >> 3;
   const long long usable = ((long long)gridDim.x * blockDim.x / groups) * groups;
   const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;

@@ -7,7 +7,7 @@
 namespace {
 
 // dst[i, :] = src[idx[i], :] for rows of `vec_per_row` 16-byte vectors; idx == nullptr: rows first .. first + n - 1
-__global__ void load_rows_vec_kernel(const uint4 *__restrict__ src, const long long *__restrict__ idx, uint4 *__restrict__ dst, long long n,
+__global__ void load_rows_vec_kernel(const uint4 *src, const long long *idx, uint4 *__restrict__ dst, long long n,
                                      long long vec_per_row, long long first, long long num_samples) {
   pdl_entry();
   const long long total = n * vec_per_row;
@@ -18,7 +18,7 @@ __global__ void load_rows_vec_kernel(const uint4 *__restrict__ src, const long l
     dst[t] = src[row * vec_per_row + v];
   }
 }
-__global__ void load_rows_byte_kernel(const unsigned char *__restrict__ src, const long long *__restrict__ idx, unsigned char *__restrict__ dst,
+__global__ void load_rows_byte_kernel(const unsigned char *src, const long long *idx, unsigned char *__restrict__ dst,
                                       long long n, long long row_bytes, long long first, long long num_samples) {
   pdl_entry();
   const long long total = n * row_bytes;

@@ -97,7 +97,7 @@ template <> struct V16<bf16> {
 };
 
 template <typename T>
-__global__ void unary_fwd_kernel(int op, const T *__restrict__ x, T *__restrict__ y, long long n, float s) {
+__global__ void unary_fwd_kernel(int op, const T *x, T *__restrict__ y, long long n, float s) {
   pdl_entry();
   constexpr int N = V16<T>::N;
   long long nv = n / N;
@@ -114,9 +114,9 @@ __global__ void unary_fwd_kernel(int op, const T *__restrict__ x, T *__restrict_
 }
 
 template <typename T>
-__global__ void unary_bwd_kernel(int op, const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ dy,
+__global__ void unary_bwd_kernel(int op, const T *x, const T *y, const T *dy,
                                  T *__restrict__ dx, long long n, float s, int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   constexpr int N = V16<T>::N;
   long long nv = n / N;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -153,7 +153,7 @@ __device__ __forceinline__ float binary_apply(int op, float a, float b) {
 // y[i] = a[i] (op) b[i % bn] ; bn == n for same-shape operands, bn == trailing
 // extent for a row-vector broadcast, bn == 1 for a scalar operand.
 template <typename T>
-__global__ void binary_fwd_kernel(int op, const T *__restrict__ a, const T *__restrict__ b, T *__restrict__ y,
+__global__ void binary_fwd_kernel(int op, const T *a, const T *b, T *__restrict__ y,
                                   long long n, long long bn) {
   pdl_entry();
   constexpr int N = V16<T>::N;
@@ -178,7 +178,7 @@ __global__ void binary_fwd_kernel(int op, const T *__restrict__ a, const T *__re
 
 // Same-shape backward.  da/db may be null; accumulate adds into them.
 template <typename T>
-__global__ void binary_bwd_kernel(int op, const T *__restrict__ a, const T *__restrict__ b, const T *__restrict__ dy,
+__global__ void binary_bwd_kernel(int op, const T *a, const T *b, const T *dy,
                                   T *da, T *db, long long n, int accumulate) {
   pdl_entry();
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -201,7 +201,7 @@ __global__ void binary_bwd_kernel(int op, const T *__restrict__ a, const T *__re
 
 // y = dropout(x) [+ r]; the keep mask is a pure function of (seed, index).
 template <typename T>
-__global__ void dropout_kernel(const T *__restrict__ x, const T *__restrict__ r, T *__restrict__ y, long long n,
+__global__ void dropout_kernel(const T *x, const T *r, T *__restrict__ y, long long n,
                                float p, float scale, unsigned long long seed, const unsigned long long *seed_ptr) {
   pdl_entry();
   // seed_ptr (optional) points at a per-step seed in device memory, so a captured CUDA graph draws a new
@@ -230,8 +230,8 @@ __global__ void dropout_kernel(const T *__restrict__ x, const T *__restrict__ r,
 }
 
 template <typename T>
-__global__ void axpby_kernel(const T *__restrict__ x, T *__restrict__ y, long long n, float a, float b) {
-  pdl_entry();
+__global__ void axpby_kernel(const T *x, T *__restrict__ y, long long n, float a, float b) {
+  pdl_entry(y);
   constexpr int N = V16<T>::N;
   long long nv = n / N;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -288,7 +288,7 @@ __global__ void cast_kernel(const void *src, int sdt, void *dst, int ddt, long l
   }
 }
 // fast paths for the two casts on the training hot path
-__global__ void cast_f32_bf16_kernel(const float *__restrict__ s, bf16 *__restrict__ d, long long n) {
+__global__ void cast_f32_bf16_kernel(const float *s, bf16 *__restrict__ d, long long n) {
   pdl_entry();
   long long nv = n / 8, stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride) {
@@ -301,8 +301,8 @@ __global__ void cast_f32_bf16_kernel(const float *__restrict__ s, bf16 *__restri
 
 // bf16 -> fp32 (written or added): the projections of fp32 attention around its bf16 core.  Through the general cast, which goes by
 // way of double one element at a time, 4096 x 2048 took 30 us.
-__global__ void cast_bf16_f32_kernel(const bf16 *__restrict__ s, float *__restrict__ d, long long n, int accumulate) {
-  pdl_entry();
+__global__ void cast_bf16_f32_kernel(const bf16 *s, float *__restrict__ d, long long n, int accumulate) {
+  pdl_entry(d);
   const long long nv = n / 8, stride = (long long)gridDim.x * blockDim.x, t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   for (long long i = t0; i < nv; i += stride) {
     const uint4 u = *reinterpret_cast<const uint4 *>(s + i * 8);
@@ -324,7 +324,7 @@ __global__ void cast_bf16_f32_kernel(const bf16 *__restrict__ s, float *__restri
 // ([gridDim.y, cols] floats) for the bias gradient.  One block handles a
 // 32-column strip over a slab of rows.
 template <typename T>
-__global__ void bias_act_bwd_kernel(const T *__restrict__ dy, const T *__restrict__ saved, T *__restrict__ dz,
+__global__ void bias_act_bwd_kernel(const T *dy, const T *saved, T *__restrict__ dz,
                                     float *__restrict__ partial, int rows, int cols, int act) {
   pdl_entry();
   __shared__ float red[8][33];
@@ -349,7 +349,7 @@ __global__ void bias_act_bwd_kernel(const T *__restrict__ dy, const T *__restric
   }
 }
 template <typename T>
-__global__ void colsum_finish_kernel(const float *__restrict__ partial, int nparts, int cols, T *out, int accumulate) {
+__global__ void colsum_finish_kernel(const float *partial, int nparts, int cols, T *out, int accumulate) {
   pdl_entry();
   int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= cols) return;

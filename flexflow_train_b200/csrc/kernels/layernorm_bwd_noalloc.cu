@@ -55,8 +55,8 @@ template <> __device__ __forceinline__ void stv<bf16>(bf16 *p, float v) { *p = f
 // partial rows in `partial` ([2][gridDim.x][cols]).  Those slots hold whatever the previous call left there,
 // so the owning thread clears them first; no other thread ever touches them.
 template <typename T>
-__global__ void ln_bwd_noalloc_kernel(const T *__restrict__ dy, const T *__restrict__ x, const T *__restrict__ gamma,
-                                      const float *__restrict__ mean, const float *__restrict__ rstd, T *__restrict__ dx,
+__global__ void ln_bwd_noalloc_kernel(const T *dy, const T *x, const T *gamma,
+                                      const float *mean, const float *rstd, T *__restrict__ dx,
                                       float *__restrict__ partial, int rows, int cols) {
   pdl_entry();
   __shared__ float red[32];
@@ -87,7 +87,7 @@ __global__ void ln_bwd_noalloc_kernel(const T *__restrict__ dy, const T *__restr
   }
 }
 template <typename T>
-__global__ void ln_bwd_noalloc_finish_kernel(const float *__restrict__ partial, int nparts, int cols, T *dgamma, T *dbeta) {
+__global__ void ln_bwd_noalloc_finish_kernel(const float *partial, int nparts, int cols, T *dgamma, T *dbeta) {
   pdl_entry();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;

@@ -24,9 +24,9 @@ template <> __device__ __forceinline__ float ldm<bf16>(const bf16 *p, long long 
 
 // pred [n, c]; sparse: label_i [n] class ids (int32 or int64 by `label64`); dense: label_d [n, c] targets (type T).
 template <typename T>
-__global__ void metrics_kernel(const T *__restrict__ pred, const void *__restrict__ label_i, const T *__restrict__ label_d, int label64,
+__global__ void metrics_kernel(const T *pred, const void *label_i, const T *label_d, int label64,
                                long long n, int c, int flags, double *__restrict__ acc) {
-  pdl_entry();
+  pdl_entry(acc);
   __shared__ float part[M_SLOTS][8];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   float sums[M_SLOTS];

@@ -23,8 +23,8 @@ template <> __device__ __forceinline__ void stf<bf16>(bf16 *p, float v) { *p = f
 // y = LN(a + b) * gamma + beta ; b optional (fused residual add); when b is
 // given and xsum is non-null the sum a + b is written too (backward needs it).
 template <typename T>
-__global__ void layernorm_fwd_kernel(const T *__restrict__ a, const T *__restrict__ b, const T *__restrict__ gamma,
-                                     const T *__restrict__ beta, T *__restrict__ xsum, T *__restrict__ y,
+__global__ void layernorm_fwd_kernel(const T *a, const T *b, const T *gamma,
+                                     const T *beta, T *__restrict__ xsum, T *__restrict__ y,
                                      float *__restrict__ mean, float *__restrict__ rstd, int rows, int cols,
                                      float eps) {
   pdl_entry();
@@ -65,11 +65,11 @@ __global__ void layernorm_fwd_kernel(const T *__restrict__ a, const T *__restric
 // dgamma / dbeta into scratch `partial` laid out [2][gridDim.x][cols].
 // Thread t owns columns t, t+blockDim, ... (at most KMAX of them).
 template <typename T, int KMAX>
-__global__ void layernorm_bwd_kernel(const T *__restrict__ dy, const T *__restrict__ x, const T *__restrict__ gamma,
-                                     const float *__restrict__ mean, const float *__restrict__ rstd,
+__global__ void layernorm_bwd_kernel(const T *dy, const T *x, const T *gamma,
+                                     const float *mean, const float *rstd,
                                      T *__restrict__ dx, T *__restrict__ dx2, float *__restrict__ partial, int rows,
                                      int cols, int accumulate_dx, int accumulate_dx2) {
-  pdl_entry();
+  pdl_entry(dx, dx2);
   __shared__ float red[32];
   float dg[KMAX], db[KMAX];
 #pragma unroll
@@ -127,7 +127,7 @@ __global__ void layernorm_bwd_kernel(const T *__restrict__ dy, const T *__restri
 // y = softmax(scale * x) over the last dim.  causal_q > 0: row r is query
 // position (r % causal_q) and keys past it are masked out.
 template <typename T>
-__global__ void softmax_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, int rows, int cols, float scale,
+__global__ void softmax_fwd_kernel(const T *x, T *__restrict__ y, int rows, int cols, float scale,
                                    int causal_q) {
   pdl_entry();
   __shared__ float red[32];
@@ -148,7 +148,7 @@ __global__ void softmax_fwd_kernel(const T *__restrict__ x, T *__restrict__ y, i
 }
 // dx = scale * y * (dy - sum(dy * y))
 template <typename T>
-__global__ void softmax_bwd_kernel(const T *__restrict__ dy, const T *__restrict__ y, T *__restrict__ dx, int rows,
+__global__ void softmax_bwd_kernel(const T *dy, const T *y, T *__restrict__ dx, int rows,
                                    int cols, float scale) {
   pdl_entry();
   __shared__ float red[32];
@@ -167,7 +167,7 @@ __global__ void softmax_bwd_kernel(const T *__restrict__ dy, const T *__restrict
 // probabilities, and dlogits = (p - onehot(label)) * grad_scale.  Rows whose
 // label is negative contribute no loss and no gradient.
 template <typename T, typename L>
-__global__ void softmax_ce_kernel(const T *__restrict__ logits, const L *__restrict__ labels, T *__restrict__ probs,
+__global__ void softmax_ce_kernel(const T *logits, const L *labels, T *__restrict__ probs,
                                   T *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols,
                                   float grad_scale) {
   pdl_entry();
@@ -196,7 +196,7 @@ __global__ void softmax_ce_kernel(const T *__restrict__ logits, const L *__restr
 // see rowwise_vec.cuh).
 constexpr int ROW_THREADS = 128;
 template <int VPT, typename L>
-__global__ void __launch_bounds__(ROW_THREADS) softmax_ce_row_kernel(const bf16 *__restrict__ logits, const L *__restrict__ labels,
+__global__ void __launch_bounds__(ROW_THREADS) softmax_ce_row_kernel(const bf16 *logits, const L *labels,
                                                                 bf16 *__restrict__ probs, bf16 *__restrict__ dlogits,
                                                                 float *__restrict__ loss, int cols, float grad_scale) {
   pdl_entry();
@@ -242,7 +242,7 @@ constexpr int WIDE_VPT = 4;
 constexpr int WIDE_SMEM = 220 * 1024;   // of one SM, shared by its blocks
 __device__ int g_rows_err = 0;
 template <bool CE, typename L>
-__global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__restrict__ x, const L *__restrict__ labels, bf16 *__restrict__ probs,
+__global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *x, const L *labels, bf16 *__restrict__ probs,
                                                                bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols,
                                                                float scale, float grad_scale, int depth, unsigned long long wait_ns) {
   pdl_entry();
@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *__res
 // the scalar kernels take 584 and 747, the row in registers (64 of them for 16 pieces alone, so it spills) 365 for 2048 x 50304,
 // this one 111.
 template <typename L>
-__global__ void __launch_bounds__(512) softmax_long_kernel(const bf16 *__restrict__ x, const L *__restrict__ labels, bf16 *__restrict__ probs,
+__global__ void __launch_bounds__(512) softmax_long_kernel(const bf16 *x, const L *labels, bf16 *__restrict__ probs,
                                                            bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols, float scale,
                                                            float grad_scale) {
   pdl_entry();
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(512) softmax_long_kernel(const bf16 *__restric
 enum { LOSS_SPARSE_CCE = 0, LOSS_CCE = 1, LOSS_MSE_AVG = 2, LOSS_IDENTITY = 3, LOSS_MSE_SUM = 4 };
 // dlogit for losses whose input is already a probability / prediction tensor.
 template <typename T, typename L>
-__global__ void loss_bwd_kernel(int kind, const T *__restrict__ pred, const void *__restrict__ target,
+__global__ void loss_bwd_kernel(int kind, const T *pred, const void *target,
                                 T *__restrict__ dpred, long long rows, int cols, float scale) {
   pdl_entry();
   long long n = rows * cols;
@@ -451,7 +451,7 @@ __global__ void loss_bwd_kernel(int kind, const T *__restrict__ pred, const void
 }
 // per-row loss values for reporting
 template <typename T, typename L>
-__global__ void loss_fwd_kernel(int kind, const T *__restrict__ pred, const void *__restrict__ target,
+__global__ void loss_fwd_kernel(int kind, const T *pred, const void *target,
                                 float *__restrict__ loss, int rows, int cols) {
   pdl_entry();
   __shared__ float red[32];

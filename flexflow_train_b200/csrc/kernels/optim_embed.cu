@@ -18,10 +18,10 @@ template <> __device__ __forceinline__ float ldg<bf16>(const bf16 *p, long long 
 
 template <typename G>
 __global__ void adam_kernel(float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
-                            const G *__restrict__ g, bf16 *__restrict__ shadow, long long n, float alpha_t,
+                            const G *g, bf16 *__restrict__ shadow, long long n, float alpha_t,
                             float beta1, float beta2, float eps, float wd, float gscale,
-                            const float *__restrict__ alpha_ptr) {
-  pdl_entry();
+                            const float *alpha_ptr) {
+  pdl_entry(w, m, v);
   // alpha_ptr (optional): bias-corrected step size kept in device memory so that a captured CUDA graph
   // sees the value of the current step.
   if (alpha_ptr) alpha_t = *alpha_ptr;
@@ -85,10 +85,10 @@ __device__ __forceinline__ float sgd_step(float wk, float gk, float *mom, float 
   return wk - lr * gt;
 }
 template <typename G>
-__global__ void __launch_bounds__(256) sgd_kernel(float *__restrict__ w, float *__restrict__ mom, const G *__restrict__ g,
+__global__ void __launch_bounds__(256) sgd_kernel(float *__restrict__ w, float *__restrict__ mom, const G *g,
                                                   bf16 *__restrict__ shadow, long long n, float lr, float momentum, int nesterov, float wd,
                                                   float gscale) {
-  pdl_entry();
+  pdl_entry(w, mom);
   // groups of four where the arenas' addresses allow it (a slice may start anywhere)
   const bool vec = (((uintptr_t)w | (uintptr_t)(momentum > 0.f ? mom : w)) & 15) == 0 && ((uintptr_t)g & (4 * sizeof(G) - 1)) == 0 &&
                    ((uintptr_t)shadow & 7) == 0;
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) sgd_kernel(float *__restrict__ w, float *
 // out[t, :] = sum_{j<bag} W[idx[t, j], :] (optionally averaged).  One warp per
 // (token, 32-column chunk group); rows are read with 16-byte loads when possible.
 template <typename W, typename I, typename O>
-__global__ void embedding_fwd_kernel(const I *__restrict__ idx, const W *__restrict__ table, O *__restrict__ out,
+__global__ void embedding_fwd_kernel(const I *idx, const W *table, O *__restrict__ out,
                                      long long tokens, int bag, int dim, long long entries, int avg) {
   pdl_entry();
   long long total = tokens * dim;
@@ -149,7 +149,7 @@ __device__ __forceinline__ void atomic_add_any(float *p, float v) { atomicAdd(p,
 __device__ __forceinline__ void atomic_add_any(bf16 *p, float v) { atomicAdd(p, f2bf(v)); }
 
 template <typename W, typename I, typename O>
-__global__ void embedding_bwd_kernel(const I *__restrict__ idx, const O *__restrict__ dout, W *__restrict__ dtable,
+__global__ void embedding_bwd_kernel(const I *idx, const O *dout, W *__restrict__ dtable,
                                      long long tokens, int bag, int dim, long long entries, int avg) {
   pdl_entry();
   long long total = tokens * dim;
@@ -196,7 +196,7 @@ __device__ __forceinline__ void red8(bf16 *p, const float (&v)[8]) {
                : "memory");
 }
 template <typename W, typename I, typename O>
-__global__ void embedding_fwd_vec_kernel(const I *__restrict__ idx, const W *__restrict__ table, O *__restrict__ out, unsigned pieces, int bag,
+__global__ void embedding_fwd_vec_kernel(const I *idx, const W *table, O *__restrict__ out, unsigned pieces, int bag,
                                          unsigned per_row, long long entries, int avg) {
   pdl_entry();
   const unsigned stride = gridDim.x * blockDim.x;
@@ -222,7 +222,7 @@ __global__ void embedding_fwd_vec_kernel(const I *__restrict__ idx, const W *__r
 }
 // dtable[idx] += scale * dout (avg: divided by the bag first), also the sparse SGD step with scale = -lr
 template <typename W, typename I, typename O>
-__global__ void embedding_scatter_vec_kernel(const I *__restrict__ idx, const O *__restrict__ dout, W *__restrict__ table, unsigned pieces,
+__global__ void embedding_scatter_vec_kernel(const I *idx, const O *dout, W *__restrict__ table, unsigned pieces,
                                              int bag, unsigned per_row, long long entries, int avg, float scale) {
   pdl_entry();
   const unsigned stride = gridDim.x * blockDim.x;
@@ -249,7 +249,7 @@ static bool emb_vec_ok(long long tokens, int dim, const void *a, const void *b) 
 // Sparse SGD for embedding tables: W[idx] -= lr * dout, applied straight from
 // the output gradient (no dense table gradient is materialised).
 template <typename I, typename O>
-__global__ void embedding_sgd_kernel(const I *__restrict__ idx, const O *__restrict__ dout, float *__restrict__ table,
+__global__ void embedding_sgd_kernel(const I *idx, const O *dout, float *__restrict__ table,
                                      long long tokens, int bag, int dim, long long entries, float lr) {
   pdl_entry();
   long long total = tokens * dim;

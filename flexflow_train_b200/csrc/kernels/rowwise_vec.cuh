@@ -40,7 +40,7 @@ __device__ __forceinline__ uint32_t keep8(unsigned long long seed, unsigned long
 // that are no multiple of 256 (sequence 500, 128 x 500 x 500 scores) used to take the block-per-row scalar kernel, which reads
 // the row three times in 2-byte pieces and left the dropped copy to a second kernel: 104 + 28 us.
 template <int VPT, bool FULL>
-__global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, bf16 *__restrict__ yd, int rows, int cols, int ld,
+__global__ void softmax_fwd_warp_kernel(const bf16 *x, bf16 *__restrict__ y, bf16 *__restrict__ yd, int rows, int cols, int ld,
                                         float scale, int causal_q, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
   pdl_entry();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -95,7 +95,7 @@ __global__ void softmax_fwd_warp_kernel(const bf16 *__restrict__ x, bf16 *__rest
 }
 // dx = scale * y * (g - sum(g * y)), g = dy (optionally first passed back through the dropout mask); rows as above
 template <int VPT, bool FULL>
-__global__ void softmax_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ y, bf16 *__restrict__ dx, int rows, int cols,
+__global__ void softmax_bwd_warp_kernel(const bf16 *dy, const bf16 *y, bf16 *__restrict__ dx, int rows, int cols,
                                         int ld, float scale, float p_drop, unsigned long long salt, const unsigned long long *seed_ptr) {
   pdl_entry();
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
@@ -139,7 +139,7 @@ __global__ void softmax_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 
   }
 }
 // y = dropout(x) over rows of `cols` at pitch `ld`, the mask of softmax_fwd_warp_kernel's yd; a thread per 8 elements
-static __global__ void dropout_rows_kernel(const bf16 *__restrict__ x, bf16 *__restrict__ y, long long rows, int cols, int ld, float p_drop,
+static __global__ void dropout_rows_kernel(const bf16 *x, bf16 *__restrict__ y, long long rows, int cols, int ld, float p_drop,
                                            unsigned long long salt, const unsigned long long *seed_ptr) {
   pdl_entry();
   const unsigned long long seed = seed_ptr ? salt * 0x9E3779B97F4A7C15ull + *seed_ptr : salt;
@@ -210,8 +210,8 @@ __device__ __forceinline__ void row_max_sum(const uint4 (&u)[VPT], int nvec, flo
 // ---------------------------------------------------------------- LayerNorm: one block per row
 // cols = 8 * blockDim.x * VPT.  y = LN(a + b) * gamma + beta, xsum = a + b (when b is given).
 template <int VPT>
-__global__ void layernorm_fwd_vec_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b, const bf16 *__restrict__ gamma,
-                                         const bf16 *__restrict__ beta, bf16 *__restrict__ xsum, bf16 *__restrict__ y,
+__global__ void layernorm_fwd_vec_kernel(const bf16 *a, const bf16 *b, const bf16 *gamma,
+                                         const bf16 *beta, bf16 *__restrict__ xsum, bf16 *__restrict__ y,
                                          float *__restrict__ mean, float *__restrict__ rstd, int rows, int cols, float eps) {
   pdl_entry();
   // two block reductions per row (mean, then centred variance), each through its own double-buffered slot so
@@ -306,8 +306,8 @@ __global__ void layernorm_fwd_vec_kernel(const bf16 *__restrict__ a, const bf16 
 // warp has VPT (2 VPT with a fused add) loads in flight and the two row reductions are warp shuffles: no
 // block-wide barrier after the one that stages gamma / beta in shared memory.
 template <int VPT>
-__global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const bf16 *__restrict__ a, const bf16 *__restrict__ b,
-                                                                    const bf16 *__restrict__ gamma, const bf16 *__restrict__ beta,
+__global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const bf16 *a, const bf16 *b,
+                                                                    const bf16 *gamma, const bf16 *beta,
                                                                     bf16 *__restrict__ xsum, bf16 *__restrict__ y, float *__restrict__ mean,
                                                                     float *__restrict__ rstd, int rows, float eps) {
   pdl_entry();
@@ -376,10 +376,10 @@ __global__ void __launch_bounds__(256, 2) layernorm_fwd_warp_kernel(const bf16 *
 }
 // dx (and optionally dx2) (+)= LN backward; per-block partial sums of dgamma/dbeta -> partial[2][grid][cols]
 template <int VPT>
-__global__ void layernorm_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ gamma,
-                                         const float *__restrict__ mean, const float *__restrict__ rstd, bf16 *__restrict__ dx,
+__global__ void layernorm_bwd_vec_kernel(const bf16 *dy, const bf16 *x, const bf16 *gamma,
+                                         const float *mean, const float *rstd, bf16 *__restrict__ dx,
                                          bf16 *__restrict__ dx2, float *__restrict__ partial, int rows, int cols, int acc1, int acc2) {
-  pdl_entry();
+  pdl_entry(dx, dx2);
   // the two row sums are reduced together through a double-buffered slot: one barrier per row
   __shared__ float2 red2[2][32];
   int parity = 0;
@@ -483,10 +483,10 @@ __global__ void layernorm_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16
 // bytes on 1184 partial rows as on the data (8.7 us and 4.5 us to fold them).
 template <int VPT>
 __global__ void __launch_bounds__(256, VPT <= 2 ? 2 : 1)
-layernorm_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ x, const bf16 *__restrict__ gamma, const float *__restrict__ mean,
-                          const float *__restrict__ rstd, bf16 *__restrict__ dx, bf16 *__restrict__ dx2, float *__restrict__ partial, int rows,
+layernorm_bwd_warp_kernel(const bf16 *dy, const bf16 *x, const bf16 *gamma, const float *mean,
+                          const float *rstd, bf16 *__restrict__ dx, bf16 *__restrict__ dx2, float *__restrict__ partial, int rows,
                           int acc1, int acc2) {
-  pdl_entry();
+  pdl_entry(dx, dx2);
   constexpr int COLS = 256 * VPT;
   __shared__ float red[8][COLS];
   __shared__ float g_s[COLS];
@@ -580,7 +580,7 @@ layernorm_bwd_warp_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ 
 // dz = dy * act'(saved); partial[blockIdx.y][col] = column sums over this block's rows.
 // With drop_p > 0 the incoming gradient first goes back through the dropout that the forward GEMM epilogue
 // applied after the activation (mask regenerated from (seed, flat index)).
-static __global__ void bias_act_bwd_vec_kernel(const bf16 *__restrict__ dy, const bf16 *__restrict__ saved, bf16 *__restrict__ dz,
+static __global__ void bias_act_bwd_vec_kernel(const bf16 *dy, const bf16 *saved, bf16 *__restrict__ dz,
                                         float *__restrict__ partial, int rows, int cols, int act, float drop_p,
                                         unsigned long long drop_salt, const unsigned long long *drop_seed_ptr) {
   pdl_entry();
@@ -636,7 +636,7 @@ static __global__ void bias_act_bwd_vec_kernel(const bf16 *__restrict__ dy, cons
 // independent loads, the lanes' sums meet in shared memory in a fixed order (deterministic).  The one-thread-per-column
 // form took 60 us for 1184 parts of 768 columns: three blocks, each thread a chain of 1184 dependent additions.
 template <typename T>
-__global__ void fold_partials_kernel(const float *__restrict__ partial, int nparts, int cols, T *out, T *out2, int accumulate) {
+__global__ void fold_partials_kernel(const float *partial, int nparts, int cols, T *out, T *out2, int accumulate) {
   pdl_entry();
   __shared__ float s1[32][33], s2[32][33];
   const int tx = threadIdx.x, ty = threadIdx.y, c = blockIdx.x * 32 + tx;

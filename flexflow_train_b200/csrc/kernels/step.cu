@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) stage_batch_kernel(const __grid
 
 // Mean of the per-row losses, written straight into page-locked host memory: one launch in the place of a reduction and a
 // device-to-host copy (5.8 us on the device at the end of every step that reports its loss, and one more launch).
-__global__ void __launch_bounds__(1024) loss_mean_kernel(const float *__restrict__ rows, long long n, float *out) {
+__global__ void __launch_bounds__(1024) loss_mean_kernel(const float *rows, long long n, float *out) {
   pdl_entry();
   __shared__ float red[32];
   float s = 0.f;

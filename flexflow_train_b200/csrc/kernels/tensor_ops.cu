@@ -32,9 +32,9 @@ struct Dims {
 };
 
 template <typename W>
-__global__ void permute_kernel(const W *__restrict__ src, W *__restrict__ dst, Dims d, long long total, int accumulate_f32,
+__global__ void permute_kernel(const W *src, W *__restrict__ dst, Dims d, long long total, int accumulate_f32,
                                int accumulate_bf16) {
-  pdl_entry();
+  pdl_entry(dst);
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     long long rem = i, off = 0;
@@ -60,9 +60,9 @@ struct Dims32 {
   long long stride[MAXD];
 };
 template <typename W>
-__global__ void permute32_kernel(const W *__restrict__ src, W *__restrict__ dst, Dims32 d, unsigned total, int accumulate_f32,
+__global__ void permute32_kernel(const W *src, W *__restrict__ dst, Dims32 d, unsigned total, int accumulate_f32,
                                  int accumulate_bf16) {
-  pdl_entry();
+  pdl_entry(dst);
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * stride) {
     W v[4];
@@ -97,7 +97,7 @@ __global__ void permute32_kernel(const W *__restrict__ src, W *__restrict__ dst,
 
 // dst[b][c][r] = src[b][r][c], 32x32 tiles through shared memory
 template <typename W>
-__global__ void transpose2d_kernel(const W *__restrict__ src, W *__restrict__ dst, int rows, int cols) {
+__global__ void transpose2d_kernel(const W *src, W *__restrict__ dst, int rows, int cols) {
   pdl_entry();
   __shared__ W tile[32][33];
   long long base = (long long)blockIdx.z * rows * cols;
@@ -116,9 +116,9 @@ __global__ void transpose2d_kernel(const W *__restrict__ src, W *__restrict__ ds
 // Copy (or add) a [outer, block] region between tensors whose rows are `src_ld` / `dst_ld` elements apart:
 // concat writes each input into its slot of the output row, split reads it back.
 template <typename T>
-__global__ void block_copy_kernel(const T *__restrict__ src, long long src_ld, T *__restrict__ dst, long long dst_ld,
+__global__ void block_copy_kernel(const T *src, long long src_ld, T *__restrict__ dst, long long dst_ld,
                                   long long outer, long long block, int accumulate) {
-  pdl_entry();
+  pdl_entry(dst);
   long long total = outer * block;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -132,7 +132,7 @@ __global__ void block_copy_kernel(const T *__restrict__ src, long long src_ld, T
 
 // Plain copy of fewer than 2^31 elements: the row / column split by multiply-high, four elements in flight per thread.
 template <typename T>
-__global__ void block_copy32_kernel(const T *__restrict__ src, long long src_ld, T *__restrict__ dst, long long dst_ld, unsigned total, CopyDiv f) {
+__global__ void block_copy32_kernel(const T *src, long long src_ld, T *__restrict__ dst, long long dst_ld, unsigned total, CopyDiv f) {
   pdl_entry();
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < total; i0 += 4 * stride) {
@@ -159,9 +159,9 @@ __global__ void block_copy32_kernel(const T *__restrict__ src, long long src_ld,
 // 16-byte form of the same copy: block, both pitches and both bases are multiples of 16 bytes and there are fewer
 // than 2^31 pieces, so the row / column split is a multiply-high instead of a 64-bit division per 2-byte element
 // (channel concatenation of channels-last activations is this case).
-__global__ void block_copy_vec_kernel(const uint4 *__restrict__ src, long long src_ld, uint4 *__restrict__ dst, long long dst_ld,
+__global__ void block_copy_vec_kernel(const uint4 *src, long long src_ld, uint4 *__restrict__ dst, long long dst_ld,
                                       unsigned total, CopyDiv f, int accumulate_bf16) {
-  pdl_entry();
+  pdl_entry(dst);
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     const unsigned o = cdiv(i, f), b = i - o * f.d;
@@ -185,7 +185,7 @@ __global__ void block_copy_vec_kernel(const uint4 *__restrict__ src, long long s
 enum { RED_SUM = 0, RED_MEAN = 1, RED_MAX = 2, RED_MIN = 3, RED_PROD = 4 };
 // x viewed as [outer, red, inner] -> y [outer, inner]
 template <typename T>
-__global__ void reduce_kernel(const T *__restrict__ x, T *__restrict__ y, long long outer, long long red, long long inner, int op) {
+__global__ void reduce_kernel(const T *x, T *__restrict__ y, long long outer, long long red, long long inner, int op) {
   pdl_entry();
   long long total = outer * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
@@ -203,9 +203,9 @@ __global__ void reduce_kernel(const T *__restrict__ x, T *__restrict__ y, long l
 }
 // backward of sum / mean: dx[o, r, in] (+)= dy[o, in] * scale
 template <typename T>
-__global__ void reduce_bwd_kernel(const T *__restrict__ dy, T *__restrict__ dx, long long outer, long long red, long long inner,
+__global__ void reduce_bwd_kernel(const T *dy, T *__restrict__ dx, long long outer, long long red, long long inner,
                                   float scale, int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   long long total = outer * red * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -220,9 +220,9 @@ __global__ void reduce_bwd_kernel(const T *__restrict__ dy, T *__restrict__ dx, 
 //             the derivative of amax/amin taken one-sided); prod: dx = dy * y / x (x == 0: product of the others
 //             recomputed).
 template <typename T>
-__global__ void reduce_select_bwd_kernel(const T *__restrict__ x, const T *__restrict__ y, const T *__restrict__ dy, T *__restrict__ dx,
+__global__ void reduce_select_bwd_kernel(const T *x, const T *y, const T *dy, T *__restrict__ dx,
                                          long long outer, long long red, long long inner, int op, int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   long long total = outer * red * inner;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -247,7 +247,7 @@ __global__ void reduce_select_bwd_kernel(const T *__restrict__ x, const T *__res
 
 // torch.gather along `dim`: x [outer, xd, inner], index/out [outer, id, inner]
 template <typename T, typename I>
-__global__ void gather_kernel(const T *__restrict__ x, const I *__restrict__ idx, T *__restrict__ y, long long outer, long long xd,
+__global__ void gather_kernel(const T *x, const I *idx, T *__restrict__ y, long long outer, long long xd,
                               long long id, long long inner) {
   pdl_entry();
   long long total = outer * id * inner;
@@ -259,7 +259,7 @@ __global__ void gather_kernel(const T *__restrict__ x, const I *__restrict__ idx
   }
 }
 template <typename I>
-__global__ void gather_bwd_kernel(const float *__restrict__ dy_f, const bf16 *__restrict__ dy_b, const I *__restrict__ idx,
+__global__ void gather_bwd_kernel(const float *dy_f, const bf16 *dy_b, const I *idx,
                                   float *dx_f, bf16 *dx_b, long long outer, long long xd, long long id, long long inner) {
   pdl_entry();
   long long total = outer * id * inner;
@@ -277,7 +277,7 @@ __global__ void gather_bwd_kernel(const float *__restrict__ dy_f, const bf16 *__
 // Top-k per row by repeated selection: one warp per row, k passes.  Rows of attention-sized tensors
 // (<= a few thousand columns) and small k are the use case; the cost is O(k * cols / 32) per row.
 template <typename T>
-__global__ void topk_kernel(const T *__restrict__ x, T *__restrict__ vals, int *__restrict__ idxs, int rows, int cols, int k) {
+__global__ void topk_kernel(const T *x, T *__restrict__ vals, int *__restrict__ idxs, int rows, int cols, int k) {
   pdl_entry();
   int warps_per_block = blockDim.x >> 5, lane = threadIdx.x & 31;
   for (int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps_per_block) {
@@ -309,9 +309,9 @@ __global__ void topk_kernel(const T *__restrict__ x, T *__restrict__ vals, int *
   }
 }
 template <typename T>
-__global__ void topk_bwd_kernel(const T *__restrict__ dvals, const int *__restrict__ idxs, T *__restrict__ dx, int rows, int cols, int k,
+__global__ void topk_bwd_kernel(const T *dvals, const int *idxs, T *__restrict__ dx, int rows, int cols, int k,
                                 int accumulate) {
-  pdl_entry();
+  pdl_entry(dx);
   long long total = (long long)rows * k;
   long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -323,7 +323,7 @@ __global__ void topk_bwd_kernel(const T *__restrict__ dvals, const int *__restri
 
 // x [outer, n, inner] -> y[o, j, :] = x[o, n-1-j, :]
 template <typename W>
-__global__ void reverse_kernel(const W *__restrict__ x, W *__restrict__ y, long long outer, long long n, long long inner) {
+__global__ void reverse_kernel(const W *x, W *__restrict__ y, long long outer, long long n, long long inner) {
   pdl_entry();
   long long total = outer * n * inner;
   long long stride = (long long)gridDim.x * blockDim.x;

@@ -60,3 +60,12 @@ def test_kernels_that_wait_for_peers_do_not_release_their_successor():
     for name, text in _sources():
         if name == "comm_kernels.cu":
             assert "pdl_" not in text and "ffk_launch" not in text
+
+
+def test_early_launched_kernels_take_no_input_for_constant():
+    """A __restrict__ pointer to const may be read through the non-coherent path, or ahead of the wait, although the
+    predecessor still writes there."""
+    bad = {k: p for k, (f, p, _) in KERNELS.items() if f != "comm_kernels.cu" for p in re.findall(r"const [\w ]+\*\s*__restrict__ \w+", p)}
+    assert not bad, bad
+    helpers = [(n, m) for n, text in _sources() if n != "comm_kernels.cu" for m in re.findall(r"const [\w ]+\*\s*__restrict__ \w+", text)]
+    assert not helpers, helpers
