@@ -1450,9 +1450,20 @@ static void gemm_plan(const FfkGemmDesc *d, long long nbatch, int *bn, int *spli
   auto l2_us = [](long long ctas, int w, float tbs) { return (float)ctas * (128.f + (float)w) * 128.f / (tbs * 1e6f); };  // a k-block of all
   float best = 1e30f;
   const bool plain32 = d->out_fp32 && !d->C2 && !d->addend && d->act == ACT_NONE && nbatch == 1 && d->alpha == 1.f;
+  // k-blocks one accumulator sums when the persistent kernel has t tiles (see launch_cfg)
+  auto range = [&](long long t) {
+    int want = plain32 && t * 2 <= sms && num_kb >= 16 ? (int)(sms / t) : 1;
+    if (want > num_kb / 8) want = num_kb / 8;
+    return want > 1 ? (num_kb + want - 1) / want : num_kb;
+  };
+  // An fp32 result of bf16 operands is as exact as its accumulators, whose error grows with the k-blocks they sum (512 x 512 x 8192: 9.1e-7 of
+  // the result at 15 blocks each, 2.1e-6 at 32), so neither a cluster nor another tile width may lengthen that range.  Rounding to bf16
+  // (1.7e-3) or of tf32 operands (7.7e-4) hides it.
+  const int most = d->out_fp32 && es == 2 ? range(tiles(d->N > 64 ? 128 : 64)) : num_kb;
   for (int w = 64; w <= (es == 4 ? 128 : 256); w *= 2) {
     if (w > 64 && d->N <= w / 2) break;
     const long long t = tiles(w);
+    if (range(t) > most) continue;
     float us;
     if (w == 256 && g_pair_mode && d->M >= 256 && (long long)((d->M + 255) / 256) * ((d->N + 255) / 256) * nbatch >= sms / 2) {
       const long long pt = (long long)((d->M + 255) / 256) * ((d->N + 255) / 256) * nbatch;
@@ -1479,6 +1490,7 @@ static void gemm_plan(const FfkGemmDesc *d, long long nbatch, int *bn, int *spli
     for (int sp = 2; sp <= 8; sp *= 2) {
       const long long ctas = tiles(w) * sp;
       if (sp > num_kb || ctas > sms - 4) break;
+      if ((num_kb + sp - 1) / sp > most) continue;
       const float l2 = l2_us(ctas, w, 15.f);
       float us = (w == 64 ? 5.8f : 6.9f) + (float)((num_kb + sp - 1) / sp) * (l2 > 0.22f ? l2 : 0.22f);
       if (sp == 8 && ctas > 96) us += 1.5f;  // more clusters of 8 than the GPCs place at once

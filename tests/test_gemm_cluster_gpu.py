@@ -105,3 +105,17 @@ def test_fp32_transposed_operands(M, N, Kd):
     if Kd % 4:  # small or repacked: no further from fp64 than the transposed copies were
         assert (K.matmul_tn(at, bt).double() - ref).norm() <= 1.01 * (K.matmul_nt(a, b).double() - ref).norm() + 1e-6
     assert K.gemm_last_error() == 0
+
+
+@pytest.mark.parametrize("M,N", [(64, 192), (256, 512), (512, 512), (768, 768), (1000, 300)])
+@pytest.mark.parametrize("Kd", [1024, 4096, 8192, 16384])
+def test_fp32_results_keep_their_accumulators_short(M, N, Kd):
+    """The chosen kernel's fp32 result is no further from fp64 than that of the split the persistent kernel makes."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + Kd)
+    a, b = torch.randn(Kd, M, generator=g, device="cuda").bfloat16(), torch.randn(Kd, N, generator=g, device="cuda").bfloat16()
+    ref = a.double().t() @ b.double()
+    off = lambda c: ((c.double() - ref).norm() / ref.norm()).item()  # noqa: E731
+    out = torch.empty(M, N, device="cuda")
+    chosen, split = off(K.matmul_tn(a, b, out=out)), off(K.matmul_tn(a, b, out=torch.empty_like(out), bn=128))
+    # errors of 1e4 and more elements average out: the ratio is that of the ranges, which are whole k-blocks
+    assert chosen <= 1.05 * split, (chosen, split)
