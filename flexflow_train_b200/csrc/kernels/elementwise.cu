@@ -429,28 +429,32 @@ FFK_API int ffk_cast(const void *src, int sdt, void *dst, int ddt, long long n, 
 }
 // Number of float slots `partial` must hold for ffk_bias_act_bwd.
 // Row chunks of the column reduction: 64 rows each and enough chunks that a narrow matrix (768 columns = three column blocks)
-// still fills the GPU; fewer rows, down to one per thread, where 64 would leave fewer than two blocks per SM (64 x 1024: 4 blocks,
-// 7.5 us of one load after another).
-static int bias_act_row_chunks(int rows, int cols) {
+// still fills the GPU; in the vector form fewer rows, down to one per thread, where 64 would leave fewer than two blocks per SM
+// (64 x 1024: 4 blocks, 7.5 us of one load after another), but not so many that a second wave begins (2048 x 2056 with 33 chunks for
+// 32: 14.2 us, 12.9).  The scalar form has eight times the column blocks and adds its chunks
+// one after another (fp32, 4096 x 128, bias only: 64 chunks 6.0 us, 296 of them 11.5).
+static int bias_act_row_chunks(int rows, int cols, bool vec) {
   const int col_blocks = (cols + 255) / 256;
   int cap = (148 * 4 + col_blocks - 1) / col_blocks;
   if (cap < 64) cap = 64;
   int gy = rows / 64;
   if (gy < 1) gy = 1;
   if (gy > cap) gy = cap;
-  const int fill = (148 * 2 + col_blocks - 1) / col_blocks, most = (rows + 7) / 8;
-  if (gy < fill) gy = fill < most ? fill : most;
+  const int fill = 148 * 2 / col_blocks, most = (rows + 7) / 8;
+  if (vec && gy < fill) gy = fill < most ? fill : most;
   return gy;
 }
-FFK_API long long ffk_bias_act_bwd_scratch(int rows, int cols) { return (long long)bias_act_row_chunks(rows, cols) * cols; }
+// of the vector form, which takes at least as many chunks as the scalar one
+FFK_API long long ffk_bias_act_bwd_scratch(int rows, int cols) { return (long long)bias_act_row_chunks(rows, cols, true) * cols; }
 // dz = dy * act'(saved); dbias (+)= column sums of dz.  dz may alias dy or be null
 // (bias gradient only); dbias may be null.  `partial` is caller-provided scratch.
 static int bias_act_bwd_impl(const void *dy, const void *saved, void *dz, void *dbias, float *partial, int rows, int cols, int act, int dt,
                              int accumulate, float drop_p, unsigned long long drop_salt, const void *drop_seed_ptr, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return 0;
   FfkTraffic traffic((long long)rows * cols * (dt == DT_BF16 ? 2 : 4) * (1 + (act != ACT_NONE) + (dz != nullptr)));
-  const int gy = bias_act_row_chunks(rows, cols);
-  if (dt == DT_BF16 && cols % 8 == 0 && (((uintptr_t)dy | (uintptr_t)saved | (uintptr_t)dz) & 15) == 0) {
+  const bool vec = dt == DT_BF16 && cols % 8 == 0 && (((uintptr_t)dy | (uintptr_t)saved | (uintptr_t)dz) & 15) == 0;
+  const int gy = bias_act_row_chunks(rows, cols, vec);
+  if (vec) {
     dim3 vgrid((cols + 255) / 256, gy), vblock(32, 8);
     ffk_launch(vec::bias_act_bwd_vec_kernel, vgrid, vblock, 0, st, (const bf16 *)dy, (const bf16 *)saved, (bf16 *)dz, dbias ? partial : nullptr, rows,
                                                           cols, act, drop_p, drop_salt, (const unsigned long long *)drop_seed_ptr);

@@ -35,6 +35,20 @@ def test_bias_gradient_of_few_rows(rows, cols):
     assert ((db.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + want.double().abs().sum(0) * rows * 2.0 ** -24 + 1e-7).all()
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 1), (7, 10), (64, 1024), (300, 33), (4096, 128), (4096, 256), (2048, 2056)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_bias_gradient_chunks(rows, cols, dtype):
+    """Scalar and vector forms, whose rows are split differently, in the scratch one function reports for both."""
+    dy = _randn(rows, cols, dtype=dtype)
+    n = K.bias_act_bwd_scratch(rows, cols)
+    scratch, db, old = torch.full((n + 64,), 7.0, device="cuda"), _randn(cols, dtype=dtype, seed=2), _randn(cols, dtype=dtype, seed=2)
+    K.bias_act_bwd(dy, None, None, db, scratch[:n], None, accumulate=True)
+    ref = dy.double().sum(0) + old.double()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+    assert ((db.double() - ref).abs() <= ref.abs() * ulp + (dy.double().abs().sum(0) + 1) * rows * 2.0 ** -24).all()
+    assert (scratch[n:] == 7).all()
+
+
 def test_bias_gradient_refuses_a_short_scratch():
     dy, db = _randn(800, 768), torch.zeros(768, device="cuda").bfloat16()
     short = torch.empty(K.bias_act_bwd_scratch(800, 768) - 1, device="cuda")
