@@ -166,31 +166,39 @@ __global__ void embedding_bwd_kernel(const I *idx, const O *dout, W *__restrict_
   }
 }
 
-// 16-byte forms: rows of a multiple of 8 elements, a thread per 8 of them, the index split in 32 bits.  Bound by HBM (tokens x dim read
-// and written); with one element and one 64-bit division per thread the lookup of 32768 x 2048 took 384 us and the scatter,
-// whose 16-bit atomics went out one by one, 586 us.  The reductions are those of the scalar form (one rounding to the table's
-// type per addition), issued eight at a time.
-__device__ __forceinline__ void load8(const float *p, float (&v)[8]) {
-  const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
-  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+// 16-byte forms: rows of a multiple of 8 elements, a thread per 16 bytes of the table (4 fp32 elements, 8 bf16), the index split in 32
+// bits.  Bound by HBM (tokens x dim read and written); with one element and one 64-bit division per thread the lookup of
+// 32768 x 2048 took 384 us and the scatter, whose 16-bit atomics went out one by one, 586 us.  The reductions are those of the scalar
+// form (one rounding to the table's type per addition), issued a piece at a time.  A warp's pieces are neighbours: with two pieces
+// of fp32 per thread each reduction covered every other 16 bytes, and a row that many tokens share took twice as long as element by element.
+template <int N> __device__ __forceinline__ void load_piece(const float *p, float (&v)[N]) {
+#pragma unroll
+  for (int k = 0; k < N; k += 4) {
+    const float4 a = *reinterpret_cast<const float4 *>(p + k);
+    v[k] = a.x; v[k + 1] = a.y; v[k + 2] = a.z; v[k + 3] = a.w;
+  }
 }
-__device__ __forceinline__ void load8(const bf16 *p, float (&v)[8]) {
+__device__ __forceinline__ void load_piece(const bf16 *p, float (&v)[8]) {
   const uint4 u = *reinterpret_cast<const uint4 *>(p);
   const float2 a = unpack_bf162(u.x), b = unpack_bf162(u.y), c = unpack_bf162(u.z), d = unpack_bf162(u.w);
   v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y; v[6] = d.x; v[7] = d.y;
 }
-__device__ __forceinline__ void store8(float *p, const float (&v)[8]) {
-  reinterpret_cast<float4 *>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
-  reinterpret_cast<float4 *>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+__device__ __forceinline__ void load_piece(const bf16 *p, float (&v)[4]) {
+  const uint2 u = *reinterpret_cast<const uint2 *>(p);
+  const float2 a = unpack_bf162(u.x), b = unpack_bf162(u.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
 }
-__device__ __forceinline__ void store8(bf16 *p, const float (&v)[8]) {
+__device__ __forceinline__ void store_piece(float *p, const float (&v)[4]) { *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void store_piece(bf16 *p, const float (&v)[4]) {
+  *reinterpret_cast<uint2 *>(p) = make_uint2(pack_bf162(v[0], v[1]), pack_bf162(v[2], v[3]));
+}
+__device__ __forceinline__ void store_piece(bf16 *p, const float (&v)[8]) {
   *reinterpret_cast<uint4 *>(p) = make_uint4(pack_bf162(v[0], v[1]), pack_bf162(v[2], v[3]), pack_bf162(v[4], v[5]), pack_bf162(v[6], v[7]));
 }
-__device__ __forceinline__ void red8(float *p, const float (&v)[8]) {
+__device__ __forceinline__ void red_piece(float *p, const float (&v)[4]) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p + 4), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
 }
-__device__ __forceinline__ void red8(bf16 *p, const float (&v)[8]) {
+__device__ __forceinline__ void red_piece(bf16 *p, const float (&v)[8]) {
   asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(pack_bf162(v[0], v[1])), "r"(pack_bf162(v[2], v[3])),
                "r"(pack_bf162(v[4], v[5])), "r"(pack_bf162(v[6], v[7]))
                : "memory");
@@ -199,25 +207,27 @@ template <typename W, typename I, typename O>
 __global__ void embedding_fwd_vec_kernel(const I *idx, const W *table, O *__restrict__ out, unsigned pieces, int bag,
                                          unsigned per_row, long long entries, int avg) {
   pdl_entry();
+  constexpr int N = 16 / sizeof(W);
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < pieces; i += stride) {
     const unsigned t = i / per_row;
-    const long long c = (long long)(i - t * per_row) * 8;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const long long c = (long long)(i - t * per_row) * N;
+    float acc[N] = {};
+#pragma unroll 4
     for (int j = 0; j < bag; ++j) {
       const long long e = (long long)idx[(long long)t * bag + j];
       if (e >= 0 && e < entries) {
-        float v[8];
-        load8(table + e * per_row * 8 + c, v);
+        float v[N];
+        load_piece(table + e * per_row * N + c, v);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] += v[k];
+        for (int k = 0; k < N; ++k) acc[k] += v[k];
       }
     }
     if (avg) {
 #pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] /= bag;
+      for (int k = 0; k < N; ++k) acc[k] /= bag;
     }
-    store8(out + (long long)i * 8, acc);
+    store_piece(out + (long long)i * N, acc);
   }
 }
 // dtable[idx] += scale * dout (avg: divided by the bag first), also the sparse SGD step with scale = -lr
@@ -225,25 +235,29 @@ template <typename W, typename I, typename O>
 __global__ void embedding_scatter_vec_kernel(const I *idx, const O *dout, W *__restrict__ table, unsigned pieces,
                                              int bag, unsigned per_row, long long entries, int avg, float scale) {
   pdl_entry();
+  constexpr int N = 16 / sizeof(W);
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < pieces; i += stride) {
     const unsigned t = i / per_row;
-    const long long c = (long long)(i - t * per_row) * 8;
-    float g[8];
-    load8(dout + (long long)i * 8, g);
+    const long long c = (long long)(i - t * per_row) * N;
+    float g[N];
+    load_piece(dout + (long long)i * N, g);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < N; ++k) {
       if (avg) g[k] /= bag;
       g[k] *= scale;
     }
+#pragma unroll 4
     for (int j = 0; j < bag; ++j) {
       const long long e = (long long)idx[(long long)t * bag + j];
-      if (e >= 0 && e < entries) red8(table + e * per_row * 8 + c, g);
+      if (e >= 0 && e < entries) red_piece(table + e * per_row * N + c, g);
     }
   }
 }
-static bool emb_vec_ok(long long tokens, int dim, const void *a, const void *b) {
-  return dim % 8 == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0 && tokens * (dim / 8) < (1ll << 31) - 148ll * 16 * 256;
+// pieces of the 16-byte forms, 0 where rows or addresses do not allow them
+template <typename W> static unsigned emb_pieces(long long tokens, int dim, const void *a, const void *b) {
+  const long long n = tokens * (dim / (int)(16 / sizeof(W)));
+  return dim % 8 == 0 && (((uintptr_t)a | (uintptr_t)b) & 15) == 0 && n < (1ll << 31) - 148ll * 16 * 256 ? (unsigned)n : 0u;
 }
 
 // Sparse SGD for embedding tables: W[idx] -= lr * dout, applied straight from
@@ -296,8 +310,8 @@ template <typename W, typename I, typename O>
 static int emb_launch(int which, const void *idx, const void *table_or_dtable, const void *out_or_dout, long long tokens,
                       int bag, int dim, long long entries, int avg, cudaStream_t st) {
   FfkTraffic traffic(tokens * dim * 4);
-  if (emb_vec_ok(tokens, dim, table_or_dtable, out_or_dout)) {
-    const unsigned per_row = (unsigned)(dim / 8), pieces = (unsigned)(tokens * per_row);
+  if (const unsigned pieces = emb_pieces<W>(tokens, dim, table_or_dtable, out_or_dout)) {
+    const unsigned per_row = (unsigned)(dim / (int)(16 / sizeof(W)));
     const int vgrid = ffk_blocks(pieces, 256);
     if (which == 0)
       ffk_launch(embedding_fwd_vec_kernel<W, I, O>, vgrid, 256, 0, st, (const I *)idx, (const W *)table_or_dtable, (O *)out_or_dout, pieces, bag,
@@ -345,8 +359,8 @@ FFK_API int ffk_embedding_bwd(const void *idx, const void *dout, void *dtable, l
 FFK_API int ffk_embedding_sgd(const void *idx, const void *dout, float *table, long long tokens, int bag, int dim,
                               long long entries, float lr, int idx_dt, int out_dt, cudaStream_t st) {
   if (tokens <= 0) return 0;
-  if (emb_vec_ok(tokens, dim, table, dout)) {
-    const unsigned per_row = (unsigned)(dim / 8), pieces = (unsigned)(tokens * per_row);
+  if (const unsigned pieces = emb_pieces<float>(tokens, dim, table, dout)) {
+    const unsigned per_row = (unsigned)(dim / 4);
     const int vgrid = ffk_blocks(pieces, 256);
 #define EMB_SGD(ID, OD, I, O)                                                                                                                \
   if (idx_dt == ID && out_dt == OD) {                                                                                                        \

@@ -131,6 +131,18 @@ def test_layernorm_backward_rows(rows, cols, acc):
     near(db, bd.grad + (ob.double() if acc else 0), sums * rows ** 0.5 + 1e-3)
 
 
+def test_scatter_into_one_row():
+    """Every token of every bag at the same row: whole numbers below 2^24, so that the sums are exact in any order."""
+    for dim in (8, 64, 768):
+        dout = torch.randint(-3, 4, (500, dim), device="cuda").float()
+        idx = torch.full((500, 3), 17, device="cuda", dtype=torch.int64)
+        table = torch.zeros(40, dim, device="cuda")
+        K.embedding_bwd(idx, dout, table)
+        assert torch.equal(table[17], 3 * dout.sum(0)) and not table[:17].any() and not table[18:].any()
+        K.embedding_sgd(idx, dout.bfloat16(), table, 1.0)
+        assert not table.any()
+
+
 @pytest.mark.parametrize("dim", [8, 64, 2048, 12])
 @pytest.mark.parametrize("bag,aggr", [(1, "sum"), (3, "sum"), (4, "avg")])
 @pytest.mark.parametrize("table_dt,out_dt", [(torch.bfloat16, torch.bfloat16), (torch.float32, torch.bfloat16), (torch.float32, torch.float32)])
