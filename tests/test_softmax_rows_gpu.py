@@ -41,6 +41,29 @@ def test_softmax_and_cross_entropy_rows(cols, rows):
     assert K.softmax_last_error() == 0
 
 
+@pytest.mark.parametrize("cols", [1536, 1544, 2040, 2048, 2056, 4088, 4096])
+@pytest.mark.parametrize("causal", [False, True])
+def test_rows_on_both_sides_of_the_warp_kernels(cols, causal):
+    """Plain softmax, forward and backward, where rows change from one warp each to one block each."""
+    gen = torch.Generator(device="cuda").manual_seed(cols)
+    x, dy = (torch.randn(70, cols, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    xd = x.double() * 0.5
+    if causal:
+        xd = xd.masked_fill(torch.arange(cols, device="cuda")[None] > (torch.arange(70, device="cuda") % 35)[:, None], float("-inf"))
+    ref = torch.softmax(xd, -1)
+    y, y2, dx, dx2 = (torch.empty_like(x) for _ in range(4))
+    K.softmax_fwd(x, out=y, scale=0.5, causal_q=35 if causal else 0)
+    K.softmax_dropout_fwd(x, y2, None, 0.0, 1, None, scale=0.5, causal_q=35 if causal else 0)
+    _near(y, ref)
+    assert torch.equal(y, y2)
+    K.softmax_bwd(dy, y, dx=dx, scale=0.5)
+    K.softmax_dropout_bwd(dy, y, dx2, 0.0, 1, None, scale=0.5)
+    g, yr = dy.double(), y.double()
+    want = 0.5 * yr * (g - (g * yr).sum(-1, keepdim=True))
+    slack = 0.5 * yr * (g * yr).abs().sum(-1, keepdim=True) * cols * 2.0 ** -24
+    assert ((dx.double() - want).abs() <= REL * want.abs() + slack + 1e-9).all() and torch.equal(dx, dx2)
+
+
 @pytest.mark.parametrize("cols", [4096, 8192, 32776, 65544, 131072])
 def test_rows_with_masked_pieces(cols):
     """Whole pieces, and a thread's and a warp's whole share of the row, masked out."""
