@@ -357,12 +357,12 @@ __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *x, co
   }
 }
 
-// Rows that the ring does not hold twice (more than 32768, cols % 8 == 0): one pass finds the row's maximum and the sum of exponentials
-// together, a second one over the row, which L2 still holds, writes the results; 16-byte accesses.  Softmax (labels null) or its
-// cross-entropy.  Bound by HBM and the second exponential: 1024 x 128256 takes 145 us (3.6 TB/s) for the loss and 141 for the softmax;
-// the scalar kernels take 584 and 747, the row in registers (64 of them for 16 pieces alone, so it spills) 365 for 2048 x 50304,
-// this one 111.
-template <typename L>
+// Rows that the ring does not hold twice (more than 32768, cols % 8 == 0), and those above 16384 of which only the loss is wanted: one
+// pass finds the row's maximum and the sum of exponentials together, a second one over the row, which L2 still holds, writes the
+// results; 16-byte accesses.  Softmax (labels null; SCALED: scale is not 1) or its cross-entropy.  Bound by HBM and the second
+// exponential: 1024 x 128256 takes 139 us for gradient and loss, 50 for the loss alone, 135 for the softmax; the scalar kernels take
+// 550, 331 and 740, the row in registers (64 of them for 16 pieces alone, so it spills) 365 for 2048 x 50304, this one 111.
+template <typename L, bool SCALED>
 __global__ void __launch_bounds__(512) softmax_long_kernel(const bf16 *x, const L *labels, bf16 *__restrict__ probs,
                                                            bf16 *__restrict__ dlogits, float *__restrict__ loss, int rows, int cols, float scale,
                                                            float grad_scale) {
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(512) softmax_long_kernel(const bf16 *x, const 
       float nm = m;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        v[j] *= scale;
+        if (SCALED) v[j] *= scale;
         nm = fmaxf(nm, v[j]);
       }
       const float sub = nm == -INFINITY ? 0.f : nm;  // nothing but masked elements so far: their exponentials are 0
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(512) softmax_long_kernel(const bf16 *x, const 
       float v[8];
       vec::ld8(px + (long long)i * 8, v);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = __expf(v[j] * scale - M) * inv;
+      for (int j = 0; j < 8; ++j) v[j] = __expf((SCALED ? v[j] * scale : v[j]) - M) * inv;
       if (probs) vec::st8(probs + at, v);
       if (dlogits) {
         const int hit = valid ? (int)label - i * 8 : -1;
@@ -726,7 +726,10 @@ FFK_API int ffk_softmax_fwd(const void *x, void *y, int rows, int cols, float sc
   if (softmax_wide_ok(cols, dt) && causal_q <= 0 && aligned16(x) && aligned16(y))
     return launch_softmax_wide<false, int>(x, nullptr, y, nullptr, nullptr, rows, cols, scale, 1.f, st);
   if (softmax_long_ok(cols, dt) && causal_q <= 0 && aligned16(x) && aligned16(y)) {
-    ffk_launch(softmax_long_kernel<int>, long_grid(rows), 512, 0, st, (const bf16 *)x, nullptr, (bf16 *)y, nullptr, nullptr, rows, cols, scale, 1.f);
+    if (scale == 1.f)
+      ffk_launch(softmax_long_kernel<int, false>, long_grid(rows), 512, 0, st, (const bf16 *)x, nullptr, (bf16 *)y, nullptr, nullptr, rows, cols, 1.f, 1.f);
+    else
+      ffk_launch(softmax_long_kernel<int, true>, long_grid(rows), 512, 0, st, (const bf16 *)x, nullptr, (bf16 *)y, nullptr, nullptr, rows, cols, scale, 1.f);
     return (int)cudaGetLastError();
   }
   return softmax_scalar_fwd(x, y, rows, cols, scale, causal_q, dt, st);
@@ -749,9 +752,12 @@ static void launch_softmax_ce_row(const void *logits, const void *labels, void *
 template <typename L>
 static int launch_softmax_ce(const void *logits, const void *labels, void *probs, void *dlogits, float *loss, int rows, int cols, float grad_scale,
                              cudaStream_t st) {
-  if (softmax_wide_ok(cols, 1)) return launch_softmax_wide<true, L>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st);
-  if (softmax_long_ok(cols, 1))
-    ffk_launch(softmax_long_kernel<L>, long_grid(rows), 512, 0, st, (const bf16 *)logits, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss, rows,
+  // The ring pays where rows are written too, and up to 16384 also for a loss alone (300 x 8192: 4.0 us, in one pass without it 6.5); beyond,
+  // where it is one block per SM, a loss alone is the faster without (8192 x 30528: 160 us through the ring, 132).
+  const bool ring = softmax_wide_ok(cols, 1) && (probs || dlogits || cols <= 16384);
+  if (ring) return launch_softmax_wide<true, L>(logits, labels, probs, dlogits, loss, rows, cols, 1.f, grad_scale, st);
+  if (softmax_long_ok(cols, 1) || softmax_wide_ok(cols, 1))
+    ffk_launch(softmax_long_kernel<L, false>, long_grid(rows), 512, 0, st, (const bf16 *)logits, (const L *)labels, (bf16 *)probs, (bf16 *)dlogits, loss, rows,
                cols, 1.f, grad_scale);
   else if (cols <= 8 * ROW_THREADS) launch_softmax_ce_row<1, L>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, st);
   else if (cols <= 16 * ROW_THREADS) launch_softmax_ce_row<2, L>(logits, labels, probs, dlogits, loss, rows, cols, grad_scale, st);

@@ -64,6 +64,19 @@ def test_rows_on_both_sides_of_the_warp_kernels(cols, causal):
     assert ((dx.double() - want).abs() <= REL * want.abs() + slack + 1e-9).all() and torch.equal(dx, dx2)
 
 
+@pytest.mark.parametrize("cols", [264, 4096, 4104, 16384, 16392, 32768, 32776])
+def test_loss_alone(cols):
+    """Cross-entropy without gradient or probabilities."""
+    x = torch.randn(300, cols, generator=torch.Generator(device="cuda").manual_seed(cols), device="cuda").bfloat16()
+    labels = torch.arange(300, device="cuda", dtype=torch.int32) * 7 % cols
+    labels[5] = -1
+    loss = torch.empty(300, device="cuda")
+    K.softmax_ce(x, labels, loss)
+    want = torch.logsumexp(x.double(), -1) - x.double().gather(1, labels.long().clamp(min=0)[:, None])[:, 0]
+    want[5] = 0
+    assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5)
+
+
 @pytest.mark.parametrize("cols", [4096, 8192, 32776, 65544, 131072])
 def test_rows_with_masked_pieces(cols):
     """Whole pieces, and a thread's and a warp's whole share of the row, masked out."""
