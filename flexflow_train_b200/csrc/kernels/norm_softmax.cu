@@ -271,6 +271,7 @@ __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *x, co
   int stage = 0;
   uint32_t phase = 0;
   for (long long row = blockIdx.x; row < rows; row += gridDim.x) {
+    const long long label = CE ? (long long)labels[row] : -1;  // asked for before the wait, which no load passes
     const bool ok = mbar_wait(&full[stage], phase, &abort_flag, &g_rows_err, FFK_ERR_TIMEOUT_PRODUCER, wait_ns);
     const uint4 *src = reinterpret_cast<const uint4 *>(wide_smem + (size_t)stage * row_bytes);
     float v[WIDE_VPT][8];
@@ -287,11 +288,9 @@ __global__ void __launch_bounds__(1024, 1) softmax_wide_kernel(const bf16 *x, co
         }
       }
     }
-    long long label = -1;
     bool valid = false;
     float at_label = 0.f;
     if (CE) {
-      label = (long long)labels[row];
       valid = label >= 0 && label < cols;
       if (valid && threadIdx.x == 0) at_label = bf2f(reinterpret_cast<const bf16 *>(src)[label]);
     }
